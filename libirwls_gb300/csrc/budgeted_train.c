@@ -140,25 +140,30 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     double *d_KC = NULL, *d_KSC = NULL, *d_K1 = NULL, *d_part = NULL, *d_sd = NULL, *d_day = NULL, *d_e = NULL,
            *d_Da = NULL, *d_beta = NULL, *d_bnew = NULL, *d_bbest = NULL, *d_nrm = NULL, *h_nrm = NULL;
     const int ld = m + 1;
-    /* split-K chunks of the Gram update: about eight CTAs per SM over the
-       lower tiles, with at least 512 rows per chunk */
+    /* The Gram runs on the tensor cores through exact integer digits of the
+       active rows (dev_gram_tc.cu): base 256 in the plain form (FP64
+       accuracy), base 128 in the precision form. P bounds the split-K chunks,
+       of which it takes as many as fill the SMs. The plain form keeps the
+       FP64 product below 128 centroids (one 128-column tile): IRWLS can
+       multiply a change of rounding in K1 by 10^8 (20000 rows, 100 SGMA
+       centroids: any other split of the same FP64 sums moves the weights by
+       1e-9 to 1e-8), and the product is small enough there to keep its
+       order, about eight CTAs per SM over the lower tiles with at least 512
+       rows per chunk (20000 x 100: 0.8 ms). At 50000 x 300 it took 2.55 ms
+       per iteration, three quarters of the training; the digits, with their
+       slicing, take 0.20. */
     const int sms = 152;
     const int tiles = ((m + 64) / 64) * ((m + 63) / 64 + 1) / 2;
-    int P = (8 * sms + tiles - 1) / tiles;
-    if (P > l / 512) P = l / 512;
-    if (P < 1) P = 1;
-    if (P > 64) P = 64;
-    /* precision form: the Gram on the tensor cores through exact integer
-       digits of the active rows (dev_gram_tc.cu), which takes as many
-       split-K chunks of the P allowed here as fill the SMs */
     const int mixed = irwls_get_precision() == IRWLS_PRECISION_MIXED;
+    const int digits = mixed || m >= 128;
     void *d_A = NULL;
-    if (mixed) {
-        P = (24 * sms + tiles - 1) / tiles;
-        if (P > l / 256) P = l / 256;
-        if (P < 1) P = 1;
-        if (P > 128) P = 128;
-        rc |= irwls_dev_malloc(&d_A, irwls_par_gram_tc_bytes(l, m));
+    int P = ((digits ? 24 : 8) * sms + tiles - 1) / tiles;
+    if (P > l / (digits ? 256 : 512)) P = l / (digits ? 256 : 512);
+    if (P < 1) P = 1;
+    if (P > (digits ? 128 : 64)) P = digits ? 128 : 64;
+    if (digits) {
+        if (!mixed && P < irwls_par_gram_min_parts(l, m)) P = irwls_par_gram_min_parts(l, m);
+        rc |= irwls_dev_malloc(&d_A, mixed ? irwls_par_gram_tc_bytes(l, m) : irwls_par_gram_bytes(l, m));
     }
     rc |= irwls_dev_malloc((void **)&d_idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_act, (size_t)l * sizeof(int));
@@ -192,8 +197,9 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
         double dW = 1e9, nW = 1.0, old = 0.0, best = 1e9;
         while ((iter < 500) && (dW / nW > 1e-6) && (since_best < 5)) {
             /* K1 = KC + KSCA^T KSCA (lower) and K2 = KSCA^T Day in row m (:401-416) */
-            if (mixed ? irwls_par_gram_tc(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P, d_A)
-                      : irwls_par_gram(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P))
+            if (mixed    ? irwls_par_gram_tc(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P, d_A)
+                : digits ? irwls_par_gram(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P, d_A)
+                         : irwls_par_gram_fp64(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P))
                 goto fail;
             g_gram_flops += (double)nact * (m + 1) * m;
             if (irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)) goto fail;
@@ -222,7 +228,7 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
         g_last_nact = nact;
     }
     if (irwls_dev_d2h(weights_out, d_bbest, (size_t)m * sizeof(double)) || irwls_dev_sync()) goto fail;
-    if (mixed) {
+    if (digits) {
         const int tc = irwls_tc_status();
         if (tc) {
             irwls_set_error(-13, "a tensor-core pipeline wait of the Gram ran out (code %d)", tc);

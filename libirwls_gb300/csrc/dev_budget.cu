@@ -10,9 +10,11 @@
 //   score_c = |r_c|^2 / eta_c    column norms reduced per CTA, then in a fixed
 //                                order; strict ">" argmax, first index wins.
 // IRWLSpar's Gram matrix K1 = KC + sum_i a_i a_i^T with a_i = sqrt(Da_i) KSC_i
-// over active rows is a split-K SYRK on the lower triangle; the right-hand
-// side K2 = sum_i a_i (sqrt(Da_i) y_i) is computed as the extra row m of the
-// same product, which is exactly where the Cholesky solver wants it.
+// over active rows is a split-K SYRK on the lower triangle (on the tensor
+// cores through exact digits in dev_gram_tc.cu; in FP64 here in the plain form
+// below 128 centroids); the right-hand side K2 = sum_i a_i (sqrt(Da_i) y_i) is
+// computed as the extra row m of the same product, which is exactly where the
+// Cholesky solver wants it.
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -905,7 +907,7 @@ extern "C" int irwls_par_first(const double *d_y, int l, double M, int *d_act, d
 
 extern "C" size_t irwls_par_gram_part_bytes(int m, int P) { return (size_t)P * (m + 1) * m * sizeof(double); }
 
-// K1 = KC + the sum of P Gram partials (the last step of both Gram forms).
+// K1 = KC + the sum of P Gram partials (the last step of both digit forms).
 extern "C" int irwls_par_gram_reduce(const double *d_part, int P, int m, const double *d_KC, double *d_K1, int ldK1) {
     const long long tot = (long long)(m + 1) * m;
     gram_reduce_kernel<<<(int)std::min<long long>(ceil_div(tot, 256), 65535), 256, 0, irwls_stream()>>>(
@@ -914,8 +916,9 @@ extern "C" int irwls_par_gram_reduce(const double *d_part, int P, int m, const d
     return 0;
 }
 
-extern "C" int irwls_par_gram(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
-                              const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part, int P) {
+extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
+                                   const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part,
+                                   int P) {
     const int T = ceil_div(m + 1, TT);
     const int Tc = ceil_div(m, TT);
     const int chunk = nact > 0 ? ceil_div(nact, P) : 1;

@@ -1,5 +1,6 @@
-// dev_gram_tc.cu -- the precision form's IRWLSpar Gram on the tensor cores,
-// through exact integer slices.
+// dev_gram_tc.cu -- IRWLSpar's Gram on the tensor cores, through exact integer
+// slices, in two digit forms: base 256 (the plain form, FP64 accuracy) and
+// base 128 (the precision form).
 //
 //   G = A'^T A',   A' = [sd * KSC[act, :], day]   (nact x (m + 1)),
 //
@@ -9,28 +10,27 @@
 //
 // 1. Each column c of A' gets a power of two sigma_c >= max_p |A'_pc| (a
 //    column-max pass), and each entry becomes the integer
-//    N_pc = round(A'_pc / sigma_c * 2^48), |N| <= 2^48, by integer operations
-//    on its bits. N is written in 7 balanced base-128 digits d_0 .. d_6
-//    (d_0 lowest), |d_s| <= 64: small integers, exact in bf16.
-// 2. sum_p N_pi N_pj = sum_u 128^u L_u(i, j), L_u = sum_{s+t=u} sum_p
-//    d_s(p,i) d_t(p,j). The levels u = 6 ... 12 are kept (28 digit pairs);
-//    the dropped levels weigh at most about 2^-46 of the top one, so each
-//    entry of G carries an error of about 2^-46 max|A'_.i| max|A'_.j| per
-//    row, the accuracy of the double-float Gram this replaces.
+//    N_pc = round(A'_pc / sigma_c * 2^F), |N| <= 2^F, F = 48 (base 128) or 55,
+//    by integer operations on its bits. N is written in 7 balanced digits
+//    d_0 .. d_6 of base B (d_0 lowest), |d_s| <= B/2: small integers, exact in
+//    bf16.
+// 2. sum_p N_pi N_pj = sum_u B^u L_u(i, j), L_u = sum_{s+t=u} sum_p
+//    d_s(p,i) d_t(p,j). The top 7 (base 128) or 8 levels are kept (28 or 33
+//    digit pairs); the dropped ones weigh at most about 2^-46 or 2^-61 of
+//    sigma_i sigma_j per row, with random signs.
 // 3. A CTA owns a 128 x 64 tile of G and one split-K chunk of the rows. Per
-//    16-row stage the 28 digit-pair products go to 7 level accumulators of
-//    128 x 64 FP32 in tensor memory (448 of its 512 columns). Every product
-//    is an integer of magnitude <= 64^2 = 4096 and a level sums at most 7
-//    pairs, so over 512 rows every partial sum is an integer below
-//    7 * 512 * 4096 < 2^24: exact in FP32, whatever the order of
-//    accumulation. Every 512 rows the epilogue drains the levels into a
-//    96-bit integer per entry (T += sum_u 128^(u-6) L_u), so the whole sum
-//    stays exact.
-// 4. G_ij = sigma_i sigma_j 2^-54 T_ij, written as the FP64 partials that
+//    16-row stage the digit-pair products go to one accumulator of 128 x 64
+//    FP32 per level in tensor memory (448 or all of its 512 columns). A level
+//    sums at most 7 pairs of products of magnitude <= (B/2)^2, so over 512
+//    (base 128) or 128 rows every partial sum is an integer below 2^24: exact
+//    in FP32, whatever the order of accumulation. After that many rows the
+//    epilogue drains the levels into a 96-bit integer per entry, so the whole
+//    sum stays exact.
+// 4. G_ij = sigma_i sigma_j 2^-GSCALE T_ij, written as the FP64 partials that
 //    gram_reduce_kernel adds to KC.
 //
 // Operands reach shared memory by bulk copies: the slices are stored in the
-// shared-memory image of a stage (per 128-column tile and 16-row block, the 8
+// shared-memory image of a stage (per 128-column tile and 16-row block, the
 // digit pieces of 128 x 16 in canonical K-major core-matrix order). Warp 0
 // copies, lane 0 of warp 1 issues the MMAs, warps 4-11 drain. Every wait is
 // bounded; a timeout sets device flag word 1.
@@ -44,22 +44,43 @@
 
 namespace {
 
+// The two digit forms, 7 balanced digits each of base 2^BITS.
+//   GramDigits<7>: the precision form. GFRAC 48, levels u >= 6 (28 digit
+//   pairs, 7 accumulators), drained every 512 rows.
+//   GramDigits<8>: the plain form. GFRAC 55, levels u >= 5 (33 pairs, 8
+//   accumulators, all of tensor memory), drained every 128 rows. Entries of at
+//   least 2^-2 of their column's scale are represented exactly, the others
+//   within 2^-56 of it, and the dropped levels weigh below 2^-61 of
+//   sigma_i sigma_j per row: together below the rounding of an FP64
+//   accumulation (up to 2^-54 of the partial sum per addition). One level less
+//   (2^-53 per row) moved the weights of 2000 to 48000-row trainings two to
+//   fifteen times further from a 64-bit reference than the FP64 product did.
+// A level sums at most 7 pairs of products of magnitude <= 2^(2 BITS - 2), so
+// over the rows between two drains every FP32 partial sum is an integer below
+// 2^24. The 33 products run on the tensor cores at about 40 TFLOP/s
+// FP64-equivalent, where the FP64 pipe of this part gives 1.06 at most.
 constexpr int GS = 7;                  // digits per entry
-constexpr int GBITS = 7;               // digit base 2^7
-constexpr int GFRAC = 48;              // N = round(v * 2^48), |v| <= 1
-constexpr int GPAIRS = GS * (GS + 1) / 2;            // digit pairs of the kept levels
-constexpr int GSCALE = 2 * GFRAC - GBITS * (GS - 1);  // G = sigma_i sigma_j 2^-GSCALE T
 constexpr int GM = 128, GN = 64;       // tile of G: rows (A' columns) x columns
 constexpr int GBK = 16;                // rows of A' per stage
 constexpr int GPIECE = GM * GBK;       // elements of one digit piece (4 KB)
-constexpr int GDRAIN = 32;             // stages between drains (512 rows)
 constexpr int GNS = 5;                 // ring stages
 constexpr int G_THREADS = 384;
 constexpr uint32_t A_STAGE = GS * GPIECE * 2;      // 28 KB: 7 pieces of 128 rows
 constexpr uint32_t B_PIECE = GN * GBK * 2;         // 2 KB: 64 rows of one piece
 constexpr uint32_t G_STAGE = A_STAGE + GS * B_PIECE;  // 42 KB
-static_assert(GS * 64 <= 512, "level accumulators exceed tensor memory");
-static_assert((long long)GS * GDRAIN * GBK * (1 << (2 * (GBITS - 1))) < (1LL << 24), "level sums must stay exact");
+
+template <int BITS>
+struct GramDigits {
+    static constexpr int HALF = 1 << (BITS - 1);        // digits in [-HALF, HALF], exact in bf16
+    static constexpr int GFRAC = BITS * GS - 1;         // N = round(v * 2^GFRAC), |v| <= 1
+    static constexpr int LOW = BITS == 7 ? GS - 1 : GS - 2;  // lowest kept level
+    static constexpr int LEVELS = 2 * (GS - 1) - LOW + 1;
+    static constexpr int GPAIRS = BITS == 7 ? 28 : 33;  // digit pairs of the kept levels
+    static constexpr int GSCALE = 2 * GFRAC - BITS * LOW;    // G = sigma_i sigma_j 2^-GSCALE T
+    static constexpr int GDRAIN = BITS == 7 ? 32 : 8;   // stages between drains
+    static_assert(LEVELS * GN <= 512, "level accumulators exceed tensor memory");
+    static_assert((long long)GS * GDRAIN * GBK * HALF * HALF < (1LL << 24), "level sums must stay exact");
+};
 
 // Element offset of (row r of the 128-row tile, k of the 16-row block) in a
 // digit piece: 8 x 8 core matrices, 128 bytes apart along k, 256 along r.
@@ -157,33 +178,37 @@ __device__ __forceinline__ int col_exp(unsigned long long mxbits) {
     return E - 1023 + (pow2 ? 0 : 1);
 }
 
-// round(v * 2^(48 - e)) for |v| <= 2^e, ties away from zero, from the bits of
-// v (no FP64 pipe).
-__device__ __forceinline__ long long fixed48(double v, int e) {
+// round(v * 2^(FRAC - e)) for |v| <= 2^e, ties away from zero, from the bits
+// of v (no FP64 pipe).
+template <int FRAC>
+__device__ __forceinline__ long long fixed_point(double v, int e) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     const int E = (int)((b >> 52) & 0x7ff);
     if (E == 0) return 0;  // zero (subnormals, below 2^-1022, are dropped)
     const unsigned long long M = (b & ((1ULL << 52) - 1)) | (1ULL << 52);
-    // v = M 2^(E - 1075); N = M 2^(E - 1075 + 47 - e) = M >> sh
-    const int sh = 1075 + e - GFRAC - E;  // >= 4 since |v| <= 2^e
+    // v = M 2^(E - 1075); N = M 2^(E - 1075 + FRAC - e) = M >> sh
+    const int sh = 1075 + e - FRAC - E;  // >= 52 - FRAC since |v| <= 2^e
     long long N = 0;
-    if (sh < 64) N = (long long)((M + (1ULL << (sh - 1))) >> sh);
+    if (FRAC > 52 && sh <= 0) N = (long long)(M << min(-sh, FRAC - 52));
+    else if (sh < 64) N = (long long)((M + (1ULL << (sh - 1))) >> sh);
     return (b >> 63) ? -N : N;
 }
 
-// The slices of A'. Thread = (column c, group of 8 rows): the 7 digits of the
+// The slices of A'. Thread = (column c, group of 8 rows): the digits of the
 // group's entries, one 16-byte store per digit piece. Rows >= nact and
 // columns > m are written as zeros.
+template <int BITS>
 __global__ void __launch_bounds__(256) gram_slice_kernel(const double *__restrict__ KSC, int m,
                                                          const int *__restrict__ act, int nact,
                                                          const double *__restrict__ sd,
                                                          const double *__restrict__ day,
                                                          const unsigned long long *__restrict__ cmax, int ncols,
                                                          int npb, __nv_bfloat16 *__restrict__ S) {
-    __shared__ uint16_t bf[129];  // bf16 bits of -64 ... 64
-    if (threadIdx.x < 129) {
-        const __nv_bfloat16 h = __float2bfloat16_rn((float)((int)threadIdx.x - 64));
-        bf[threadIdx.x] = *(const uint16_t *)&h;
+    constexpr int HALF = GramDigits<BITS>::HALF;
+    __shared__ uint16_t bf[2 * HALF + 1];  // bf16 bits of -HALF ... HALF
+    for (int t = threadIdx.x; t <= 2 * HALF; t += 256) {
+        const __nv_bfloat16 h = __float2bfloat16_rn((float)(t - HALF));
+        bf[t] = *(const uint16_t *)&h;
     }
     __syncthreads();
     const long long items = (long long)ncols * npb * 2;
@@ -200,19 +225,19 @@ __global__ void __launch_bounds__(256) gram_slice_kernel(const double *__restric
             long long N = 0;
             if (p < nact && c <= m && e > -1100) {
                 const double v = c < m ? __dmul_rn(sd[p], KSC[(size_t)act[p] * m + c]) : day[p];
-                N = fixed48(v, e);
+                N = fixed_point<GramDigits<BITS>::GFRAC>(v, e);
             }
 #pragma unroll
             for (int s = 0; s < GS; ++s) {
                 int d;
                 if (s < GS - 1) {
-                    d = (int)(N & 127);
-                    if (d >= 64) d -= 128;
-                    N = (N - d) >> 7;
+                    d = (int)(N & (2 * HALF - 1));
+                    if (d >= HALF) d -= 2 * HALF;
+                    N = (N - d) >> BITS;
                 } else {
-                    d = (int)N;  // |d| <= 64
+                    d = (int)N;  // |d| <= HALF
                 }
-                const uint32_t hb = bf[d + 64];
+                const uint32_t hb = bf[d + HALF];
                 if (k & 1) w[s][k >> 1] |= hb << 16;
                 else w[s][k >> 1] = hb;
             }
@@ -259,9 +284,12 @@ __device__ __forceinline__ void acc_add(Acc96 &a, long long xh, uint32_t xl) {
 
 // Tile (I, J) of G for split-K chunk z: rows 128 I ... of G (columns of A'),
 // columns 64 J ...; stages [z * spc, min(npb, (z + 1) * spc)) of 16 rows.
+template <int BITS>
 __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat16 *__restrict__ S, int npb, int spc,
                                                                int m, const unsigned long long *__restrict__ cmax,
                                                                double *__restrict__ part, int *flags) {
+    using Cfg = GramDigits<BITS>;
+    constexpr int LOW = Cfg::LOW, LEVELS = Cfg::LEVELS, GSCALE = Cfg::GSCALE, GDRAIN = Cfg::GDRAIN;
     const int J = blockIdx.x, I = blockIdx.y, z = blockIdx.z;
     if (GN * J > GM * I + GM - 1 || GN * J >= m) return;  // above the diagonal or past the last column
     extern __shared__ __align__(1024) unsigned char g_smem[];
@@ -295,7 +323,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat
     const uint32_t tmem = tmem_slot;
 
     if (warp == 0) {
-        // producer: the A tile's 8 pieces in one copy, the B half-pieces in 8
+        // producer: the A tile's pieces in one copy, the B half-pieces one by one
         if (lane == 0) {
             const uint32_t base = smem_u32(smem);
             const __nv_bfloat16 *Ab = S + ((size_t)I * npb + k0) * GS * GPIECE;
@@ -324,7 +352,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat
         }
         __syncwarp();
     } else if (warp == 1) {
-        // MMA issue: level u - 6 += sum_{s+t=u} A_s B_t, u = 6 ... 12
+        // MMA issue: level u - LOW += sum_{s+t=u} A_s B_t, u = LOW ... 2 GS - 2
         if (lane == 0) {
             const uint32_t base = smem_u32(smem);
             for (int k = 0; k < nst && !abort_flag; ++k) {
@@ -344,24 +372,25 @@ __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
                 const uint32_t sa = base + slot * G_STAGE, sbb = sa + A_STAGE;
-                // A piece s against the B pieces t = GS-1-s ... GS-1, which lie
+                // A piece s against the B pieces t = LOW-s ... GS-1, which lie
                 // consecutively in shared memory and so form one operand of
-                // 64 (s + 1) rows whose products land on the consecutive
-                // levels 0 ... s: ten MMAs of N <= 256 for the 28 pairs, each A
-                // piece read once per MMA instead of once per pair. Piece GS-1
-                // comes first and covers every level, so it alone starts a
-                // drain block. The sums are exact integers, so the grouping
-                // does not change them.
+                // up to 64 GS rows whose products land on consecutive levels:
+                // ten MMAs of N <= 256 for the 28 pairs (thirteen for 33), each
+                // A piece read once per MMA instead of once per pair. The
+                // first product of a drain block on each level starts it:
+                // piece GS-1 covers all levels with LOW = GS - 1, all but the
+                // lowest with LOW = GS - 2, whose first is (GS-2, 0). The sums
+                // are exact integers, so the grouping does not change them.
 #pragma unroll
                 for (int s = GS - 1; s >= 0; --s) {
                     const uint64_t da = tc_desc_lbo_sbo(sa + s * (GPIECE * 2), 128, 256);
+                    const bool lone = LOW == GS - 2 && s == GS - 2;  // piece 0 by itself
 #pragma unroll
-                    for (int t0 = GS - 1 - s; t0 < GS; t0 += 4) {
-                        const int np = GS - t0 < 4 ? GS - t0 : 4;  // B pieces of this MMA
+                    for (int t0 = LOW > s ? LOW - s : 0; t0 < GS; t0 += (lone && t0 == 0) ? 1 : 4) {
+                        const int np = lone && t0 == 0 ? 1 : GS - t0 < 4 ? GS - t0 : 4;  // B pieces of this MMA
                         const uint64_t db = tc_desc_lbo_sbo(sbb + t0 * B_PIECE, 128, 256);
-                        const bool acc = kin > 0 || s < GS - 1;
-                        mma_bf16(tmem + (uint32_t)(s + t0 - (GS - 1)) * GN, da, db, tc_idesc(GM, GN * np),
-                                 acc ? 1u : 0u);
+                        const bool acc = kin > 0 || !(s == GS - 1 || (lone && t0 == 0));
+                        mma_bf16(tmem + (uint32_t)(s + t0 - LOW) * GN, da, db, tc_idesc(GM, GN * np), acc ? 1u : 0u);
                     }
                 }
                 tc_commit(&empty[slot]);
@@ -397,21 +426,24 @@ __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat
             const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16) + 32 * h;
 #pragma unroll
             for (int c4 = 0; c4 < 32; c4 += 4) {
-                float L[GS][4];
+                float L[LEVELS][4];
 #pragma unroll
-                for (int v = 0; v < GS; ++v) tc_ld4(lanes + v * GN + c4, L[v]);
+                for (int v = 0; v < LEVELS; ++v) tc_ld4(lanes + v * GN + c4, L[v]);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    // levels 9-12 and 6-8 by Horner in 64-bit integers (below
-                    // 2^45 and 2^38), then T += t_hi 2^21 + t_lo
-                    long long th = __float2int_rn(L[6][j]);
-                    th = th * 128 + __float2int_rn(L[5][j]);
-                    th = th * 128 + __float2int_rn(L[4][j]);
-                    th = th * 128 + __float2int_rn(L[3][j]);
-                    long long tl = __float2int_rn(L[2][j]);
-                    tl = tl * 128 + __float2int_rn(L[1][j]);
-                    tl = tl * 128 + __float2int_rn(L[0][j]);
-                    acc_add(T[c4 + j], th >> 11, (uint32_t)th << 21);
+                    // the upper four levels and the lower three or four by
+                    // Horner in 64-bit integers (at most 2^48 and a little),
+                    // then T += t_hi 2^UP + t_lo
+                    constexpr int UP = BITS * (LEVELS - 4);  // 21 or 32
+                    constexpr int B = 1 << BITS;
+                    long long th = __float2int_rn(L[LEVELS - 1][j]);
+#pragma unroll
+                    for (int v = LEVELS - 2; v >= LEVELS - 4; --v) th = th * B + __float2int_rn(L[v][j]);
+                    long long tl = __float2int_rn(L[LEVELS - 5][j]);
+#pragma unroll
+                    for (int v = LEVELS - 6; v >= 0; --v) tl = tl * B + __float2int_rn(L[v][j]);
+                    if constexpr (UP == 32) T[c4 + j].hi += th;
+                    else acc_add(T[c4 + j], th >> (32 - UP), (uint32_t)th << UP);
                     acc_add(T[c4 + j], tl >> 32, (uint32_t)tl);
                 }
             }
@@ -446,16 +478,77 @@ __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
 }
 
-size_t slices_bytes(int l, int m) {
-    const size_t ct = (size_t)ceil_div(m + 1, GM), npb = (size_t)ceil_div(std::max(l, 1), GBK);
+size_t slices_bytes(int rows, int m) {
+    const size_t ct = (size_t)ceil_div(m + 1, GM), npb = (size_t)ceil_div(std::max(rows, 1), GBK);
     return ct * npb * GS * GPIECE * sizeof(__nv_bfloat16);
+}
+
+// bf16 tensor-core flops issued by gram_tc_kernel since the last read (28 or
+// 33 digit-pair products per 128 x 64 x 16 step of every tile).
+double g_tc_flops = 0.0;
+
+// The Gram in digit form BITS, the active rows taken in slabs of at most
+// `slab` rows (the slices of one slab are the workspace; the column scales
+// are those of all rows). P >= the number of slabs bounds the partials.
+template <int BITS>
+int gram_run(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd, const double *d_day,
+             const double *d_KC, double *d_K1, int ldK1, double *d_part, int P, void *d_ws, int slab) {
+    using Cfg = GramDigits<BITS>;
+    const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
+    const int ct = ceil_div(m + 1, GM), nt = ceil_div(m, GN);
+    const int nslab = std::max(1, ceil_div(nact, slab));
+    __nv_bfloat16 *S = (__nv_bfloat16 *)d_ws;
+    unsigned long long *cmax = (unsigned long long *)((char *)d_ws + slices_bytes(std::min(nact, slab), m));
+    // tiles of the lower part, and enough chunks to give every SM one CTA
+    int tiles = 0;
+    for (int I = 0; I < ct; ++I)
+        for (int J = 0; J < nt; ++J)
+            if (GN * J <= GM * I + GM - 1) ++tiles;
+    if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM_SLICE);
+    if (irwls_dev_memset(cmax, 0, (size_t)(m + 1) * sizeof(unsigned long long))) return -1;
+    if (nact > 0) {
+        gram_colmax_kernel<<<dim3(ceil_div(nact, GCM), ceil_div(m + 1, 1024)), 256, 0, irwls_stream()>>>(
+            d_KSC, m, d_act, nact, d_sd, d_day, cmax);
+        IRWLS_LAUNCH_CHECK("gram_colmax");
+    }
+    const size_t smem = (size_t)GNS * G_STAGE + 1024;
+    cudaFuncSetAttribute(gram_tc_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int parts = 0;
+    for (int a = 0, n = 0; n < nslab; a += slab, ++n) {
+        const int rows = std::min(slab, nact - a);
+        const int npb = ceil_div(std::max(rows, 1), GBK);
+        int pz = std::max(1, std::min(P / nslab, sms / std::max(tiles, 1)));
+        pz = std::min(pz, npb);
+        const int spc = ceil_div(npb, pz);
+        pz = ceil_div(npb, spc);
+        if (irwls_prof_on() && n > 0) irwls_prof_begin(IRWLS_PROF_GRAM_SLICE);
+        const long long items = (long long)ct * GM * npb * 2;
+        gram_slice_kernel<BITS><<<(int)std::min<long long>(ceil_div(items, 256), 16LL * sms), 256, 0, irwls_stream()>>>(
+            d_KSC, m, d_act + a, rows, d_sd + a, d_day + a, cmax, ct * GM, npb, S);
+        if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM_SLICE);
+        IRWLS_LAUNCH_CHECK("gram_slice");
+        if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
+        gram_tc_kernel<BITS><<<dim3(nt, ct, pz), G_THREADS, smem, irwls_stream()>>>(
+            S, npb, spc, m, cmax, d_part + (size_t)parts * (m + 1) * m, irwls_dev_flags());
+        g_tc_flops += (double)tiles * npb * GBK * GM * GN * 2.0 * Cfg::GPAIRS;
+        if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
+        IRWLS_LAUNCH_CHECK("gram_tc");
+        parts += pz;
+    }
+    return irwls_par_gram_reduce(d_part, parts, m, d_KC, d_K1, ldK1);
+}
+
+// Rows per slab of the plain form: 4 GB of slices at most, so that the
+// workspace stays small beside K_nm itself (14 bytes of digits per 8-byte
+// entry) whatever the number of rows.
+constexpr size_t SLAB_BYTES = 4ULL << 30;
+int slab_rows(int m) {
+    const size_t per = slices_bytes(GBK, m);  // one 16-row block of every column tile
+    return (int)std::min<size_t>(std::max<size_t>(SLAB_BYTES / per, 1) * GBK, 1u << 30);
 }
 
 }  // namespace
 
-// bf16 tensor-core flops issued by gram_tc_kernel since the last read (28
-// digit-pair products per 128 x 64 x 16 step of every tile).
-static double g_tc_flops = 0.0;
 extern "C" double irwls_gram_tc_flops(int reset) {
     const double f = g_tc_flops;
     if (reset) g_tc_flops = 0.0;
@@ -469,44 +562,22 @@ extern "C" size_t irwls_par_gram_tc_bytes(int l, int m) {
 }
 
 // K1 (column-major, leading dimension ldK1, lower part) = KC + the Gram of
-// the active rows, row m = K2, as irwls_par_gram gives; P bounds the
-// split-K chunks (part holds at least P partials).
+// the active rows, row m = K2; P bounds the split-K chunks (part holds at
+// least P partials).
 extern "C" int irwls_par_gram_tc(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
                                  const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part,
                                  int P, void *d_ws) {
-    const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
-    const int ct = ceil_div(m + 1, GM), nt = ceil_div(m, GN);
-    const int npb = ceil_div(std::max(nact, 1), GBK);
-    __nv_bfloat16 *S = (__nv_bfloat16 *)d_ws;
-    unsigned long long *cmax = (unsigned long long *)((char *)d_ws + slices_bytes(nact, m));
-    // tiles of the lower part, and enough chunks to give every SM one CTA
-    int tiles = 0;
-    for (int I = 0; I < ct; ++I)
-        for (int J = 0; J < nt; ++J)
-            if (GN * J <= GM * I + GM - 1) ++tiles;
-    int pz = std::max(1, std::min(P, sms / std::max(tiles, 1)));
-    pz = std::min(pz, npb);
-    const int spc = ceil_div(npb, pz);
-    pz = ceil_div(npb, spc);
-    if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM_SLICE);
-    if (irwls_dev_memset(cmax, 0, (size_t)(m + 1) * sizeof(unsigned long long))) return -1;
-    if (nact > 0) {
-        gram_colmax_kernel<<<dim3(ceil_div(nact, GCM), ceil_div(m + 1, 1024)), 256, 0, irwls_stream()>>>(
-            d_KSC, m, d_act, nact, d_sd, d_day, cmax);
-        IRWLS_LAUNCH_CHECK("gram_colmax");
-    }
-    const long long items = (long long)ct * GM * npb * 2;
-    gram_slice_kernel<<<(int)std::min<long long>(ceil_div(items, 256), 16LL * sms), 256, 0, irwls_stream()>>>(
-        d_KSC, m, d_act, nact, d_sd, d_day, cmax, ct * GM, npb, S);
-    if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM_SLICE);
-    IRWLS_LAUNCH_CHECK("gram_slice");
-    if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
-    const size_t smem = (size_t)GNS * G_STAGE + 1024;
-    cudaFuncSetAttribute(gram_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    gram_tc_kernel<<<dim3(nt, ct, pz), G_THREADS, smem, irwls_stream()>>>(S, npb, spc, m, cmax, d_part,
-                                                                          irwls_dev_flags());
-    g_tc_flops += (double)tiles * npb * GBK * GM * GN * 2.0 * GPAIRS;
-    if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
-    IRWLS_LAUNCH_CHECK("gram_tc");
-    return irwls_par_gram_reduce(d_part, pz, m, d_KC, d_K1, ldK1);
+    return gram_run<7>(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ldK1, d_part, P, d_ws, std::max(nact, 1));
+}
+
+// The plain form's Gram, its workspace and the fewest partials
+// that P may allow for l rows (one per slab).
+extern "C" size_t irwls_par_gram_bytes(int l, int m) {
+    return slices_bytes(std::min(l, slab_rows(m)), m) + (size_t)(m + 1) * sizeof(unsigned long long) + 256;
+}
+extern "C" int irwls_par_gram_min_parts(int l, int m) { return std::max(1, ceil_div(l, slab_rows(m))); }
+extern "C" int irwls_par_gram(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
+                              const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part, int P,
+                              void *d_ws) {
+    return gram_run<8>(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ldK1, d_part, P, d_ws, slab_rows(m));
 }

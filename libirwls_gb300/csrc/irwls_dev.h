@@ -195,12 +195,21 @@ int irwls_sgma_extend(const irwls_dev_set *X, int l, int s, const int *d_cent, c
 int irwls_par_build(const irwls_dev_set *X, int l, const int *d_idx, int m, double *d_KC, double *d_KSC);
 int irwls_par_first(const double *d_y, int l, double M, int *d_act, double *d_sd, double *d_day);
 size_t irwls_par_gram_part_bytes(int m, int P);
+/* The Gram on the tensor cores (dev_gram_tc.cu): A' as exact integer digits
+   per column scale, digit-pair products summed exactly in FP32 tensor
+   memory and drained into 96-bit integers. irwls_par_gram is the plain form
+   (base 256, FP64 accuracy): d_ws holds irwls_par_gram_bytes(l, m) bytes and
+   d_part P >= irwls_par_gram_min_parts(l, m) partials for up to l active rows. */
+size_t irwls_par_gram_bytes(int l, int m);
+int irwls_par_gram_min_parts(int l, int m);
 int irwls_par_gram(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
-                   const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part, int P);
-/* Precision form of the Gram on the tensor cores (dev_gram_tc.cu): A' as
-   exact base-128 integer digits per column scale, digit-pair products summed
-   exactly in FP32 tensor memory and drained into 96-bit integers; d_ws holds
-   irwls_par_gram_tc_bytes(l, m) bytes for up to l active rows. */
+                   const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part, int P,
+                   void *d_ws);
+/* The same product on the FP64 pipe (dev_budget.cu), the rows in P chunks. */
+int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
+                        const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part, int P);
+/* The precision form's (base 128); d_ws holds irwls_par_gram_tc_bytes(l, m)
+   bytes for up to l active rows. */
 size_t irwls_par_gram_tc_bytes(int l, int m);
 /* Reads and clears device flag word 1: 0, or the code a tensor-core kernel
    left when one of its bounded waits ran out. */
