@@ -34,16 +34,36 @@ constexpr int CT = 1024;
 
 // Per candidate: KNC row, forward then backward substitution with L, eta.
 // smem: v[s] (working vector), A row of the candidate (ld doubles).
+// With `need` (the screened selection) the kernel returns unless need[0] is
+// set; its CTAs from NCAND on then form the columns of KSC that no earlier
+// step formed (from built[0] on).
 __global__ void __launch_bounds__(256) sgma_cand_kernel(KView X, const int *__restrict__ cand,
                                                         const int *__restrict__ cent, int s,
                                                         const double *__restrict__ L, int ldL,
                                                         double *__restrict__ W, double *__restrict__ Z,
                                                         double *__restrict__ KN, int ldz,
-                                                        double *__restrict__ eta) {
+                                                        double *__restrict__ eta, const int *__restrict__ need,
+                                                        const int *__restrict__ built, int l,
+                                                        double *__restrict__ KSC) {
+    chain_wait();
+    chain_open();
+    if (need && !need[0]) return;
     extern __shared__ double sm[];
     double *v = sm;
     double *sA = sm + s;
     const int c = blockIdx.x, tid = threadIdx.x;
+    if (c >= NCAND) {
+        for (int t = built[0]; t < s; ++t) {
+            const int g = cent[t];
+            for (int k = tid; k < X.ld; k += blockDim.x) sA[k] = X.X[(size_t)g * X.ld + k];
+            __syncthreads();
+            const double qg = X.q[g];
+            for (int i = (c - NCAND) * blockDim.x + tid; i < l; i += (gridDim.x - NCAND) * blockDim.x)
+                KSC[(size_t)t * l + i] = kentry(X, sA, qg, i);
+            __syncthreads();
+        }
+        return;
+    }
     const int gc = cand[c];
     for (int t = tid; t < X.ld; t += blockDim.x) sA[t] = X.X[(size_t)gc * X.ld + t];
     __syncthreads();
@@ -220,15 +240,22 @@ __global__ void __launch_bounds__(256) w_gemm_kernel(const double *__restrict__ 
 // Per candidate c: w_e = sum of the chunks of row e in chunk order, W (FP64),
 // eta = 1 - |w|^2 (fixed-order block reduction), and w as the bf16 hi/mid/lo
 // pieces of its FP32 rounding in the blocked layout (zero up to the padded
-// width kpad).
+// width kpad). With eps (the screened selection): the candidates are training
+// rows, whose row of Q = K_nm L^-T is w itself, so |Q_c - w_c| measures the
+// error that Q has picked up; eps[0] keeps its maximum (float bits).
 __global__ void __launch_bounds__(256) w_finish_kernel(const double *__restrict__ part, int ldp, int s,
                                                        double *__restrict__ W, int ldz, __nv_bfloat16 *Wb, int kpad,
-                                                       double *__restrict__ eta) {
+                                                       double *__restrict__ eta, const int *__restrict__ cand,
+                                                       const __nv_bfloat16 *__restrict__ Qb, int kbn,
+                                                       unsigned *__restrict__ eps) {
     chain_wait();
     chain_open();
     __shared__ double red[256];
+    __shared__ float dred[8];
     const int c = blockIdx.x;
+    const int gc = eps ? cand[c] : 0;
     double ss = 0.0;
+    float dd = 0.f;
     for (int e = threadIdx.x; e < kpad; e += blockDim.x) {
         float xf = 0.f;
         if (e < s) {
@@ -245,6 +272,11 @@ __global__ void __launch_bounds__(256) w_finish_kernel(const double *__restrict_
             W[(size_t)c * ldz + e] = w;
             ss = fma(w, w, ss);
             xf = (float)w;
+            if (eps) {
+                const float d = xf - bf16_join3(Qb[qb_index(gc, e, kbn, 0)], Qb[qb_index(gc, e, kbn, 1)],
+                                                Qb[qb_index(gc, e, kbn, 2)]);
+                dd = fmaf(d, d, dd);
+            }
         }
         __nv_bfloat16 pc[3];
         bf16_pieces3(xf, pc);
@@ -252,12 +284,24 @@ __global__ void __launch_bounds__(256) w_finish_kernel(const double *__restrict_
         for (int k = 0; k < QB_NP; ++k) Wb[wb_index(c, e, k)] = pc[k];
     }
     red[threadIdx.x] = ss;
+    if (eps) {
+        for (int o = 16; o > 0; o >>= 1) dd += __shfl_xor_sync(0xffffffffu, dd, o);
+        if ((threadIdx.x & 31) == 0) dred[threadIdx.x >> 5] = dd;
+    }
     __syncthreads();
     for (int o = 128; o > 0; o >>= 1) {
         if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) eta[c] = 1.0 - red[0];
+    if (threadIdx.x == 0) {
+        eta[c] = 1.0 - red[0];
+        if (eps) {
+            float t = 0.f;
+            for (int k = 0; k < 8; ++k) t += dred[k];
+            // a NaN keeps its (large) bits in the maximum
+            atomicMax(eps, __float_as_uint(fabsf(sqrtf(t))));
+        }
+    }
 }
 
 // New row s of Linv from row s of L (l2, pivot L3):
@@ -331,7 +375,10 @@ constexpr int GM = 32, GK = 16;
 __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const int *__restrict__ cand, int s,
                                                            const double *__restrict__ KSC,
                                                            const double *__restrict__ Z, int ldz,
-                                                           double *__restrict__ part) {
+                                                           double *__restrict__ part, const int *__restrict__ need) {
+    chain_wait();
+    chain_open();
+    if (need && !need[0]) return;
     __shared__ __align__(16) double As[2][GK][GM];
     __shared__ __align__(16) double Bs[2][GK][NCAND + 1];
     __shared__ double red[16][NCAND + 1];
@@ -419,7 +466,11 @@ __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const
 __global__ void __launch_bounds__(NCAND) sgma_select_kernel(const double *__restrict__ part, int nblk,
                                                             const double *__restrict__ eta,
                                                             const int *__restrict__ cand, int s, int *cent,
-                                                            int *best, double *bestval) {
+                                                            int *best, double *bestval, const int *__restrict__ need,
+                                                            int *built) {
+    chain_wait();
+    chain_open();
+    if (need && !need[0]) return;
     __shared__ double sc[NCAND];
     const int c = threadIdx.x;
     double v = 0.0;
@@ -438,6 +489,7 @@ __global__ void __launch_bounds__(NCAND) sgma_select_kernel(const double *__rest
         cent[s] = cand[bb];
         best[0] = bb;
         bestval[s] = val;
+        if (built) built[0] = s;
     }
 }
 
@@ -804,12 +856,12 @@ extern "C" int irwls_sgma_score(const irwls_dev_set *X, int l, const int *d_cand
     if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_SGMA_CAND);
     sgma_cand_kernel<<<NCAND, 256, smem, irwls_stream()>>>(kview(X), d_cand, d_cent, s, d_L, ldL, d_W, d_Z, d_KN, ldz,
-                                                          d_eta);
+                                                          d_eta, nullptr, nullptr, l, nullptr);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_SGMA_CAND);
     IRWLS_LAUNCH_CHECK("sgma_cand");
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_SGMA_GEMM);
     sgma_gemm_kernel<<<sgma_gemm_grid(l), 256, 0, irwls_stream()>>>(kview(X), l, d_cand, s, d_KSC, d_Z, ldz,
-                                                                     d_part);
+                                                                     d_part, nullptr);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_SGMA_GEMM);
     IRWLS_LAUNCH_CHECK("sgma_gemm");
     return 0;
@@ -817,14 +869,41 @@ extern "C" int irwls_sgma_score(const irwls_dev_set *X, int l, const int *d_cand
 
 extern "C" int irwls_sgma_partials(int l) { return sgma_gemm_grid(l); }
 
-// Precision form: W = K_CN L^-T for the 64 candidates of step s, eta and the
-// bf16 split of W. wpart: irwls_sgma_wpart_count(m) doubles.
+// The FP64 scores of one step of the screened selection, taken on the device
+// only when need[0] is set (see irwls_sgma_tc_select): the columns of KSC not
+// formed yet, the candidate solves, the score GEMM and the selection.
+extern "C" int irwls_sgma_rescore(const irwls_dev_set *X, int l, const int *d_cand, int *d_cent, int s,
+                                  const double *d_L, int ldL, double *d_KSC, double *d_W, double *d_Z, double *d_KN,
+                                  int ldz, double *d_eta, double *d_part, int *d_best, double *d_bestval,
+                                  const int *d_need, int *d_built) {
+    const size_t smem = ((size_t)s + X->ld) * sizeof(double);
+    if (smem > 200 * 1024) {
+        irwls_set_error(-7, "SGMA budget %d with feature width %d exceeds the substitution tile", s, X->width);
+        return -7;
+    }
+    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
+    launch_chained(sgma_cand_kernel, dim3(NCAND + sms), dim3(256), smem, kview(X), d_cand, d_cent, s, d_L, ldL, d_W,
+                   d_Z, d_KN, ldz, d_eta, d_need, d_built, l, d_KSC);
+    IRWLS_LAUNCH_CHECK("sgma_cand");
+    launch_chained(sgma_gemm_kernel, dim3(sgma_gemm_grid(l)), dim3(256), 0, kview(X), l, d_cand, s, d_KSC, d_Z, ldz,
+                   d_part, d_need);
+    IRWLS_LAUNCH_CHECK("sgma_gemm");
+    launch_chained(sgma_select_kernel, dim3(1), dim3(NCAND), 0, d_part, sgma_gemm_grid(l), d_eta, d_cand, s, d_cent,
+                   d_best, d_bestval, d_need, d_built);
+    IRWLS_LAUNCH_CHECK("sgma_select");
+    return 0;
+}
+
+// Tensor-core scores: W = K_CN L^-T for the 64 candidates of step s, eta and
+// the bf16 split of W. wpart: irwls_sgma_wpart_count(m) doubles. d_eps (or
+// NULL): the running maximum of |Q_c - w_c| over the candidates.
 extern "C" size_t irwls_sgma_wpart_count(int m) { return ((size_t)m / WT + 2) * NCAND * (size_t)(m > 0 ? m : 1); }
 extern "C" size_t irwls_sgma_lpart_count(int m) { return ((size_t)ceil_div(m, LE) + 1) * (size_t)(m > 0 ? m : 1); }
 
 extern "C" int irwls_sgma_cand_inv(const irwls_dev_set *X, const int *d_cand, const int *d_cent, int s,
                                    const double *d_Linv, int ldi, double *d_KN, int ldz, double *d_wpart, int ldp,
-                                   double *d_W, void *Wb, int ldq, double *d_eta) {
+                                   double *d_W, void *Wb, int ldq, double *d_eta, const void *Qb, unsigned *d_eps) {
     if (s < 1) return 0;
     const size_t smem = (size_t)X->ld * sizeof(double);
     if (smem > 48 * 1024) cudaFuncSetAttribute(cand_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -841,7 +920,7 @@ extern "C" int irwls_sgma_cand_inv(const irwls_dev_set *X, const int *d_cand, co
                    d_wpart, ldp);
     IRWLS_LAUNCH_CHECK("w_gemm");
     launch_chained(w_finish_kernel, dim3(NCAND), dim3(256), 0, d_wpart, ldp, s, d_W, ldz, (__nv_bfloat16 *)Wb, kpad,
-                   d_eta);
+                   d_eta, d_cand, (const __nv_bfloat16 *)Qb, ldq / 32, d_eps);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_SGMA_CAND);
     IRWLS_LAUNCH_CHECK("w_finish");
     return 0;
@@ -876,7 +955,7 @@ extern "C" int irwls_sgma_factor(const irwls_dev_set *X, int s, const int *d_cen
 extern "C" int irwls_sgma_select(const double *d_part, int l, const double *d_eta, const int *d_cand, int s,
                                  int *d_cent, int *d_best, double *d_bestval) {
     sgma_select_kernel<<<1, NCAND, 0, irwls_stream()>>>(d_part, sgma_gemm_grid(l), d_eta, d_cand, s, d_cent, d_best,
-                                                        d_bestval);
+                                                        d_bestval, nullptr, nullptr);
     IRWLS_LAUNCH_CHECK("sgma_select");
     return 0;
 }

@@ -521,14 +521,25 @@ constexpr int CAT_LD = 68;
 // Scores of the precision form: per candidate, the tile sums in 16 strided
 // groups with Kahan-compensated FP32 adds, the 16 group sums in FP64 in a
 // fixed order, score = sum / eta; strict ">" argmax, first index wins.
+//
+// With eps (the plain form's screened selection) the scores only screen: the
+// residuals r = Q w - k carry an absolute error of at most about
+// E = 8 eps + 2^-19 (eps: the largest |Q_c - w_c| seen on 64 random rows per
+// step, 8: a margin for the rows not seen, 2^-19: the FP32 kernel values and
+// products), so sum r^2 over l rows is known to a factor 1 +- d,
+// d = 2x + x^2 + 2^-18, x = E / sqrt(sum r^2 / l). If another row's score can
+// reach the best one's within those bounds, or a bound is not finite, need[0]
+// asks for the FP64 scores of the step (irwls_sgma_rescore).
 __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__restrict__ part, int nblk,
                                                               const double *__restrict__ eta,
                                                               const int *__restrict__ cand, int s, int *cent,
-                                                              int *best, double *bestval, float *scores) {
+                                                              int *best, double *bestval, float *scores,
+                                                              const unsigned *__restrict__ eps, int l, int *need) {
     chain_wait();
     chain_open();
     __shared__ double grp[16][64];
     __shared__ double sc[64];
+    __shared__ float dl[64];
     const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
     float sum = 0.f, comp = 0.f;
     for (int b = g; b < nblk; b += 16) {
@@ -545,6 +556,11 @@ __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__re
         const double et = eta[threadIdx.x];
         sc[threadIdx.x] = (et > 0.0) ? v / et : 0.0;
         if (scores) scores[threadIdx.x] = (float)sc[threadIdx.x];
+        if (eps) {
+            const float x = (8.f * __uint_as_float(eps[0]) + 0x1p-19f) / sqrtf((float)v / (float)l);
+            // eta below 2^-24 in magnitude: its sign is not settled
+            dl[threadIdx.x] = fabs(et) > 0x1p-24 ? 2.f * x + x * x + 0x1p-18f : INFINITY;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -558,6 +574,13 @@ __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__re
         cent[s] = cand[bb];
         best[0] = bb;
         bestval[s] = val;
+        if (eps) {
+            const float low = (float)val * (1.f - dl[bb]);
+            int ask = !(low > 0.f);
+            for (int i = 0; i < 64; ++i)
+                if (i != bb && cand[i] != cand[bb] && !((float)sc[i] * (1.f + dl[i]) < low)) ask = 1;
+            need[0] = ask;
+        }
     }
 }
 
@@ -1065,16 +1088,9 @@ extern "C" void irwls_f32_mirror_free(void *h) {
     free(f);
 }
 
-extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb,
-                                   int ldq, const void *Wb, int s, float *d_part, float *d_resid) {
-    constexpr size_t XS = 24 * 1024;  // largest row-staging buffer (one of two)
-    const int kst = (s + WS_BK - 1) / WS_BK;
-    if (kst * WS_BK > ldq || ldq % WS_BK) {
-        irwls_set_error(-12, "Q leading dimension %d does not hold order %d in 32-column blocks", ldq, s);
-        return -12;
-    }
-    // dynamic shared memory of a CTA: the device's opt-in limit less the
-    // kernel's static shared memory (all instantiations have the same)
+// Dynamic shared memory of a score CTA: the device's opt-in limit less the
+// kernel's static shared memory (all instantiations have the same).
+static size_t score_smem_limit() {
     static size_t limit = 0;
     if (!limit) {
         int dev = 0, optin = 0;
@@ -1088,7 +1104,24 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
         }
         limit = (size_t)optin - fa.sharedSizeBytes;
     }
-    const size_t fixed = 1024 + (size_t)CAT_LD * X->ld * sizeof(float);
+    return limit;
+}
+static size_t score_smem_fixed(const irwls_dev_set *X) { return 1024 + (size_t)CAT_LD * X->ld * sizeof(float); }
+
+// Whether the candidate rows of this feature width fit the score kernel.
+extern "C" int irwls_sgma_tc_fits(const irwls_dev_set *X) {
+    return score_smem_fixed(X) + 2 * TcRing<64, QB_NP, WS_BK>::BYTES <= score_smem_limit();
+}
+
+extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb,
+                                   int ldq, const void *Wb, int s, float *d_part, float *d_resid) {
+    constexpr size_t XS = 24 * 1024;  // largest row-staging buffer (one of two)
+    const int kst = (s + WS_BK - 1) / WS_BK;
+    if (kst * WS_BK > ldq || ldq % WS_BK) {
+        irwls_set_error(-12, "Q leading dimension %d does not hold order %d in 32-column blocks", ldq, s);
+        return -12;
+    }
+    const size_t limit = score_smem_limit(), fixed = score_smem_fixed(X);
     const size_t stage = TcRing<64, QB_NP, WS_BK>::BYTES;
     if (fixed + 2 * stage > limit) {
         irwls_set_error(-12, "feature width %d too wide for the precision-form SGMA tile", X->width);
@@ -1142,10 +1175,12 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
 
 extern "C" int irwls_sgma_tc_partials(int l) { return ceil_div(l, TC_BM); }
 
+// eps, need: the screened selection's error measure and its answer, or NULL.
 extern "C" int irwls_sgma_tc_select(const float *d_part, int nblk, const double *d_eta, const int *d_cand, int s,
-                                    int *d_cent, int *d_best, double *d_bestval, float *d_scores) {
+                                    int *d_cent, int *d_best, double *d_bestval, float *d_scores,
+                                    const unsigned *d_eps, int l, int *d_need) {
     launch_chained(sgma_select_f32_kernel, dim3(1), dim3(1024), 0, d_part, nblk, d_eta, d_cand, s, d_cent, d_best,
-                   d_bestval, d_scores);
+                   d_bestval, d_scores, d_eps, l, d_need);
     IRWLS_LAUNCH_CHECK("sgma_select_f32");
     return 0;
 }

@@ -19,7 +19,8 @@
  *   objective was off by a factor of 4e6), while the digit products' error
  *   (about 2^-45 of the column scales per row) keeps it definite.
  * Selected with irwls_set_precision(IRWLS_PRECISION_MIXED) or the
- * environment variable IRWLS_PRECISION=mixed; plain FP64 is the default.
+ * environment variable IRWLS_PRECISION=mixed; plain FP64 is the default. The
+ * plain form's SGMA uses the same kernels to screen its candidates (below).
  */
 #include <stdio.h>
 #include <stdlib.h>
@@ -30,13 +31,16 @@
 
 int irwls_sgma_cand_inv(const irwls_dev_set *X, const int *d_cand, const int *d_cent, int s, const double *d_Linv,
                         int ldi, double *d_KN, int ldz, double *d_wpart, int ldp, double *d_W, void *Wb, int ldq,
-                        double *d_eta);
+                        double *d_eta, const void *Qb, unsigned *d_eps);
 int irwls_sgma_linv_update(const double *d_L, int ldL, double *d_Linv, int ldi, int s, double *d_lpart,
                            float *d_lrow);
 size_t irwls_sgma_wpart_count(int m);
 size_t irwls_sgma_lpart_count(int m);
 int irwls_sgma_tc_select(const float *d_part, int nblk, const double *d_eta, const int *d_cand, int s, int *d_cent,
-                         int *d_best, double *d_bestval, float *d_scores);
+                         int *d_best, double *d_bestval, float *d_scores, const unsigned *d_eps, int l, int *d_need);
+int irwls_sgma_rescore(const irwls_dev_set *X, int l, const int *d_cand, int *d_cent, int s, const double *d_L, int ldL,
+                       double *d_KSC, double *d_W, double *d_Z, double *d_KN, int ldz, double *d_eta, double *d_part,
+                       int *d_best, double *d_bestval, const int *d_need, int *d_built);
 int irwls_sgma_factor(const irwls_dev_set *X, int s, const int *d_cent, const int *d_best, const double *d_W, int ldz,
                       double *d_L, int ldL);
 /* Qb, Wb: the blocked bf16 hi/mid/lo layout of Q and W (blocked_bf16.cuh);
@@ -45,6 +49,7 @@ int irwls_sgma_factor(const irwls_dev_set *X, int s, const int *d_cent, const in
 int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb, int ldq,
                         const void *Wb, int s, float *d_part, float *d_rq);
 int irwls_sgma_tc_partials(int l);
+int irwls_sgma_tc_fits(const irwls_dev_set *X);
 int irwls_q_column(const irwls_dev_set *X, const void *F, int l, const int *d_cent, int s, const float *lrow, void *Qb,
                    int ldq, float *d_qn);
 int irwls_q_column_resid(int l, const float *d_rq, const int *d_best, int s, const float *lrow, void *Qb, int ldq,
@@ -101,7 +106,14 @@ static void draw_label_rows(const svm_dataset *ds, double want, int n, int *out)
     }
 }
 
-int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out) {
+/* SGMA with tensor-core scores. screen = 0: the precision form. screen = 1:
+ * the plain form -- the tensor-core scores and a measured bound of their error
+ * settle the steps whose best candidate stands clear of the others; the other
+ * steps (a fraction of a percent on the workloads) take the FP64 scores of
+ * all 64 candidates on the device, with the columns of K_nm they need formed
+ * then. The selection is the FP64 one either way. verbose == 1 prints the
+ * scores, so every step then takes the FP64 ones. */
+static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out, int screen) {
     const int m = props.size, l = ds->l;
     if (m <= 0) return 0;
     int *cand = irwls_draw_sgma_candidates(ds, m);
@@ -118,8 +130,10 @@ int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properti
     double *d_resid = NULL;
     void *Qb = NULL, *Wb = NULL;
     /* proposals and traces need the RBF kernel's k(x, x) = 1 */
-    const int learn = g_proposer != NULL && X->mode != IRWLS_K_LINEAR && m > 2;
-    const int trace = g_trace_feat != NULL && m > 2;
+    const int learn = !screen && g_proposer != NULL && X->mode != IRWLS_K_LINEAR && m > 2;
+    const int trace = !screen && g_trace_feat != NULL && m > 2;
+    double *d_KSC = NULL, *d_Z = NULL, *d_part64 = NULL;
+    int *d_need = NULL; /* need, the columns of K_nm formed, and the error measure (float bits) */
     const int nf = irwls_mlp_feature_count(), pool = g_pool, half = g_pool / 2;
     void *F = irwls_f32_mirror(X);
     if (!F) {
@@ -145,6 +159,12 @@ int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properti
     rc |= irwls_dev_malloc((void **)&d_lpart, irwls_sgma_lpart_count(m) * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_qn, (size_t)(l + 2) * sizeof(float));
     rc |= irwls_dev_malloc((void **)&d_resid, sizeof(double));
+    if (screen) {
+        rc |= irwls_dev_malloc((void **)&d_KSC, (size_t)l * m * sizeof(double));
+        rc |= irwls_dev_malloc((void **)&d_Z, (size_t)64 * ldz * sizeof(double));
+        rc |= irwls_dev_malloc((void **)&d_part64, (size_t)irwls_sgma_partials(l) * 64 * sizeof(double));
+        rc |= irwls_dev_malloc((void **)&d_need, 3 * sizeof(int));
+    }
     if (learn || trace) {
         rc |= irwls_dev_malloc((void **)&d_probe, NPROBE * sizeof(int));
         rc |= irwls_dev_malloc((void **)&d_F, (size_t)pool * nf * sizeof(float));
@@ -167,6 +187,8 @@ int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properti
         rc |= irwls_dev_memset(d_W, 0, (size_t)64 * ldz * sizeof(double));
         rc |= irwls_dev_memset(Qb, 0, qb_bytes);
         rc |= irwls_dev_memset(d_qn, 0, (size_t)(l + 2) * sizeof(float));
+        if (screen) rc |= irwls_dev_memset(d_need, 0, 3 * sizeof(int));
+        unsigned *d_eps = screen ? (unsigned *)d_need + 2 : NULL;
         if (learn || trace) {
             /* probe rows and the proposal pools, drawn after the reference's
                candidates so that those stay the plain run's */
@@ -207,19 +229,25 @@ int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properti
             if (trace)
                 rc |= irwls_learn_features(X32, X->ld, X->width, raw, q32, (float)X->neg_gamma, X->y, cs, NCAND,
                                            d_probe, NPROBE, d_qn, d_tfeat + (size_t)(s - 2) * NCAND * nf);
-            rc |= irwls_sgma_cand_inv(X, cs, d_cent, s, d_Linv, ldL, d_KN, ldz, d_wpart, m, d_W, Wb, ldq, d_eta);
+            rc |= irwls_sgma_cand_inv(X, cs, d_cent, s, d_Linv, ldL, d_KN, ldz, d_wpart, m, d_W, Wb, ldq, d_eta, Qb,
+                                      d_eps);
             rc |= irwls_sgma_tc_score(X, F, l, cs, Qb, ldq, Wb, s, d_part, d_rq);
             irwls_prof_begin(IRWLS_PROF_SGMA_UPDATE);
             rc |= irwls_sgma_tc_select(d_part, nblk, d_eta, cs, s, d_cent, d_best, d_val,
-                                       trace ? d_tscore + (size_t)(s - 2) * NCAND : NULL);
+                                       trace ? d_tscore + (size_t)(s - 2) * NCAND : NULL, d_eps, l, d_need);
+            if (screen) {
+                if (props.verbose == 1) rc |= irwls_dev_memset(d_need, 1, sizeof(int));
+                rc |= irwls_sgma_rescore(X, l, cs, d_cent, s, d_L, ldL, d_KSC, d_W, d_Z, d_KN, ldz, d_eta, d_part64,
+                                         d_best, d_val, d_need, d_need + 1);
+            }
             rc |= irwls_sgma_factor(X, s, d_cent, d_best, d_W, ldz, d_L, ldL);
             rc |= irwls_sgma_linv_update(d_L, ldL, d_Linv, ldL, s, d_lpart, lrow);
             rc |= irwls_q_column_resid(l, d_rq, d_best, s, lrow, Qb, ldq, d_qn);
             irwls_prof_end(IRWLS_PROF_SGMA_UPDATE);
         }
         /* Nystrom residual trace(K - K_nm K_mm^-1 K_mn) = sum_i (k_ii - |Q_i|^2) */
-        g_last_residual = -1.0;
-        if (!rc && X->mode != IRWLS_K_LINEAR && !irwls_learn_residual_trace(d_qn, l, d_resid))
+        if (!screen) g_last_residual = -1.0;
+        if (!rc && !screen && X->mode != IRWLS_K_LINEAR && !irwls_learn_residual_trace(d_qn, l, d_resid))
             rc |= irwls_dev_d2h(&g_last_residual, d_resid, sizeof(double));
         if (!rc && trace) {
             rc |= irwls_dev_d2h(g_trace_feat, d_tfeat, (size_t)(m - 2) * NCAND * nf * sizeof(float));
@@ -250,11 +278,26 @@ done:
     free(cand);
     {
         void *bufs[] = {d_cand, d_cent, d_best, d_L, d_W, d_KN, d_eta, d_part, d_val, d_rq, Qb, Wb, lrow,
-                        d_Linv, d_wpart, d_lpart, d_qn, d_resid, d_probe, d_F, d_pool, d_pred, d_tfeat, d_tscore};
+                        d_Linv, d_wpart, d_lpart, d_qn, d_resid, d_probe, d_F, d_pool, d_pred, d_tfeat, d_tscore,
+                        d_KSC, d_Z, d_part64, d_need};
         for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
         irwls_f32_mirror_free(F);
     }
     return rc ? -1 : 0;
+}
+
+int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out) {
+    return sgma_tc_dev(X, ds, props, cent_out, 0);
+}
+
+/* The plain form through the screened selection; -100 when it does not apply:
+ * a linear kernel (Q is not bounded there), a feature width beyond the score
+ * kernel's tile, or K_nm and Q together above 96 GB (the FP64 selection needs
+ * K_nm alone). */
+int irwls_sgma_screened_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out) {
+    const double bytes = (double)ds->l * (14.0 * round_up(props.size, 128) + 256.0);
+    if (X->mode == IRWLS_K_LINEAR || !irwls_sgma_tc_fits(X) || bytes > 96e9) return -100;
+    return sgma_tc_dev(X, ds, props, cent_out, 1);
 }
 
 /* Records the features and exact scores of the candidates of a precision-form
