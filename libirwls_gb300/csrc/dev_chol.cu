@@ -72,28 +72,31 @@ __device__ void factor_block(double (*D)[NB + 1], double *rp, int nb, int k0, in
 // dot product split over 8 lanes of a warp (column j by threads 8 j ..
 // 8 j + 7), Di[c][j] = -(sum_{j <= t < c} D[c][t] Di[t][j]) rp[c].
 // blockDim.x == 256; ends synced.
-__device__ void invert_block(double (*D)[NB + 1], double (*Di)[NB + 1], const double *rp, int nb) {
+__device__ void invert_columns(double (*D)[NB + 1], double (*Di)[NB + 1], const double *rp, int nb) {
     const int tid = threadIdx.x;
-    for (int t = tid; t < NB * NB; t += blockDim.x) Di[t / NB][t % NB] = 0.0;
-    __syncthreads();
     // (every lane of a warp runs the same iterations so that the shuffles
-    // always see the whole warp)
-    {
-        const int j = tid >> 3, q = tid & 7;
-        if (q == 0 && j < nb) Di[j][j] = rp[j];
+    // always see the whole warp; the first row below a warp's four columns
+    // is the first it has to form)
+    const int j = tid >> 3, q = tid & 7;
+    if (q == 0 && j < nb) Di[j][j] = rp[j];
+    __syncwarp();
+    for (int c = (tid >> 5) * 4 + 1; c < nb; ++c) {
+        const bool live = j < nb && c > j;
+        double acc = 0.0;
+        if (live)
+            for (int t = j + q; t < c; t += 8) acc = fma(D[c][t], Di[t][j], acc);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4, 8);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2, 8);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1, 8);
+        if (live && q == 0) Di[c][j] = -acc * rp[c];
         __syncwarp();
-        for (int c = 1; c < NB; ++c) {
-            const bool live = j < nb && c < nb && c > j;
-            double acc = 0.0;
-            if (live)
-                for (int t = j + q; t < c; t += 8) acc = fma(D[c][t], Di[t][j], acc);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 4, 8);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 2, 8);
-            acc += __shfl_xor_sync(0xffffffffu, acc, 1, 8);
-            if (live && q == 0) Di[c][j] = -acc * rp[c];
-            __syncwarp();
-        }
     }
+}
+
+__device__ void invert_block(double (*D)[NB + 1], double (*Di)[NB + 1], const double *rp, int nb) {
+    for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) Di[t / NB][t % NB] = 0.0;
+    __syncthreads();
+    invert_columns(D, Di, rp, nb);
     __syncthreads();
 }
 
@@ -295,24 +298,32 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // The lower blocked matrix (32 x 32 tiles (i, j), i >= j, the right-hand-side
 // row n included as a row) is a list of tasks in column-major order; task t
 // belongs to CTA t mod G, and each CTA runs its tasks in order, keeping its
-// tile in shared memory. A tile takes the updates of panels k = 0 ... j - 1
-// as soon as their tiles L(i, k) and L(j, k) are published, then either
-// factors and inverts itself (i == j) or solves against the published inverse
-// of diagonal block j; it then publishes itself (a release store of a ready
-// word after its data; readers poll with acquire loads and read the data
-// from L2). Every dependency of a task has a smaller index, and all CTAs are
+// tile in shared memory. A tile takes the updates of panels k = 0 ... j - 1,
+// then either factors itself (i == j) or solves against diagonal block j.
+// Every tile is published eight columns at a time (a release store of its
+// column count after the data; readers poll it, fence, and read the data from
+// L2), and its readers take the columns as they come: the panel
+// solves run eight columns behind the pivots, and the next diagonal tile's
+// last update eight columns behind the panel solves, so that a panel costs its
+// pivot chain plus one trailing step of each instead of the sum of whole
+// tiles. Every dependency of a task has a smaller index, and all CTAs are
 // resident (cooperative launch), so the smallest unfinished task can always
-// run: no wait is circular. There are no grid-wide barriers, so a panel's
-// diagonal block is factored as soon as its last update lands while other
-// CTAs are still applying earlier panels elsewhere.
+// run: no wait is circular.
+//
+// What bounds it: an FP64 instruction of one warp takes 65 cycles on this part
+// and holds its SM quarter's FP64 unit for that long (76 with all four busy),
+// so a panel of 32 pivots is a chain of 32 (reciprocal square root 370 cycles,
+// scale, diagonal update). One warp runs that chain on a quarter of its own
+// (factor_stream); six warps on the other three apply the rank-1 updates.
+// Whole tiles at a time, with three CTA barriers per pivot, a panel took 40 to
+// 48 us.
 //
 // Every element gets the multi-launch path's operations in the same order:
 // per panel, acc = sum over the panel's 32 columns by FMA from zero, then
-// M - acc; the diagonal blocks through factor_block; the panel solves by
-// forward substitution against the factored block (subst_block). The
-// results are the same bits. A diagonal block's factor is published before
-// its inverse is formed: only the backward sweep, after this launch, reads
-// the inverse.
+// M - acc; the diagonal blocks as factor_block; the panel solves by forward
+// substitution (subst_block's operations). The results are the same bits. A
+// diagonal block is published before its inverse is formed: only the backward
+// sweep, after this launch, reads the inverse.
 //
 // The waits are bounded: one that runs out (which needs a fault in this
 // schedule) sets the pivot status to -1 and the tensor-core status word to
@@ -320,54 +331,186 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // ---------------------------------------------------------------------------
 constexpr long long DF_WAIT_LIMIT = 1LL << 22;
 constexpr int CHOL_WAIT_CODE = 0x40000000;
+constexpr int DFC = 8;  // columns per published step
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
+__device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
     unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
-
-// Thread 0 polls *p until it is nonzero (or `abort` is set elsewhere); the
-// CTA learns the outcome at the barrier. False if the wait ran out.
-__device__ bool df_wait(const unsigned *p, const volatile int *abort, int *ok_sh) {
-    if (threadIdx.x == 0) {
-        int ok = 0;
-        for (long long it = 0; it < DF_WAIT_LIMIT; ++it) {
-            if (ld_acquire_u32(p)) {
-                ok = 1;
-                break;
-            }
-            if (*abort) break;
-            __nanosleep(64);
-        }
-        *ok_sh = ok;
-    }
-    __syncthreads();
-    return *ok_sh != 0;
+__device__ __forceinline__ void bar_sync(int id, int count) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int count) {
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
 
-// Publishes the tile just stored by the whole CTA.
-__device__ __forceinline__ void df_publish(unsigned *p) {
+// Waits until both column counts exceed `done` and returns the smaller one
+// (thread 0 polls, the CTA learns it at the barrier); 0 if the wait ran out
+// or `abort` is set elsewhere. `got` is a CTA word: two consecutive calls
+// take different ones.
+__device__ int df_wait(const unsigned *p, const unsigned *q, int done, const int *abort, int *got) {
+    if (threadIdx.x == 0) {
+        int v = 0;
+        for (long long it = 0; it < DF_WAIT_LIMIT; ++it) {
+            // (relaxed, so that the three loads overlap; the fence below
+            // orders the data's loads after them)
+            const int a = (int)ld_relaxed_u32(p), b = (int)ld_relaxed_u32(q);
+            const int stop = (int)ld_relaxed_u32((const unsigned *)abort);
+            v = min(a, b);
+            if (v > done) break;
+            v = 0;
+            if (stop) break;
+            if (it > 64) __nanosleep(32);
+        }
+        __threadfence();
+        *got = v;
+    }
+    __syncthreads();
+    return *got;
+}
+
+// Publishes `cols` columns of the tile whose data the whole CTA has stored.
+__device__ __forceinline__ void df_publish(unsigned *p, unsigned cols) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        st_release_u32(p, 1u);
+        st_release_u32(p, cols);
     }
 }
 
-// ready: diag[j] at ready[j] (j < nbc), tile L(i, j) at ready[nbc + j * nbr + i].
-__global__ void __launch_bounds__(256) chol_df_kernel(double *__restrict__ M, int n, int ld, int nrows,
-                                                      int *__restrict__ flags, double *__restrict__ Dinv,
-                                                      unsigned *__restrict__ ready, int *__restrict__ abort) {
+// Factors the nb x nb diagonal block in D (lower part valid) with
+// factor_block's operations, publishing its columns as they are finished.
+// Warp 0 holds the diagonal (lane = row) and runs the pivots: it waits for
+// the next column (barrier 2), scales it by the pivot's reciprocal root and
+// hands it out (barrier 1; barriers 3 to 6 pass eight finished columns each to
+// the publishing warp). Warps 1, 2, 3, 5, 6 and 7 hold the 496 elements
+// below the diagonal, in column order, 32 to a register: group g on warp
+// g mod 6 (so on the three SM quarters warp 0 is not on), the first of a
+// step's live groups holding the next column. Warp 4, beside warp 0, stores
+// and publishes. blockDim.x == 256; ends synced.
+struct FactorShared {
+    double col[2][NB];  // the scaled column, by step parity
+    int failed;
+};
+__device__ void factor_stream(double (*D)[NB + 1], double *rp, int nb, int k0, int *flags, FactorShared &fs, double *M,
+                              int ld, double *Dinv, unsigned *ready) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int ALL = 32 * 7;
+    if (warp == 0) {
+        double dg = lane < nb ? D[lane][lane] : 0.0;
+        int failed = -1;
+        for (int t = 0; t < nb; ++t) {
+            const double s = __shfl_sync(0xffffffffu, dg, t);
+            double r, d;
+            if (s > 0.0) {
+                r = rsqrt(s);
+                d = s * r;
+            } else {
+                if (failed < 0) failed = t;  // stored without its root, as dpotrf leaves it
+                r = 1.0 / s;
+                d = s;
+            }
+            if (t > 0) bar_sync(2, ALL);  // column t is final below the diagonal
+            const double l = lane > t && lane < nb ? D[lane][t] * r : 0.0;
+            fs.col[t & 1][lane] = l;
+            if (lane > t) D[lane][t] = l;
+            if (lane == t) {
+                D[t][t] = d;
+                rp[t] = r;
+            }
+            __syncwarp();
+            if (t + 1 < nb) bar_arrive(1, ALL);
+            if ((t & (DFC - 1)) == DFC - 1 || t == nb - 1) bar_arrive(3 + t / DFC, 64);
+            if (lane > t) dg = fma(-l, l, dg);
+        }
+        if (lane == 0 && failed >= 0) atomicCAS(flags, 0, k0 + failed + 1);
+    } else if (warp == 4) {
+        for (int c0 = 0; c0 < nb; c0 += DFC) {
+            bar_sync(3 + c0 / DFC, 64);
+            const int c1 = min(nb, c0 + DFC);
+            for (int c = c0; c < c1; ++c)
+                if (lane >= c && lane < nb) M[(size_t)(k0 + c) * ld + k0 + lane] = D[lane][c];
+            if (lane >= c0 && lane < c1) Dinv[lane * (NB + 1)] = rp[lane];
+            __syncwarp();
+            if (lane == 0) {
+                __threadfence();
+                st_release_u32(ready, c1 == nb ? NB : c1);
+            }
+        }
+        if (lane >= nb) Dinv[lane * (NB + 1)] = 0.0;
+    } else {
+        const int u = warp < 4 ? warp - 1 : warp - 2;  // 0 ... 5
+        double v[3];
+        int er[3], ec[3];
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            // element e of the strictly lower part in column order
+            int e = (u + 6 * x) * 32 + lane, c = 0;
+            while (c < NB - 1 && e >= NB - 1 - c) {
+                e -= NB - 1 - c;
+                ++c;
+            }
+            ec[x] = c < NB - 1 ? c : -1;  // past the last element: never live
+            er[x] = c < NB - 1 ? c + 1 + e : 0;
+            v[x] = ec[x] >= 0 ? D[er[x]][ec[x]] : 0.0;
+        }
+        for (int t = 0; t + 1 < nb; ++t) {
+            bar_sync(1, ALL);
+            const double *l = fs.col[t & 1];
+            bool told = false;
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+                const bool live = ec[x] > t;
+                if (!__any_sync(0xffffffffu, live)) continue;
+                // the next column lies in this warp's first live groups
+                if (!told && !__any_sync(0xffffffffu, ec[x] == t + 1)) {
+                    bar_arrive(2, ALL);
+                    told = true;
+                }
+                if (live) v[x] = fma(-l[er[x]], l[ec[x]], v[x]);
+                if (ec[x] == t + 1) D[er[x]][ec[x]] = v[x];
+            }
+            if (!told) {
+                __syncwarp();
+                bar_arrive(2, ALL);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// ready: columns published of diag[j] at ready[j] (j < nbc), of tile L(i, j)
+// at ready[nbc + j * nbr + i]. b: the right-hand side (row n), or NULL when
+// it is in row n of M already.
+__global__ void __launch_bounds__(256, 1) chol_df_kernel(double *__restrict__ M, int n, int ld, int nrows,
+                                                      const double *__restrict__ b, int *__restrict__ flags,
+                                                      double *__restrict__ Dinv, unsigned *__restrict__ ready,
+                                                      int *__restrict__ abort) {
     __shared__ double T[NB][NB + 1], Li[NB][NB + 1], Lj[NB][NB + 1];
     __shared__ double rp[NB];
-    __shared__ int failed_at, ok_sh;
+    __shared__ FactorShared fs;
+    __shared__ int got[2];
     const int tid = threadIdx.x;
     const int nbc = (n + NB - 1) / NB, nbr = (nrows + NB - 1) / NB;
-    int t = 0;
+    int t = 0, w = 0;
+    // the pivot status; every block that can fail comes after tile 0 (this
+    // CTA's) by the chain of published tiles
+    if (blockIdx.x == 0 && tid == 0) *flags = 0;
+    // this thread's elements of a diagonal tile's lower triangle
+    int dr[3], dc[3];
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        const int e = tid + 256 * x;
+        int r = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+        while (r * (r + 1) / 2 > e) --r;
+        while ((r + 1) * (r + 2) / 2 <= e) ++r;
+        dr[x] = r;
+        dc[x] = e - r * (r + 1) / 2;
+    }
     for (int j = 0; j < nbc; ++j) {
         for (int i = j; i < nbr; ++i, ++t) {
             if (t % (int)gridDim.x != (int)blockIdx.x) continue;
@@ -375,92 +518,120 @@ __global__ void __launch_bounds__(256) chol_df_kernel(double *__restrict__ M, in
             const int nr = min(NB, nrows - r0), nc = min(NB, n - c0);
             for (int e = tid; e < NB * NB; e += 256) {
                 const int r = e % NB, c = e / NB;
-                T[r][c] = (r < nr && c < nc && (i != j || c <= r)) ? __ldcg(M + (size_t)(c0 + c) * ld + r0 + r) : 0.0;
+                double v = 0.0;
+                if (r < nr && c < nc && (i != j || c <= r))
+                    v = b && r0 + r == n ? b[c0 + c] : __ldcg(M + (size_t)(c0 + c) * ld + r0 + r);
+                T[r][c] = v;
             }
             for (int k = 0; k < j; ++k) {
                 const int kc = NB * k;
-                if (!df_wait(ready + nbc + (size_t)k * nbr + i, abort, &ok_sh) ||
-                    !df_wait(ready + nbc + (size_t)k * nbr + j, abort, &ok_sh))
-                    goto fail;
-                for (int e = tid; e < NB * NB; e += 256) {
-                    const int r = e % NB, kk = e / NB;
-                    Li[r][kk] = r < nr ? __ldcg(M + (size_t)(kc + kk) * ld + r0 + r) : 0.0;
-                    Lj[r][kk] = r < nc ? __ldcg(M + (size_t)(kc + kk) * ld + c0 + r) : 0.0;
+                const unsigned *pi = ready + nbc + (size_t)k * nbr + i, *pj = ready + nbc + (size_t)k * nbr + j;
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                for (int done = 0; done < NB;) {
+                    const int have = df_wait(pi, pj, done, abort, got + (w++ & 1));
+                    if (have == 0) goto fail;
+                    for (int e = tid; e < NB * (have - done); e += 256) {
+                        const int r = e % NB, kk = done + e / NB;
+                        Li[r][kk] = r < nr ? __ldcg(M + (size_t)(kc + kk) * ld + r0 + r) : 0.0;
+                        if (i != j) Lj[r][kk] = r < nc ? __ldcg(M + (size_t)(kc + kk) * ld + c0 + r) : 0.0;
+                    }
+                    __syncthreads();
+                    if (i != j) {
+                        const int r = tid % NB, u = tid / NB;
+                        for (int kk = done; kk < have; kk += DFC)
+#pragma unroll
+                            for (int h = 0; h < DFC; ++h)
+#pragma unroll
+                                for (int x = 0; x < 4; ++x)
+                                    acc[x] = fma(Li[r][kk + h], Lj[u + 8 * x][kk + h], acc[x]);
+                    } else {
+                        for (int kk = done; kk < have; kk += DFC)
+#pragma unroll
+                            for (int h = 0; h < DFC; ++h)
+#pragma unroll
+                                for (int x = 0; x < 3; ++x)
+                                    if (x < 2 || tid < NB * (NB + 1) / 2 - 512)
+                                        acc[x] = fma(Li[dr[x]][kk + h], Li[dc[x]][kk + h], acc[x]);
+                    }
+                    done = have;
                 }
-                __syncthreads();
                 if (i != j) {
-                    const int r = tid % NB;
-                    for (int cc = tid / NB; cc < NB; cc += 8) {
-                        if (r >= nr || cc >= nc) continue;
-                        double acc = 0.0;
-#pragma unroll 8
-                        for (int kk = 0; kk < NB; ++kk) acc = fma(Li[r][kk], Lj[cc][kk], acc);
-                        T[r][cc] = T[r][cc] - acc;
-                    }
+                    const int r = tid % NB, u = tid / NB;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                        if (r < nr && u + 8 * x < nc) T[r][u + 8 * x] = T[r][u + 8 * x] - acc[x];
                 } else {
-                    // a diagonal tile needs only its lower triangle: threads
-                    // take its NB (NB + 1) / 2 elements (the same FMAs per
-                    // element), not the full tile's divergent columns, which
-                    // halves this step on the factorization's critical path
-                    for (int e = tid; e < NB * (NB + 1) / 2; e += 256) {
-                        int r = (int)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
-                        while (r * (r + 1) / 2 > e) --r;
-                        while ((r + 1) * (r + 2) / 2 <= e) ++r;
-                        const int cc = e - r * (r + 1) / 2;
-                        if (r >= nr || cc >= nc) continue;
-                        double acc = 0.0;
-#pragma unroll 8
-                        for (int kk = 0; kk < NB; ++kk) acc = fma(Li[r][kk], Lj[cc][kk], acc);
-                        T[r][cc] = T[r][cc] - acc;
-                    }
+#pragma unroll
+                    for (int x = 0; x < 3; ++x)
+                        if ((x < 2 || tid < NB * (NB + 1) / 2 - 512) && dr[x] < nr && dc[x] < nc)
+                            T[dr[x]][dc[x]] = T[dr[x]][dc[x]] - acc[x];
                 }
                 __syncthreads();
             }
             if (i == j) {
-                // rows >= n of this tile (the right-hand side) wait in Lj
+                // row nc of this tile (the right-hand side) waits in Li
                 for (int e = tid; e < NB * NB; e += 256) {
                     const int r = e % NB, c = e / NB;
-                    Lj[r][c] = (r >= nc && r < nr && c < nc) ? T[r][c] : 0.0;
+                    if (r == nc && r < nr && c < nc) Li[0][c] = T[r][c];
                     if (r >= nc || c > r) T[r][c] = 0.0;
                 }
                 __syncthreads();
-                factor_block(T, rp, nc, c0, flags, &failed_at);
-                // the factor and its reciprocal pivots (the inverse's
-                // diagonal) are all the panel solves read: publish them now
-                for (int e = tid; e < NB * NB; e += 256) {
-                    const int r = e / NB, c = e % NB;
-                    if (r < nc && c <= r) M[(size_t)(c0 + c) * ld + c0 + r] = T[r][c];
-                }
-                if (tid < NB) Dinv[(size_t)j * NB * NB + tid * (NB + 1)] = tid < nc ? rp[tid] : 0.0;
-                df_publish(ready + j);
-                // the right-hand-side row, by the same substitution
-                if (nr > nc) {
-                    for (int e = tid; e < NB * NB; e += 256) {
-                        const int r = e / NB, c = e % NB;
-                        if (r < nr - nc) Li[r][c] = Lj[nc + r][c];
+                factor_stream(T, rp, nc, c0, flags, fs, M, ld, Dinv + (size_t)j * NB * NB, ready + j);
+                for (int e = tid; e < NB * NB; e += 256) Lj[e / NB][e % NB] = 0.0;
+                __syncthreads();
+                // the right-hand-side row, by the panel solves' substitution:
+                // warp 7 (whose columns of the inverse are the shortest) with
+                // lane = column
+                if (nr > nc && tid >= 224) {
+                    const int c = tid - 224;
+                    double v = c < nc ? Li[0][c] : 0.0;
+                    for (int q = 0; q < nc; ++q) {
+                        if (c == q) v = v * rp[q];
+                        const double x = __shfl_sync(0xffffffffu, v, q);
+                        if (c > q && c < nc) v = fma(-x, T[c][q], v);
                     }
-                    __syncthreads();
-                    subst_block(Li, nr - nc, T, rp, nc);
-                    for (int c = tid; c < nc; c += 256) M[(size_t)(c0 + c) * ld + r0 + nc] = Li[0][c];
-                    df_publish(ready + nbc + (size_t)j * nbr + i);
+                    if (c < nc) M[(size_t)(c0 + c) * ld + r0 + nc] = v;
                 }
                 // the inverse (for the backward sweep after this launch)
-                invert_block(T, Lj, rp, nc);
+                invert_columns(T, Lj, rp, nc);
+                __syncthreads();
                 for (int e = tid; e < NB * NB; e += 256) Dinv[(size_t)j * NB * NB + e] = Lj[e / NB][e % NB];
             } else {
-                if (!df_wait(ready + j, abort, &ok_sh)) goto fail;
-                for (int e = tid; e < NB * NB; e += 256) {
-                    const int r = e / NB, c = e % NB;
-                    Li[r][c] = (r < nc && c <= r) ? __ldcg(M + (size_t)(c0 + c) * ld + c0 + r) : 0.0;
+                // the panel solve, eight columns at a time: within them by the
+                // 32 x 8 threads (row, column), then the later columns
+                // (nc == NB: a tile below a diagonal block has whole columns)
+                const int r = tid % NB, u = tid / NB;
+                for (int done = 0; done < NB;) {
+                    const int have = df_wait(ready + j, ready + j, done, abort, got + (w++ & 1));
+                    if (have == 0) goto fail;
+                    for (int e = tid; e < NB * (have - done); e += 256) {
+                        const int rr = e % NB, c = done + e / NB;
+                        Li[rr][c] = c <= rr ? __ldcg(M + (size_t)(c0 + c) * ld + c0 + rr) : 0.0;
+                    }
+                    if (tid >= done && tid < have) rp[tid] = __ldcg(Dinv + (size_t)j * NB * NB + tid * (NB + 1));
+                    __syncthreads();
+                    for (; done < have; done += DFC) {
+                        double v = T[r][done + u];
+#pragma unroll
+                        for (int q = 0; q < DFC; ++q) {
+                            if (u == q) {
+                                v = v * rp[done + q];
+                                T[r][done + q] = v;
+                            }
+                            __syncthreads();
+                            if (u > q) v = fma(-T[r][done + q], Li[done + u][done + q], v);
+                        }
+                        if (r < nr) M[(size_t)(c0 + done + u) * ld + r0 + r] = v;
+                        df_publish(ready + nbc + (size_t)j * nbr + i, done + DFC);
+                        for (int c = done + DFC + u; c < NB; c += 8) {
+                            double z = T[r][c];
+#pragma unroll
+                            for (int q = 0; q < DFC; ++q) z = fma(-T[r][done + q], Li[c][done + q], z);
+                            T[r][c] = z;
+                        }
+                        __syncthreads();
+                    }
                 }
-                if (tid < NB) rp[tid] = __ldcg(Dinv + (size_t)j * NB * NB + tid * (NB + 1));
-                __syncthreads();
-                subst_block(T, nr, Li, rp, nc);
-                for (int e = tid; e < NB * NB; e += 256) {
-                    const int c = e / NB, r = e % NB;
-                    if (c < nc && r < nr) M[(size_t)(c0 + c) * ld + r0 + r] = T[r][c];
-                }
-                df_publish(ready + nbc + (size_t)j * nbr + i);
             }
             __syncthreads();
         }
@@ -553,6 +724,105 @@ __global__ void __launch_bounds__(256) chol_backsolve_coop_kernel(double *__rest
     }
 }
 
+// The same sweep in one thread-block cluster of ceil(n / 256) CTAs (orders up
+// to 2048), block b of 32 rows on CTA b mod g with its z in shared memory. Per
+// block from the bottom its owner forms x_b and stores it into every CTA's
+// shared memory; a split cluster barrier hands it out. The owner of block
+// b - 1 applies x_b to it at once and goes on to x_(b-1); the other blocks
+// take x_b between their CTA's arrival at the next barrier and its wait, so
+// the chain per block is one block's update and dot product. A dot product's
+// four partial chains (sweep_dot, sweep_row) run on four lanes, eight FMAs
+// each, instead of one after another on one: 65 cycles per FP64 instruction
+// whatever the lanes. x_b lives in one of four slots: it is last read before
+// the wait of block b - 1, and block b - 4 writes the slot next.
+__device__ __forceinline__ double chains_sum(double a) {
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    return a + __shfl_xor_sync(0xffffffffu, a, 2);  // (a0 + a1) + (a2 + a3)
+}
+
+constexpr int SWB = 8;  // blocks of a CTA
+__global__ void __launch_bounds__(256) chol_sweep_cluster_kernel(const double *__restrict__ M, int n, int ld,
+                                                                 const double *__restrict__ Dinv,
+                                                                 double *__restrict__ x, const int *__restrict__ flags,
+                                                                 int *__restrict__ info) {
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    __shared__ double z[SWB][NB], xb[4][NB], Di[2][NB][NB + 1];
+    const int g = (int)cl.num_blocks(), me = (int)cl.block_rank();
+    const int tid = threadIdx.x, half = tid >> 7;
+    const int row = 8 * ((tid >> 5) & 3) + ((tid & 31) >> 2), ch = tid & 3;  // row of a block, partial chain
+    const int nblk = (n + NB - 1) / NB;
+    for (int e = tid; e < SWB * NB; e += 256) {
+        const int c = ((e / NB) * g + me) * NB + e % NB;
+        z[e / NB][e % NB] = c < n ? M[(size_t)c * ld + n] : 0.0;
+    }
+    auto load_inv = [&](int b) {
+        for (int t = tid; t < NB * NB; t += 256) Di[b & 1][t / NB][t % NB] = Dinv[(size_t)b * NB * NB + t];
+    };
+    if ((nblk - 1) % g == me) load_inv(nblk - 1);
+    if (info && me == 0 && tid == 0) *info = *flags;
+    cl.sync();
+    // z of block q minus its rows of L_b^T times x_b; l: the row's values
+    // 4 k + ch when they are loaded already
+    auto update = [&](int q, int b, const double *l) {
+        const int nb = min(NB, n - NB * b);
+        const double *col = M + (size_t)(NB * q + row) * ld + NB * b, *xs = xb[b & 3];
+        double a = 0.0;
+        if (nb == NB) {
+            double v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = l ? l[k] : col[4 * k + ch];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) a = fma(v[k], xs[4 * k + ch], a);
+        } else {
+            for (int k = 0; k < nb / 4; ++k) a = fma(col[4 * k + ch], xs[4 * k + ch], a);
+            if (ch == 0)
+                for (int c = nb / 4 * 4; c < nb; ++c) a = fma(col[c], xs[c], a);
+        }
+        a = chains_sum(a);
+        if (ch == 0) z[q / g][row] = z[q / g][row] - a;
+    };
+    for (int b = nblk - 1; b >= 0; --b) {
+        if (b % g == me && half == 0) {
+            const int nb = min(NB, n - NB * b), t = row, K = t < nb ? (nb - t) / 4 : 0;
+            const double(*D)[NB + 1] = Di[b & 1];
+            const double *yb = z[b / g];
+            double a = 0.0;
+            for (int k = 0; k < K; ++k) a = fma(D[t + 4 * k + ch][t], yb[t + 4 * k + ch], a);
+            if (ch == 0)
+                for (int c = t + 4 * K; c < nb; ++c) a = fma(D[c][t], yb[c], a);
+            a = chains_sum(a);
+            if (ch == 0 && t < nb) {
+                x[NB * b + t] = a;
+                if (b > 0)
+                    for (int r = 0; r < g; ++r) *cl.map_shared_rank(&xb[b & 3][t], r) = a;
+            }
+        }
+        if (b == 0) break;
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+        const bool next = (b - 1) % g == me;
+        double pre[8];
+        if (next) {
+            load_inv(b - 1);
+            if (half == 0 && NB * b + NB <= n) {
+                const double *col = M + (size_t)(NB * (b - 1) + row) * ld + NB * b;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) pre[k] = col[4 * k + ch];
+            }
+        }
+        // the previous block's x for this CTA's blocks below b (block b has it)
+        if (b + 1 < nblk)
+            for (int s = half; s * g + me < b; s += 2) update(s * g + me, b + 1, nullptr);
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+        if (next) {
+            __syncthreads();
+            if (half == 0) update(b - 1, b, pre);
+            __syncthreads();
+        }
+    }
+}
+
 // CTAs of the cooperative sweep for order n on the current device, or 0 when
 // they cannot all be resident at once (the single-CTA sweep is used then).
 // The capacity is computed per device from the device's own attributes (the
@@ -584,25 +854,52 @@ int coop_backsolve_ctas(int n) {
     return g <= c - 1 ? g : 0;
 }
 
+// Whether a cluster of g <= 8 CTAs of the sweep can run on the current device.
+bool sweep_cluster_ok() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> state[kDevices];  // 0: not known, 1: no, 2: yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (dev < 0 || dev >= kDevices) return false;
+    int v = state[dev].load(std::memory_order_acquire);
+    if (v == 0) {
+        int has = 0;
+        if (cudaDeviceGetAttribute(&has, cudaDevAttrClusterLaunch, dev) != cudaSuccess) {
+            cudaGetLastError();
+            has = 0;
+        }
+        v = has ? 2 : 1;
+        state[dev].store(v, std::memory_order_release);
+    }
+    return v == 2;
+}
+
 int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, double *Dinv, cudaStream_t st);
-int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, cudaStream_t st);
+int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
+                           cudaStream_t st);
 
 // ready: the data-flow path's list (df_ready_words words), or NULL for the
-// multi-launch path.
-int chol_enqueue(double *d_M, int n, int ld, double *d_x, int *flags, double *Dinv, cudaStream_t st,
-                 unsigned *ready = nullptr) {
+// multi-launch path. d_b: the right-hand side, or NULL when row n of M holds
+// it. The pivot status starts at zero here; it goes to d_info (or NULL) too.
+int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int *flags, double *Dinv, int *d_info,
+                 cudaStream_t st, unsigned *ready = nullptr) {
     const int has_b = d_x != nullptr;
     const int nrows = n + has_b;
     const int G = ready && g_chol_path != 1 ? df_capacity() : 0;
+    cudaError_t e = cudaSuccess;
     if (G > 0) {
         // one cooperative launch of the data-flow factorization
         const size_t words = df_ready_words(n, has_b);
-        cudaError_t e = cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
+        e = cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
         const int nbc = (n + NB - 1) / NB, nbr = (nrows + NB - 1) / NB;
         const int tasks = nbc * (2 * nbr - nbc + 1) / 2;
         int grid = std::min(G, tasks);
         int *abort = (int *)(ready + words - 1);
-        void *args[] = {&d_M, &n, &ld, (void *)&nrows, &flags, &Dinv, &ready, &abort};
+        const double *b = has_b ? d_b : nullptr;
+        void *args[] = {&d_M, &n, &ld, (void *)&nrows, &b, &flags, &Dinv, &ready, &abort};
         if (e == cudaSuccess)
             e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(256), args, 0, st);
         if (e != cudaSuccess) {
@@ -614,10 +911,23 @@ int chol_enqueue(double *d_M, int n, int ld, double *d_x, int *flags, double *Di
         irwls_set_error(-2, "the data-flow Cholesky needs a cooperative launch");
         return -2;
     } else {
+        e = cudaMemsetAsync(flags, 0, sizeof(int), st);
+        if (e == cudaSuccess && d_b && has_b)  // b becomes row n: M[c*ld + n] = b[c]
+            e = cudaMemcpy2DAsync(d_M + n, (size_t)ld * sizeof(double), d_b, sizeof(double), sizeof(double), n,
+                                  cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) {
+            irwls_set_error(-2, "rhs copy: %s", cudaGetErrorString(e));
+            return -2;
+        }
         const int rc = chol_enqueue_panels(d_M, n, ld, nrows, flags, Dinv, st);
         if (rc) return rc;
     }
-    return has_b ? chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, st) : 0;
+    if (has_b) return chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st);
+    if (d_info && (e = cudaMemcpyAsync(d_info, flags, sizeof(int), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) {
+        irwls_set_error(-2, "pivot status: %s", cudaGetErrorString(e));
+        return -2;
+    }
+    return 0;
 }
 
 // The multi-launch factorization: per panel a solve launch and an update
@@ -642,9 +952,38 @@ int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, doubl
     return 0;
 }
 
-// The backward sweep L^T x = z (z in row n of M).
-int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, cudaStream_t st) {
+// The backward sweep L^T x = z (z in row n of M): the cluster form up to order
+// 2048, the cooperative one above, one CTA where neither can run. They give
+// the same bits.
+int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
+                           cudaStream_t st) {
     {
+        if (n <= 8 * SWB * NB && sweep_cluster_ok()) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((n + SWB * NB - 1) / (SWB * NB));
+            cfg.blockDim = dim3(256);
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cfg.gridDim.x;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_sweep_cluster_kernel, (const double *)d_M, n, ld,
+                                                     (const double *)Dinv, d_x, flags, d_info);
+            if (e != cudaSuccess) {
+                irwls_set_error(-2, "CUDA error in chol_sweep (cluster): %s", cudaGetErrorString(e));
+                return -2;
+            }
+            irwls_count_launch(1);
+            return 0;
+        }
+        cudaError_t ei = cudaSuccess;
+        if (d_info) ei = cudaMemcpyAsync(d_info, flags, sizeof(int), cudaMemcpyDeviceToDevice, st);
+        if (ei != cudaSuccess) {
+            irwls_set_error(-2, "pivot status: %s", cudaGetErrorString(ei));
+            return -2;
+        }
         const int g = coop_backsolve_ctas(n);
         if (g > 0) {
             void *args[] = {&d_M, &n, &ld, &Dinv, &d_x};
@@ -689,16 +1028,6 @@ extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_
         return -6;
     }
     int *flags = irwls_dev_flags();
-    if (irwls_dev_memset(flags, 0, sizeof(int))) return -2;
-    if (d_b) {
-        // b becomes row n: M[c*ld + n] = b[c]
-        cudaError_t e = cudaMemcpy2DAsync(d_M + n, (size_t)ld * sizeof(double), d_b, sizeof(double), sizeof(double), n,
-                                          cudaMemcpyDeviceToDevice, irwls_stream());
-        if (e != cudaSuccess) {
-            irwls_set_error(-2, "rhs copy: %s", cudaGetErrorString(e));
-            return -2;
-        }
-    }
     const int npanel = ceil_div(n, NB);
     // factored diagonal blocks: the context's grow-only scratch slot 0
     double *diag = (double *)irwls_ctx_scratch(0, (size_t)npanel * NB * NB * sizeof(double));
@@ -707,7 +1036,7 @@ extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_
     unsigned *ready = (unsigned *)irwls_ctx_scratch(3, df_ready_words(n, d_x != nullptr) * sizeof(unsigned));
     if (!ready) return -3;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_CHOL);
-    int rc = chol_enqueue(d_M, n, ld, d_x, flags, diag, irwls_stream(), ready);
+    int rc = chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, nullptr, irwls_stream(), ready);
     if (rc) return rc;
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_CHOL);
     return 0;
@@ -828,26 +1157,6 @@ extern "C" int irwls_chol_solve_noalloc(double *d_M, int n, int ld, const double
     int *flags = (int *)(diag + IRWLS_NOALLOC_PANELS * NB * NB);
     unsigned *ready = (unsigned *)(diag + IRWLS_NOALLOC_PANELS * NB * NB + 32);
     cudaStream_t st = (cudaStream_t)stream;
-    // the pivot status must start at zero; the diagonal blocks are fully
-    // rewritten before they are read
-    if ((e = cudaMemsetAsync(flags, 0, sizeof(int), st)) != cudaSuccess) {
-        irwls_set_error(-2, "irwls_chol_solve_noalloc: %s", cudaGetErrorString(e));
-        return -2;
-    }
-    if (d_b) {
-        e = cudaMemcpy2DAsync(d_M + n, (size_t)ld * sizeof(double), d_b, sizeof(double), sizeof(double), n,
-                              cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) {
-            irwls_set_error(-2, "irwls_chol_solve_noalloc: rhs copy: %s", cudaGetErrorString(e));
-            return -2;
-        }
-    }
     // order <= 4096: the backward sweep's vector fits the default 48 KiB
-    const int rc = chol_enqueue(d_M, n, ld, d_x, flags, diag, st, ready);
-    if (rc) return rc;
-    if (d_info && (e = cudaMemcpyAsync(d_info, flags, sizeof(int), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) {
-        irwls_set_error(-2, "irwls_chol_solve_noalloc: %s", cudaGetErrorString(e));
-        return -2;
-    }
-    return 0;
+    return chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, d_info, st, ready);
 }
