@@ -277,8 +277,10 @@ double irwls_fp32_peak_tflops(int reps);
  * Returns 0 on success. */
 int irwls_chol_solve_noalloc(double *d_M, int n, int ld, const double *d_b, double *d_x, int *d_info,
                              void *stream);
-/* CTAs of the cooperative backward sweep that a solve of order n uses on the
- * current device (0: the single-CTA sweep); no counterpart in the reference. */
+/* CTAs of the cooperative backward sweep for order n on the current device
+ * (0: the single-CTA sweep); orders up to 2048 take a sweep in one thread-block
+ * cluster instead where the device has clusters. No counterpart in the
+ * reference. */
 int irwls_chol_sweep_ctas(int n);
 /* Test hook, no counterpart in the reference: which Cholesky factorization
  * the solves use. 0 (default): one cooperative launch scheduled by data flow

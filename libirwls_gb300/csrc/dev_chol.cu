@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "dev_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace {
 
@@ -300,13 +301,15 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // belongs to CTA t mod G, and each CTA runs its tasks in order, keeping its
 // tile in shared memory. A tile takes the updates of panels k = 0 ... j - 1,
 // then either factors itself (i == j) or solves against diagonal block j.
-// Every tile is published eight columns at a time (a release store of its
-// column count after the data; readers poll it, fence, and read the data from
-// L2), and its readers take the columns as they come: the panel
-// solves run eight columns behind the pivots, and the next diagonal tile's
-// last update eight columns behind the panel solves, so that a panel costs its
+// Every tile is published four columns at a time (a release store of its
+// column count after the data; readers poll it with acquire loads and read the
+// data from L2), and its readers take the columns as they come: the panel
+// solves run four columns behind the pivots, and the next diagonal tile's
+// last update four columns behind the panel solves, so that a panel costs its
 // pivot chain plus one trailing step of each instead of the sum of whole
-// tiles. Every dependency of a task has a smaller index, and all CTAs are
+// tiles. In each CTA one warp polls and loads ahead into a ring of steps, one
+// stores and publishes, and eight compute: a poll and its loads take about
+// 1300 cycles and a publication 1400, which would otherwise add to each step. Every dependency of a task has a smaller index, and all CTAs are
 // resident (cooperative launch), so the smallest unfinished task can always
 // run: no wait is circular.
 //
@@ -331,11 +334,23 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // ---------------------------------------------------------------------------
 constexpr long long DF_WAIT_LIMIT = 1LL << 22;
 constexpr int CHOL_WAIT_CODE = 0x40000000;
-constexpr int DFC = 8;  // columns per published step
+constexpr int DFC = 4;               // columns per published step
+constexpr int DFQ = NB / DFC;        // steps of a tile
+constexpr int DFR = 6;               // ring slots of steps
+constexpr int DF_THREADS = 320;      // warps 0-7 compute, 8 loads, 9 publishes
+// named barriers: 1 and 2 the pivots' (factor_stream), 3 ... finished columns
+// of a diagonal block, then the compute warps' own two
+constexpr int BAR_ALL = 3 + DFQ, BAR_STEP = BAR_ALL + 1;
+static_assert(BAR_STEP < 16, "named barriers");
 
 __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
     unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
@@ -348,101 +363,58 @@ __device__ __forceinline__ void bar_arrive(int id, int count) {
     asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
 
-// Waits until both column counts exceed `done` and returns the smaller one
-// (thread 0 polls, the CTA learns it at the barrier); 0 if the wait ran out
-// or `abort` is set elsewhere. `got` is a CTA word: two consecutive calls
-// take different ones.
-__device__ int df_wait(const unsigned *p, const unsigned *q, int done, const int *abort, int *got) {
-    if (threadIdx.x == 0) {
-        int v = 0;
-        for (long long it = 0; it < DF_WAIT_LIMIT; ++it) {
-            // (relaxed, so that the three loads overlap; the fence below
-            // orders the data's loads after them)
-            const int a = (int)ld_relaxed_u32(p), b = (int)ld_relaxed_u32(q);
-            const int stop = (int)ld_relaxed_u32((const unsigned *)abort);
-            v = min(a, b);
-            if (v > done) break;
-            v = 0;
-            if (stop) break;
-            if (it > 64) __nanosleep(32);
-        }
-        __threadfence();
-        *got = v;
-    }
-    __syncthreads();
-    return *got;
-}
-
-// Publishes `cols` columns of the tile whose data the whole CTA has stored.
-__device__ __forceinline__ void df_publish(unsigned *p, unsigned cols) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        st_release_u32(p, cols);
-    }
-}
-
-// Factors the nb x nb diagonal block in D (lower part valid) with
-// factor_block's operations, publishing its columns as they are finished.
-// Warp 0 holds the diagonal (lane = row) and runs the pivots: it waits for
-// the next column (barrier 2), scales it by the pivot's reciprocal root and
-// hands it out (barrier 1; barriers 3 to 6 pass eight finished columns each to
-// the publishing warp). Warps 1, 2, 3, 5, 6 and 7 hold the 496 elements
-// below the diagonal, in column order, 32 to a register: group g on warp
-// g mod 6 (so on the three SM quarters warp 0 is not on), the first of a
-// step's live groups holding the next column. Warp 4, beside warp 0, stores
-// and publishes. blockDim.x == 256; ends synced.
-struct FactorShared {
-    double col[2][NB];  // the scaled column, by step parity
-    int failed;
+// One step of columns in shared memory: rows of the tile's own block row (or
+// of the diagonal block), rows of the other block row, the reciprocal pivots.
+struct DfSlot {
+    double a[NB][DFC + 1], b[NB][DFC + 1], rp[DFC];
 };
-__device__ void factor_stream(double (*D)[NB + 1], double *rp, int nb, int k0, int *flags, FactorShared &fs, double *M,
-                              int ld, double *Dinv, unsigned *ready) {
+struct DfShared {
+    double T[NB][NB + 1], Di[NB][NB + 1];
+    double rp[NB], rhs[NB];
+    double col[2][NB];  // factor_stream: the scaled column, by step parity
+    DfSlot slot[DFR];
+    // pub: one per step of a tile, so that the computing warps may run ahead
+    // of the publisher; used again after done, the publisher's end of a tile
+    uint64_t full[DFR], empty[DFR], pub[DFQ], done;
+    volatile int bad[DFR], stop;  // the loader gave up in a slot; the computing warps did
+};
+
+// Factors the nb x nb diagonal block in T (lower part valid) with
+// factor_block's operations, handing its columns to the publishing warp as
+// they are finished. Warp 0 holds the diagonal (lane = row) and runs the
+// pivots: it waits for the next column (barrier 2), scales it by the pivot's
+// reciprocal root and hands it out (barrier 1; one barrier from 3 on per DFC
+// finished columns, for the publisher). Warps 1, 2, 3, 5, 6 and 7 hold the 496
+// elements below the diagonal, in column order, 32 to a register: group g on
+// warp g mod 6 (so on the three SM quarters warp 0 is not on), the first of a
+// step's live groups holding the next column. Signs are tested on the bits: an
+// FP64 compare would take the unit for 65 cycles.
+__device__ void factor_stream(DfShared &sh, int nb, int k0, int *flags) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int ALL = 32 * 7;
+    double(*D)[NB + 1] = sh.T;
     if (warp == 0) {
         double dg = lane < nb ? D[lane][lane] : 0.0;
         int failed = -1;
         for (int t = 0; t < nb; ++t) {
             const double s = __shfl_sync(0xffffffffu, dg, t);
-            double r, d;
-            if (s > 0.0) {
-                r = rsqrt(s);
-                d = s * r;
-            } else {
-                if (failed < 0) failed = t;  // stored without its root, as dpotrf leaves it
-                r = 1.0 / s;
-                d = s;
-            }
-            if (t > 0) bar_sync(2, ALL);  // column t is final below the diagonal
-            const double l = lane > t && lane < nb ? D[lane][t] * r : 0.0;
-            fs.col[t & 1][lane] = l;
-            if (lane > t) D[lane][t] = l;
-            if (lane == t) {
-                D[t][t] = d;
-                rp[t] = r;
-            }
+            const long long bits = __double_as_longlong(s);
+            const bool ok = bits > 0 && bits <= 0x7ff0000000000000LL;  // s > 0.0
+            const double r = ok ? rsqrt(s) : 1.0 / s;
+            if (!ok && failed < 0) failed = t;  // stored without its root, as dpotrf leaves it
+            if (t > 0) bar_sync(2, ALL);        // column t is final below the diagonal
+            const double a = lane == t ? s : lane > t && lane < nb ? D[lane][t] : 0.0;
+            const double l = a * r;
+            sh.col[t & 1][lane] = l;
+            if (lane >= t) D[lane][t] = lane == t && !ok ? s : l;
+            if (lane == t) sh.rp[t] = r;
             __syncwarp();
             if (t + 1 < nb) bar_arrive(1, ALL);
             if ((t & (DFC - 1)) == DFC - 1 || t == nb - 1) bar_arrive(3 + t / DFC, 64);
-            if (lane > t) dg = fma(-l, l, dg);
+            dg = fma(-l, l, dg);  // (of use for lanes > t)
         }
         if (lane == 0 && failed >= 0) atomicCAS(flags, 0, k0 + failed + 1);
-    } else if (warp == 4) {
-        for (int c0 = 0; c0 < nb; c0 += DFC) {
-            bar_sync(3 + c0 / DFC, 64);
-            const int c1 = min(nb, c0 + DFC);
-            for (int c = c0; c < c1; ++c)
-                if (lane >= c && lane < nb) M[(size_t)(k0 + c) * ld + k0 + lane] = D[lane][c];
-            if (lane >= c0 && lane < c1) Dinv[lane * (NB + 1)] = rp[lane];
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence();
-                st_release_u32(ready, c1 == nb ? NB : c1);
-            }
-        }
-        if (lane >= nb) Dinv[lane * (NB + 1)] = 0.0;
-    } else {
+    } else if (warp != 4) {
         const int u = warp < 4 ? warp - 1 : warp - 2;  // 0 ... 5
         double v[3];
         int er[3], ec[3];
@@ -460,13 +432,13 @@ __device__ void factor_stream(double (*D)[NB + 1], double *rp, int nb, int k0, i
         }
         for (int t = 0; t + 1 < nb; ++t) {
             bar_sync(1, ALL);
-            const double *l = fs.col[t & 1];
+            const double *l = sh.col[t & 1];
             bool told = false;
 #pragma unroll
             for (int x = 0; x < 3; ++x) {
                 const bool live = ec[x] > t;
                 if (!__any_sync(0xffffffffu, live)) continue;
-                // the next column lies in this warp's first live groups
+                // the next column lies in the first live groups
                 if (!told && !__any_sync(0xffffffffu, ec[x] == t + 1)) {
                     bar_arrive(2, ALL);
                     told = true;
@@ -480,26 +452,142 @@ __device__ void factor_stream(double (*D)[NB + 1], double *rp, int nb, int k0, i
             }
         }
     }
-    __syncthreads();
+    bar_sync(BAR_ALL, 256);
 }
 
 // ready: columns published of diag[j] at ready[j] (j < nbc), of tile L(i, j)
 // at ready[nbc + j * nbr + i]. b: the right-hand side (row n), or NULL when
 // it is in row n of M already.
-__global__ void __launch_bounds__(256, 1) chol_df_kernel(double *__restrict__ M, int n, int ld, int nrows,
-                                                      const double *__restrict__ b, int *__restrict__ flags,
-                                                      double *__restrict__ Dinv, unsigned *__restrict__ ready,
-                                                      int *__restrict__ abort) {
-    __shared__ double T[NB][NB + 1], Li[NB][NB + 1], Lj[NB][NB + 1];
-    __shared__ double rp[NB];
-    __shared__ FactorShared fs;
-    __shared__ int got[2];
-    const int tid = threadIdx.x;
+__global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restrict__ M, int n, int ld, int nrows,
+                                                                const double *__restrict__ b, int *__restrict__ flags,
+                                                                double *__restrict__ Dinv,
+                                                                unsigned *__restrict__ ready, int *__restrict__ abort) {
+    extern __shared__ __align__(16) unsigned char df_smem[];
+    DfShared &sh = *(DfShared *)df_smem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nbc = (n + NB - 1) / NB, nbr = (nrows + NB - 1) / NB;
-    int t = 0, w = 0;
-    // the pivot status; every block that can fail comes after tile 0 (this
-    // CTA's) by the chain of published tiles
-    if (blockIdx.x == 0 && tid == 0) *flags = 0;
+    if (tid == 0) {
+        for (int q = 0; q < DFR; ++q) {
+            mbar_init(&sh.full[q], 32);
+            mbar_init(&sh.empty[q], 8);
+        }
+        for (int q = 0; q < DFQ; ++q) mbar_init(&sh.pub[q], 8);
+        mbar_init(&sh.done, 1);
+        sh.stop = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+        // the pivot status; every block that can fail comes after tile 0 (CTA
+        // 0's) by the chain of published tiles
+        if (blockIdx.x == 0) *flags = 0;
+    }
+    __syncthreads();
+    int step = 0;  // ring steps so far, the same in the loading and computing warps
+
+    if (warp == 8) {
+        // the loader: per step, polls the two column counts (lanes 0 and 1),
+        // then brings the columns into a ring slot
+        int t = 0;
+        for (int j = 0; j < nbc; ++j) {
+            for (int i = j; i < nbr; ++i, ++t) {
+                if (t % (int)gridDim.x != (int)blockIdx.x) continue;
+                const int r0 = NB * i, c0 = NB * j;
+                const int nr = min(NB, nrows - r0), nc = min(NB, n - c0);
+                for (int k = 0; k <= j; ++k) {
+                    if (k == j && i == j) break;
+                    const int kc = NB * k;
+                    const unsigned *p = k == j ? ready + j : ready + nbc + (size_t)k * nbr + (lane == 1 ? j : i);
+                    int have = 0;
+                    for (int q = 0; q < DFQ; ++q, ++step) {
+                        const int s = step % DFR, done = DFC * q;
+                        bool ok = step < DFR || mbar_wait(smem_u32(&sh.empty[s]), (unsigned)(step / DFR - 1) & 1u);
+                        if (have <= done) {
+                            for (long long it = 0; ok; ++it) {
+                                const int v = lane < 2 ? (int)ld_acquire_u32(p) : NB;
+                                have = __reduce_min_sync(0xffffffffu, v);
+                                if (have > done) break;
+                                if (it >= DF_WAIT_LIMIT || ld_relaxed_u32((const unsigned *)abort)) ok = false;
+                                ok = __all_sync(0xffffffffu, ok);
+                                if (it > 64) __nanosleep(32);
+                            }
+                            __syncwarp();
+                        }
+                        DfSlot &sl = sh.slot[s];
+                        if (lane == 0) sh.bad[s] = !ok;
+                        if (ok) {
+                            double va[DFC], vb[DFC], vr = 0.0;
+#pragma unroll
+                            for (int h = 0; h < DFC; ++h) {
+                                const double *col = M + (size_t)(kc + done + h) * ld;
+                                if (k == j) {
+                                    va[h] = __ldcg(col + c0 + lane);
+                                } else {
+                                    va[h] = lane < nr ? __ldcg(col + r0 + lane) : 0.0;
+                                    vb[h] = i != j && lane < nc ? __ldcg(col + c0 + lane) : 0.0;
+                                }
+                            }
+                            if (k == j && lane < DFC)
+                                vr = __ldcg(Dinv + (size_t)j * NB * NB + (done + lane) * (NB + 1));
+#pragma unroll
+                            for (int h = 0; h < DFC; ++h) {
+                                sl.a[lane][h] = va[h];
+                                if (k < j && i != j) sl.b[lane][h] = vb[h];
+                            }
+                            if (k == j && lane < DFC) sl.rp[lane] = vr;
+                        }
+                        mbar_arrive(&sh.full[s]);
+                        if (!ok) {
+                            if (lane == 0) {
+                                *(volatile int *)abort = 1;
+                                atomicExch(flags, -1);
+                                atomicExch(flags + 1, CHOL_WAIT_CODE | (int)blockIdx.x);
+                            }
+                            return;
+                        }
+                    }
+                }
+            }
+        }
+        return;
+    }
+
+    if (warp == 9) {
+        // the publisher: stores finished columns and releases their count
+        int t = 0, tasks = 0, below = 0;  // tiles so far, and those below the diagonal
+        for (int j = 0; j < nbc; ++j) {
+            for (int i = j; i < nbr; ++i, ++t) {
+                if (t % (int)gridDim.x != (int)blockIdx.x) continue;
+                const int r0 = NB * i, c0 = NB * j;
+                const int nr = min(NB, nrows - r0), nc = min(NB, n - c0);
+                for (int q = 0; DFC * q < nc; ++q) {
+                    const int q1 = min(nc, DFC * q + DFC);
+                    bool ok = true;
+                    if (i == j) {
+                        // (a diagonal tile gives up before it is factored)
+                        if (q == 0) ok = mbar_wait(smem_u32(&sh.pub[0]), (unsigned)tasks & 1u) && !sh.stop;
+                        if (ok) bar_sync(3 + q, 64);
+                    } else {
+                        ok = mbar_wait(smem_u32(&sh.pub[q]), (unsigned)(q == 0 ? tasks : below) & 1u) && !sh.stop;
+                    }
+                    if (!__all_sync(0xffffffffu, ok)) return;
+                    for (int c = DFC * q; c < q1; ++c)
+                        if (lane < nr && (i != j || (lane >= c && lane < nc)))
+                            M[(size_t)(c0 + c) * ld + r0 + lane] = sh.T[lane][c];
+                    if (i == j && lane >= DFC * q && lane < q1)
+                        Dinv[(size_t)j * NB * NB + lane * (NB + 1)] = sh.rp[lane];
+                    __syncwarp();
+                    if (lane == 0) {
+                        __threadfence();
+                        st_release_u32(i == j ? ready + j : ready + nbc + (size_t)j * nbr + i, q1 == nc ? NB : q1);
+                    }
+                }
+                if (lane == 0) mbar_arrive(&sh.done);
+                ++tasks;
+                below += i != j;
+            }
+        }
+        return;
+    }
+
+    int t = 0, tasks = 0, told = 0;  // told: publication steps of the current tile
     // this thread's elements of a diagonal tile's lower triangle
     int dr[3], dc[3];
 #pragma unroll
@@ -511,137 +599,144 @@ __global__ void __launch_bounds__(256, 1) chol_df_kernel(double *__restrict__ M,
         dr[x] = r;
         dc[x] = e - r * (r + 1) / 2;
     }
-    for (int j = 0; j < nbc; ++j) {
-        for (int i = j; i < nbr; ++i, ++t) {
+    const bool third = tid < NB * (NB + 1) / 2 - 512;
+    const int r = tid % NB, u = tid / NB;
+    bool good = true;
+    // the slot of the next step, or false when the loader gave up
+    auto take = [&](int s) {
+        return mbar_wait(smem_u32(&sh.full[s]), (unsigned)(step / DFR) & 1u) && !sh.bad[s];
+    };
+    auto give = [&](int s) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.empty[s]);
+        ++step;
+    };
+    for (int j = 0; j < nbc && good; ++j) {
+        for (int i = j; i < nbr && good; ++i, ++t) {
             if (t % (int)gridDim.x != (int)blockIdx.x) continue;
             const int r0 = NB * i, c0 = NB * j;
             const int nr = min(NB, nrows - r0), nc = min(NB, n - c0);
+            // T is free when the publisher has stored the previous tile
+            if (tasks > 0) good = mbar_wait(smem_u32(&sh.done), (unsigned)(tasks - 1) & 1u);
+            ++tasks;
+            told = 0;
             for (int e = tid; e < NB * NB; e += 256) {
-                const int r = e % NB, c = e / NB;
+                const int rr = e % NB, c = e / NB;
                 double v = 0.0;
-                if (r < nr && c < nc && (i != j || c <= r))
-                    v = b && r0 + r == n ? b[c0 + c] : __ldcg(M + (size_t)(c0 + c) * ld + r0 + r);
-                T[r][c] = v;
+                if (rr < nr && c < nc && (i != j || c <= rr))
+                    v = b && r0 + rr == n ? b[c0 + c] : __ldcg(M + (size_t)(c0 + c) * ld + r0 + rr);
+                sh.T[rr][c] = v;
             }
-            for (int k = 0; k < j; ++k) {
-                const int kc = NB * k;
-                const unsigned *pi = ready + nbc + (size_t)k * nbr + i, *pj = ready + nbc + (size_t)k * nbr + j;
+            bar_sync(BAR_ALL, 256);
+            for (int k = 0; k < j && good; ++k) {
                 double acc[4] = {0.0, 0.0, 0.0, 0.0};
-                for (int done = 0; done < NB;) {
-                    const int have = df_wait(pi, pj, done, abort, got + (w++ & 1));
-                    if (have == 0) goto fail;
-                    for (int e = tid; e < NB * (have - done); e += 256) {
-                        const int r = e % NB, kk = done + e / NB;
-                        Li[r][kk] = r < nr ? __ldcg(M + (size_t)(kc + kk) * ld + r0 + r) : 0.0;
-                        if (i != j) Lj[r][kk] = r < nc ? __ldcg(M + (size_t)(kc + kk) * ld + c0 + r) : 0.0;
-                    }
-                    __syncthreads();
+                for (int q = 0; q < DFQ; ++q) {
+                    const int s = step % DFR;
+                    good = take(s);
+                    if (!good) break;
+                    const DfSlot &sl = sh.slot[s];
                     if (i != j) {
-                        const int r = tid % NB, u = tid / NB;
-                        for (int kk = done; kk < have; kk += DFC)
 #pragma unroll
-                            for (int h = 0; h < DFC; ++h)
+                        for (int h = 0; h < DFC; ++h)
 #pragma unroll
-                                for (int x = 0; x < 4; ++x)
-                                    acc[x] = fma(Li[r][kk + h], Lj[u + 8 * x][kk + h], acc[x]);
+                            for (int x = 0; x < 4; ++x) acc[x] = fma(sl.a[r][h], sl.b[u + 8 * x][h], acc[x]);
                     } else {
-                        for (int kk = done; kk < have; kk += DFC)
 #pragma unroll
-                            for (int h = 0; h < DFC; ++h)
+                        for (int h = 0; h < DFC; ++h)
 #pragma unroll
-                                for (int x = 0; x < 3; ++x)
-                                    if (x < 2 || tid < NB * (NB + 1) / 2 - 512)
-                                        acc[x] = fma(Li[dr[x]][kk + h], Li[dc[x]][kk + h], acc[x]);
+                            for (int x = 0; x < 3; ++x)
+                                if (x < 2 || third) acc[x] = fma(sl.a[dr[x]][h], sl.a[dc[x]][h], acc[x]);
                     }
-                    done = have;
+                    give(s);
                 }
+                if (!good) break;
+                // (each element is its thread's own until the barrier below)
                 if (i != j) {
-                    const int r = tid % NB, u = tid / NB;
 #pragma unroll
                     for (int x = 0; x < 4; ++x)
-                        if (r < nr && u + 8 * x < nc) T[r][u + 8 * x] = T[r][u + 8 * x] - acc[x];
+                        if (r < nr && u + 8 * x < nc) sh.T[r][u + 8 * x] = sh.T[r][u + 8 * x] - acc[x];
                 } else {
 #pragma unroll
                     for (int x = 0; x < 3; ++x)
-                        if ((x < 2 || tid < NB * (NB + 1) / 2 - 512) && dr[x] < nr && dc[x] < nc)
-                            T[dr[x]][dc[x]] = T[dr[x]][dc[x]] - acc[x];
+                        if ((x < 2 || third) && dr[x] < nr && dc[x] < nc)
+                            sh.T[dr[x]][dc[x]] = sh.T[dr[x]][dc[x]] - acc[x];
                 }
-                __syncthreads();
             }
+            // every thread has seen the same slots, so `good` is the CTA's
+            if (!good) break;
+            bar_sync(BAR_ALL, 256);
             if (i == j) {
-                // row nc of this tile (the right-hand side) waits in Li
+                if (lane == 0) mbar_arrive(&sh.pub[0]);  // the publisher may join the factor
+                // row nc of this tile is the right-hand side
                 for (int e = tid; e < NB * NB; e += 256) {
-                    const int r = e % NB, c = e / NB;
-                    if (r == nc && r < nr && c < nc) Li[0][c] = T[r][c];
-                    if (r >= nc || c > r) T[r][c] = 0.0;
+                    const int rr = e % NB, c = e / NB;
+                    if (rr == nc && rr < nr && c < nc) sh.rhs[c] = sh.T[rr][c];
+                    if (rr >= nc || c > rr) sh.T[rr][c] = 0.0;
+                    sh.Di[rr][c] = 0.0;
                 }
-                __syncthreads();
-                factor_stream(T, rp, nc, c0, flags, fs, M, ld, Dinv + (size_t)j * NB * NB, ready + j);
-                for (int e = tid; e < NB * NB; e += 256) Lj[e / NB][e % NB] = 0.0;
-                __syncthreads();
+                bar_sync(BAR_ALL, 256);
+                factor_stream(sh, nc, c0, flags);
                 // the right-hand-side row, by the panel solves' substitution:
                 // warp 7 (whose columns of the inverse are the shortest) with
                 // lane = column
-                if (nr > nc && tid >= 224) {
-                    const int c = tid - 224;
-                    double v = c < nc ? Li[0][c] : 0.0;
+                if (nr > nc && warp == 7) {
+                    double v = lane < nc ? sh.rhs[lane] : 0.0;
                     for (int q = 0; q < nc; ++q) {
-                        if (c == q) v = v * rp[q];
+                        if (lane == q) v = v * sh.rp[q];
                         const double x = __shfl_sync(0xffffffffu, v, q);
-                        if (c > q && c < nc) v = fma(-x, T[c][q], v);
+                        if (lane > q && lane < nc) v = fma(-x, sh.T[lane][q], v);
                     }
-                    if (c < nc) M[(size_t)(c0 + c) * ld + r0 + nc] = v;
+                    if (lane < nc) M[(size_t)(c0 + lane) * ld + r0 + nc] = v;
                 }
                 // the inverse (for the backward sweep after this launch)
-                invert_columns(T, Lj, rp, nc);
-                __syncthreads();
-                for (int e = tid; e < NB * NB; e += 256) Dinv[(size_t)j * NB * NB + e] = Lj[e / NB][e % NB];
+                invert_columns(sh.T, sh.Di, sh.rp, nc);
+                bar_sync(BAR_ALL, 256);
+                for (int e = tid; e < NB * NB; e += 256) Dinv[(size_t)j * NB * NB + e] = sh.Di[e / NB][e % NB];
             } else {
-                // the panel solve, eight columns at a time: within them by the
-                // 32 x 8 threads (row, column), then the later columns
-                // (nc == NB: a tile below a diagonal block has whole columns)
-                const int r = tid % NB, u = tid / NB;
-                for (int done = 0; done < NB;) {
-                    const int have = df_wait(ready + j, ready + j, done, abort, got + (w++ & 1));
-                    if (have == 0) goto fail;
-                    for (int e = tid; e < NB * (have - done); e += 256) {
-                        const int rr = e % NB, c = done + e / NB;
-                        Li[rr][c] = c <= rr ? __ldcg(M + (size_t)(c0 + c) * ld + c0 + rr) : 0.0;
-                    }
-                    if (tid >= done && tid < have) rp[tid] = __ldcg(Dinv + (size_t)j * NB * NB + tid * (NB + 1));
-                    __syncthreads();
-                    for (; done < have; done += DFC) {
-                        double v = T[r][done + u];
+                // the panel solve, DFC columns at a time: within them by
+                // warps 0 to DFC - 1 (one column each, lane = row), then the
+                // later columns (a tile below a diagonal block has whole
+                // columns, nc == NB). Column c is updated by warps c mod 8 and
+                // (c + 4) mod 8 in turn; BAR_ALL is between them.
+                for (int q = 0; q < DFQ; ++q) {
+                    const int s = step % DFR, done = DFC * q;
+                    good = take(s);
+                    if (!good) break;
+                    const DfSlot &sl = sh.slot[s];
+                    if (u < DFC) {
+                        double v = sh.T[r][done + u];
 #pragma unroll
-                        for (int q = 0; q < DFC; ++q) {
-                            if (u == q) {
-                                v = v * rp[done + q];
-                                T[r][done + q] = v;
+                        for (int h = 0; h < DFC; ++h) {
+                            if (u == h) {
+                                v = v * sl.rp[h];
+                                sh.T[r][done + h] = v;
                             }
-                            __syncthreads();
-                            if (u > q) v = fma(-T[r][done + q], Li[done + u][done + q], v);
+                            if (h < DFC - 1) {
+                                bar_sync(BAR_STEP, 32 * DFC);
+                                if (u > h) v = fma(-sh.T[r][done + h], sl.a[done + u][h], v);
+                            }
                         }
-                        if (r < nr) M[(size_t)(c0 + done + u) * ld + r0 + r] = v;
-                        df_publish(ready + nbc + (size_t)j * nbr + i, done + DFC);
-                        for (int c = done + DFC + u; c < NB; c += 8) {
-                            double z = T[r][c];
-#pragma unroll
-                            for (int q = 0; q < DFC; ++q) z = fma(-T[r][done + q], Li[c][done + q], z);
-                            T[r][c] = z;
-                        }
-                        __syncthreads();
                     }
+                    bar_sync(BAR_ALL, 256);
+                    if (lane == 0) mbar_arrive(&sh.pub[q]);
+                    told = q + 1;
+                    for (int c = done + DFC + u; c < NB; c += 8) {
+                        double z = sh.T[r][c];
+#pragma unroll
+                        for (int h = 0; h < DFC; ++h) z = fma(-sh.T[r][done + h], sl.a[c][h], z);
+                        sh.T[r][c] = z;
+                    }
+                    give(s);
                 }
             }
-            __syncthreads();
         }
     }
-    return;
-fail:
-    if (tid == 0) {
-        *(volatile int *)abort = 1;
-        atomicExch(flags, -1);
-        atomicExch(flags + 1, CHOL_WAIT_CODE | (int)blockIdx.x);
+    if (!good) {
+        // tell the publisher to stop
+        sh.stop = 1;
+        __syncwarp();
+        if (lane == 0)
+            for (int q = told; q < DFQ; ++q) mbar_arrive(&sh.pub[q]);
     }
 }
 
@@ -662,7 +757,10 @@ int df_capacity() {
         int coop = 0, per_sm = 0, sms = 0, cap = 0;
         if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chol_df_kernel, 256, 0) != cudaSuccess)
+            cudaFuncSetAttribute(chol_df_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(DfShared)) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chol_df_kernel, DF_THREADS, sizeof(DfShared)) !=
+                cudaSuccess)
             cudaGetLastError();
         else if (coop && per_sm > 0)
             cap = sms;
@@ -724,8 +822,8 @@ __global__ void __launch_bounds__(256) chol_backsolve_coop_kernel(double *__rest
     }
 }
 
-// The same sweep in one thread-block cluster of ceil(n / 256) CTAs (orders up
-// to 2048), block b of 32 rows on CTA b mod g with its z in shared memory. Per
+// The same sweep in one thread-block cluster of g <= 8 CTAs (orders up to
+// 2048), block b of 32 rows on CTA b mod g with its z in shared memory. Per
 // block from the bottom its owner forms x_b and stores it into every CTA's
 // shared memory; a split cluster barrier hands it out. The owner of block
 // b - 1 applies x_b to it at once and goes on to x_(b-1); the other blocks
@@ -901,7 +999,8 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
         const double *b = has_b ? d_b : nullptr;
         void *args[] = {&d_M, &n, &ld, (void *)&nrows, &b, &flags, &Dinv, &ready, &abort};
         if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(256), args, 0, st);
+            e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(DF_THREADS), args,
+                                            sizeof(DfShared), st);
         if (e != cudaSuccess) {
             irwls_set_error(-2, "CUDA error in chol_df (cooperative): %s", cudaGetErrorString(e));
             return -2;
@@ -959,8 +1058,10 @@ int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv
                            cudaStream_t st) {
     {
         if (n <= 8 * SWB * NB && sweep_cluster_ok()) {
+            // two blocks a CTA, up to eight CTAs: one block's update holds the
+            // FP64 units for 0.45 us, the chain of a block takes about 1.3
             cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((n + SWB * NB - 1) / (SWB * NB));
+            cfg.gridDim = dim3(std::min(8, (n + 2 * NB - 1) / (2 * NB)));
             cfg.blockDim = dim3(256);
             cfg.stream = st;
             cudaLaunchAttribute at[1];
