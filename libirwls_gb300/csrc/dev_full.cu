@@ -30,6 +30,7 @@ extern "C" void irwls_ws_mixed_counts(long long *solves, long long *fallbacks, i
 namespace {
 
 constexpr int CT = 1024;  // threads of the single-CTA bookkeeping kernels
+constexpr int SUB_K = 4096;  // largest working set whose kernel matrix is kept
 
 // Exclusive scan of per-thread counts in shared memory; returns the total.
 __device__ int block_exclusive_scan(int *s, int v) {
@@ -52,18 +53,30 @@ __device__ int block_exclusive_scan(int *s, int v) {
 
 // Ordered compaction: writes, in ascending i, every i < n with pred(i) to
 // out (through emit(pos, i)); returns the count (same in every thread).
+// Rounds of one i per thread, placed by warp ballots and a scan of the warps'
+// counts (two barriers a round; the 20 barriers of a scan over all threads
+// took most of a bookkeeping kernel's time).
 template <class Pred, class Emit>
-__device__ int block_compact(int n, Pred pred, Emit emit, int *s_scan) {
-    const int ch = (n + CT - 1) / CT;
-    const int b = threadIdx.x * ch, e = min(n, b + ch);
-    int c = 0;
-    for (int i = b; i < e; ++i) c += pred(i) ? 1 : 0;
-    const int total = block_exclusive_scan(s_scan, c);
-    int off = s_scan[threadIdx.x];
-    for (int i = b; i < e; ++i)
-        if (pred(i)) emit(off++, i);
-    __syncthreads();
-    return total;
+__device__ int block_compact(int n, Pred pred, Emit emit, int *s_cnt) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int base = 0;
+    for (int i0 = 0; i0 < n; i0 += blockDim.x) {
+        const int i = i0 + threadIdx.x;
+        const bool on = i < n && pred(i);
+        const unsigned bal = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) s_cnt[warp] = __popc(bal);
+        __syncthreads();
+        int v = lane < nw ? s_cnt[lane] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, v, o);
+            v += lane >= o ? x : 0;
+        }
+        const int before = __shfl_sync(0xffffffffu, v, warp > 0 ? warp - 1 : 0);
+        if (on) emit(base + (warp > 0 ? before : 0) + __popc(bal & ((1u << lane) - 1u)), i);
+        base += __shfl_sync(0xffffffffu, v, 31);
+        __syncthreads();
+    }
+    return base;
 }
 
 // Deterministic CTA-wide sum of f(i), i < n: each thread adds its contiguous
@@ -91,33 +104,63 @@ __device__ double block_sum_ordered(int n, F f, double *red) {
     return r;
 }
 
-template <class F, class Op>
-__device__ double block_reduce(int n, F f, Op op, double init, double *red) {
-    double v = init;
-    for (int i = threadIdx.x; i < n; i += CT) v = op(v, f(i));
-    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// --- inner IRWLS -----------------------------------------------------------
+//
+// The bookkeeping kernels run on one CTA of NT = 512 threads for working sets
+// below 512 (one round per pass), else 1024. What costs in them is FP64
+// instructions, 65 cycles each per warp and SM quarter: the sums go through
+// shared memory to four warps, and extrema compare bit patterns.
+
+// Sums of v1 and v2 over the CTA's threads, in every thread: thread values in
+// shared memory, four warps each add every fourth group of 32 and reduce by a
+// butterfly, the four partial sums in order.
+template <int NT>
+__device__ void block_sum2(double &v1, double &v2, double (*buf)[NT], double (*part)[4]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    buf[0][threadIdx.x] = v1;
+    buf[1][threadIdx.x] = v2;
     __syncthreads();
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        double t = red[lane];
-        for (int o = 16; o > 0; o >>= 1) t = op(t, __shfl_xor_sync(0xffffffffu, t, o));
-        if (lane == 0) red[32] = t;
+    if (warp < 4) {
+        double a = 0.0, b = 0.0;
+#pragma unroll
+        for (int g = 0; g < NT / 128; ++g) {
+            a = __dadd_rn(a, buf[0][128 * g + 32 * warp + lane]);
+            b = __dadd_rn(b, buf[1][128 * g + 32 * warp + lane]);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            a = __dadd_rn(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = __dadd_rn(b, __shfl_xor_sync(0xffffffffu, b, o));
+        }
+        if (lane < 2) part[lane][warp] = lane == 0 ? a : b;
     }
     __syncthreads();
-    const double r = red[32];
+    if (threadIdx.x < 2)
+        part[threadIdx.x][0] = __dadd_rn(__dadd_rn(part[threadIdx.x][0], part[threadIdx.x][1]),
+                                         __dadd_rn(part[threadIdx.x][2], part[threadIdx.x][3]));
     __syncthreads();
-    return r;
+    v1 = part[0][0];
+    v2 = part[1][0];
 }
 
-// --- inner IRWLS -----------------------------------------------------------
+// Order-preserving map of a double to an integer, and back (NaN maps as 0.0,
+// which no "greater" or "less" test against a NaN would have picked either).
+__device__ __forceinline__ long long order_key(double v) {
+    const long long b = __double_as_longlong(v);
+    if ((b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL) return 0;
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double key_value(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
 
 // a_i and groups at entry (src/full-train.c:131-155).
-__global__ void __launch_bounds__(CT) sub_init_kernel(irwls_sub_ws ws, const double *__restrict__ yg, double C) {
-    __shared__ int s_scan[CT];
+template <int NT>
+__global__ void __launch_bounds__(NT) sub_init_kernel(irwls_sub_ws ws, const double *__restrict__ yg, double C) {
+    __shared__ int s_scan[32];
+    chain_wait();
+    chain_open();
     const int w = ws.w;
-    for (int i = threadIdx.x; i < w; i += CT) {
+    for (int i = threadIdx.x; i < w; i += NT) {
         const double yi = yg[ws.map[i]];
         ws.y[i] = yi;
         const double ei = ws.e[i];
@@ -125,7 +168,7 @@ __global__ void __launch_bounds__(CT) sub_init_kernel(irwls_sub_ws ws, const dou
         ws.a[i] = ai;
         ws.grp[i] = (ai == 0) ? 2 : ((ws.beta[i] == __dmul_rn(yi, C)) ? 3 : 1);
     }
-    for (int i = threadIdx.x; i <= w; i += CT) ws.G13[i] = 0.0;
+    for (int i = threadIdx.x; i <= w; i += NT) ws.G13[i] = 0.0;
     __syncthreads();
     const int n1 = block_compact(w, [&](int i) { return ws.grp[i] == 1; },
                                  [&](int p, int i) { ws.S1[p] = i; ws.gl1[p] = ws.map[i]; }, s_scan);
@@ -186,30 +229,134 @@ __global__ void build_border_kernel(irwls_sub_ws ws, int n1) {
     }
 }
 
+// The working set's kernel matrix K (row-major, w x w), formed once per run of
+// the inner loop and read by every iteration's H, G13 and error update, which
+// had each formed the values they needed again (at 500 rows and 20 features
+// 81 us per inner iteration, against 31 us once and 5 us to read them). Row i,
+// columns j <= i, and their mirror images: both orders of a pair give the same
+// bits (the raw form's squares; the norm form's products of shared entries in
+// index order).
+__global__ void __launch_bounds__(64) sub_kmat_kernel(irwls_sub_ws ws, KView X) {
+    chain_wait();
+    chain_open();
+    extern __shared__ double sA[];
+    const int i = blockIdx.y, w = ws.w;
+    if ((int)blockIdx.x * 64 > i) return;
+    const int gi = ws.map[i];
+    for (int t = threadIdx.x; t < X.ld; t += 64) sA[t] = X.X[(size_t)gi * X.ld + t];
+    __syncthreads();
+    const int j = blockIdx.x * 64 + threadIdx.x;
+    if (j > i) return;
+    const double kv = kentry(X, sA, X.q[gi], ws.map[j]);
+    ws.K[(size_t)i * w + j] = kv;
+    ws.K[(size_t)j * w + i] = kv;
+}
+
+// One iteration's system from K (src/full-train.c:165-186, :327-344): CTA
+// j < n1 writes column j of H (rows j .. n1 - 1, the border row) and
+// rhs_j = 1 - G13_j - GIN_j with G13_j = sum over S3 of C k y_j y_o (use13),
+// CTA n1 the border's corner.
+__global__ void __launch_bounds__(128) sub_system_kernel(irwls_sub_ws ws, double C, int n1, int n3, int use13) {
+    chain_wait();
+    chain_open();
+    __shared__ double red[4];
+    const int j = blockIdx.x, w = ws.w;
+    if (j == n1) {
+        if (threadIdx.x == 0) {
+            ws.H[(size_t)n1 * ws.ldH + n1] = 0.0;
+            ws.rhs[n1] = __dsub_rn(-ws.G13[n1], ws.GIN[w]);
+        }
+        return;
+    }
+    const int lj = ws.S1[j];
+    const double yj = ws.y[lj];
+    const double *row = ws.K + (size_t)lj * w;
+    double *col = ws.H + (size_t)j * ws.ldH;
+    for (int i = j + threadIdx.x; i < n1; i += 128) {
+        const int li = ws.S1[i];
+        double h = __dmul_rn(__dmul_rn(row[li], ws.y[li]), yj);
+        if (i == j) h = __dadd_rn(h, __ddiv_rn(1.0, ws.a[lj]));
+        col[i] = h;
+    }
+    double g = 0.0;
+    if (use13) {
+        for (int o = threadIdx.x; o < n3; o += 128) {
+            const int lo = ws.S3[o];
+            g = __dadd_rn(g, __dmul_rn(__dmul_rn(__dmul_rn(C, row[lo]), yj), ws.y[lo]));
+        }
+        for (int o = 16; o > 0; o >>= 1) g = __dadd_rn(g, __shfl_xor_sync(0xffffffffu, g, o));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = g;
+        __syncthreads();
+        g = __dadd_rn(__dadd_rn(red[0], red[1]), __dadd_rn(red[2], red[3]));
+    }
+    if (threadIdx.x == 0) {
+        col[n1] = yj;
+        ws.rhs[j] = __dsub_rn(__dsub_rn(1.0, g), ws.GIN[lj]);
+    }
+}
+
+// e_i -= sum over the changed weights of k(i, j) (bnew_j - beta_j), then the
+// bias change, from K: a warp per row.
+__global__ void __launch_bounds__(128) sub_errors_kernel(irwls_sub_ws ws) {
+    chain_wait();
+    chain_open();
+    const int lane = threadIdx.x & 31, i = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (i >= ws.w) return;
+    const int nl = ws.cnt[0];
+    const double *row = ws.K + (size_t)i * ws.w;
+    double acc = 0.0;
+    for (int p = lane; p < nl; p += 32) acc = fma(ws.dlt[p], row[ws.lloc[p]], acc);
+    for (int o = 16; o > 0; o >>= 1) acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    if (lane == 0) ws.e[i] = __dsub_rn(__dsub_rn(ws.e[i], acc), ws.scal[0]);
+}
+
 // New weights, convergence sums and the list of changed weights
 // (src/full-train.c:205-230 and the skip test of :242).
-__global__ void __launch_bounds__(CT) sub_update_kernel(irwls_sub_ws ws, double C, int n1, int n3) {
-    __shared__ int s_scan[CT];
-    const int w = ws.w;
-    for (int i = threadIdx.x; i <= w; i += CT) ws.bnew[i] = 0.0;
+template <int NT>
+__global__ void __launch_bounds__(NT) sub_update_kernel(irwls_sub_ws ws, double C, int n1, int n3) {
+    chain_wait();
+    chain_open();
+    __shared__ double buf[2][NT], part[2][4];
+    __shared__ long long kmax[32], kmin[32];
+    __shared__ int s_scan[32];
+    const int w = ws.w, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i <= w; i += NT) ws.bnew[i] = 0.0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n1; i += CT) ws.bnew[ws.S1[i]] = __dmul_rn(ws.bsol[i], ws.y[ws.S1[i]]);
-    for (int i = threadIdx.x; i < n3; i += CT) ws.bnew[ws.S3[i]] = __dmul_rn(C, ws.y[ws.S3[i]]);
+    long long hi = 0, lo = 0;  // the keys of 0.0
+    for (int i = threadIdx.x; i < n1; i += NT) {
+        const int li = ws.S1[i];
+        const double b = ws.bsol[i];
+        const long long k = order_key(b);
+        hi = k > hi ? k : hi;
+        lo = k < lo ? k : lo;
+        ws.bnew[li] = __dmul_rn(b, ws.y[li]);
+    }
+    for (int i = threadIdx.x; i < n3; i += NT) ws.bnew[ws.S3[i]] = __dmul_rn(C, ws.y[ws.S3[i]]);
     if (threadIdx.x == 0) ws.bnew[w] = ws.bsol[n1];
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long h2 = __shfl_xor_sync(0xffffffffu, hi, o), l2 = __shfl_xor_sync(0xffffffffu, lo, o);
+        hi = h2 > hi ? h2 : hi;
+        lo = l2 < lo ? l2 : lo;
+    }
+    if (lane == 0) {
+        kmax[warp] = hi;
+        kmin[warp] = lo;
+    }
     __syncthreads();
-    __shared__ double red[33];
-    const double bmax = block_reduce(n1, [&](int i) { return ws.bsol[i]; },
-                                     [](double a, double b) { return b > a ? b : a; }, 0.0, red);
-    const double bmin = block_reduce(n1, [&](int i) { return ws.bsol[i]; },
-                                     [](double a, double b) { return b < a ? b : a; }, 0.0, red);
-    const double dW = block_sum_ordered(w + 1, [&](int i) {
-        const double d = __dsub_rn(ws.bnew[i], ws.beta[i]);
-        return __dmul_rn(d, d);
-    }, red);
-    const double nW = block_sum_ordered(w + 1, [&](int i) { return __dmul_rn(ws.beta[i], ws.beta[i]); }, red);
+    double dW = 0.0, nW = 0.0;
+    for (int i = threadIdx.x; i <= w; i += NT) {
+        const double b = ws.beta[i], d = __dsub_rn(ws.bnew[i], b);
+        dW = fma(d, d, dW);
+        nW = fma(b, b, nW);
+    }
+    block_sum2<NT>(dW, nW, buf, part);
     if (threadIdx.x == 0) {
-        ws.stats->bmax = bmax;
-        ws.stats->bmin = bmin;
+        for (int k = 0; k < NT / 32; ++k) {
+            hi = kmax[k] > hi ? kmax[k] : hi;
+            lo = kmin[k] < lo ? kmin[k] : lo;
+        }
+        ws.stats->bmax = key_value(hi);
+        ws.stats->bmin = key_value(lo);
         ws.stats->dW = dW;
         ws.stats->nW = nW;
         ws.scal[0] = __dsub_rn(ws.bnew[w], ws.beta[w]);
@@ -217,6 +364,7 @@ __global__ void __launch_bounds__(CT) sub_update_kernel(irwls_sub_ws ws, double 
     const int nl = block_compact(w, [&](int j) { return ws.bnew[j] != ws.beta[j]; },
                                  [&](int p, int j) {
                                      ws.lst[p] = ws.map[j];
+                                     ws.lloc[p] = j;
                                      ws.dlt[p] = __dsub_rn(ws.bnew[j], ws.beta[j]);
                                  },
                                  s_scan);
@@ -224,10 +372,14 @@ __global__ void __launch_bounds__(CT) sub_update_kernel(irwls_sub_ws ws, double 
 }
 
 // a_i, groups, beta <- bnew, S1/S3 lists, G13[n1] (src/full-train.c:264-344).
-__global__ void __launch_bounds__(CT) sub_groups_kernel(irwls_sub_ws ws, double C) {
-    __shared__ int s_scan[CT];
+template <int NT>
+__global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double C) {
+    chain_wait();
+    chain_open();
+    __shared__ double buf[2][NT], part[2][4];
+    __shared__ int s_scan[32];
     const int w = ws.w;
-    for (int i = threadIdx.x; i < w; i += CT) {
+    for (int i = threadIdx.x; i < w; i += NT) {
         const double yi = ws.y[i], ei = ws.e[i];
         const double ey = __dmul_rn(ei, yi);
         double ai;
@@ -259,10 +411,10 @@ __global__ void __launch_bounds__(CT) sub_groups_kernel(irwls_sub_ws ws, double 
                                      ws.rhs[p] = C;
                                  },
                                  s_scan);
-    for (int i = threadIdx.x; i <= n1; i += CT) ws.G13[i] = 0.0;
-    __syncthreads();
-    __shared__ double red[33];
-    const double g13 = block_sum_ordered(n3, [&](int o) { return __dmul_rn(ws.rhs[o], ws.y[ws.S3[o]]); }, red);
+    for (int i = threadIdx.x; i <= n1; i += NT) ws.G13[i] = 0.0;
+    double g13 = 0.0, none = 0.0;
+    for (int o = threadIdx.x; o < n3; o += NT) g13 = __dadd_rn(g13, __dmul_rn(C, ws.y[ws.S3[o]]));
+    block_sum2<NT>(g13, none, buf, part);
     if (threadIdx.x == 0) {
         if (n3 > 0) ws.G13[n1] = g13;
         ws.stats->nS1 = n1;
@@ -744,9 +896,14 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
     double **dbl[] = {&ws->a, &ws->e, &ws->beta, &ws->bnew, &ws->bsol, &ws->bbest, &ws->G13, &ws->rhs, &ws->GIN,
                       &ws->y, &ws->dlt, &ws->scal};
     for (double **p : dbl) rc |= irwls_dev_malloc((void **)p, nd * sizeof(double));
-    int **ints[] = {&ws->grp, &ws->S1, &ws->S3, &ws->lst, &ws->gl1, &ws->gl3, &ws->cnt, &ws->mapbuf};
+    int **ints[] = {&ws->grp, &ws->S1, &ws->S3, &ws->lst, &ws->lloc, &ws->gl1, &ws->gl3, &ws->cnt,
+                    &ws->mapbuf};
     for (int **p : ints) rc |= irwls_dev_malloc((void **)p, nd * sizeof(int));
     rc |= irwls_dev_malloc((void **)&ws->H, nd * nd * sizeof(double));
+    // the kernel matrix of working sets up to SUB_K rows (134 MB at most)
+    // (the six first violators can exceed a working set below six)
+    const size_t nk = (size_t)cap + 6;
+    if (cap <= SUB_K) rc |= irwls_dev_malloc((void **)&ws->K, nk * nk * sizeof(double));
     rc |= irwls_dev_malloc((void **)&ws->stats, sizeof(irwls_sub_stats));
     rc |= irwls_dev_host_alloc((void **)&ws->h_stats, sizeof(irwls_sub_stats));
     ws->map = ws->mapbuf;
@@ -756,24 +913,41 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
 extern "C" void irwls_sub_release(irwls_sub_ws *ws) {
     irwls_dev_sync();
     void *ptrs[] = {ws->a, ws->e, ws->beta, ws->bnew, ws->bsol, ws->bbest, ws->G13, ws->rhs, ws->GIN, ws->y,
-                    ws->dlt, ws->scal, ws->grp, ws->S1, ws->S3, ws->lst, ws->gl1, ws->gl3, ws->cnt, ws->mapbuf,
-                    ws->H, ws->stats};
+                    ws->dlt, ws->scal, ws->grp, ws->S1, ws->S3, ws->lst, ws->lloc, ws->gl1, ws->gl3, ws->cnt,
+                    ws->mapbuf, ws->H, ws->K, ws->stats};
     for (void *p : ptrs) irwls_dev_free(p);
     irwls_dev_host_free(ws->h_stats);
     memset(ws, 0, sizeof *ws);
 }
 
 extern "C" int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C) {
-    sub_init_kernel<<<1, CT, 0, irwls_stream()>>>(*ws, X->y, C);
+    const int w = ws->w;
+    if (w < 512) launch_chained(sub_init_kernel<512>, dim3(1), dim3(512), 0, *ws, X->y, C);
+    else launch_chained(sub_init_kernel<CT>, dim3(1), dim3(CT), 0, *ws, X->y, C);
     IRWLS_LAUNCH_CHECK("sub_init");
+    ws->use13 = 0;
+    if (!ws->K || w <= 0) return 0;
+    // precision form on integer-valued data: from exact tensor-core dot
+    // products (FP64 exp), else the FP64 kernels
+    const int ex = irwls_tc_exact_block(ws->tcs, X, ws->map, w, ws->map, w, nullptr, nullptr, ws->K, w, 0);
+    if (ex < 0) return -2;
+    if (ex == 1) {
+        const size_t smem = (size_t)X->ld * sizeof(double);
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(sub_kmat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        launch_chained(sub_kmat_kernel, dim3(ceil_div(w, 64), w), dim3(64), smem, *ws, kview(X));
+        IRWLS_LAUNCH_CHECK("sub_kmat");
+    }
     return 0;
 }
 
 // G13 of the current S1/S3 lists (src/full-train.c:327-344). The reference
 // computes it at the end of an iteration for use in the next one; it is
-// issued here at the start of the next iteration, when n1/n3 are known.
+// issued here at the start of the next iteration, when n1/n3 are known (with
+// K, as a part of that iteration's system).
 extern "C" int irwls_sub_g13(irwls_sub_ws *ws, const irwls_dev_set *X, int n1, int n3) {
-    if (n3 <= 0 || n1 <= 0) return 0;
+    ws->use13 = n3 > 0 && n1 > 0;
+    if (!ws->use13 || ws->K) return 0;
     const int ex = irwls_tc_exact_rowsum(ws->tcs, X, ws->gl1, n1, ws->gl3, n3, nullptr, n3, ws->rhs, X->y, X->y, +1,
                                          nullptr, nullptr, ws->G13);
     if (ex != 1) return ex;
@@ -781,8 +955,8 @@ extern "C" int irwls_sub_g13(irwls_sub_ws *ws, const irwls_dev_set *X, int n1, i
                                    ws->G13);
 }
 
-extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, double C, int n1, int n3) {
-    const int n = n1 + 1;
+// The system of one iteration without K (working sets above SUB_K rows).
+static int sub_system_direct(irwls_sub_ws *ws, const irwls_dev_set *X, int n1) {
     KView kv = kview(X);
     if (n1 > 0) {
         // precision form on integer-valued data: the kernel block from exact
@@ -803,6 +977,17 @@ extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, doubl
     }
     build_border_kernel<<<ceil_div(n1 + 1, 256), 256, 0, irwls_stream()>>>(*ws, n1);
     IRWLS_LAUNCH_CHECK("build_border");
+    return 0;
+}
+
+extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, double C, int n1, int n3) {
+    const int n = n1 + 1, w = ws->w;
+    if (ws->K) {
+        launch_chained(sub_system_kernel, dim3(n1 + 1), dim3(128), 0, *ws, C, n1, n3, ws->use13);
+        IRWLS_LAUNCH_CHECK("sub_system");
+    } else if (sub_system_direct(ws, X, n1)) {
+        return -2;
+    }
     // precision form: FP32 factor + FP64 refinement in one cluster launch,
     // the FP64 factorization where that cannot run or does not converge
     int solve = 1;
@@ -813,18 +998,27 @@ extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, doubl
         g_ws_mixed_fallbacks += solve == 1 && n1 >= 1 && n1 <= irwls_ws_mixed_max();
     }
     if (solve == 1 && irwls_dev_chol_solve(ws->H, n, ws->ldH, ws->rhs, ws->bsol)) return -2;
-    sub_update_kernel<<<1, CT, 0, irwls_stream()>>>(*ws, C, n1, n3);
+    if (w < 512) launch_chained(sub_update_kernel<512>, dim3(1), dim3(512), 0, *ws, C, n1, n3);
+    else launch_chained(sub_update_kernel<CT>, dim3(1), dim3(CT), 0, *ws, C, n1, n3);
     IRWLS_LAUNCH_CHECK("sub_update");
     // e_i -= k(i, j) (bnew_j - beta_j) over changed j, then the bias change
-    // (exact tensor-core dot products in the precision form where the data
-    // allow them: at most w changed entries)
-    const int ex = irwls_tc_exact_rowsum(ws->tcs, X, ws->map, ws->w, ws->lst, 0, ws->cnt, ws->w, ws->dlt, nullptr,
-                                         nullptr, -1, ws->e, ws->scal, ws->e);
-    if (ex < 0) return -2;
-    if (ex == 1 && irwls_dev_kernel_rowsum_n(X, ws->map, ws->w, X, ws->lst, ws->cnt, ws->dlt, nullptr, nullptr, -1,
-                                             ws->e, ws->scal, ws->e))
-        return -2;
-    sub_groups_kernel<<<1, CT, 0, irwls_stream()>>>(*ws, C);
+    // (without K: exact tensor-core dot products in the precision form where
+    // the data allow them: at most w changed entries)
+    if (ws->K) {
+        if (w > 0) {
+            launch_chained(sub_errors_kernel, dim3(ceil_div(w, 4)), dim3(128), 0, *ws);
+            IRWLS_LAUNCH_CHECK("sub_errors");
+        }
+    } else {
+        const int ex = irwls_tc_exact_rowsum(ws->tcs, X, ws->map, w, ws->lst, 0, ws->cnt, w, ws->dlt, nullptr, nullptr,
+                                             -1, ws->e, ws->scal, ws->e);
+        if (ex < 0) return -2;
+        if (ex == 1 && irwls_dev_kernel_rowsum_n(X, ws->map, w, X, ws->lst, ws->cnt, ws->dlt, nullptr, nullptr, -1,
+                                                 ws->e, ws->scal, ws->e))
+            return -2;
+    }
+    if (w < 512) launch_chained(sub_groups_kernel<512>, dim3(1), dim3(512), 0, *ws, C);
+    else launch_chained(sub_groups_kernel<CT>, dim3(1), dim3(CT), 0, *ws, C);
     IRWLS_LAUNCH_CHECK("sub_groups");
     return 0;
 }
@@ -873,8 +1067,9 @@ extern "C" int irwls_full_norms(const double *d_beta, const double *d_bnew, int 
 
 extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, const double *d_y, int l, double C,
                                    int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *d_counts) {
-    if (l < 4 * CB) {
-        // small sets: one CTA is faster than four launches
+    if (l <= CT) {
+        // one round of one CTA is faster than four launches (at 4000 rows it
+        // took 94 us: every row's FP64 tests four times on one SM)
         classify_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_e, d_y, l, C, d_SW, d_SC, d_SIN, d_counts);
         IRWLS_LAUNCH_CHECK("classify");
         return 0;

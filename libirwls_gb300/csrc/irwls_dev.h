@@ -144,7 +144,9 @@ typedef struct irwls_sub_ws {
     int cap;
     int *map;             /* device, w entries (points at mapbuf or a caller list) */
     double *a, *e, *beta, *bnew, *bsol, *bbest, *G13, *rhs, *GIN, *y, *dlt, *scal, *H;
-    int *grp, *S1, *S3, *lst, *gl1, *gl3, *cnt, *mapbuf;
+    double *K;            /* kernel matrix of the working set, w x w (NULL: too large to keep) */
+    int *grp, *S1, *S3, *lst, *lloc, *gl1, *gl3, *cnt, *mapbuf;   /* lst, lloc: changed weights, as rows of X and of the set */
+    int use13;            /* this iteration's G13 is not zero */
     irwls_sub_stats *stats;   /* device */
     irwls_sub_stats *h_stats; /* pinned host mirror */
     int ldH;
@@ -156,7 +158,8 @@ void irwls_sub_release(irwls_sub_ws *ws);
 /* a_i and the groups at entry (src/full-train.c:131-155); e, beta and map
  * must be set; stats->nS1/nS3 filled. */
 int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C);
-/* G13 of the current S1/S3 lists (src/full-train.c:327-344). */
+/* G13 of the current S1/S3 lists (src/full-train.c:327-344), for the next
+ * irwls_sub_iterate. */
 int irwls_sub_g13(irwls_sub_ws *ws, const irwls_dev_set *X, int n1, int n3);
 /* One inner iteration: H and rhs, solve, weights, working-set error update,
  * a_i and groups (src/full-train.c:160-307). */
