@@ -835,7 +835,7 @@ extern "C" int irwls_sgma_first(const irwls_dev_set *X, int l, int *d_cent, doub
     // centroid 0 = row l (the positive class mean), set by the caller in d_cent
     if (irwls_dev_kernel_block_t(X, d_cent, 1, X, nullptr, l, d_KSC, l, 0)) return -2;
     const size_t smem = (size_t)X->ld * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(sgma_factor_kernel);
     sgma_factor_kernel<<<1, 128, smem, irwls_stream()>>>(kview(X), 0, d_cent, nullptr, nullptr, 0, d_L, ldL, 0);
     IRWLS_LAUNCH_CHECK("sgma_factor");
     return 0;
@@ -853,7 +853,7 @@ extern "C" int irwls_sgma_score(const irwls_dev_set *X, int l, const int *d_cand
         irwls_set_error(-7, "SGMA budget %d with feature width %d exceeds the substitution tile", s, X->width);
         return -7;
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(sgma_cand_kernel);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_SGMA_CAND);
     sgma_cand_kernel<<<NCAND, 256, smem, irwls_stream()>>>(kview(X), d_cand, d_cent, s, d_L, ldL, d_W, d_Z, d_KN, ldz,
                                                           d_eta, nullptr, nullptr, l, nullptr);
@@ -881,7 +881,7 @@ extern "C" int irwls_sgma_rescore(const irwls_dev_set *X, int l, const int *d_ca
         irwls_set_error(-7, "SGMA budget %d with feature width %d exceeds the substitution tile", s, X->width);
         return -7;
     }
-    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_cand_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(sgma_cand_kernel);
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
     launch_chained(sgma_cand_kernel, dim3(NCAND + sms), dim3(256), smem, kview(X), d_cand, d_cent, s, d_L, ldL, d_W,
                    d_Z, d_KN, ldz, d_eta, d_need, d_built, l, d_KSC);
@@ -906,7 +906,7 @@ extern "C" int irwls_sgma_cand_inv(const irwls_dev_set *X, const int *d_cand, co
                                    double *d_W, void *Wb, int ldq, double *d_eta, const void *Qb, unsigned *d_eps) {
     if (s < 1) return 0;
     const size_t smem = (size_t)X->ld * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(cand_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(cand_rows_kernel);
     const int kpad = ceil_div(s, 64) * 64;
     if (kpad > ldq) {
         irwls_set_error(-12, "candidate width %d exceeds the split leading dimension %d", kpad, ldq);
@@ -944,7 +944,7 @@ extern "C" int irwls_sgma_linv_update(const double *d_L, int ldL, double *d_Linv
 extern "C" int irwls_sgma_factor(const irwls_dev_set *X, int s, const int *d_cent, const int *d_best, const double *d_W,
                                  int ldz, double *d_L, int ldL) {
     const size_t smem = (size_t)X->ld * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(sgma_factor_kernel);
     launch_chained(sgma_factor_kernel, dim3(1), dim3(128), smem, kview(X), s, d_cent, d_best, d_W, ldz, d_L, ldL, 1);
     IRWLS_LAUNCH_CHECK("sgma_factor");
     return 0;
@@ -964,7 +964,7 @@ extern "C" int irwls_sgma_extend(const irwls_dev_set *X, int l, int s, const int
                                  const double *d_W, int ldz, double *d_L, int ldL, double *d_KSC) {
     if (irwls_dev_kernel_block_t(X, d_cent + s, 1, X, nullptr, l, d_KSC + (size_t)s * l, l, 0)) return -2;
     const size_t smem = (size_t)X->ld * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(sgma_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(sgma_factor_kernel);
     sgma_factor_kernel<<<1, 128, smem, irwls_stream()>>>(kview(X), s, d_cent, d_best, d_W, ldz, d_L, ldL, 0);
     IRWLS_LAUNCH_CHECK("sgma_factor");
     return 0;

@@ -42,6 +42,20 @@ inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block,
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// Lets `kern` use as much dynamic shared memory as the device allows beside its
+// static shared memory. The attribute belongs to the function, not to a launch:
+// set to one launch's size, another thread's larger launch of the same kernel
+// between the two calls of this one was refused.
+template <typename K>
+inline void allow_smem(K kern) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+        cudaFuncGetAttributes(&fa, kern) == cudaSuccess)
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+}
+
 // Device-side status words (dev_context.cu), a device array of 8 ints:
 // [0] first failed Cholesky pivot of the last factorization (1-based, 0 if none).
 int *irwls_dev_flags();

@@ -934,7 +934,7 @@ extern "C" int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C
     if (ex == 1) {
         const size_t smem = (size_t)X->ld * sizeof(double);
         if (smem > 48 * 1024)
-            cudaFuncSetAttribute(sub_kmat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(sub_kmat_kernel);
         launch_chained(sub_kmat_kernel, dim3(ceil_div(w, 64), w), dim3(64), smem, *ws, kview(X));
         IRWLS_LAUNCH_CHECK("sub_kmat");
     }
@@ -970,7 +970,7 @@ static int sub_system_direct(irwls_sub_ws *ws, const irwls_dev_set *X, int n1) {
             dim3 grid(ceil_div(n1, 64), n1);
             const size_t smem = (size_t)X->ld * sizeof(double);
             if (smem > 48 * 1024)
-                cudaFuncSetAttribute(build_H_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                allow_smem(build_H_kernel);
             build_H_kernel<<<grid, 64, smem, irwls_stream()>>>(*ws, kv, n1);
             IRWLS_LAUNCH_CHECK("build_H");
         }

@@ -512,7 +512,7 @@ int gram_run(const double *d_KSC, int m, const int *d_act, int nact, const doubl
         IRWLS_LAUNCH_CHECK("gram_colmax");
     }
     const size_t smem = (size_t)GNS * G_STAGE + 1024;
-    cudaFuncSetAttribute(gram_tc_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(gram_tc_kernel<BITS>);
     int parts = 0;
     for (int a = 0, n = 0; n < nslab; a += slab, ++n) {
         const int rows = std::min(slab, nact - a);

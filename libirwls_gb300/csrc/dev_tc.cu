@@ -406,13 +406,13 @@ extern "C" int irwls_tc_gemm(const void *Ahi, const void *Alo, int lda, int M, c
     int *flags = irwls_dev_flags();
     const size_t smem = irwls_tc_smem_bytes(bn);
     if (bn == 64) {
-        cudaFuncSetAttribute(tc_gemm_store_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(tc_gemm_store_kernel<64>);
         dim3 grid(ceil_div(N, 64), ceil_div(M, TC_BM), splits);
         tc_gemm_store_kernel<64><<<grid, TC_THREADS, smem, irwls_stream()>>>(
             (const __nv_bfloat16 *)Ahi, (const __nv_bfloat16 *)Alo, lda, M, (const __nv_bfloat16 *)Bhi,
             (const __nv_bfloat16 *)Blo, ldb, N, kst, per, C, ldc, zstride, lower_only, flags);
     } else {
-        cudaFuncSetAttribute(tc_gemm_store_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(tc_gemm_store_kernel<128>);
         dim3 grid(ceil_div(N, 128), ceil_div(M, TC_BM), splits);
         tc_gemm_store_kernel<128><<<grid, TC_THREADS, smem, irwls_stream()>>>(
             (const __nv_bfloat16 *)Ahi, (const __nv_bfloat16 *)Alo, lda, M, (const __nv_bfloat16 *)Bhi,
@@ -1156,7 +1156,7 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
     const KViewF kv = kviewf(X, (const F32Mirror *)F);
     const __nv_bfloat16 *qb = (const __nv_bfloat16 *)Qb, *wb = (const __nv_bfloat16 *)Wb;
     auto launch = [&](auto kern) {
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kern);
         launch_chained(kern, dim3(grid), dim3(128 + 128 * WS_EG), smem, kv, l, d_cand, qb, ldq / 32, wb, kst, d_part,
                        d_resid, (int)xs, irwls_dev_flags());
     };
@@ -1195,7 +1195,7 @@ extern "C" int irwls_q_column(const irwls_dev_set *X, const void *F, int l, cons
     }
     const size_t smem = (size_t)X->ld * sizeof(float);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute(q_column_direct_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(q_column_direct_kernel);
     const int blocks = std::max(1, std::min(ceil_div(l, 256), 4 * (irwls_num_sms() > 0 ? irwls_num_sms() : 148)));
     q_column_direct_kernel<<<blocks, 256, smem, irwls_stream()>>>(kviewf(X, (const F32Mirror *)F), l, d_cent, s, lrow,
                                                                    (__nv_bfloat16 *)Qb, ldq, d_qn);
@@ -1819,7 +1819,7 @@ int rs_launch(TcSet *t, int M, const int *d_idx, const int *d_n, const double *d
     constexpr int NS = rs_stages<P>();
     const size_t smem = NS * RsStage<P>::BYTES + 1024;
     static_assert(NS * RsStage<P>::BYTES + 1024 <= 227 * 1024, "ring exceeds shared memory");
-    cudaFuncSetAttribute(tc_rowsum_ws_kernel<P, NS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(tc_rowsum_ws_kernel<P, NS, MODE>);
     const int ntiles = ceil_div(M, RS_BM);
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
     const int slot = MODE == 0 ? IRWLS_PROF_ROWSUM : IRWLS_PROF_PREDICT;
@@ -2095,7 +2095,7 @@ int ex_launch(TcSet *t, const irwls_dev_set *X, int nA, const int *d_ia, const i
               const double *d_cb, const double *d_sa, const double *d_sb, double *out, long long ldo, int lower) {
     const int ntiles = ceil_div(nA, RS_BM), nchx = ceil_div(nmax, CW);
     const size_t smem = (size_t)EX_NS * (RS_APIECE * 2 + CW * RS_BK * 2) + 1024;
-    cudaFuncSetAttribute(tc_exact_rowsum_kernel<CW, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(tc_exact_rowsum_kernel<CW, STORE>);
     tc_exact_rowsum_kernel<CW, STORE><<<ntiles * nchx, EX_THREADS, smem, irwls_stream()>>>(
         t->Ag, nA, t->kbn, t->B, d_n, nmax, nchx, X->q, d_ia, d_ib, t->rbf, X->neg_gamma, 1.0 / (t->scale * t->scale),
         d_cb, d_sa, d_sb, out, ldo, lower, irwls_dev_flags(), g_rs_wait_limit);

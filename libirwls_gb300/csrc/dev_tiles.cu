@@ -118,7 +118,7 @@ extern "C" int irwls_dev_kernel_block_t(const irwls_dev_set *A, const int *d_ia,
         return -5;
     }
     const size_t smem = ((size_t)R * A->ld + 16) * sizeof(double);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kernel_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) allow_smem(kernel_block_kernel);
     dim3 grid(ceil_div(nB, 128), ceil_div(nA, R));
     kernel_block_kernel<<<grid, kThreads, smem, irwls_stream()>>>(kview(A), d_ia, nA, kview(B), d_ib, nB, R, d_out,
                                                                    ld_out, trans);
@@ -146,7 +146,7 @@ static int rowsum_launch(const irwls_dev_set *A, const int *d_ia, int nA, const 
     }
     const size_t smem = ((size_t)R * A->ld + 8 + 1024) * sizeof(double);
     if (smem > 48 * 1024)
-        cudaFuncSetAttribute(kernel_rowsum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem(kernel_rowsum_kernel);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
     kernel_rowsum_kernel<<<ceil_div(nA, R), kThreads, smem, irwls_stream()>>>(
         kview(A), d_ia, nA, kview(B), d_ib, nB > 0 ? nB : 0, d_nB, R, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
