@@ -70,22 +70,33 @@ __device__ void factor_block(double (*D)[NB + 1], double *rp, int nb, int k0, in
 }
 
 // Inverse of the factored block (its reciprocal pivots in rp): each entry a
-// dot product split over 8 lanes of a warp (column j by threads 8 j ..
-// 8 j + 7), Di[c][j] = -(sum_{j <= t < c} D[c][t] Di[t][j]) rp[c].
-// blockDim.x == 256; ends synced.
+// dot product split over 8 lanes of a warp, four columns to a warp,
+// Di[c][j] = -(sum_{j <= t < c} D[c][t] Di[t][j]) rp[c], entry (c, j)'s lane q
+// summing t = j + q, j + q + 8, ... Warps w and w + 4, which share an SM
+// quarter's FP64 unit, take column groups w and 7 - w: 34 rows to form
+// between them everywhere (46 and 22 at the ends with groups in warp order,
+// where a 32-column inverse took 28000 cycles).
+// Di zeroed by the caller; blockDim.x >= 256, the first eight warps call.
 __device__ void invert_columns(double (*D)[NB + 1], double (*Di)[NB + 1], const double *rp, int nb) {
-    const int tid = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // (every lane of a warp runs the same iterations so that the shuffles
     // always see the whole warp; the first row below a warp's four columns
     // is the first it has to form)
-    const int j = tid >> 3, q = tid & 7;
+    const int j0 = 4 * (warp < 4 ? warp : 11 - warp), j = j0 + (lane >> 3), q = lane & 7;
     if (q == 0 && j < nb) Di[j][j] = rp[j];
     __syncwarp();
-    for (int c = (tid >> 5) * 4 + 1; c < nb; ++c) {
+    for (int c = j0 + 1; c < nb; ++c) {
         const bool live = j < nb && c > j;
-        double acc = 0.0;
-        if (live)
-            for (int t = j + q; t < c; t += 8) acc = fma(D[c][t], Di[t][j], acc);
+        double acc = 0.0, d[4], e[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {  // (all of the row's loads before its FMAs)
+            const int t = min(j + q + 8 * k, NB - 1);
+            d[k] = D[c][t];
+            e[k] = Di[t][j];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (live && j + q + 8 * k < c) acc = fma(d[k], e[k], acc);
         acc += __shfl_xor_sync(0xffffffffu, acc, 4, 8);
         acc += __shfl_xor_sync(0xffffffffu, acc, 2, 8);
         acc += __shfl_xor_sync(0xffffffffu, acc, 1, 8);
@@ -317,7 +328,8 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // and holds its SM quarter's FP64 unit for that long (76 with all four busy),
 // so a panel of 32 pivots is a chain of 32 (reciprocal square root 370 cycles,
 // scale, diagonal update). One warp runs that chain on a quarter of its own
-// (factor_stream); six warps on the other three apply the rank-1 updates.
+// (factor_stream); six warps on the other three scale the columns and apply the
+// rank-1 updates.
 // Whole tiles at a time, with three CTA barriers per pivot, a panel took 40 to
 // 48 us.
 //
@@ -338,10 +350,11 @@ constexpr int DFC = 4;               // columns per published step
 constexpr int DFQ = NB / DFC;        // steps of a tile
 constexpr int DFR = 6;               // ring slots of steps
 constexpr int DF_THREADS = 320;      // warps 0-7 compute, 8 loads, 9 publishes
-// named barriers: 1 and 2 the pivots' (factor_stream), 3 ... finished columns
-// of a diagonal block, then the compute warps' own two
-constexpr int BAR_ALL = 3 + DFQ, BAR_STEP = BAR_ALL + 1;
-static_assert(BAR_STEP < 16, "named barriers");
+// named barriers: the pivots' three (factor_stream), finished columns of a
+// diagonal block, the compute warps' own two
+constexpr int BAR_ROOT = 1, BAR_COL = 2, BAR_NEXT = 3, BAR_PUB = 4;
+constexpr int BAR_ALL = BAR_PUB + DFQ, BAR_STEP = BAR_ALL + 1, BAR_ROOT2 = BAR_STEP + 1;
+static_assert(BAR_ROOT2 < 16, "named barriers");
 
 __device__ __forceinline__ unsigned ld_relaxed_u32(const unsigned *p) {
     unsigned v;
@@ -356,10 +369,19 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void bar_sync(int id, int count) {
+template <int ID, int COUNT>
+__device__ __forceinline__ void bar_sync() {
+    asm volatile("bar.sync %0, %1;\n" ::"n"(ID), "n"(COUNT) : "memory");
+}
+template <int ID, int COUNT>
+__device__ __forceinline__ void bar_arrive() {
+    asm volatile("bar.arrive %0, %1;\n" ::"n"(ID), "n"(COUNT) : "memory");
+}
+// (barrier numbers known at run time only)
+__device__ __forceinline__ void bar_sync_at(int id, int count) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
-__device__ __forceinline__ void bar_arrive(int id, int count) {
+__device__ __forceinline__ void bar_arrive_at(int id, int count) {
     asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(count) : "memory");
 }
 
@@ -371,7 +393,9 @@ struct DfSlot {
 struct DfShared {
     double T[NB][NB + 1], Di[NB][NB + 1];
     double rp[NB], rhs[NB];
-    double col[2][NB];  // factor_stream: the scaled column, by step parity
+    // factor_stream, by step parity: the scaled column, the next unscaled one,
+    // the diagonal, the pivot and its reciprocal root
+    double col[2][NB], next[2][NB], diag[2][NB], piv[2], root[2];
     DfSlot slot[DFR];
     // pub: one per step of a tile, so that the computing warps may run ahead
     // of the publisher; used again after done, the publisher's end of a tile
@@ -381,78 +405,130 @@ struct DfShared {
 
 // Factors the nb x nb diagonal block in T (lower part valid) with
 // factor_block's operations, handing its columns to the publishing warp as
-// they are finished. Warp 0 holds the diagonal (lane = row) and runs the
-// pivots: it waits for the next column (barrier 2), scales it by the pivot's
-// reciprocal root and hands it out (barrier 1; one barrier from 3 on per DFC
-// finished columns, for the publisher). Warps 1, 2, 3, 5, 6 and 7 hold the 496
-// elements below the diagonal, in column order, 32 to a register: group g on
-// warp g mod 6 (so on the three SM quarters warp 0 is not on), the first of a
-// step's live groups holding the next column. Signs are tested on the bits: an
-// FP64 compare would take the unit for 65 cycles.
-__device__ void factor_stream(DfShared &sh, int nb, int k0, int *flags) {
+// they are finished. The pivots are one dependent chain -- reciprocal root of
+// s_t, the scaled element below it, s_(t+1) = D - l l -- which warp 0 alone
+// runs, on scalars, an SM quarter to itself: about 650 cycles a pivot (501 the
+// chain alone, 806 when that warp also scaled the column and held the
+// diagonal). Warp 1 (lane =
+// row) scales column t, keeps the diagonal and signals the publisher; warps 2,
+// 3, 5, 6 and 7 hold the 496 elements below the diagonal, in column order, 32
+// to a register: group g on warp number g mod 5, the first of a step's live
+// groups holding the next column. Barriers: BAR_ROOT and BAR_ROOT2 pass r_t for
+// even and odd t (warps 0, 1), BAR_COL the scaled column t (1, updates),
+// BAR_NEXT the unscaled column t + 1 and the diagonal (updates, 1, 0); one
+// barrier from BAR_PUB on per DFC finished columns. A warp that only arrives
+// must not arrive at a barrier again before those that wait at it have: warp 0
+// passes BAR_NEXT of step t, which warp 1 joins after BAR_ROOT of step t, between
+// its arrivals of steps t and t + 2 but not of t and t + 1, hence the two. What a step hands out lies in one of two buffers by its
+// parity: each is written again only after its readers have passed a later
+// barrier. Signs are tested on the bits: an FP64 compare would take the unit
+// for 65 cycles.
+struct FactorPart {
+    int er[4], ec[4];  // an update thread's elements (row, column; column -1: none)
+    int c0[4], c1[4];  // first and last column of the warp's groups (the warp's)
+};
+__device__ void factor_part(FactorPart &f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int ALL = 32 * 7;
+    const int u = warp < 4 ? warp - 2 : warp - 3;  // 0 ... 4 on the update warps
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        // element e of the strictly lower part in column order
+        int e = (u + 5 * x) * 32 + lane, c = 0;
+        while (c < NB - 1 && e >= NB - 1 - c) {
+            e -= NB - 1 - c;
+            ++c;
+        }
+        f.ec[x] = c < NB - 1 ? c : -1;  // past the last element: never live
+        f.er[x] = c < NB - 1 ? c + 1 + e : 0;
+        f.c0[x] = __shfl_sync(0xffffffffu, f.ec[x], 0);
+        f.c1[x] = __reduce_max_sync(0xffffffffu, f.ec[x]);
+    }
+}
+__device__ void factor_stream(DfShared &sh, const FactorPart &f, int nb, int k0, int *flags) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NEXT = 32 * 7, COL = 32 * 6;
     double(*D)[NB + 1] = sh.T;
     if (warp == 0) {
-        double dg = lane < nb ? D[lane][lane] : 0.0;
+        double s = D[0][0], a = D[1][0], g = D[1][1];  // (read before warp 1 may scale column 0)
         int failed = -1;
         for (int t = 0; t < nb; ++t) {
-            const double s = __shfl_sync(0xffffffffu, dg, t);
             const long long bits = __double_as_longlong(s);
             const bool ok = bits > 0 && bits <= 0x7ff0000000000000LL;  // s > 0.0
             const double r = ok ? rsqrt(s) : 1.0 / s;
             if (!ok && failed < 0) failed = t;  // stored without its root, as dpotrf leaves it
-            if (t > 0) bar_sync(2, ALL);        // column t is final below the diagonal
-            const double a = lane == t ? s : lane > t && lane < nb ? D[lane][t] : 0.0;
-            const double l = a * r;
-            sh.col[t & 1][lane] = l;
-            if (lane >= t) D[lane][t] = lane == t && !ok ? s : l;
-            if (lane == t) sh.rp[t] = r;
-            __syncwarp();
-            if (t + 1 < nb) bar_arrive(1, ALL);
-            if ((t & (DFC - 1)) == DFC - 1 || t == nb - 1) bar_arrive(3 + t / DFC, 64);
-            dg = fma(-l, l, dg);  // (of use for lanes > t)
+            sh.root[t & 1] = r;  // (every lane: the same value)
+            sh.piv[t & 1] = s;
+            if (t & 1) bar_arrive<BAR_ROOT2, 64>();
+            else bar_arrive<BAR_ROOT, 64>();
+            if (t + 1 < nb) {
+                if (t > 0) {
+                    bar_sync<BAR_NEXT, NEXT>();  // of step t - 1: column t and the diagonal
+                    a = sh.next[t & 1][t + 1];
+                    g = sh.diag[(t - 1) & 1][t + 1];
+                }
+                const double l = a * r;
+                s = fma(-l, l, g);
+            } else if (t > 0) {
+                bar_arrive<BAR_NEXT, NEXT>();
+            }
         }
         if (lane == 0 && failed >= 0) atomicCAS(flags, 0, k0 + failed + 1);
-    } else if (warp != 4) {
-        const int u = warp < 4 ? warp - 1 : warp - 2;  // 0 ... 5
-        double v[3];
-        int er[3], ec[3];
-#pragma unroll
-        for (int x = 0; x < 3; ++x) {
-            // element e of the strictly lower part in column order
-            int e = (u + 6 * x) * 32 + lane, c = 0;
-            while (c < NB - 1 && e >= NB - 1 - c) {
-                e -= NB - 1 - c;
-                ++c;
-            }
-            ec[x] = c < NB - 1 ? c : -1;  // past the last element: never live
-            er[x] = c < NB - 1 ? c + 1 + e : 0;
-            v[x] = ec[x] >= 0 ? D[er[x]][ec[x]] : 0.0;
+    } else if (warp == 1) {
+        double dg = lane < nb ? D[lane][lane] : 0.0;
+        for (int t = 0; t < nb; ++t) {
+            const double c0 = t == 0 ? D[lane][0] : 0.0;
+            if (t > 0) bar_sync<BAR_NEXT, NEXT>();
+            const double c = t == 0 ? c0 : sh.next[t & 1][lane];
+            if (t & 1) bar_sync<BAR_ROOT2, 64>();
+            else bar_sync<BAR_ROOT, 64>();
+            const double r = sh.root[t & 1], s = sh.piv[t & 1];
+            const long long bits = __double_as_longlong(s);
+            const bool ok = bits > 0 && bits <= 0x7ff0000000000000LL;
+            const double a = lane == t ? s : lane > t && lane < nb ? c : 0.0;
+            const double l = a * r;
+            sh.col[t & 1][lane] = l;
+            __syncwarp();
+            if (t + 1 < nb) bar_arrive<BAR_COL, COL>();
+            if (lane >= t) D[lane][t] = lane == t && !ok ? s : l;
+            if (lane == t) sh.rp[t] = r;
+            dg = fma(-l, l, dg);  // (of use for lanes > t)
+            sh.diag[t & 1][lane] = dg;
+            __syncwarp();
+            if ((t & (DFC - 1)) == DFC - 1 || t == nb - 1) bar_arrive_at(BAR_PUB + t / DFC, 64);
         }
+    } else if (warp != 4) {
+        double v[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) v[x] = f.ec[x] > 0 ? D[f.er[x]][f.ec[x]] : 0.0;
         for (int t = 0; t + 1 < nb; ++t) {
-            bar_sync(1, ALL);
+            bar_sync<BAR_COL, COL>();
             const double *l = sh.col[t & 1];
+            double lr[4], lc[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                lr[x] = l[f.er[x]];
+                lc[x] = l[max(f.ec[x], 0)];
+            }
             bool told = false;
 #pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                const bool live = ec[x] > t;
-                if (!__any_sync(0xffffffffu, live)) continue;
+            for (int x = 0; x < 4; ++x) {
+                if (f.c1[x] <= t) continue;  // no live element
                 // the next column lies in the first live groups
-                if (!told && !__any_sync(0xffffffffu, ec[x] == t + 1)) {
-                    bar_arrive(2, ALL);
+                const bool now = f.c0[x] <= t + 1;
+                if (!told && !now) {
+                    bar_arrive<BAR_NEXT, NEXT>();
                     told = true;
                 }
-                if (live) v[x] = fma(-l[er[x]], l[ec[x]], v[x]);
-                if (ec[x] == t + 1) D[er[x]][ec[x]] = v[x];
+                if (f.ec[x] > t) v[x] = fma(-lr[x], lc[x], v[x]);
+                if (now) {
+                    if (f.ec[x] == t + 1) sh.next[(t + 1) & 1][f.er[x]] = v[x];
+                    __syncwarp();
+                }
             }
-            if (!told) {
-                __syncwarp();
-                bar_arrive(2, ALL);
-            }
+            if (!told) bar_arrive<BAR_NEXT, NEXT>();
         }
     }
-    bar_sync(BAR_ALL, 256);
+    bar_sync<BAR_ALL, 256>();
 }
 
 // ready: columns published of diag[j] at ready[j] (j < nbc), of tile L(i, j)
@@ -504,9 +580,12 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                                 const int v = lane < 2 ? (int)ld_acquire_u32(p) : NB;
                                 have = __reduce_min_sync(0xffffffffu, v);
                                 if (have > done) break;
-                                if (it >= DF_WAIT_LIMIT || ld_relaxed_u32((const unsigned *)abort)) ok = false;
+                                if (it >= DF_WAIT_LIMIT) ok = false;
+                                if ((it & 63) == 63) {
+                                    if (ld_relaxed_u32((const unsigned *)abort)) ok = false;
+                                    __nanosleep(32);
+                                }
                                 ok = __all_sync(0xffffffffu, ok);
-                                if (it > 64) __nanosleep(32);
                             }
                             __syncwarp();
                         }
@@ -563,7 +642,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                     if (i == j) {
                         // (a diagonal tile gives up before it is factored)
                         if (q == 0) ok = mbar_wait(smem_u32(&sh.pub[0]), (unsigned)tasks & 1u) && !sh.stop;
-                        if (ok) bar_sync(3 + q, 64);
+                        if (ok) bar_sync_at(BAR_PUB + q, 64);
                     } else {
                         ok = mbar_wait(smem_u32(&sh.pub[q]), (unsigned)(q == 0 ? tasks : below) & 1u) && !sh.stop;
                     }
@@ -574,10 +653,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                     if (i == j && lane >= DFC * q && lane < q1)
                         Dinv[(size_t)j * NB * NB + lane * (NB + 1)] = sh.rp[lane];
                     __syncwarp();
-                    if (lane == 0) {
-                        __threadfence();
+                    if (lane == 0)
                         st_release_u32(i == j ? ready + j : ready + nbc + (size_t)j * nbr + i, q1 == nc ? NB : q1);
-                    }
                 }
                 if (lane == 0) mbar_arrive(&sh.done);
                 ++tasks;
@@ -599,6 +676,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
         dr[x] = r;
         dc[x] = e - r * (r + 1) / 2;
     }
+    FactorPart part;
+    factor_part(part);
     const bool third = tid < NB * (NB + 1) / 2 - 512;
     const int r = tid % NB, u = tid / NB;
     bool good = true;
@@ -627,7 +706,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                     v = b && r0 + rr == n ? b[c0 + c] : __ldcg(M + (size_t)(c0 + c) * ld + r0 + rr);
                 sh.T[rr][c] = v;
             }
-            bar_sync(BAR_ALL, 256);
+            bar_sync<BAR_ALL, 256>();
             for (int k = 0; k < j && good; ++k) {
                 double acc[4] = {0.0, 0.0, 0.0, 0.0};
                 for (int q = 0; q < DFQ; ++q) {
@@ -664,7 +743,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
             }
             // every thread has seen the same slots, so `good` is the CTA's
             if (!good) break;
-            bar_sync(BAR_ALL, 256);
+            bar_sync<BAR_ALL, 256>();
             if (i == j) {
                 if (lane == 0) mbar_arrive(&sh.pub[0]);  // the publisher may join the factor
                 // row nc of this tile is the right-hand side
@@ -674,12 +753,12 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                     if (rr >= nc || c > rr) sh.T[rr][c] = 0.0;
                     sh.Di[rr][c] = 0.0;
                 }
-                bar_sync(BAR_ALL, 256);
-                factor_stream(sh, nc, c0, flags);
+                bar_sync<BAR_ALL, 256>();
+                factor_stream(sh, part, nc, c0, flags);
                 // the right-hand-side row, by the panel solves' substitution:
-                // warp 7 (whose columns of the inverse are the shortest) with
+                // warp 4 (whose columns of the inverse are the shortest) with
                 // lane = column
-                if (nr > nc && warp == 7) {
+                if (nr > nc && warp == 4) {
                     double v = lane < nc ? sh.rhs[lane] : 0.0;
                     for (int q = 0; q < nc; ++q) {
                         if (lane == q) v = v * sh.rp[q];
@@ -690,7 +769,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                 }
                 // the inverse (for the backward sweep after this launch)
                 invert_columns(sh.T, sh.Di, sh.rp, nc);
-                bar_sync(BAR_ALL, 256);
+                bar_sync<BAR_ALL, 256>();
                 for (int e = tid; e < NB * NB; e += 256) Dinv[(size_t)j * NB * NB + e] = sh.Di[e / NB][e % NB];
             } else {
                 // the panel solve, DFC columns at a time: within them by
@@ -712,12 +791,12 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                                 sh.T[r][done + h] = v;
                             }
                             if (h < DFC - 1) {
-                                bar_sync(BAR_STEP, 32 * DFC);
+                                bar_sync<BAR_STEP, 32 * DFC>();
                                 if (u > h) v = fma(-sh.T[r][done + h], sl.a[done + u][h], v);
                             }
                         }
                     }
-                    bar_sync(BAR_ALL, 256);
+                    bar_sync<BAR_ALL, 256>();
                     if (lane == 0) mbar_arrive(&sh.pub[q]);
                     told = q + 1;
                     for (int c = done + DFC + u; c < NB; c += 8) {
@@ -824,101 +903,144 @@ __global__ void __launch_bounds__(256) chol_backsolve_coop_kernel(double *__rest
 
 // The same sweep in one thread-block cluster of g <= 8 CTAs (orders up to
 // 2048), block b of 32 rows on CTA b mod g with its z in shared memory. Per
-// block from the bottom its owner forms x_b and stores it into every CTA's
-// shared memory; a split cluster barrier hands it out. The owner of block
-// b - 1 applies x_b to it at once and goes on to x_(b-1); the other blocks
-// take x_b between their CTA's arrival at the next barrier and its wait, so
-// the chain per block is one block's update and dot product. A dot product's
-// four partial chains (sweep_dot, sweep_row) run on four lanes, eight FMAs
-// each, instead of one after another on one: 65 cycles per FP64 instruction
-// whatever the lanes. x_b lives in one of four slots: it is last read before
-// the wait of block b - 1, and block b - 4 writes the slot next.
+// block from the bottom its owner forms x_b and sends it into every CTA's
+// shared memory (st.async, one mbarrier and one place per block, so nothing is
+// reused and no CTA waits for a slower one). Warps 0 to 3 of the owner of
+// block b - 1 apply x_b to it as it arrives and go on to x_(b-1): that is the
+// chain, one block's update and dot product per block. Warps 4 to 7 apply x_b
+// to the CTA's blocks further up (in a CTA whose chain warps are at work, once
+// they have sent x_(b-1): they share the FP64 units) and hand block q to the
+// chain warps when x_(q+2) is in it. A dot product's four partial chains
+// (sweep_dot, sweep_row) run on four lanes, eight FMAs each, instead of one
+// after another on one: 65 cycles per FP64 instruction whatever the lanes.
 __device__ __forceinline__ double chains_sum(double a) {
     a += __shfl_xor_sync(0xffffffffu, a, 1);
     return a + __shfl_xor_sync(0xffffffffu, a, 2);  // (a0 + a1) + (a2 + a3)
 }
 
-constexpr int SWB = 8;  // blocks of a CTA
-__global__ void __launch_bounds__(256) chol_sweep_cluster_kernel(const double *__restrict__ M, int n, int ld,
-                                                                 const double *__restrict__ Dinv,
-                                                                 double *__restrict__ x, const int *__restrict__ flags,
-                                                                 int *__restrict__ info) {
+constexpr int SWB = 8;                // blocks of a CTA
+constexpr int SWN = 8 * SWB;          // blocks of the largest order
+struct SweepShared {
+    double z[SWB][NB], xb[SWN][NB], Di[2][NB][NB + 1];
+    uint64_t got[SWN], ready[SWB];  // x_b has arrived; a block has all but its last update
+};
+__global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double *__restrict__ M, int n, int ld,
+                                                                    const double *__restrict__ Dinv,
+                                                                    double *__restrict__ x,
+                                                                    const int *__restrict__ flags,
+                                                                    int *__restrict__ info) {
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-    __shared__ double z[SWB][NB], xb[4][NB], Di[2][NB][NB + 1];
+    __shared__ SweepShared sh;
     const int g = (int)cl.num_blocks(), me = (int)cl.block_rank();
-    const int tid = threadIdx.x, half = tid >> 7;
-    const int row = 8 * ((tid >> 5) & 3) + ((tid & 31) >> 2), ch = tid & 3;  // row of a block, partial chain
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int row = 8 * ((tid >> 5) & 3) + (lane >> 2), ch = tid & 3;  // row of a block, partial chain
     const int nblk = (n + NB - 1) / NB;
     for (int e = tid; e < SWB * NB; e += 256) {
         const int c = ((e / NB) * g + me) * NB + e % NB;
-        z[e / NB][e % NB] = c < n ? M[(size_t)c * ld + n] : 0.0;
+        sh.z[e / NB][e % NB] = c < n ? M[(size_t)c * ld + n] : 0.0;
     }
-    auto load_inv = [&](int b) {
-        for (int t = tid; t < NB * NB; t += 256) Di[b & 1][t / NB][t % NB] = Dinv[(size_t)b * NB * NB + t];
+    if (tid < SWB) mbar_init(&sh.ready[tid], 4);
+    if (tid < nblk) {
+        mbar_init(&sh.got[tid], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(&sh.got[tid])),
+                     "r"(8 * min(NB, n - NB * tid)));
+    }
+    auto load_inv = [&](int b, int t0, int nt) {
+        for (int t = t0; t < NB * NB; t += nt) sh.Di[b & 1][t / NB][t % NB] = Dinv[(size_t)b * NB * NB + t];
     };
-    if ((nblk - 1) % g == me) load_inv(nblk - 1);
+    if ((nblk - 1) % g == me) load_inv(nblk - 1, tid, 256);
     if (info && me == 0 && tid == 0) *info = *flags;
     cl.sync();
-    // z of block q minus its rows of L_b^T times x_b; l: the row's values
-    // 4 k + ch when they are loaded already
-    auto update = [&](int q, int b, const double *l) {
+    // this thread's values of rows of L_b^T for block q (4 k + ch)
+    auto load_row = [&](int q, int b, double *v) {
+        const double *col = M + (size_t)(NB * q + row) * ld + NB * b;
+        if (NB * b + NB <= n)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = col[4 * k + ch];
+    };
+    // z of block q minus those rows times x_b
+    auto update = [&](int q, int b, const double *v) {
         const int nb = min(NB, n - NB * b);
-        const double *col = M + (size_t)(NB * q + row) * ld + NB * b, *xs = xb[b & 3];
+        const double *xs = sh.xb[b];
         double a = 0.0;
         if (nb == NB) {
-            double v[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = l ? l[k] : col[4 * k + ch];
 #pragma unroll
             for (int k = 0; k < 8; ++k) a = fma(v[k], xs[4 * k + ch], a);
         } else {
+            const double *col = M + (size_t)(NB * q + row) * ld + NB * b;
             for (int k = 0; k < nb / 4; ++k) a = fma(col[4 * k + ch], xs[4 * k + ch], a);
             if (ch == 0)
                 for (int c = nb / 4 * 4; c < nb; ++c) a = fma(col[c], xs[c], a);
         }
         a = chains_sum(a);
-        if (ch == 0) z[q / g][row] = z[q / g][row] - a;
+        if (ch == 0) sh.z[q / g][row] = sh.z[q / g][row] - a;
     };
-    for (int b = nblk - 1; b >= 0; --b) {
-        if (b % g == me && half == 0) {
-            const int nb = min(NB, n - NB * b), t = row, K = t < nb ? (nb - t) / 4 : 0;
-            const double(*D)[NB + 1] = Di[b & 1];
-            const double *yb = z[b / g];
-            double a = 0.0;
-            for (int k = 0; k < K; ++k) a = fma(D[t + 4 * k + ch][t], yb[t + 4 * k + ch], a);
-            if (ch == 0)
-                for (int c = t + 4 * K; c < nb; ++c) a = fma(D[c][t], yb[c], a);
-            a = chains_sum(a);
-            if (ch == 0 && t < nb) {
-                x[NB * b + t] = a;
-                if (b > 0)
-                    for (int r = 0; r < g; ++r) *cl.map_shared_rank(&xb[b & 3][t], r) = a;
-            }
-        }
-        if (b == 0) break;
-        __syncwarp();
-        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
-        const bool next = (b - 1) % g == me;
+    if (tid < 128) {
         double pre[8];
-        if (next) {
-            load_inv(b - 1);
-            if (half == 0 && NB * b + NB <= n) {
-                const double *col = M + (size_t)(NB * (b - 1) + row) * ld + NB * b;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) pre[k] = col[4 * k + ch];
+        bool ok = true;
+        for (int b = nblk - 1; b >= 0 && ok; --b) {
+            if (b % g == me) {
+                const int nb = min(NB, n - NB * b), t = row, K = t < nb ? (nb - t) / 4 : 0;
+                const double(*D)[NB + 1] = sh.Di[b & 1];
+                const double *yb = sh.z[b / g];
+                double a = 0.0;
+                for (int k = 0; k < K; ++k) a = fma(D[t + 4 * k + ch][t], yb[t + 4 * k + ch], a);
+                if (ch == 0)
+                    for (int c = t + 4 * K; c < nb; ++c) a = fma(D[c][t], yb[c], a);
+                a = chains_sum(a);
+                if (t < nb) {
+                    // lane ch of the row sends to CTAs ch, ch + 4
+                    if (b > 0)
+                        for (int r = ch; r < g; r += 4) {
+                            uint32_t dst, bar;
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                                         : "=r"(dst)
+                                         : "r"(smem_u32(&sh.xb[b][t])), "r"(r));
+                            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                                         : "=r"(bar)
+                                         : "r"(smem_u32(&sh.got[b])), "r"(r));
+                            asm volatile(
+                                "st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];\n" ::"r"(dst),
+                                "l"(__double_as_longlong(a)), "r"(bar)
+                                : "memory");
+                        }
+                    if (ch == 0) x[NB * b + t] = a;
+                }
+                asm volatile("bar.sync 1, 128;\n" ::: "memory");  // all have read the inverse: its buffer is free
+            }
+            if (b > 0 && (b - 1) % g == me) {
+                load_inv(b - 1, tid, 128);
+                load_row(b - 1, b, pre);
+                // x_(b+1) and all before it are in the block (none when b is the last)
+                if (b + 1 < nblk) ok = mbar_wait(smem_u32(&sh.ready[(b - 1) / g]), 0u);
+                ok = ok && mbar_wait(smem_u32(&sh.got[b]), 0u);
+                update(b - 1, b, pre);
+                asm volatile("bar.sync 1, 128;\n" ::: "memory");
             }
         }
-        // the previous block's x for this CTA's blocks below b (block b has it)
-        if (b + 1 < nblk)
-            for (int s = half; s * g + me < b; s += 2) update(s * g + me, b + 1, nullptr);
-        __syncwarp();
-        asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-        if (next) {
-            __syncthreads();
-            if (half == 0) update(b - 1, b, pre);
-            __syncthreads();
+    } else {
+        bool ok = true;
+        for (int b = nblk - 1; b >= 2 && ok; --b) {
+            // this CTA's blocks q <= b - 2, the next to be handed over first
+            int q = b - 2 - ((b - 2 - me) % g + g) % g;
+            if (q < 0) continue;
+            double v[8];
+            load_row(q, b, v);
+            ok = mbar_wait(smem_u32(&sh.got[b]), 0u);
+            if ((b - 1) % g == me) ok = ok && mbar_wait(smem_u32(&sh.got[b - 1]), 0u);
+            if (!ok) break;
+            for (; q >= 0; q -= g) {
+                update(q, b, v);
+                if (q == b - 2) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh.ready[q / g]);
+                }
+                if (q >= g) load_row(q - g, b, v);
+            }
         }
     }
+    cl.sync();  // no CTA leaves while others may send to it
 }
 
 // CTAs of the cooperative sweep for order n on the current device, or 0 when
@@ -1103,7 +1225,7 @@ int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv
                 irwls_set_error(-6, "system of order %d exceeds the backward-solve tile", n);
                 return -6;
             }
-            cudaFuncSetAttribute(chol_backsolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(chol_backsolve_kernel);
         }
         chol_backsolve_kernel<<<1, 256, smem, st>>>(d_M, n, ld, Dinv, d_x);
         IRWLS_LAUNCH_CHECK("chol_backsolve");
