@@ -510,7 +510,7 @@ extern "C" double *irwls_dmodel_predict(const irwls_dmodel *m, svm_dataset ds, p
     double *out = (double *)malloc((size_t)std::max(1, n) * sizeof(double));
     if (!out) return nullptr;
     if (n > 0) {
-        const int w = std::max(irwls_feature_width(&ds, n), m->S.width);
+        const int w = m->S.width;  // at least: a wider set keeps its own width
         irwls_dev_set T;
         const int fast = m->kernelType == 0 && irwls_get_linear_fast_path();
         int rc = fast ? irwls_dev_upload_csr(&ds, n, m->kernelType, m->Kgamma, w, &T)

@@ -74,6 +74,7 @@ typedef struct irwls_dev_set {
     double *q;        /* quadratic_value per row */
     double *y;        /* labels per row */
     long long nnz;
+    void *block;      /* the allocation that holds the arrays, or NULL: each is its own */
 } irwls_dev_set;
 
 /* Uploads rows 0..n_rows-1 of `ds`. kernelType/gamma pick the mode as the
@@ -89,8 +90,7 @@ int irwls_dev_upload_csr(const svm_dataset *ds, int n_rows, int kernelType, doub
 /* Same upload from the rows of a model. */
 int irwls_dev_upload_model(const model *m, int width_hint, irwls_dev_set *out);
 void irwls_dev_release(irwls_dev_set *s);
-int irwls_feature_width(const svm_dataset *ds, int n_rows);   /* max index + 1 over rows */
-int irwls_model_feature_width(const model *m);
+int irwls_model_feature_width(const model *m);   /* max index + 1 over the support vectors */
 
 /* ---- kernel tiles (dev_tiles.cu) ----------------------------------------- */
 /* out[i*ld_out + j] = k(A[ia_i], B[ib_j]) for i < nA, j < nB. ia/ib may be

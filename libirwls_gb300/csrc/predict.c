@@ -35,19 +35,18 @@ static double *predict(svm_dataset ds, model m, predictProperties props, int har
     const int n = ds.l;
     double *out = (double *)malloc((size_t)(n > 0 ? n : 1) * sizeof(double));
     if (n > 0) {
-        int w = irwls_feature_width(&ds, n);
+        /* one column space: the rows take the model's width, the model theirs */
         const int wm = irwls_model_feature_width(&m);
-        if (wm > w) w = wm;
         irwls_dev_set T, S;
         double *d_w = NULL, *d_out = NULL;
         const int fast = m.kernelType == 0 && irwls_get_linear_fast_path();
-        int rc = fast ? irwls_dev_upload_csr(&ds, n, m.kernelType, m.Kgamma, w, &T)
-                      : irwls_dev_upload(&ds, n, m.kernelType, m.Kgamma, 1, w, &T);
+        int rc = fast ? irwls_dev_upload_csr(&ds, n, m.kernelType, m.Kgamma, wm, &T)
+                      : irwls_dev_upload(&ds, n, m.kernelType, m.Kgamma, 1, wm, &T);
         if (rc) {
             free(out);
             return NULL;
         }
-        rc = irwls_dev_upload_model(&m, w, &S);
+        rc = irwls_dev_upload_model(&m, T.width, &S);
         if (rc) {
             irwls_dev_release(&T);
             free(out);
