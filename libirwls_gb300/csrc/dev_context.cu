@@ -18,6 +18,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -415,22 +417,33 @@ int stage_give(Stage s) {
     return rc;
 }
 
-// fn(first row, last row, part) over `n` rows in `parts` contiguous parts, one
-// thread each (the caller's runs the first, and any the system has no thread
-// for). fn does not throw.
-template <class F>
-void over_rows(int n, int parts, F fn) {
-    std::vector<std::thread> team;
-    team.reserve((size_t)parts);
-    auto part = [=](int t) { fn((int)((long long)n * t / parts), (int)((long long)n * (t + 1) / parts), t); };
-    int started = 1;
-    try {
-        for (; started < parts; ++started) team.emplace_back(part, started);
-    } catch (...) {
+// fn(first row, last row, chunk) over `n` rows in `chunks` contiguous chunks,
+// taken in turn by the caller and helpers - 1 other threads. The caller waits for
+// the chunks, not for the threads: one that the system starts late (behind
+// another library's spinning threads that cost up to 6 ms) finds nothing left
+// and ends by itself. fn does not throw.
+struct RowTeam {
+    std::atomic<int> next{0}, done{0};
+    int n = 0, chunks = 0;
+    std::function<void(int, int, int)> fn;
+    void work() {
+        for (int c; (c = next.fetch_add(1)) < chunks;) {
+            fn((int)((long long)n * c / chunks), (int)((long long)n * (c + 1) / chunks), c);
+            done.fetch_add(1);
+        }
     }
-    part(0);
-    for (int t = started; t < parts; ++t) part(t);
-    for (auto &t : team) t.join();
+};
+void over_rows(int n, int chunks, int helpers, std::function<void(int, int, int)> fn) {
+    auto team = std::make_shared<RowTeam>();
+    team->n = n;
+    team->chunks = chunks;
+    team->fn = std::move(fn);
+    try {
+        for (int t = 1; t < helpers; ++t) std::thread([team] { team->work(); }).detach();
+    } catch (...) {  // (no thread to be had: the caller does it all)
+    }
+    team->work();
+    while (team->done.load() < chunks) std::this_thread::yield();
 }
 
 // The dense rows by feature index from the CSR: a warp per row writes its
@@ -472,18 +485,22 @@ static int upload_rows_(svm_sample *const *rows, const double *q, const double *
     out->n_rows = n_rows;
     out->mode = mode;
     out->neg_gamma = -gamma;
-    // threads: one per 40000 entries by the first row's length (a thread costs
-    // about as much as walking 10000), one in the batching form's workers
-    int parts = 1;
+    // threads: one more per 250000 entries by the first row's length, one in
+    // the batching form's workers. (From 40000 on the warm time fell by 0.3 ms
+    // of 6.3 at 240000 entries, but where another library's threads still spin
+    // after a call of its own, a helper in the middle of a chunk can lose its
+    // core for 6 ms: not worth it below a walk of several milliseconds.)
+    int helpers = 1;
     if (!t_ctx && n_rows >= 64) {
         long long len = 1;
         for (const svm_sample *p = rows[0]; p->index != -1; ++p) ++len;
         const int hw = (int)std::thread::hardware_concurrency();
-        parts = (int)std::min<long long>(std::min(8, hw > 0 ? hw : 1), 1 + len * n_rows / 40000);
+        helpers = (int)std::min<long long>(std::min(8, hw > 0 ? hw : 1), 1 + len * n_rows / 250000);
     }
+    const int chunks = helpers > 1 ? 4 * helpers : 1;
     std::vector<int> count((size_t)n_rows + 1);
-    std::vector<RowScan> scan(parts);
-    over_rows(n_rows, parts, [&, rows](int i0, int i1, int t) {
+    std::vector<RowScan> scan(chunks);
+    over_rows(n_rows, chunks, helpers, [&, rows](int i0, int i1, int t) {
         RowScan r;
         for (int i = i0; i < i1; ++i) {
             const svm_sample *p = rows[i];
@@ -540,7 +557,7 @@ static int upload_rows_(svm_sample *const *rows, const double *q, const double *
     hrp[0] = 0;
     for (int i = 0; i < n_rows; ++i) hrp[i + 1] = hrp[i] + count[i];
     const int ld = out->ld;
-    over_rows(n_rows, parts, [=](int i0, int i1, int) {
+    over_rows(n_rows, chunks, helpers, [=](int i0, int i1, int) {
         if (i1 > i0) {
             if (q) memcpy(hq + i0, q + i0, (size_t)(i1 - i0) * sizeof(double));
             else memset(hq + i0, 0, (size_t)(i1 - i0) * sizeof(double));

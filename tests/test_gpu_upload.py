@@ -1,4 +1,4 @@
-"""The dataset upload: rows walked by several threads (sets above 40000 entries),
+"""The dataset upload: rows walked by several threads (sets above 250000 entries),
 the dense copy made on the device, rows that name a feature twice or out of
 order (the last entry stays), and the first bad row reported."""
 import ctypes as C
@@ -35,7 +35,7 @@ def _rows(n, d, seed):
     return out
 
 
-@pytest.mark.parametrize("n,d,nsv", [(1, 3, 2), (70, 9, 64), (6000, 41, 130)])
+@pytest.mark.parametrize("n,d,nsv", [(1, 3, 2), (70, 9, 64), (6000, 41, 130), (20000, 60, 33)])
 def test_predictions_from_uploaded_rows(n, d, nsv):
     lib = load()
     rng = np.random.default_rng(n)
@@ -61,7 +61,7 @@ def test_predictions_from_uploaded_rows(n, d, nsv):
 
 def test_the_first_bad_row_is_reported():
     lib = load()
-    rows = _rows(9000, 30, 3)
+    rows = _rows(24000, 60, 3)
     for k in (8000, 4321, 8999):
         rows[k] = ([1], [float("nan")])
     d = _set(rows)
