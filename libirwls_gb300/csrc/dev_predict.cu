@@ -1,7 +1,7 @@
 // dev_predict.cu -- batched prediction f(x_i) = bias + sum_j w_j k(x_i, sv_j)
-// (reference src/LIBIRWLS-predict.c:56-131): an ordered kernel row sum, so
-// every decision value accumulates its support vectors in the reference's
-// order; the sign is taken on the device.
+// (reference src/LIBIRWLS-predict.c:56-131): small batches as an ordered kernel
+// row sum in FP64, the support vectors in the reference's order; large ones from
+// the tensor cores (dev_predict_tc.cu). The sign is taken on the device.
 #include <algorithm>
 
 #include "dev_common.cuh"
@@ -92,17 +92,23 @@ extern "C" int irwls_predict_linear(const irwls_dev_set *T, int n, const irwls_d
     return 0;
 }
 
+// f_i of every row, or its sign: on the tensor cores where that path takes the
+// sizes and values (dev_predict_tc.cu), else as ordered FP64 row sums.
 extern "C" int irwls_predict_soft(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                                   double bias, int hard, double *d_out) {
     if (n <= 0) return 0;
-    fill_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n, bias);
-    IRWLS_LAUNCH_CHECK("fill");
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_PREDICT);
-    int rc = irwls_dev_kernel_rowsum(T, nullptr, n, S, nullptr, nSV, d_w, nullptr, nullptr, 0, +1, d_out, nullptr,
+    int rc = irwls_predict_exact(T, n, S, nSV, d_w, bias, hard, d_out);
+    const bool ordered = rc == 1;
+    if (ordered) {
+        fill_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n, bias);
+        IRWLS_LAUNCH_CHECK("fill");
+        rc = irwls_dev_kernel_rowsum(T, nullptr, n, S, nullptr, nSV, d_w, nullptr, nullptr, 0, +1, d_out, nullptr,
                                      d_out);
+    }
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_PREDICT);
     if (rc) return rc;
-    if (hard) {
+    if (hard && ordered) {
         sign_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n);
         IRWLS_LAUNCH_CHECK("sign");
     }

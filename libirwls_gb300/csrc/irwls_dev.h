@@ -278,6 +278,10 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
 /* ---- prediction (dev_predict.cu) ----------------------------------------- */
 int irwls_predict_soft(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                        double bias, int hard, double *d_out);
+/* the tensor-core form of irwls_predict_soft (dev_predict_tc.cu); 1: not for
+ * these sizes or values */
+int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
+                        double bias, int hard, double *d_out);
 size_t irwls_predict_linear_scratch(int width, int nsv);
 int irwls_predict_linear(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                          double bias, int hard, double *d_W, double *d_out);
