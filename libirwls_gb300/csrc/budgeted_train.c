@@ -153,8 +153,8 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
        multiply a change of rounding in K1 by 10^8 (20000 rows, 100 SGMA
        centroids: any other split of the same FP64 sums moves the weights by
        1e-9 to 1e-8), and the product is small enough there to keep its
-       order, about eight CTAs per SM over the lower tiles with at least 512
-       rows per chunk (20000 x 100: 0.8 ms). At 50000 x 300 it took 2.55 ms
+       order and its chunks, about eight per SM and 64 x 64 lower tile with at
+       least 512 rows each (20000 x 100: 0.27 ms). At 50000 x 300 it took 2.55 ms
        per iteration, three quarters of the training; the digits, with their
        slicing, take 0.20. */
     const int sms = 152;

@@ -559,64 +559,55 @@ __global__ void add_diag_kernel(double *KC, int m, double v) {
         KC[(size_t)i * m + i] = __dadd_rn(KC[(size_t)i * m + i], v);
 }
 
-// Partial Gram tiles. A' row p = [sd_p * KSC[act_p, :], day_p] (m + 1 values).
-// Tile (bi, bj), bi >= bj, of the lower triangle of A'^T A' restricted to
-// columns < m; chunk z of the active rows. part layout: [P][m+1 rows][m cols]
-// row-major by output row. Row chunks of TK are copied with cp.async into a
-// double buffer, then scaled in place (each thread scales the values it
-// copied) so that the products use fl(sd * KSC) as the reference does.
-constexpr int TT = 64, TK = 16;
-__global__ void __launch_bounds__(256) gram_kernel(const double *__restrict__ KSC, int m, const int *__restrict__ act,
-                                                   int nact, const double *__restrict__ sd,
-                                                   const double *__restrict__ day, int chunk,
-                                                   double *__restrict__ part) {
-    const int bj = blockIdx.x, bi = blockIdx.y, z = blockIdx.z;
-    if (bi < bj) return;
-    const int r0 = bi * TT, c0 = bj * TT;  // output rows (0..m), output cols (0..m-1)
+// Partial Gram of the FP64 form (fewer than 128 columns). A' row p =
+// [sd_p * KSC[act_p, :], day_p] (m + 1 values); chunk z of the active rows, the
+// lower part of A'^T A' restricted to columns < m. part layout:
+// [P][m+1 rows][m cols] row-major by output row. A thread keeps a micro-tile of
+// 4 rows by 2 columns of the lower triangle (tile t: row group R, the largest
+// with R (R + 1) <= t, column group t - R (R + 1)); CTA y of a chunk takes
+// blockDim.x tiles. Row chunks of TK are copied with cp.async into a double
+// buffer, then scaled in place (each thread scales the values it copied) so
+// that the products use fl(sd * KSC) as the reference does; every output adds
+// its products row by row.
+// Bound: the FP64 pipe. Micro-tiles instead of 64 x 64 tiles of the square leave
+// 5600 multiply-adds per row at m = 100 where those had 12288, and one scaling
+// per value and CTA: 20000 rows take 266 us, they took 790.
+constexpr int TK = 16, GW = 132;  // rows per copy, columns of the buffer
+constexpr int GT_MAX = 544;       // threads of a CTA at most
+__global__ void __launch_bounds__(GT_MAX) gram_kernel(const double *__restrict__ KSC, int m, const int *__restrict__ act,
+                                                      int nact, const double *__restrict__ sd,
+                                                      const double *__restrict__ day, int chunk,
+                                                      double *__restrict__ part) {
+    const int z = blockIdx.x;
     const int p0 = z * chunk, p1 = min(nact, p0 + chunk);
-    __shared__ __align__(16) double Ai[2][TK][TT + 1];
-    __shared__ __align__(16) double Aj[2][TK][TT + 1];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    double acc[4][4];
+    __shared__ __align__(16) double A[2][TK][GW];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int t = blockIdx.y * blockDim.x + threadIdx.x;
+    int R = (int)((sqrtf(4.f * t + 1.f) - 1.f) * 0.5f);
+    while (R * (R + 1) > t) --R;
+    while ((R + 1) * (R + 2) <= t) ++R;
+    const int r0 = 4 * R, c0 = 2 * (t - R * (R + 1));  // c0 <= r0 + 2
+    const bool live = r0 <= m && c0 < m;
+    const int ra = live ? r0 : 0, ca = live ? c0 : 0;
+    const int wp = (m + 4) & ~3;  // columns copied: 0 ... m, zeros behind
+    double acc[4][2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+    for (int a = 0; a < 4; ++a) acc[a][0] = acc[a][1] = 0.0;
     auto load = [&](int buf, int p) {
-        for (int t = tid; t < TK * TT; t += 256) {
-            const int kk = t / TT, cc = t % TT;
+        for (int kk = warp; kk < TK; kk += nw) {
             const int pp = p + kk;
-            const int ci = r0 + cc, cj = c0 + cc;
-            const double *si = KSC, *sj = KSC;
-            int ni = 0, nj = 0;
-            if (pp < p1) {
-                const double *row = KSC + (size_t)act[pp] * m;
-                if (ci < m) {
-                    si = row + ci;
-                    ni = 8;
-                } else if (ci == m) {
-                    si = day + pp;
-                    ni = 8;
-                }
-                if (cj < m) {
-                    sj = row + cj;
-                    nj = 8;
-                }
+            const double *row = pp < p1 ? KSC + (size_t)act[pp] * m : KSC;
+            for (int c = lane; c < wp; c += 32) {
+                const bool k = pp < p1 && c < m, d = pp < p1 && c == m;
+                cp_async8(&A[buf][kk][c], k ? row + c : d ? day + pp : KSC, k || d ? 8 : 0);
             }
-            cp_async8(&Ai[buf][kk][cc], si, ni);
-            cp_async8(&Aj[buf][kk][cc], sj, nj);
         }
         cp_async_commit();
     };
     auto scale = [&](int buf, int p) {
-        for (int t = tid; t < TK * TT; t += 256) {
-            const int kk = t / TT, cc = t % TT;
-            const int pp = p + kk;
-            if (pp < p1) {
-                const double sc = sd[pp];
-                if (r0 + cc < m) Ai[buf][kk][cc] = __dmul_rn(sc, Ai[buf][kk][cc]);
-                if (c0 + cc < m) Aj[buf][kk][cc] = __dmul_rn(sc, Aj[buf][kk][cc]);
-            }
+        for (int kk = warp; kk < TK && p + kk < p1; kk += nw) {
+            const double sc = sd[p + kk];
+            for (int c = lane; c < m; c += 32) A[buf][kk][c] = __dmul_rn(sc, A[buf][kk][c]);
         }
     };
     if (p0 < p1) load(0, p0);
@@ -631,28 +622,28 @@ __global__ void __launch_bounds__(256) gram_kernel(const double *__restrict__ KS
         }
         scale(buf, p);
         __syncthreads();
-#pragma unroll
+#pragma unroll 4
         for (int kk = 0; kk < TK; ++kk) {
-            double ai[4], aj[4];
+            const double2 x = *(const double2 *)&A[buf][kk][ra], y = *(const double2 *)&A[buf][kk][ra + 2];
+            const double2 b = *(const double2 *)&A[buf][kk][ca];
+            const double ai[4] = {x.x, x.y, y.x, y.y};
 #pragma unroll
-            for (int a = 0; a < 4; ++a) ai[a] = Ai[buf][kk][ty + 16 * a];
-#pragma unroll
-            for (int b = 0; b < 4; ++b) aj[b] = Aj[buf][kk][tx + 16 * b];
-#pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] = fma(ai[a], aj[b], acc[a][b]);
+            for (int a = 0; a < 4; ++a) {
+                acc[a][0] = fma(ai[a], b.x, acc[a][0]);
+                acc[a][1] = fma(ai[a], b.y, acc[a][1]);
+            }
         }
         __syncthreads();
     }
+    if (!live) return;
     double *out = part + (size_t)z * (m + 1) * m;
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
-        const int r = r0 + ty + 16 * a;
+        const int r = r0 + a;
         if (r > m) continue;
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int c = c0 + tx + 16 * b;
+        for (int b = 0; b < 2; ++b) {
+            const int c = c0 + b;
             if (c < m && c <= r) out[(size_t)r * m + c] = acc[a][b];
         }
     }
@@ -998,12 +989,28 @@ extern "C" int irwls_par_gram_reduce(const double *d_part, int P, int m, const d
 extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
                                    const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part,
                                    int P) {
-    const int T = ceil_div(m + 1, TT);
-    const int Tc = ceil_div(m, TT);
+    if (m > 127) {
+        irwls_set_error(-5, "the FP64 Gram takes fewer than 128 columns");
+        return -5;
+    }
     const int chunk = nact > 0 ? ceil_div(nact, P) : 1;
-    dim3 grid(Tc, T, P);
+    // micro-tiles of the lower triangle, in warps; CTAs per chunk so that the
+    // busiest SM has the least to do (8 multiply-adds per warp and row, and the
+    // chunk's scaling in each of its CTAs)
+    const int R = ceil_div(m + 1, 4), W = ceil_div(R * (R + 1), 32);
+    const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
+    int ns = ceil_div(W, GT_MAX / 32), best = 1 << 30;
+    for (int s = ns; s <= W; ++s) {
+        const int load = ceil_div((long long)P * s, sms) * (8 * ceil_div(W, s) + ceil_div(m, 32));
+        if (load < best) {
+            best = load;
+            ns = s;
+        }
+    }
+    const int wpc = ceil_div(W, ns);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
-    gram_kernel<<<grid, 256, 0, irwls_stream()>>>(d_KSC, m, d_act, nact, d_sd, d_day, chunk, d_part);
+    gram_kernel<<<dim3(P, ceil_div(W, wpc)), 32 * wpc, 0, irwls_stream()>>>(d_KSC, m, d_act, nact, d_sd, d_day, chunk,
+                                                                          d_part);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
     IRWLS_LAUNCH_CHECK("gram");
     const long long total = (long long)(m + 1) * m;
