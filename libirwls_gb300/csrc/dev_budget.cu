@@ -665,41 +665,53 @@ __global__ void gram_reduce_kernel(const double *__restrict__ part, int P, int m
     }
 }
 
-// e = y - KSC beta, then Da (src/budgeted-train.c:431-457). A warp per row,
-// two rows in flight (their loads interleaved); per row each lane's terms in
-// increasing j, then a butterfly over the lanes.
-__global__ void residual_kernel(const double *__restrict__ KSC, int l, int m, const double *__restrict__ beta,
-                                const double *__restrict__ y, double C, double M, double *__restrict__ e,
-                                double *__restrict__ Da) {
+// e = y - KSC beta, then Da (src/budgeted-train.c:431-457). A warp takes RROWS
+// consecutive rows (their loads in flight together); per row each lane's terms
+// in increasing j, then the pairwise tree over the lanes (16 apart, 8 apart,
+// ...). Halves of the warp reduce different rows: the same sums as a butterfly
+// per row, in 9 instead of 40 FP64 instructions for 8 rows, and the weights'
+// division runs once for the 8 rows. The FP64 pipe bounds it (an instruction
+// costs it the same with one lane active as with 32): 50000 x 300 takes 47 us,
+// a butterfly per row and a division per two rows took 80.
+constexpr int RROWS = 8;
+__global__ void __launch_bounds__(256) residual_kernel(const double *__restrict__ KSC, int l, int m,
+                                                       const double *__restrict__ beta, const double *__restrict__ y,
+                                                       double C, double M, double *__restrict__ e,
+                                                       double *__restrict__ Da) {
     const int lane = threadIdx.x & 31;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int i0 = warp; i0 < l; i0 += 2 * nw) {
-        const int i1 = i0 + nw;
-        const bool two = i1 < l;
-        const double *r0 = KSC + (size_t)i0 * m, *r1 = KSC + (size_t)(two ? i1 : i0) * m;
-        double a0 = 0.0, a1 = 0.0;
-        int j = lane;
-        for (; j + 32 < m; j += 64) {
-            const double b0 = beta[j], b1 = beta[j + 32];
-            const double x0 = r0[j], x1 = r1[j], y0 = r0[j + 32], y1 = r1[j + 32];
-            a0 = fma(x0, b0, a0);
-            a1 = fma(x1, b0, a1);
-            a0 = fma(y0, b1, a0);
-            a1 = fma(y1, b1, a1);
+    for (int i0 = RROWS * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i0 < l; i0 += RROWS * nw) {
+        const double *r[RROWS];
+        double a[RROWS];
+#pragma unroll
+        for (int k = 0; k < RROWS; ++k) {
+            r[k] = KSC + (size_t)min(i0 + k, l - 1) * m;
+            a[k] = 0.0;
         }
-        if (j < m) {
-            const double b0 = beta[j];
-            a0 = fma(r0[j], b0, a0);
-            a1 = fma(r1[j], b0, a1);
+#pragma unroll 2
+        for (int j = lane; j < m; j += 32) {
+            const double b = beta[j];
+            double x[RROWS];
+#pragma unroll
+            for (int k = 0; k < RROWS; ++k) x[k] = r[k][j];
+#pragma unroll
+            for (int k = 0; k < RROWS; ++k) a[k] = fma(x[k], b, a[k]);
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 += __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+        // lane bits 4, 3, 2 choose the row kept at each level
+#pragma unroll
+        for (int o = 16, h = RROWS / 2; h > 0; o >>= 1, h >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int k = 0; k < RROWS / 2; ++k)
+                if (k < h) {
+                    const double mine = up ? a[k + h] : a[k], other = up ? a[k] : a[k + h];
+                    a[k] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+                }
         }
-        if (lane < 2 && (lane == 0 || two)) {
-            const int i = lane == 0 ? i0 : i1;
-            const double acc = lane == 0 ? a0 : a1;
+        double acc = a[0] + __shfl_xor_sync(0xffffffffu, a[0], 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+        const int i = i0 + ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);
+        if ((lane & 3) == 0 && i < l) {
             const double yi = y[i];
             const double ei = yi - acc;
             e[i] = ei;
@@ -1022,7 +1034,7 @@ extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act,
 
 extern "C" int irwls_par_residual(const double *d_KSC, int l, int m, const double *d_beta, const double *d_y, double C,
                                   double M, double *d_e, double *d_Da) {
-    const int blocks = std::min(ceil_div(l, 8), 8 * (irwls_num_sms() > 0 ? irwls_num_sms() : 148));
+    const int blocks = std::min(ceil_div(l, 8 * RROWS), 8 * (irwls_num_sms() > 0 ? irwls_num_sms() : 148));
     residual_kernel<<<blocks, 256, 0, irwls_stream()>>>(d_KSC, l, m, d_beta, d_y, C, M, d_e, d_Da);
     IRWLS_LAUNCH_CHECK("residual");
     return 0;
