@@ -1,6 +1,6 @@
 // blocked_bf16.cuh -- blocked bf16 layout of the precision form's SGMA
 // operands, shared by the kernels that write them (dev_budget.cu: W;
-// dev_tc.cu: Q) and the tcgen05 score kernel that streams them.
+// dev_tc.cu: Q; dev_sgma_ahead.cu: both) and the tcgen05 score kernel that streams them.
 #pragma once
 #include <stddef.h>
 
@@ -39,4 +39,13 @@ __device__ __forceinline__ void bf16_pieces3(float x, __nv_bfloat16 p[3]) {
 // x from its pieces (exact).
 __device__ __forceinline__ float bf16_join3(__nv_bfloat16 h, __nv_bfloat16 m, __nv_bfloat16 l) {
     return (__bfloat162float(h) + __bfloat162float(m)) + __bfloat162float(l);
+}
+
+// Q's column s written as its three pieces, and |Q_i|^2 updated.
+__device__ __forceinline__ void put_q(int row, int s, float q, __nv_bfloat16 *Qb, int kbn, float *qn) {
+    if (qn) qn[row] = fmaf(q, q, qn[row]);  // |Q_i|^2: the Nystrom residual of row i is k_ii - qn[i]
+    __nv_bfloat16 pc[3];
+    bf16_pieces3(q, pc);
+#pragma unroll
+    for (int k = 0; k < QB_NP; ++k) Qb[qb_index(row, s, kbn, k)] = pc[k];
 }

@@ -542,6 +542,7 @@ __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__re
     __shared__ float dl[64];
     const int c = threadIdx.x & 63, g = threadIdx.x >> 6;
     float sum = 0.f, comp = 0.f;
+#pragma unroll 8
     for (int b = g; b < nblk; b += 16) {
         const float y = __fsub_rn(part[(size_t)b * 64 + c], comp);
         const float t = __fadd_rn(sum, y);
@@ -563,23 +564,42 @@ __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__re
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double val = sc[0];
-        int bb = 0;
-        for (int i = 1; i < 64; ++i)
-            if (sc[i] > val) {
-                val = sc[i];
-                bb = i;
+    if (threadIdx.x < 32) {
+        // the largest score, the first of equals; scores are sums of squares over
+        // a positive eta, or 0, so their bits order them; a NaN loses to all but wins
+        // in the first place, as sc[i] > sc[0] has it
+        const int i = threadIdx.x;
+        auto key = [&](int k) {
+            const long long b = __double_as_longlong(sc[k]);
+            return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL ? (k == 0 ? 0x7fffffffffffffffLL : -1LL) : b;
+        };
+        long long v = key(i), w = key(i + 32);
+        int bb = i;
+        if (w > v) {
+            v = w;
+            bb = i + 32;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int ob = __shfl_xor_sync(0xffffffffu, bb, o);
+            if (ov > v || (ov == v && ob < bb)) {
+                v = ov;
+                bb = ob;
             }
-        cent[s] = cand[bb];
-        best[0] = bb;
-        bestval[s] = val;
+        }
+        const int cb = cand[bb];
+        if (i == 0) {
+            cent[s] = cb;
+            best[0] = bb;
+            bestval[s] = sc[bb];
+        }
         if (eps) {
-            const float low = (float)val * (1.f - dl[bb]);
-            int ask = !(low > 0.f);
-            for (int i = 0; i < 64; ++i)
-                if (i != bb && cand[i] != cand[bb] && !((float)sc[i] * (1.f + dl[i]) < low)) ask = 1;
-            need[0] = ask;
+            const float low = (float)sc[bb] * (1.f - dl[bb]);
+            bool ask = !(low > 0.f);
+            for (int k = i; k < 64; k += 32)
+                ask |= k != bb && cand[k] != cb && !((float)sc[k] * (1.f + dl[k]) < low);
+            ask = __any_sync(0xffffffffu, ask);
+            if (i == 0) need[0] = ask;
         }
     }
 }
@@ -981,15 +1001,6 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
 }
 
-// Q's column s written as its three pieces, and |Q_i|^2 updated.
-__device__ __forceinline__ void put_q(int row, int s, float q, __nv_bfloat16 *Qb, int ldq, float *qn) {
-    if (qn) qn[row] = fmaf(q, q, qn[row]);  // |Q_i|^2: the Nystrom residual of row i is k_ii - qn[i]
-    __nv_bfloat16 pc[3];
-    bf16_pieces3(q, pc);
-#pragma unroll
-    for (int k = 0; k < QB_NP; ++k) Qb[qb_index(row, s, ldq >> 5, k)] = pc[k];
-}
-
 // Column s of Q from the score step's residuals r = Q w - k of the winning
 // candidate (slot best[0]; the residuals of candidate c at resid + c * l):
 // q_i = -r_i / L3. lrow[s] holds 1 / L3.
@@ -1001,7 +1012,7 @@ __global__ void q_column_resid_kernel(int l, const float *__restrict__ resid, co
     const int c = best[0];
     const float inv_l3 = lrow[s];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < l; i += gridDim.x * blockDim.x)
-        put_q(i, s, -resid[(size_t)c * l + i] * inv_l3, Qb, ldq, qn);
+        put_q(i, s, -resid[(size_t)c * l + i] * inv_l3, Qb, ldq >> 5, qn);
 }
 
 // Column s of Q directly, q_i = (k(x_i, c_s) - sum_{t<s} Q_it l2_t) / L3,
@@ -1036,7 +1047,7 @@ __global__ void __launch_bounds__(256) q_column_direct_kernel(KViewF X, int l, c
             for (int p = X.rp[i]; p < X.rp[i + 1]; ++p) kd = fmaf(X.cv[p], sc[X.ci[p]], kd);
             kv = X.mode == IRWLS_K_LINEAR ? kd : __expf(X.ng * fmaxf(qa + X.q[i] - 2.f * kd, 0.f));
         }
-        put_q(i, s, (kv - dot) * inv_l3, Qb, ldq, qn);
+        put_q(i, s, (kv - dot) * inv_l3, Qb, ldq >> 5, qn);
     }
 }
 

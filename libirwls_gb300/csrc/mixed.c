@@ -34,6 +34,13 @@ int irwls_sgma_cand_inv(const irwls_dev_set *X, const int *d_cand, const int *d_
                         double *d_eta, const void *Qb, unsigned *d_eps);
 int irwls_sgma_linv_update(const double *d_L, int ldL, double *d_Linv, int ldi, int s, double *d_lpart,
                            float *d_lrow);
+size_t irwls_sgma_ahead_bytes(int m, int ldq);
+const void *irwls_sgma_ahead_image(const void *ws, int m, int ldq, int s);
+int irwls_sgma_ahead_init(const irwls_dev_set *X, const int *d_cand, int m, int ldq, void *ws);
+int irwls_sgma_ahead_lrow(const double *d_L, int ldL, int s, float *d_lrow);
+int irwls_sgma_ahead_step(const irwls_dev_set *X, int l, const int *d_cand, const int *d_cent, const int *d_best, int s,
+                          int m, int ldq, double *d_L, void *ws, void *Qb, float *d_qn, const float *d_rq,
+                          double *d_eta, unsigned *d_eps);
 size_t irwls_sgma_wpart_count(int m);
 size_t irwls_sgma_lpart_count(int m);
 int irwls_sgma_tc_select(const float *d_part, int nblk, const double *d_eta, const int *d_cand, int s, int *d_cent,
@@ -128,7 +135,7 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     float *d_rq = NULL, *lrow = NULL, *d_qn = NULL, *d_F = NULL, *d_pred = NULL, *d_tfeat = NULL, *d_tscore = NULL;
     int *d_probe = NULL, *d_pool = NULL;
     double *d_resid = NULL;
-    void *Qb = NULL, *Wb = NULL;
+    void *Qb = NULL, *Wb = NULL, *ahead = NULL;
     /* proposals and traces need the RBF kernel's k(x, x) = 1 */
     const int learn = !screen && g_proposer != NULL && X->mode != IRWLS_K_LINEAR && m > 2;
     const int trace = !screen && g_trace_feat != NULL && m > 2;
@@ -139,6 +146,14 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     if (!F) {
         free(cand);
         return -1;
+    }
+    /* the candidates' rows ahead of their steps (dev_sgma_ahead.cu), where the
+       candidates are known then and the workspace (64 m (8 m + 6 ldq) bytes) is
+       at most 4 GB, m about 2100, and can be had; else the explicit inverse */
+    if (!learn && irwls_sgma_ahead_bytes(m, ldq) <= (size_t)4 << 30 &&
+        irwls_dev_malloc(&ahead, irwls_sgma_ahead_bytes(m, ldq))) {
+        irwls_clear_error();
+        ahead = NULL;
     }
     rc |= irwls_dev_malloc((void **)&d_cand, (size_t)m * 64 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_cent, (size_t)m * sizeof(int));
@@ -152,11 +167,13 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     rc |= irwls_dev_malloc((void **)&d_rq, (size_t)l * 64 * sizeof(float));
     const size_t qb_bytes = (size_t)nblk * 128 * ldq * 6; /* whole 128-row tiles, three pieces */
     rc |= irwls_dev_malloc(&Qb, qb_bytes);
-    rc |= irwls_dev_malloc(&Wb, (size_t)64 * ldq * 6);
+    if (!ahead) rc |= irwls_dev_malloc(&Wb, (size_t)64 * ldq * 6);
     rc |= irwls_dev_malloc((void **)&lrow, (size_t)(m + 1) * sizeof(float));
-    rc |= irwls_dev_malloc((void **)&d_Linv, (size_t)m * ldL * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_wpart, irwls_sgma_wpart_count(m) * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_lpart, irwls_sgma_lpart_count(m) * sizeof(double));
+    if (!ahead) {
+        rc |= irwls_dev_malloc((void **)&d_Linv, (size_t)m * ldL * sizeof(double));
+        rc |= irwls_dev_malloc((void **)&d_wpart, irwls_sgma_wpart_count(m) * sizeof(double));
+        rc |= irwls_dev_malloc((void **)&d_lpart, irwls_sgma_lpart_count(m) * sizeof(double));
+    }
     rc |= irwls_dev_malloc((void **)&d_qn, (size_t)(l + 2) * sizeof(float));
     rc |= irwls_dev_malloc((void **)&d_resid, sizeof(double));
     if (screen) {
@@ -183,7 +200,8 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
         rc |= irwls_dev_h2d(d_cand, cand, (size_t)m * 64 * sizeof(int));
         rc |= irwls_dev_h2d(d_cent, first, (m > 1 ? 2 : 1) * sizeof(int));
         rc |= irwls_dev_memset(d_L, 0, (size_t)m * ldL * sizeof(double));
-        rc |= irwls_dev_memset(d_Linv, 0, (size_t)m * ldL * sizeof(double));
+        if (ahead) rc |= irwls_sgma_ahead_init(X, d_cand, m, ldq, ahead);
+        else rc |= irwls_dev_memset(d_Linv, 0, (size_t)m * ldL * sizeof(double));
         rc |= irwls_dev_memset(d_W, 0, (size_t)64 * ldz * sizeof(double));
         rc |= irwls_dev_memset(Qb, 0, qb_bytes);
         rc |= irwls_dev_memset(d_qn, 0, (size_t)(l + 2) * sizeof(float));
@@ -210,8 +228,12 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
         /* centroids 0 and 1 are the class means (src/budgeted-train.c:127-147) */
         for (int s = 0; s < 2 && s < m && !rc; s++) {
             rc |= irwls_sgma_factor(X, s, d_cent, d_best, d_W, ldz, d_L, ldL);
-            rc |= irwls_sgma_linv_update(d_L, ldL, d_Linv, ldL, s, d_lpart, lrow);
+            if (ahead) rc |= irwls_sgma_ahead_lrow(d_L, ldL, s, lrow);
+            else rc |= irwls_sgma_linv_update(d_L, ldL, d_Linv, ldL, s, d_lpart, lrow);
             rc |= irwls_q_column(X, F, l, d_cent, s, lrow, Qb, ldq, d_qn);
+            if (ahead)
+                rc |= irwls_sgma_ahead_step(X, l, d_cand, d_cent, NULL, s, m, ldq, d_L, ahead, Qb, NULL, NULL, d_eta,
+                                            d_eps);
         }
         const float *X32 = NULL, *q32 = NULL;
         irwls_f32_mirror_view(F, &X32, &q32);
@@ -229,9 +251,11 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
             if (trace)
                 rc |= irwls_learn_features(X32, X->ld, X->width, raw, q32, (float)X->neg_gamma, X->y, cs, NCAND,
                                            d_probe, NPROBE, d_qn, d_tfeat + (size_t)(s - 2) * NCAND * nf);
-            rc |= irwls_sgma_cand_inv(X, cs, d_cent, s, d_Linv, ldL, d_KN, ldz, d_wpart, m, d_W, Wb, ldq, d_eta, Qb,
-                                      d_eps);
-            rc |= irwls_sgma_tc_score(X, F, l, cs, Qb, ldq, Wb, s, d_part, d_rq);
+            if (!ahead)
+                rc |= irwls_sgma_cand_inv(X, cs, d_cent, s, d_Linv, ldL, d_KN, ldz, d_wpart, m, d_W, Wb, ldq, d_eta,
+                                          Qb, d_eps);
+            rc |= irwls_sgma_tc_score(X, F, l, cs, Qb, ldq, ahead ? irwls_sgma_ahead_image(ahead, m, ldq, s) : Wb, s,
+                                      d_part, d_rq);
             irwls_prof_begin(IRWLS_PROF_SGMA_UPDATE);
             rc |= irwls_sgma_tc_select(d_part, nblk, d_eta, cs, s, d_cent, d_best, d_val,
                                        trace ? d_tscore + (size_t)(s - 2) * NCAND : NULL, d_eps, l, d_need);
@@ -240,9 +264,14 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
                 rc |= irwls_sgma_rescore(X, l, cs, d_cent, s, d_L, ldL, d_KSC, d_W, d_Z, d_KN, ldz, d_eta, d_part64,
                                          d_best, d_val, d_need, d_need + 1);
             }
-            rc |= irwls_sgma_factor(X, s, d_cent, d_best, d_W, ldz, d_L, ldL);
-            rc |= irwls_sgma_linv_update(d_L, ldL, d_Linv, ldL, s, d_lpart, lrow);
-            rc |= irwls_q_column_resid(l, d_rq, d_best, s, lrow, Qb, ldq, d_qn);
+            if (ahead) {
+                rc |= irwls_sgma_ahead_step(X, l, d_cand, d_cent, d_best, s, m, ldq, d_L, ahead, Qb, d_qn, d_rq, d_eta,
+                                            d_eps);
+            } else {
+                rc |= irwls_sgma_factor(X, s, d_cent, d_best, d_W, ldz, d_L, ldL);
+                rc |= irwls_sgma_linv_update(d_L, ldL, d_Linv, ldL, s, d_lpart, lrow);
+                rc |= irwls_q_column_resid(l, d_rq, d_best, s, lrow, Qb, ldq, d_qn);
+            }
             irwls_prof_end(IRWLS_PROF_SGMA_UPDATE);
         }
         /* Nystrom residual trace(K - K_nm K_mm^-1 K_mn) = sum_i (k_ii - |Q_i|^2) */
@@ -279,7 +308,7 @@ done:
     {
         void *bufs[] = {d_cand, d_cent, d_best, d_L, d_W, d_KN, d_eta, d_part, d_val, d_rq, Qb, Wb, lrow,
                         d_Linv, d_wpart, d_lpart, d_qn, d_resid, d_probe, d_F, d_pool, d_pred, d_tfeat, d_tscore,
-                        d_KSC, d_Z, d_part64, d_need};
+                        d_KSC, d_Z, d_part64, d_need, ahead};
         for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
         irwls_f32_mirror_free(F);
     }
