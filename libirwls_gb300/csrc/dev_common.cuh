@@ -21,8 +21,10 @@ int irwls_num_sms();
 // Chained launches (programmatic dependent launch): a kernel launched with
 // launch_chained may be scheduled while the kernel before it on the stream
 // is finishing, and starts with chain_wait(), which returns once that kernel
-// has completed and its writes are visible; nothing before chain_wait() may
-// touch global memory. chain_open() lets the next chained kernel be scheduled.
+// has completed and its writes are visible. Every chained kernel calls
+// chain_open() after its chain_wait(), so before chain_wait() a kernel may read
+// what was complete before the kernel before it, and touch nothing else in
+// global memory. chain_open() lets the next chained kernel be scheduled.
 // Outside a chained launch both are no-ops.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }

@@ -15,6 +15,7 @@
 // later candidates' w (64 s (m - s) doubles per step) where that read L^-1.
 #include <cuda_bf16.h>
 #include <math.h>
+#include <stdint.h>
 
 #include <algorithm>
 
@@ -25,6 +26,7 @@ namespace {
 
 constexpr int NCAND = 64;
 constexpr int SG = 8;  // warps of a CTA: they split the sums over t and over the features
+constexpr int WP = 128;  // rows of W copied to shared memory before the choice is known
 
 struct AheadArgs {
     KView X;
@@ -98,15 +100,30 @@ __global__ void ahead_lrow_kernel(const double *__restrict__ L, int ldL, int s, 
 // CTA b < ncta: 32 candidates of the later steps, a lane each; warp g adds every
 // SG-th term of the sum over t and its share of the kernel value's features. The
 // others: Q's column s, q_i = -r_i / L_ss from the residuals of the chosen candidate.
-// Latency bounds it (the chosen candidate's row, the sums, one exponential).
+// Latency bounds it (the chosen candidate's row, the sums, one exponential), so what
+// does not depend on the choice -- W up to row s - 1, written by the kernel of step
+// s - 1, three launches back -- is fetched while the selection runs.
 __global__ void __launch_bounds__(32 * SG) sgma_ahead_kernel(AheadArgs p) {
-    chain_wait();
-    chain_open();
-    extern __shared__ double l2[];  // row s of L
-    __shared__ double piv[2];       // L_ss, its reciprocal
+    extern __shared__ __align__(16) double wbuf[];  // WP rows of W at most, then row s of L
+    __shared__ double piv[2];                       // L_ss, its reciprocal
     __shared__ double red[2][SG][33];
     const int s = p.s, lane = threadIdx.x & 31, g = threadIdx.x >> 5;
     const size_t nc = (size_t)NCAND * p.m;
+    const int sp = min(s, WP);
+    double *l2 = wbuf + 32 * sp;
+    const size_t j0 = (size_t)NCAND * max(2, s + 1) + 32 * blockIdx.x;
+    if ((int)blockIdx.x < p.ncta) {
+        for (int t = threadIdx.x; t < 16 * sp; t += blockDim.x)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(wbuf + 2 * t)),
+                         "l"(p.W + (t >> 4) * nc + j0 + 2 * (t & 15)));
+        for (int t = WP + g; t < s; t += SG)
+            if (lane < 2) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.W + t * nc + j0 + 16 * lane));
+        if (p.X.ld <= 128)
+            for (int k = 16 * g; k < p.X.ld; k += 16 * SG)
+                asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p.X.X + (size_t)p.cand[j0 + lane] * p.X.ld + k));
+    }
+    chain_wait();
+    chain_open();
     const bool chosen = p.best != nullptr;
     const int bb = chosen ? p.best[0] : 0, gc = p.cent[s];
     const size_t jb = (size_t)NCAND * s + bb;
@@ -132,12 +149,18 @@ __global__ void __launch_bounds__(32 * SG) sgma_ahead_kernel(AheadArgs p) {
     }
     for (int t = threadIdx.x; t < s; t += blockDim.x)
         l2[t] = chosen ? p.W[t * nc + jb] : p.L[(size_t)s * p.m + t];
-    const size_t j = (size_t)NCAND * max(2, s + 1) + 32 * blockIdx.x + lane;  // < nc: ncta covers 64 each
+    const size_t j = j0 + lane;  // < nc: ncta covers 64 each
     const int gj = p.cand[j];
     const double kp = part_kernel(p.X, p.X.X + (size_t)gj * p.X.ld, gc, g);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     double a0 = 0.0, a1 = 0.0;
     int t = g;
+    for (; t + SG < sp; t += 2 * SG) {
+        a0 = fma(l2[t], wbuf[32 * t + lane], a0);
+        a1 = fma(l2[t + SG], wbuf[32 * (t + SG) + lane], a1);
+    }
+    for (; t < sp; t += SG) a0 = fma(l2[t], wbuf[32 * t + lane], a0);
     for (; t + 7 * SG < s; t += 8 * SG) {
         double w[8];
 #pragma unroll
@@ -252,7 +275,7 @@ extern "C" int irwls_sgma_ahead_step(const irwls_dev_set *X, int l, const int *d
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
     const int nq = d_best ? std::max(1, std::min(ceil_div(l, 256), 4 * sms)) : 0;
     if (a.ncta + nq == 0) return 0;
-    const size_t smem = (size_t)std::max(1, s) * sizeof(double);
+    const size_t smem = ((size_t)32 * std::min(s, WP) + std::max(1, s)) * sizeof(double);
     if (smem > 40 * 1024) allow_smem(sgma_ahead_kernel);
     launch_chained(sgma_ahead_kernel, dim3(a.ncta + nq), dim3(32 * SG), smem, a);
     IRWLS_LAUNCH_CHECK("sgma_ahead");

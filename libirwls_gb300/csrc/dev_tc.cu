@@ -639,7 +639,7 @@ __device__ __forceinline__ void cp_async4(uint32_t saddr, const void *gmem) {
 // stride (conflict-free row-per-lane reads); kind 0: too large for the
 // buffer, entries read from global memory.
 struct TileRows {
-    int kind, lds;
+    int kind, lds, p0;  // p0: the slice's first entry
     const int *rp;
     const float *q;
     const int *ci;
@@ -648,12 +648,17 @@ struct TileRows {
 };
 
 // Issues the staging copies of rows m0 ... m0 + nr - 1 (threads et = 0 ... 255
-// of the epilogue); the caller waits for them (cp.async.wait_all + barrier).
-__device__ __forceinline__ TileRows stage_tile_rows(const KViewF &X, int m0, int nr, unsigned char *buf, int buf_bytes,
+// of the epilogue), entries p0 ... p1 - 1; the caller waits for them
+// (cp.async.wait_all + barrier) and has read p0 and p1 a tile earlier, so that
+// nothing here waits for memory: with the row pointers and norms loaded through
+// registers a tile stood still for three trips to L2.
+__device__ __forceinline__ TileRows stage_tile_rows(const KViewF &X, int m0, int nr, int p0, int p1,
+                                                    unsigned char *buf, int buf_bytes,
                                                     int *srp, float *sq, int et, int nthr) {
     TileRows t;
     t.kind = 0;
     t.lds = 0;
+    t.p0 = p0;
     t.rp = srp;
     t.q = sq;
     if (X.mode == IRWLS_K_RAW_RBF) {
@@ -671,15 +676,14 @@ __device__ __forceinline__ TileRows stage_tile_rows(const KViewF &X, int m0, int
         }
         return t;
     }
-    const int p0 = X.rp[m0], p1 = X.rp[m0 + nr];
     const int nnz = p1 - p0;
     int *ci = (int *)buf;
     float *cv = (float *)(buf + (buf_bytes / 8) * 4);
     t.ci = ci;
     t.cv = cv;
-    for (int k = et; k <= nr; k += nthr) srp[k] = X.rp[m0 + k] - p0;
+    for (int k = et; k <= nr; k += nthr) cp_async4(smem_u32(srp + k), X.rp + m0 + k);
     if (X.mode == IRWLS_K_NORM_RBF)
-        for (int k = et; k < nr; k += nthr) sq[k] = X.q[m0 + k];
+        for (int k = et; k < nr; k += nthr) cp_async4(smem_u32(sq + k), X.q + m0 + k);
     if (nnz <= buf_bytes / 8) {
         t.kind = 1;
         for (int k = et; k < nnz; k += nthr) {
@@ -731,8 +735,8 @@ __device__ __forceinline__ void kentry32_tile(const KViewF &B, const TileRows &T
     if (T.kind == 1) {
         ci = T.ci;
         cv = T.cv;
-        p0 = T.rp[r];
-        p1 = T.rp[r + 1];
+        p0 = T.rp[r] - T.p0;
+        p1 = T.rp[r + 1] - T.p0;
         qb = B.mode == IRWLS_K_NORM_RBF ? T.q[r] : 0.f;
     } else {
         ci = B.ci;
@@ -808,14 +812,18 @@ __device__ __forceinline__ void score_mma_stage(unsigned char *sb, uint32_t tmem
 }
 
 // EG epilogue groups of four warps (warps 4 ... 4 EG + 3), each scoring 64 / EG
-// of the candidates for all 128 rows of a tile.
+// of the candidates for all 128 rows of a tile. early: all but the last stage of W
+// and Q were complete before the kernel before this one; the first tile's other
+// stages are loaded while that one ends (X and the candidates always are).
 template <int NS, int EG>
 __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
     KViewF X, int l, const int *__restrict__ cand, const __nv_bfloat16 *__restrict__ Qb, int kbn,
     const __nv_bfloat16 *__restrict__ Wb, int kst, float *__restrict__ part, float *__restrict__ resid, int xs_bytes,
-    int *flags) {
-    chain_wait();
-    chain_open();
+    int early, int *flags) {
+    if (!early) {
+        chain_wait();
+        chain_open();
+    }
     using S = TcRing<64, QB_NP, WS_BK>;
     static_assert(S::A_BYTES == 2 * QB_PIECE && S::B_BYTES == 2 * WB_PIECE, "blocked pieces are stage images");
     extern __shared__ __align__(1024) unsigned char tc_smem[];
@@ -869,10 +877,15 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
         if (lane == 0) {
             const uint32_t base = smem_u32(smem);
             int issued = 0;
+            bool waited = !early;
             for (int j = 0; j < my_tiles && !abort_flag; ++j) {
                 const size_t tile = (size_t)blockIdx.x + (size_t)j * gridDim.x;
                 for (int k = 0; k < kst; ++k) {
                     const int u = j * kst + k, slot = u % NS;
+                    if (!waited && k == kst - 1) {
+                        chain_wait();
+                        waited = true;
+                    }
                     if (u >= NS && !mbar_wait(smem_u32(&empty[slot]), (uint32_t)(u / NS - 1) & 1u)) abort_flag = 1;
                     if (abort_flag) break;
                     const uint32_t sb = base + slot * S::BYTES, fb = smem_u32(&full[slot]);
@@ -883,6 +896,7 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
                     issued = u + 1;
                 }
             }
+            if (!waited) chain_wait();
             // no copy is left in flight: the last NS stages issued have landed
             for (int u = issued > NS ? issued - NS : 0; u < issued; ++u)
                 if (!mbar_wait(smem_u32(&full[u % NS]), (uint32_t)(u / NS) & 1u)) abort_flag = 1;
@@ -918,13 +932,23 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
         const int ew = warp & 3, g = (warp - 4) >> 2;
         const int et = threadIdx.x - 128;
         // the rows of tile j + 1 are copied in while tile j is scored
-        auto stage = [&](int jt) {
+        auto entries = [&](int jt) {
             const int m0 = ((int)blockIdx.x + jt * (int)gridDim.x) * TC_BM;
-            return stage_tile_rows(X, m0, min(TC_BM, l - m0), xs + (jt & 1) * xs_bytes, xs_bytes, srp[jt & 1],
+            return jt < my_tiles && X.mode != IRWLS_K_RAW_RBF ? make_int2(X.rp[m0], X.rp[min(m0 + TC_BM, l)])
+                                                              : make_int2(0, 0);
+        };
+        auto stage = [&](int jt, int2 pe) {
+            const int m0 = ((int)blockIdx.x + jt * (int)gridDim.x) * TC_BM;
+            return stage_tile_rows(X, m0, min(TC_BM, l - m0), pe.x, pe.y, xs + (jt & 1) * xs_bytes, xs_bytes, srp[jt & 1],
                                    sq[jt & 1], et, EPI);
         };
         TileRows T = {};
-        if (my_tiles > 0) T = stage(0);
+        if (my_tiles > 0) T = stage(0, entries(0));
+        int2 pn = entries(1);
+        if (early) {
+            chain_wait();
+            chain_open();
+        }
         for (int j = 0; j < my_tiles; ++j) {
             const int b = j & 1, tile = (int)blockIdx.x + j * (int)gridDim.x;
             const int m0 = tile * TC_BM, r = 32 * ew + lane, row = m0 + r;
@@ -945,25 +969,25 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
             }
             // the other buffer was last read by tile j - 1, which every epilogue
             // thread finished before the barriers that closed it
-            const TileRows Tn = j + 1 < my_tiles ? stage(j + 1) : T;
+            const TileRows Tn = j + 1 < my_tiles ? stage(j + 1, pn) : T;
+            pn = entries(j + 2);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
             {
                 // this row's kernel values against the group's 32 candidates
                 float v[32], acc[32];
                 if (row < l) kentry32_tile(X, T, cat + CPG * g, qc + CPG * g, r, row, v);
                 // Q w: the three accumulators (terms of order 1, 2^-8 and
-                // 2^-16) added smallest first, eight candidates at a time
+                // 2^-16) added smallest first
                 const uint32_t tb = tmem + b * SC_COLS;
+                {
+                    float s1[32];
+                    tc_ld32_lanes(tb + 128, 32 * ew, CPG * g, acc);
+                    tc_ld32_lanes(tb + 64, 32 * ew, CPG * g, s1);
 #pragma unroll
-                for (int c8 = 0; c8 < 32; c8 += 8) {
-                    float s1[8], s2[8];
-                    tc_ld8_lanes(tb + 128, 32 * ew, CPG * g + c8, s2);
-                    tc_ld8_lanes(tb + 64, 32 * ew, CPG * g + c8, s1);
+                    for (int jj = 0; jj < 32; ++jj) acc[jj] = __fadd_rn(s1[jj], acc[jj]);
+                    tc_ld32_lanes(tb, 32 * ew, CPG * g, s1);
 #pragma unroll
-                    for (int jj = 0; jj < 8; ++jj) s2[jj] = __fadd_rn(s1[jj], s2[jj]);
-                    tc_ld8_lanes(tb, 32 * ew, CPG * g + c8, s1);
-#pragma unroll
-                    for (int jj = 0; jj < 8; ++jj) acc[c8 + jj] = __fadd_rn(s1[jj], s2[jj]);
+                    for (int jj = 0; jj < 32; ++jj) acc[jj] = __fadd_rn(s1[jj], acc[jj]);
                 }
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
                 if (lane == 0) mbar_arrive(&acce[b]);  // this warp's reads of accumulator b are done
@@ -1124,8 +1148,9 @@ extern "C" int irwls_sgma_tc_fits(const irwls_dev_set *X) {
     return score_smem_fixed(X) + 2 * TcRing<64, QB_NP, WS_BK>::BYTES <= score_smem_limit();
 }
 
+// early: as the kernel's.
 extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb,
-                                   int ldq, const void *Wb, int s, float *d_part, float *d_resid) {
+                                   int ldq, const void *Wb, int s, float *d_part, float *d_resid, int early) {
     constexpr size_t XS = 24 * 1024;  // largest row-staging buffer (one of two)
     const int kst = (s + WS_BK - 1) / WS_BK;
     if (kst * WS_BK > ldq || ldq % WS_BK) {
@@ -1169,7 +1194,7 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
     auto launch = [&](auto kern) {
         allow_smem(kern);
         launch_chained(kern, dim3(grid), dim3(128 + 128 * WS_EG), smem, kv, l, d_cand, qb, ldq / 32, wb, kst, d_part,
-                       d_resid, (int)xs, irwls_dev_flags());
+                       d_resid, (int)xs, early, irwls_dev_flags());
     };
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_SGMA_GEMM);
     switch (ns) {

@@ -54,7 +54,7 @@ int irwls_sgma_factor(const irwls_dev_set *X, int s, const int *d_cent, const in
    d_rq: the residuals r = Q w - k of every row against the step's 64
    candidates (64 x rows, candidate-major) */
 int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb, int ldq,
-                        const void *Wb, int s, float *d_part, float *d_rq);
+                        const void *Wb, int s, float *d_part, float *d_rq, int early);
 int irwls_sgma_tc_partials(int l);
 int irwls_sgma_tc_fits(const irwls_dev_set *X);
 int irwls_q_column(const irwls_dev_set *X, const void *F, int l, const int *d_cent, int s, const float *lrow, void *Qb,
@@ -255,7 +255,7 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
                 rc |= irwls_sgma_cand_inv(X, cs, d_cent, s, d_Linv, ldL, d_KN, ldz, d_wpart, m, d_W, Wb, ldq, d_eta,
                                           Qb, d_eps);
             rc |= irwls_sgma_tc_score(X, F, l, cs, Qb, ldq, ahead ? irwls_sgma_ahead_image(ahead, m, ldq, s) : Wb, s,
-                                      d_part, d_rq);
+                                      d_part, d_rq, ahead != NULL);
             irwls_prof_begin(IRWLS_PROF_SGMA_UPDATE);
             rc |= irwls_sgma_tc_select(d_part, nblk, d_eta, cs, s, d_cent, d_best, d_val,
                                        trace ? d_tscore + (size_t)(s - 2) * NCAND : NULL, d_eps, l, d_need);
