@@ -128,6 +128,14 @@ __device__ __forceinline__ double sparse_dot(const double *a_dense, const KView 
     return s;
 }
 
+// The same with one rounding per entry.
+__device__ __forceinline__ double sparse_dot_fused(const double *a_dense, const KView &B, int jb) {
+    double s = 0.0;
+    const int p0 = B.rp[jb], p1 = B.rp[jb + 1];
+    for (int p = p0; p < p1; ++p) s = fma(B.cv[p], a_dense[B.ci[p]], s);
+    return s;
+}
+
 // k(A row held densely in a_dense (shared memory), B row jb).
 __device__ __forceinline__ double kentry(const KView &B, const double *a_dense, double qa, int jb) {
     if (B.mode == IRWLS_K_RAW_RBF) {

@@ -103,8 +103,7 @@ extern "C" int irwls_predict_soft(const irwls_dev_set *T, int n, const irwls_dev
     if (ordered) {
         fill_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n, bias);
         IRWLS_LAUNCH_CHECK("fill");
-        rc = irwls_dev_kernel_rowsum(T, nullptr, n, S, nullptr, nSV, d_w, nullptr, nullptr, 0, +1, d_out, nullptr,
-                                     d_out);
+        rc = irwls_dev_predict_rowsum(T, n, S, nSV, d_w, d_out);
     }
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_PREDICT);
     if (rc) return rc;
