@@ -1024,7 +1024,8 @@ extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, doubl
 }
 
 extern "C" int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, const int *d_SIN, int nSIN,
-                              const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN) {
+                              const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN,
+                              void *exact) {
     // scratch slot 2: the chunk counts (then offsets) and chunk sums
     unsigned char *sc = (unsigned char *)irwls_ctx_scratch(2, (size_t)CT * (sizeof(int) + sizeof(double)));
     if (!sc) return -3;
@@ -1036,6 +1037,8 @@ extern "C" int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, 
     IRWLS_LAUNCH_CHECK("gin_scan");
     gin_write_kernel<<<CT / PC, PC, 0, irwls_stream()>>>(d_SIN, nSIN, d_bnew, ccount, d_lst, d_cb);
     IRWLS_LAUNCH_CHECK("gin_write");
+    const int rc = irwls_exact_rowsum(exact, d_SW, nSW, d_lst, d_cnt, nSIN, d_cb, X->y, +1, nullptr, nullptr, d_GIN);
+    if (rc != 1) return rc;
     return irwls_dev_kernel_rowsum_n(X, d_SW, nSW, X, d_lst, d_cnt, d_cb, X->y, nullptr, +1, nullptr, nullptr,
                                      d_GIN);
 }

@@ -1,6 +1,7 @@
-// dev_predict_tc.cu -- plain-form RBF prediction f_i = b + sum_j w_j k(t_i, s_j)
-// (reference src/LIBIRWLS-predict.c:56-131) with FP64-accurate kernel values
-// from the tensor cores and the integer pipe.
+// dev_predict_tc.cu -- RBF row sums f_i = b + sum_j w_j k(t_i, s_j) with
+// FP64-accurate kernel values from the tensor cores and the integer pipe: the
+// plain form's prediction (reference src/LIBIRWLS-predict.c:56-131) and the error
+// updates of its full training (src/full-train.c:436-510).
 //
 // On the FP64 pipe a kernel value costs two instructions per stored feature and
 // 16 for its exponential, 5.5 ms for 20000 rows against 3000 vectors of 12
@@ -18,8 +19,8 @@
 //    weigh below 2^-61 sigma sigma' per feature).
 // 3. y = log2(e) gamma (q_i + q_j) - 2 log2(e) gamma sigma_i sigma_j 2^-62 T
 //    in 64-bit fixed point (its unit 2^-56, or below 2^-56 of the largest term), then
-//    2^-y by exp2_fixed. The value times w_j is added in FP64, in vector order per 16- or 32-vector strip;
-//    the strips' sums are added in a fixed order.
+//    2^-y by exp2_fixed. The value times w_j is added in FP64, in vector order
+//    per strip of 16 of every 64 vectors; the strips' sums in a fixed order.
 //
 // Against a 64-bit evaluation the decision values are within 2.5e-16 of their
 // size, the ordered FP64 sums within 1.5e-15 (20000 one-hot rows of 54 features,
@@ -56,9 +57,10 @@ static_assert((5LL * 256 + 6) * PDRAIN * PK * 128 * 128 < (1LL << 31), "levels 3
 __device__ __forceinline__ int ppiece_off(int r, int k) { return (r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7); }
 
 // Per row: e with 2^e >= |x| (-2000: a zero row), and over the set the largest
-// |q| and the largest |x|^2 (floats rounded up a little, as bits) and, with w,
-// the high half of the largest |w| (that of infinity where a row's indices do
-// not increase). One warp per row.
+// |q| (with q) and the largest |x|^2 (floats rounded up a little, as bits) and, with w,
+// the high half of the largest |w|; with rp that of infinity where a row's
+// indices do not increase (a vector that names a feature twice: its products add
+// both). One warp per row.
 __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restrict__ X, int ld, int width,
                                                          const double *__restrict__ q,
                                                          const double *__restrict__ w, const int *__restrict__ rp,
@@ -95,9 +97,8 @@ __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restric
             }
             for (int o = 16; o > 0; o >>= 1) rho += __shfl_xor_sync(0xffffffffu, rho, o);
         }
-        // a vector that names a feature twice (its product adds both): not for this path
         bool bad = false;
-        if (w)
+        if (rp)
             for (int t = rp[i] + 1 + lane; t < rp[i + 1]; t += 32) bad |= ci[t] <= ci[t - 1];
         bad = __any_sync(0xffffffffu, bad);
         if (lane == 0) {
@@ -107,13 +108,27 @@ __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restric
             ex[i] = E == 0 ? -2000 : e + max(grow, 0);
             // (the order of non-negative floats is that of their bits; an
             // overflow to infinity makes the caller take the other path)
-            atomicMax(big, __float_as_uint(fabsf((float)q[i]) * up));
+            if (q) atomicMax(big, __float_as_uint(fabsf((float)q[i]) * up));
             atomicMax(big + 1, __float_as_uint(E == 0 ? 0.f : ldexpf(rho * up, 2 * e)));
-            if (w) atomicMax(big + 2, bad ? 0x7ff00000u : (unsigned)__double2hiint(w[i]) & 0x7fffffffu);
+            if (w || bad) atomicMax(big + 2, bad ? 0x7ff00000u : (unsigned)__double2hiint(w[i]) & 0x7fffffffu);
         }
     }
     __syncthreads();
     if (threadIdx.x < 3 && big[threadIdx.x]) atomicMax(top + threadIdx.x, big[threadIdx.x]);
+}
+
+// round(x 2^(55 - e)) for |x| <= 2^e, ties away from zero.
+__device__ __forceinline__ long long fixed55(double x, int e) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int E = (int)((b >> 52) & 0x7ff);
+    if (E == 0) return 0;
+    // x = M 2^(E - 1075)
+    const unsigned long long M = (b & ((1ULL << 52) - 1)) | (1ULL << 52);
+    const int sh = 1075 + e - 55 - E;  // >= -3 since |x| <= 2^e
+    long long N = 0;
+    if (sh <= 0) N = (long long)(M << min(-sh, 3));
+    else if (sh < 64) N = (long long)((M + (1ULL << (sh - 1))) >> sh);
+    return (b >> 63) ? -N : N;
 }
 
 // The digits of 8 features of a row in one 16-byte store per piece. Rows >= n
@@ -138,18 +153,7 @@ __global__ void __launch_bounds__(256) row_slice_kernel(const double *__restrict
         for (int k = 0; k < 8; ++k) {
             const int c = (int)g * 8 + k;
             long long N = 0;
-            if (e > -2000 && c < width) {
-                const unsigned long long b = (unsigned long long)__double_as_longlong(X[(size_t)i * ld + c]);
-                const int E = (int)((b >> 52) & 0x7ff);
-                if (E != 0) {
-                    // x = M 2^(E - 1075); N = x 2^(55 - e), ties away from zero
-                    const unsigned long long M = (b & ((1ULL << 52) - 1)) | (1ULL << 52);
-                    const int sh = 1075 + e - 55 - E;  // >= -3 since |x| <= 2^e
-                    if (sh <= 0) N = (long long)(M << min(-sh, 3));
-                    else if (sh < 64) N = (long long)((M + (1ULL << (sh - 1))) >> sh);
-                    if (b >> 63) N = -N;
-                }
-            }
+            if (e > -2000 && c < width) N = fixed55(X[(size_t)i * ld + c], e);
 #pragma unroll
             for (int s = 0; s < PS; ++s) {
                 int d;
@@ -192,10 +196,34 @@ __global__ void row_norms_kernel(const double *__restrict__ q, int n, unsigned l
     a[i] = v;
 }
 
+// The same of the row's own fixed point, for raw rows (their kernel is that of the
+// differences: FP64 norms would leave c |x|^2 2^-53 of them, the integers leave
+// units of y): T_ii = sum N N 2^-48, in the products' unit. A warp per row.
+__global__ void __launch_bounds__(256) row_norms_raw_kernel(const double *__restrict__ X, int ld, int width, int n,
+                                                            const int *__restrict__ ex, unsigned long long cg, int ec,
+                                                            int fb, long long *__restrict__ a) {
+    const int lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const int e = ex[i];
+        long long T = 0;
+        if (e > -2000)
+            for (int t = lane; t < width; t += 32) {
+                const long long N = fixed55(X[(size_t)i * ld + t], e) << 8;
+                T += __mul64hi(N, N);
+            }
+        for (int o = 16; o > 0; o >>= 1) T += __shfl_xor_sync(0xffffffffu, T, o);
+        // c |x|^2 2^fb = T cg 2^(2 e - 62 - ec + fb)
+        const int sh = -(2 * e + 2 - ec + fb);
+        const long long m = (long long)__umul64hi((unsigned long long)T, cg);
+        if (lane == 0) a[i] = e <= -2000 ? 0 : sh <= 0 ? m << min(-sh, 3) : sh < 64 ? (m >> (sh - 1)) + 1 >> 1 : 0;
+    }
+}
+
 struct PredictArgs {
     const __nv_bfloat16 *T, *S;  // digit slices of the rows and of the vectors
     int npb;                     // 16-feature blocks
     int n, nsv, per, P;          // rows, vectors, vector tiles per chunk, chunks
+    const int *nsvp;             // the number of vectors on the device (at most nsv), or NULL
     const int *et, *es;          // row and vector scales
     const long long *at, *as;    // norm terms
     const double *w;
@@ -219,7 +247,8 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
     unsigned char *smem = p_smem + ((1024 - (smem_u32(p_smem) & 1023)) & 1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int I = blockIdx.x, z = blockIdx.y;
-    const int nt = (p.nsv + PN - 1) / PN;
+    const int nsv = p.nsvp ? p.nsvp[0] : p.nsv;
+    const int nt = (nsv + PN - 1) / PN;
     const int j0 = z * p.per, jn = max(0, min(nt, j0 + p.per) - j0);
     const int nd = (p.npb + PDRAIN - 1) / PDRAIN;  // drains per tile pair
     const int nst = jn * p.npb;
@@ -320,9 +349,9 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
         // vector et of tile t into registers (past the end: weight 0, 2^-y <= 1)
         auto fetch = [&](int t) {
             const int j = PN * t + et;
-            nw = j < p.nsv ? p.w[j] : 0.0;
-            ng.x = j < p.nsv ? (unsigned long long)p.as[j] : 1ULL << 62;
-            ng.y = j < p.nsv ? p.g >> min(p.emax - p.es[j], 63) : 0;
+            nw = j < nsv ? p.w[j] : 0.0;
+            ng.x = j < nsv ? (unsigned long long)p.as[j] : 1ULL << 62;
+            ng.y = j < nsv ? p.g >> min(p.emax - p.es[j], 63) : 0;
         };
         if (et < PN && jn > 0) {
             fetch(j0);
@@ -416,6 +445,48 @@ __global__ void predict_finish_kernel(const double *__restrict__ part, int strip
     out[i] = hard ? (f >= 0.0 ? 1.0 : -1.0) : f;
 }
 
+// out_i = init_i +- (the strips in order) sa_i - tail, as kernel_rowsum_kernel.
+__global__ void rowsum_finish_kernel(const double *__restrict__ part, int strips, int n, const int *__restrict__ ia,
+                                     const double *__restrict__ sa, int op, const double *init,  // may alias out
+                                     const double *__restrict__ tail, double *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double f = 0.0;
+#pragma unroll 8
+    for (int s = 0; s < strips; ++s) f = __dadd_rn(f, part[(size_t)s * n + i]);
+    if (sa) f = __dmul_rn(f, sa[ia ? ia[i] : i]);
+    const double f0 = init ? init[i] : 0.0;
+    f = op > 0 ? __dadd_rn(f0, f) : __dsub_rn(f0, f);
+    out[i] = tail ? __dsub_rn(f, tail[0]) : f;
+}
+
+// The digits, scales and norm terms of the rows idx[0 ... n - 1] of a sliced set as
+// a sliced set of their own (zero digits up to whole 128-row tiles).
+__global__ void __launch_bounds__(256) gather_slices_kernel(const uint4 *__restrict__ S, const int *__restrict__ ex,
+                                                            const long long *__restrict__ a, int npb,
+                                                            const int *__restrict__ idx, int n,
+                                                            const int *__restrict__ np, uint4 *__restrict__ oS,
+                                                            int *__restrict__ oex, long long *__restrict__ oa) {
+    if (np) n = np[0];
+    constexpr int TILE = PS * PPIECE / 8;  // 16-byte units of a 16-feature block of a tile
+    const int units = npb * PS * 2;        // of a row
+    const long long items = (long long)((n + PM - 1) / PM * PM) * units;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < items;
+         t += (long long)gridDim.x * blockDim.x) {
+        // (neighbouring threads: the rows of a core matrix, 128 contiguous bytes)
+        const int i = (int)(t / (8 * units)) * 8 + (int)(t & 7), u = (int)(t / 8 % units);
+        const int pb = u / (2 * PS), s = u % (2 * PS) >> 1, h = u & 1;
+        const int r = i < n ? idx[i] : 0;
+        const uint4 v = i < n ? S[((size_t)(r >> 7) * npb + pb) * TILE + s * (PPIECE / 8) + ppiece_off(r & 127, 8 * h) / 8]
+                              : make_uint4(0, 0, 0, 0);
+        oS[((size_t)(i >> 7) * npb + pb) * TILE + s * (PPIECE / 8) + ppiece_off(i & 127, 8 * h) / 8] = v;
+        if (u == 0 && i < n) {
+            oex[i] = ex[r];
+            oa[i] = a[r];
+        }
+    }
+}
+
 // gamma log2(e) = g 2^-e with g in [2^62, 2^63): the 53-bit mantissa of gamma
 // times log2(e) 2^62, exactly.
 void scaled_gamma(double gamma, unsigned long long *g, int *e) {
@@ -430,11 +501,76 @@ void scaled_gamma(double gamma, unsigned long long *g, int *e) {
 
 size_t slice_bytes(long long rows, int npb) { return (size_t)((rows + PM - 1) / PM) * npb * PS * PPIECE * 2; }
 
+// The fixed point of y from the maxima of the two sets (row_scales_kernel: |q|,
+// |x|^2 and, for the vectors, |w|), and cg 2^-ec = gamma log2(e); false: not for it.
+// Raw rows (no q) take it in units of 2^-53 at most: there it is as close as the
+// differences' squares summed in FP64 (units of y each, about 3 to a value's 1 to
+// 2 ulp), in larger units close rows would not be.
+bool fixed_point_of(double gamma, bool raw, const float *ht, const float *hs, PredictArgs *a, unsigned long long *cg,
+                    int *ec) {
+    unsigned wtop;
+    memcpy(&wtop, hs + 2, sizeof wtop);
+    if (!(ht[1] < 1e30f && hs[1] < 1e30f) || wtop >= 0x7ff00000u) return false;
+    // |y| <= c (|q_i| + |q_j|) + 2 c |x_i| |x_j| < 2^(62 - fb), c = gamma log2(e)
+    const double ym = gamma * 1.4426950408889634 *
+                      ((double)ht[raw] + (double)hs[raw] + 2.0 * sqrt((double)ht[1] * (double)hs[1]));
+    if (!(ym < 1e8)) return false;
+    a->fb = ym < 32.0 ? 56 : 60 - ilogb(ym);
+    scaled_gamma(gamma, cg, ec);
+    // sigma < 2 |x| (1.001): the largest exponents (of zero rows: never less than -74)
+    const int ei = ht[1] > 0.f ? (ilogb((double)ht[1]) >> 1) + 1 : -74;
+    a->emax = hs[1] > 0.f ? (ilogb((double)hs[1]) >> 1) + 1 : -74;
+    // y's product part = 2 c 2^(e_i + e_j) 2^-62 T 2^fb; no left shift in it
+    a->fb = std::min(a->fb, *ec - 3 - ei - a->emax);
+    if (a->fb < (raw ? 53 : 32)) return false;
+    a->g = *cg;
+    a->shr = *ec - 3 - a->fb - a->emax;
+    return true;
+}
+
+// Chunks of nt vector tiles for `it` row tiles: the fewest rounds of items over the
+// SMs, an item's start taken as a quarter of a tile.
+int best_chunks(int it, int nt, int sms, long long most = 1 << 30) {
+    int best = 1;
+    double cost = 1e300;
+    for (int P = 1; P <= nt && P <= most && P <= std::max(64, 16 * sms / it); ++P) {
+        const int per = ceil_div(nt, P);
+        const double c = ceil_div((long long)it * ceil_div(nt, per), sms) * (per + 0.25);
+        if (c < cost * 0.999) {
+            cost = c;
+            best = P;
+        }
+    }
+    return best;
+}
+
+constexpr int GR = 4;  // strips of a chunk (column groups of predict_tc_kernel)
+
+void launch_predict(const PredictArgs &a, int tiles) {
+    auto kern = a.npb > PDRAIN ? (a.fb == 56 ? predict_tc_kernel<true, 56> : predict_tc_kernel<true, 0>)
+                               : (a.fb == 56 ? predict_tc_kernel<false, 56> : predict_tc_kernel<false, 0>);
+    allow_smem(kern);
+    kern<<<dim3(tiles, a.P), 128 + 32 * 16, (size_t)PNS * P_STAGE + 1024, irwls_stream()>>>(a, irwls_dev_flags());
+    irwls_count_launch(1);
+}
+
+void launch_norms(const irwls_dev_set *X, bool raw, int n, const int *ex, unsigned long long cg, int ec, int fb,
+                  long long *a) {
+    if (raw)
+        row_norms_raw_kernel<<<std::min(ceil_div(n, 8), 2048), 256, 0, irwls_stream()>>>(X->X, X->ld, X->width, n, ex,
+                                                                                       cg, ec, fb, a);
+    else row_norms_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(X->q, n, cg, ec, fb, a);
+    irwls_count_launch(1);
+}
+
+int slice_grid(long long rows, int npb, int sms) {
+    return (int)std::max<long long>(1, std::min<long long>(ceil_div(rows * npb * 2, 256), 16LL * sms));
+}
+
 }  // namespace
 
 // The plain form's prediction on the tensor cores; 1 when the sizes or values
-// are not for it (the caller then sums on the FP64 pipe): not the RBF kernel by
-// norms, more than 12288 features (what the FP64 path takes) or 4 GB of vector
+// are not for it (the caller then sums on the FP64 pipe): not the RBF kernel, more than 12288 features (what the FP64 path takes) or 4 GB of vector
 // slices, a vector that names a feature twice, a gamma outside (1e-30, 1e6),
 // features or weights that are not finite, values whose squares leave FP32's
 // range or whose y does not fit its fixed point, no room for the workspace, or
@@ -445,10 +581,11 @@ size_t slice_bytes(long long rows, int npb) { return (size_t)((rows + PM - 1) / 
 extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                                    double bias, int hard, double *d_out) {
     constexpr double MIN_VALUES = 5.0e5;
-    if (n < 1 || nSV < 1 || (double)n * nSV < MIN_VALUES || T->mode != IRWLS_K_NORM_RBF ||
-        S->mode != IRWLS_K_NORM_RBF || !T->X ||
-        !S->X || !S->rp || !S->ci)
+    if (n < 1 || nSV < 1 || (double)n * nSV < MIN_VALUES || T->mode != S->mode ||
+        S->mode == IRWLS_K_LINEAR || !T->X || !S->X)
         return 1;
+    const bool raw = S->mode == IRWLS_K_RAW_RBF;
+    if (raw ? T->width != S->width : !S->rp || !S->ci) return 1;
     const int width = std::max(T->width, S->width);
     const int npb = ceil_div(width, PK);
     const double gamma = -S->neg_gamma;
@@ -459,12 +596,7 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     const long long tiles_fit = std::max<long long>(1, ((long long)2 << 30) / (long long)slice_bytes(PM, npb));
     const int slab = (int)std::min<long long>((long long)PM * tiles_fit, (long long)ceil_div(n, PM) * PM);
     const int nt = ceil_div(nSV, PN), it = ceil_div(std::min(n, slab), PM);
-    // chunks of the vectors: about eight items per SM, at least two tiles each
-    int P = std::max(1, std::min(ceil_div(8 * sms, it), (nt + 1) / 2));
-    const int per = ceil_div(nt, P);
-    P = ceil_div(nt, per);
-    const bool multi = npb > PDRAIN;
-    constexpr int GR = 4;  // strips of a chunk
+    const int per = ceil_div(nt, best_chunks(it, nt, sms)), P = ceil_div(nt, per);
     const size_t rn = (size_t)std::min(n, slab);
     const size_t off_s = (slice_bytes(slab, npb) + 255) & ~(size_t)255;
     const size_t off_et = off_s + ((slice_bytes(nSV, npb) + 255) & ~(size_t)255);
@@ -487,40 +619,23 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     };
     if (rc) return fail(rc);
     const int gt = std::min(ceil_div(n, 8), 4 * sms), gs = std::min(ceil_div(nSV, 8), 4 * sms);
-    row_scales_kernel<<<gt, 256, 0, irwls_stream()>>>(T->X, T->ld, T->width, T->q, nullptr, nullptr, nullptr, n, et, top);
+    row_scales_kernel<<<gt, 256, 0, irwls_stream()>>>(T->X, T->ld, T->width, raw ? nullptr : T->q, nullptr, nullptr, nullptr, n,
+                                                     et, top);
     irwls_count_launch(1);
-    row_scales_kernel<<<gs, 256, 0, irwls_stream()>>>(S->X, S->ld, S->width, S->q, d_w, S->rp, S->ci, nSV, es, top + 3);
+    row_scales_kernel<<<gs, 256, 0, irwls_stream()>>>(S->X, S->ld, S->width, raw ? nullptr : S->q, d_w, raw ? nullptr : S->rp, S->ci,
+                                                     nSV, es, top + 3);
     irwls_count_launch(1);
-    row_slice_kernel<<<std::min(ceil_div((long long)ceil_div(nSV, PM) * PM * npb * 2, 256), 16 * sms), 256, 0,
-                       irwls_stream()>>>(S->X, S->ld, S->width, nSV, es, ceil_div(nSV, PM) * PM, npb, dS);
+    row_slice_kernel<<<slice_grid((long long)ceil_div(nSV, PM) * PM, npb, sms), 256, 0, irwls_stream()>>>(S->X, S->ld, S->width, nSV, es, ceil_div(nSV, PM) * PM, npb, dS);
     irwls_count_launch(1);
     if ((rc = irwls_check_launch("predict_prepare"))) return fail(rc);
     float h[6];
     if (irwls_dev_d2h(h, top, sizeof h) || irwls_dev_sync()) return fail(-2);
-    unsigned wtop;
-    memcpy(&wtop, h + 5, sizeof wtop);
-    if (!(h[1] < 1e30f && h[4] < 1e30f) || wtop >= 0x7ff00000u) return fail(1);
     PredictArgs a = {};
-    // |y| <= c (|q_i| + |q_j|) + 2 c |x_i| |x_j| < 2^(62 - fb), c = gamma log2(e)
-    const double ym = gamma * 1.4426950408889634 *
-                      ((double)h[0] + (double)h[3] + 2.0 * sqrt((double)h[1] * (double)h[4]));
-    if (!(ym < 1e8)) return fail(1);
-    a.fb = ym < 32.0 ? 56 : 60 - ilogb(ym);
     unsigned long long cg;
     int ec;
-    scaled_gamma(gamma, &cg, &ec);  // c = cg 2^-ec
-    // sigma < 2 |x| (1.001): the largest exponents (of zero rows: never less than -74)
-    const int ei = h[1] > 0.f ? (ilogb((double)h[1]) >> 1) + 1 : -74;
-    a.emax = h[4] > 0.f ? (ilogb((double)h[4]) >> 1) + 1 : -74;
-    // y's product part = 2 c 2^(e_i + e_j) 2^-62 T 2^fb; no left shift in it
-    a.fb = std::min(a.fb, ec - 3 - ei - a.emax);
-    if (a.fb < 32) return fail(1);
-    a.g = cg;
-    a.shr = ec - 3 - a.fb - a.emax;
-    row_norms_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(T->q, n, cg, ec, a.fb, at);
-    irwls_count_launch(1);
-    row_norms_kernel<<<ceil_div(nSV, 256), 256, 0, irwls_stream()>>>(S->q, nSV, cg, ec, a.fb, as);
-    irwls_count_launch(1);
+    if (!fixed_point_of(gamma, raw, h, h + 3, &a, &cg, &ec)) return fail(1);
+    launch_norms(T, raw, n, et, cg, ec, a.fb, at);
+    launch_norms(S, raw, nSV, es, cg, ec, a.fb, as);
     a.T = dT;
     a.S = dS;
     a.npb = npb;
@@ -531,20 +646,14 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     a.as = as;
     a.w = d_w;
     a.part = (double *)(ws + off_part);
-    const size_t smem = (size_t)PNS * P_STAGE + 1024;
     for (int r0 = 0; r0 < n && !rc; r0 += slab) {
         const int rows = std::min(slab, n - r0), tiles = ceil_div(rows, PM);
         a.n = rows;
         a.et = et + r0;
         a.at = at + r0;
-        row_slice_kernel<<<(int)std::min<long long>(ceil_div((long long)tiles * PM * npb * 2, 256), 16LL * sms), 256, 0,
-                           irwls_stream()>>>(T->X + (size_t)r0 * T->ld, T->ld, T->width, rows, et + r0, tiles * PM, npb, dT);
+        row_slice_kernel<<<slice_grid((long long)tiles * PM, npb, sms), 256, 0, irwls_stream()>>>(T->X + (size_t)r0 * T->ld, T->ld, T->width, rows, et + r0, tiles * PM, npb, dT);
         irwls_count_launch(1);
-        auto kern = multi ? (a.fb == 56 ? predict_tc_kernel<true, 56> : predict_tc_kernel<true, 0>)
-                          : (a.fb == 56 ? predict_tc_kernel<false, 56> : predict_tc_kernel<false, 0>);
-        allow_smem(kern);
-        kern<<<dim3(tiles, P), 128 + 32 * 16, smem, irwls_stream()>>>(a, irwls_dev_flags());
-        irwls_count_launch(1);
+        launch_predict(a, tiles);
         predict_finish_kernel<<<ceil_div(rows, 256), 256, 0, irwls_stream()>>>(a.part, P * GR, rows, bias, hard, d_out + r0);
         irwls_count_launch(1);
         rc = irwls_check_launch("predict_tc");
@@ -557,4 +666,127 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
         return -13;
     }
     return 0;
+}
+
+// ---- row sums within one set ------------------------------------------------
+
+// A set's digits, kept over a training, and room for lists of its rows.
+struct ExactRows {
+    unsigned char *ws;
+    __nv_bfloat16 *S, *bS, *aS;  // all rows; a list of vectors; a list of rows
+    int *ex, *bex, *aex;
+    long long *q, *bq, *aq;
+    double *part;
+    int n, npb, na, sms;
+    size_t nparts;
+    PredictArgs p;
+};
+
+extern "C" void irwls_exact_rows_free(void *h) {
+    ExactRows *E = (ExactRows *)h;
+    if (!E) return;
+    irwls_dev_free(E->ws);
+    free(E);
+}
+
+// Rows 0 ... n - 1 of X for row sums of all or up to na listed rows against lists
+// of rows; NULL where irwls_predict_exact would return 1, or above 4 GB.
+extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) {
+    const double gamma = -X->neg_gamma;
+    const bool raw = X->mode == IRWLS_K_RAW_RBF;
+    if (n < 1 || X->mode == IRWLS_K_LINEAR || !X->X || (!raw && (!X->rp || !X->ci)) || X->ld > 12288 ||
+        !(gamma > 1e-30 && gamma < 1e6))
+        return nullptr;
+    const int npb = ceil_div(X->width, PK), sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
+    na = std::min(na, n);
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t sb = up(slice_bytes(n, npb)), ab = up(slice_bytes(na, npb)), n4 = up((size_t)n * 4), n8 = up((size_t)n * 8);
+    // partial sums: all rows in up to 16 chunks, or a list of rows against any
+    const size_t nparts = (size_t)GR * std::max<size_t>((size_t)n * 16, (size_t)na * ceil_div(n, PN));
+    const size_t total = 2 * sb + ab + 3 * (n4 + n8) + 256 + up(nparts * sizeof(double));
+    if (total > ((size_t)4 << 30)) return nullptr;
+    ExactRows *E = (ExactRows *)calloc(1, sizeof(ExactRows));
+    if (!E) return nullptr;
+    if (irwls_dev_malloc((void **)&E->ws, total)) {
+        irwls_clear_error();
+        free(E);
+        return nullptr;
+    }
+    unsigned char *w = E->ws;
+    auto take = [&](size_t b) {
+        unsigned char *r = w;
+        w += b;
+        return r;
+    };
+    E->S = (__nv_bfloat16 *)take(sb);
+    E->bS = (__nv_bfloat16 *)take(sb);
+    E->aS = (__nv_bfloat16 *)take(ab);
+    E->ex = (int *)take(n4), E->bex = (int *)take(n4), E->aex = (int *)take(n4);
+    E->q = (long long *)take(n8), E->bq = (long long *)take(n8), E->aq = (long long *)take(n8);
+    unsigned *top = (unsigned *)take(256);
+    E->part = (double *)w;
+    E->nparts = nparts;
+    E->n = n, E->npb = npb, E->na = na, E->sms = sms;
+    float h[3];
+    int rc = irwls_dev_memset(top, 0, 3 * sizeof(unsigned));
+    row_scales_kernel<<<std::min(ceil_div(n, 8), 4 * sms), 256, 0, irwls_stream()>>>(X->X, X->ld, X->width,
+                                                                                  raw ? nullptr : X->q, nullptr,
+                                                                                  raw ? nullptr : X->rp, X->ci, n,
+                                                                                  E->ex, top);
+    irwls_count_launch(1);
+    row_slice_kernel<<<slice_grid((long long)ceil_div(n, PM) * PM, npb, sms), 256, 0, irwls_stream()>>>(
+        X->X, X->ld, X->width, n, E->ex, ceil_div(n, PM) * PM, npb, E->S);
+    irwls_count_launch(1);
+    rc = rc || irwls_check_launch("exact_rows") || irwls_dev_d2h(h, top, sizeof h) || irwls_dev_sync();
+    unsigned long long cg;
+    int ec;
+    if (rc || !fixed_point_of(gamma, raw, h, h, &E->p, &cg, &ec)) {
+        irwls_exact_rows_free(E);
+        return nullptr;
+    }
+    launch_norms(X, raw, n, E->ex, cg, ec, E->p.fb, E->q);
+    E->p.npb = npb;
+    return E;
+}
+
+// The arguments of irwls_dev_kernel_rowsum_n with the vectors' signs in cb; the list
+// has at most nBmax rows. 1: fewer than 500000 kernel values (the caller then takes
+// the FP64 kernel; the line is the predictions'). 4000 raw rows of 20 values, 500
+// in the working set: 30 us a call with its gathers and sums, there 286.
+extern "C" int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d_ib, const int *d_nB, int nBmax,
+                                  const double *d_cb, const double *d_sa, int op, const double *d_init,
+                                  const double *d_tail, double *d_out) {
+    ExactRows *E = (ExactRows *)h;
+    if (!E || nA < 1 || nBmax < 1 || (double)nA * nBmax < 5.0e5 || (d_ia ? nA > E->na : nA > E->n) || nBmax > E->n)
+        return 1;
+    PredictArgs a = E->p;
+    const int it = ceil_div(nA, PM), nt = ceil_div(nBmax, PN);
+    a.per = ceil_div(nt, best_chunks(it, nt, E->sms, (long long)(E->nparts / GR / nA)));
+    a.P = ceil_div(nt, a.per);
+    if (d_ia) {
+        gather_slices_kernel<<<slice_grid((long long)nA * PS, E->npb, E->sms), 256, 0, irwls_stream()>>>(
+            (const uint4 *)E->S, E->ex, E->q, E->npb, d_ia, nA, nullptr, (uint4 *)E->aS, E->aex, E->aq);
+        irwls_count_launch(1);
+    }
+    gather_slices_kernel<<<slice_grid((long long)nBmax * PS, E->npb, E->sms), 256, 0, irwls_stream()>>>(
+        (const uint4 *)E->S, E->ex, E->q, E->npb, d_ib, nBmax, d_nB, (uint4 *)E->bS, E->bex, E->bq);
+    irwls_count_launch(1);
+    a.T = d_ia ? E->aS : E->S;
+    a.et = d_ia ? E->aex : E->ex;
+    a.at = d_ia ? E->aq : E->q;
+    a.S = E->bS;
+    a.es = E->bex;
+    a.as = E->bq;
+    a.n = nA;
+    a.nsv = nBmax;
+    a.nsvp = d_nB;
+    a.w = d_cb;
+    a.part = E->part;
+    if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
+    launch_predict(a, it);
+    if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_ROWSUM);
+    rowsum_finish_kernel<<<ceil_div(nA, 256), 256, 0, irwls_stream()>>>(E->part, a.P * GR, nA, d_ia, d_sa, op, d_init,
+                                                                       d_tail, d_out);
+    irwls_count_launch(1);
+    return irwls_check_launch("exact_rowsum");
 }

@@ -122,6 +122,10 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
        solves, GIN and the in-set updates are the FP64 form's. */
     void *tcs = NULL;
     if (irwls_get_precision() == IRWLS_PRECISION_MIXED && !(tcs = irwls_tc_set_create(X, l, W))) return -1;
+    /* plain form: the row sums from the tensor cores where they are large enough
+       (at most W changed weights per update, or W rows); the errors are as close
+       to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu) */
+    void *exact = !tcs && (double)l * W >= 5.0e5 ? irwls_exact_rows_create(X, l, W) : NULL;
     const double band = 0.05, eps = 2e-5 * (tcs ? irwls_tc_set_kbound(tcs) : 1.0);
     int *xflag = NULL, *xmark = NULL, *xS = NULL, *xSnew = NULL, *svlst = NULL, *svcnt = NULL, *xcnt = NULL,
         *h_xcnt = NULL;
@@ -196,7 +200,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     double best = 1e20;
     while (stop == 0 && since_best < 300) {
         /* GIN of the inactive set; kept as is when the set is empty (:436-456) */
-        if (nSIN > 0 && irwls_full_gin(X, SW, nSW, SIN, nSIN, bnew, lst, cb, cnt, ws.GIN)) goto fail;
+        if (nSIN > 0 && irwls_full_gin(X, SW, nSW, SIN, nSIN, bnew, lst, cb, cnt, ws.GIN, exact)) goto fail;
         ws.w = nSW;
         ws.map = SW;
         ws.tcs = tcs;
@@ -219,8 +223,10 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
             }
             if (irwls_tc_kernel_rowsum(tcs, lst, cnt, cb, e, dbias, e)) goto fail;
             if (irwls_dev_scatter(eS, xS, nS, e) || irwls_dev_d2h(h_l1, dbias + 1, sizeof(double))) goto fail;
-        } else if (irwls_dev_kernel_rowsum_n(X, NULL, l, X, lst, cnt, cb, NULL, NULL, -1, e, dbias, e)) {
-            goto fail;
+        } else {
+            const int ex = irwls_exact_rowsum(exact, NULL, l, lst, cnt, nSW, cb, NULL, -1, e, dbias, e);
+            if (ex < 0 || (ex == 1 && irwls_dev_kernel_rowsum_n(X, NULL, l, X, lst, cnt, cb, NULL, NULL, -1, e, dbias, e)))
+                goto fail;
         }
         if (irwls_full_norms(beta, bnew, l + 1, norms)) goto fail;
         if (irwls_dev_d2h(h_norms, norms, 2 * sizeof(double)) || irwls_dev_sync()) goto fail;
@@ -296,7 +302,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         }
     }
     if (irwls_dev_d2h(beta_out, bnew, L1 * sizeof(double)) || irwls_dev_sync()) goto fail;
-    if (tcs) {
+    if (tcs || exact) {
         const int tc = irwls_tc_status();
         if (tc) {
             irwls_set_error(-13, "a tensor-core pipeline wait of the error update ran out (code %d)", tc);
@@ -309,6 +315,7 @@ fail:
 done:
     irwls_sub_release(&ws);
     irwls_tc_set_free(tcs);
+    irwls_exact_rows_free(exact);
     void *xbufs[] = {xflag, xmark, xS, xSnew, svlst, svcnt, xcnt, eS, svcb};
     for (size_t k = 0; k < sizeof xbufs / sizeof xbufs[0]; k++) irwls_dev_free(xbufs[k]);
     irwls_dev_host_free(h_xcnt);

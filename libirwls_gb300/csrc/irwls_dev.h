@@ -174,7 +174,7 @@ typedef struct irwls_outer_counts {
     int nSW, nSIN, nSC, pad;
 } irwls_outer_counts;
 int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, const int *d_SIN, int nSIN,
-                   const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN);
+                   const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN, void *exact);
 int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e, const double *d_beta, int l,
                          double *d_esub, double *d_bsub);
 int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt, const double *d_beta, int l,
@@ -285,6 +285,12 @@ int irwls_predict_soft(const irwls_dev_set *T, int n, const irwls_dev_set *S, in
  * these sizes or values */
 int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                         double bias, int hard, double *d_out);
+/* row sums within one set on the same kernels (full training, plain form) */
+void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na);
+void irwls_exact_rows_free(void *h);
+int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d_ib, const int *d_nB, int nBmax,
+                       const double *d_cb, const double *d_sa, int op, const double *d_init, const double *d_tail,
+                       double *d_out);
 size_t irwls_predict_linear_scratch(int width, int nsv);
 int irwls_predict_linear(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                          double bias, int hard, double *d_W, double *d_out);
