@@ -141,9 +141,10 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     const double C = props.C;
     if (m <= 0) return 0;
     int rc = 0;
-    int *d_idx = NULL, *d_act = NULL, *d_nact = NULL, *h_nact = NULL;
+    int *d_idx = NULL, *d_act = NULL;
+    irwls_par_post *h_post = NULL;
     double *d_KC = NULL, *d_KSC = NULL, *d_K1 = NULL, *d_part = NULL, *d_sd = NULL, *d_day = NULL, *d_e = NULL,
-           *d_Da = NULL, *d_beta = NULL, *d_bnew = NULL, *d_bbest = NULL, *d_nrm = NULL, *h_nrm = NULL;
+           *d_Da = NULL, *d_beta = NULL, *d_bnew = NULL, *d_bbest = NULL;
     const int ld = m + 1;
     /* The Gram runs on the tensor cores through exact integer digits of the
        active rows (dev_gram_tc.cu): base 256 in the plain form (FP64
@@ -172,8 +173,6 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     }
     rc |= irwls_dev_malloc((void **)&d_idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_act, (size_t)l * sizeof(int));
-    rc |= irwls_dev_malloc((void **)&d_nact, sizeof(int));
-    rc |= irwls_dev_host_alloc((void **)&h_nact, sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_KC, (size_t)m * m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_KSC, (size_t)l * m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_K1, (size_t)ld * ld * sizeof(double));
@@ -185,9 +184,9 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     rc |= irwls_dev_malloc((void **)&d_beta, (size_t)m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_bnew, (size_t)m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_bbest, (size_t)m * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_nrm, 2 * sizeof(double));
-    rc |= irwls_dev_host_alloc((void **)&h_nrm, 2 * sizeof(double));
+    rc |= irwls_dev_host_alloc((void **)&h_post, sizeof(irwls_par_post));
     if (rc) goto done;
+    h_post->seq = 0;
     double M = 10000.0;
     rc |= irwls_dev_h2d(d_idx, idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_memset(d_beta, 0, (size_t)m * sizeof(double));
@@ -208,15 +207,13 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
                 goto fail;
             g_gram_flops += (double)nact * (m + 1) * m;
             if (irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)) goto fail;
-            if (irwls_par_delta(d_bnew, d_beta, m, d_nrm)) goto fail;
+            if (irwls_par_delta(d_bnew, d_beta, m, h_post)) goto fail;
             if (irwls_par_residual(d_KSC, l, m, d_beta, X->y, C, M, d_e, d_Da)) goto fail;
-            if (irwls_par_weights(d_Da, X->y, l, d_act, d_sd, d_day, d_nact)) goto fail;
-            if (irwls_dev_d2h(h_nrm, d_nrm, 2 * sizeof(double)) || irwls_dev_d2h(h_nact, d_nact, sizeof(int)) ||
-                irwls_dev_sync())
-                goto fail;
-            dW = h_nrm[0];
-            nW = h_nrm[1];
-            nact = *h_nact;
+            if (irwls_par_weights(d_Da, X->y, l, d_act, d_sd, d_day, h_post, (unsigned)iter + 1)) goto fail;
+            if (irwls_dev_wait_post(&h_post->seq, (unsigned)iter + 1, 2 * sizeof(double) + sizeof(int))) goto fail;
+            dW = h_post->dW;
+            nW = h_post->nW;
+            nact = h_post->nact;
             ++iter;
             if (props.verbose == 1) printf("Iteration %d, nSVs %d, ||deltaW||^2/||W||^2=%f\n", iter, nact, dW / nW);
             if (iter > 10 && dW / nW > 100 * old) M = M / 10.0;
@@ -245,11 +242,11 @@ fail:
     rc = -1;
 done:
     {
-        void *bufs[] = {d_idx, d_act, d_nact, d_KC, d_KSC, d_K1, d_part, d_sd, d_day, d_e, d_Da, d_beta, d_bnew,
-                        d_bbest, d_nrm, d_A};
+        void *bufs[] = {d_idx, d_act, d_KC, d_KSC, d_K1, d_part, d_sd, d_day, d_e, d_Da, d_beta, d_bnew,
+                        d_bbest, d_A};
         for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
-        irwls_dev_host_free(h_nact);
-        irwls_dev_host_free(h_nrm);
+        if (rc) irwls_dev_sync(); /* (a kernel may still post) */
+        irwls_dev_host_free(h_post);
     }
     return rc ? -1 : 0;
 }

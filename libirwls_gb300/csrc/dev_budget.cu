@@ -752,13 +752,17 @@ __global__ void __launch_bounds__(256) weights_count_kernel(const double *__rest
 __global__ void __launch_bounds__(256) weights_write_kernel(const double *__restrict__ Da, const double *__restrict__ y,
                                                             int l, const int *__restrict__ cnt, int nb,
                                                             int *__restrict__ act, double *__restrict__ sd,
-                                                            double *__restrict__ day, int *__restrict__ nact) {
+                                                            double *__restrict__ day, irwls_par_post *h,
+                                                            unsigned seq) {
     __shared__ int ws[8];
     __shared__ int woff[8];
     int part = 0;
     for (int k = threadIdx.x; k < (int)blockIdx.x; k += 256) part += cnt[k];
     int base = block_sum256(part, ws);
-    if (blockIdx.x == nb - 1 && threadIdx.x == 0) nact[0] = base + cnt[nb - 1];
+    if (blockIdx.x == nb - 1 && threadIdx.x == 0) {
+        h->nact = base + cnt[nb - 1];
+        post_seq(&h->seq, seq);
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r0 = blockIdx.x * WB, r1 = min(l, r0 + WB);
     for (int i0 = r0; i0 < r1; i0 += 256) {
@@ -801,7 +805,7 @@ __global__ void first_weights_kernel(const double *__restrict__ y, int l, double
 
 // dW = |bnew - beta|^2, nW = |bnew|^2 (chunked, fixed order), beta <- bnew.
 __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bnew, double *beta, int m,
-                                                   double *out2) {
+                                                   irwls_par_post *h) {
     __shared__ double red[33];
     const int ch = (m + CT - 1) / CT;
     const int b = threadIdx.x * ch, e = min(m, b + ch);
@@ -816,8 +820,9 @@ __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bn
     __syncthreads();
     for (int i = b; i < e; ++i) beta[i] = bnew[i];
     if (threadIdx.x == 0) {
-        out2[0] = dW;
-        out2[1] = nW;
+        h->dW = dW;
+        h->nW = nW;
+        __threadfence_system();
     }
 }
 
@@ -1041,19 +1046,19 @@ extern "C" int irwls_par_residual(const double *d_KSC, int l, int m, const doubl
 }
 
 extern "C" int irwls_par_weights(const double *d_Da, const double *d_y, int l, int *d_act, double *d_sd,
-                                 double *d_day, int *d_nact) {
+                                 double *d_day, irwls_par_post *h, unsigned seq) {
     const int nb = std::max(1, ceil_div(l, WB));
     int *cnt = (int *)irwls_ctx_scratch(2, (size_t)nb * sizeof(int));
     if (!cnt) return -3;
     weights_count_kernel<<<nb, 256, 0, irwls_stream()>>>(d_Da, l, cnt);
     IRWLS_LAUNCH_CHECK("weights_count");
-    weights_write_kernel<<<nb, 256, 0, irwls_stream()>>>(d_Da, d_y, l, cnt, nb, d_act, d_sd, d_day, d_nact);
+    weights_write_kernel<<<nb, 256, 0, irwls_stream()>>>(d_Da, d_y, l, cnt, nb, d_act, d_sd, d_day, h, seq);
     IRWLS_LAUNCH_CHECK("weights_write");
     return 0;
 }
 
-extern "C" int irwls_par_delta(const double *d_bnew, double *d_beta, int m, double *d_out2) {
-    delta_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_beta, m, d_out2);
+extern "C" int irwls_par_delta(const double *d_bnew, double *d_beta, int m, irwls_par_post *h) {
+    delta_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_beta, m, h);
     IRWLS_LAUNCH_CHECK("delta");
     return 0;
 }

@@ -538,6 +538,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                                                                 const double *__restrict__ b, int *__restrict__ flags,
                                                                 double *__restrict__ Dinv,
                                                                 unsigned *__restrict__ ready, int *__restrict__ abort) {
+    chain_open();  // (the sweep may be made resident; it waits for the whole of this)
     extern __shared__ __align__(16) unsigned char df_smem[];
     DfShared &sh = *(DfShared *)df_smem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -928,13 +929,18 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
                                                                     const double *__restrict__ Dinv,
                                                                     double *__restrict__ x,
                                                                     const int *__restrict__ flags,
-                                                                    int *__restrict__ info) {
+                                                                    int *__restrict__ info,
+                                                                    unsigned *__restrict__ clear, int words) {
+    chain_wait();
+    chain_open();
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     __shared__ SweepShared sh;
     const int g = (int)cl.num_blocks(), me = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31;
     const int row = 8 * ((tid >> 5) & 3) + (lane >> 2), ch = tid & 3;  // row of a block, partial chain
     const int nblk = (n + NB - 1) / NB;
+    // the factorization's ready list, done with: zeros for the next one
+    for (int t = 256 * me + tid; t < words; t += 256 * g) clear[t] = 0;
     for (int e = tid; e < SWB * NB; e += 256) {
         const int c = ((e / NB) * g + me) * NB + e % NB;
         sh.z[e / NB][e % NB] = c < n ? M[(size_t)c * ld + n] : 0.0;
@@ -1099,13 +1105,19 @@ bool sweep_cluster_ok() {
 
 int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, double *Dinv, cudaStream_t st);
 int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
-                           cudaStream_t st);
+                           cudaStream_t st, unsigned *clear, size_t words, bool chained);
 
-// ready: the data-flow path's list (df_ready_words words), or NULL for the
-// multi-launch path. d_b: the right-hand side, or NULL when row n of M holds
+// Whether the cluster sweep takes order n.
+bool cluster_sweep_for(int n) { return n <= 8 * SWB * NB && sweep_cluster_ok(); }
+
+// ready: the data-flow path's list (df_ready_words words, all zero; it is left all
+// zero, by the cluster sweep or a memset: clearing it before the factorization
+// instead cost each solve 4 us), or NULL for the multi-launch path. chained: the
+// sweep may be a chained launch (a stream of this library).
+// d_b: the right-hand side, or NULL when row n of M holds
 // it. The pivot status starts at zero here; it goes to d_info (or NULL) too.
 int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int *flags, double *Dinv, int *d_info,
-                 cudaStream_t st, unsigned *ready = nullptr) {
+                 cudaStream_t st, unsigned *ready = nullptr, bool chained = false) {
     const int has_b = d_x != nullptr;
     const int nrows = n + has_b;
     const int G = ready && g_chol_path != 1 ? df_capacity() : 0;
@@ -1113,21 +1125,29 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
     if (G > 0) {
         // one cooperative launch of the data-flow factorization
         const size_t words = df_ready_words(n, has_b);
-        e = cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
         const int nbc = (n + NB - 1) / NB, nbr = (nrows + NB - 1) / NB;
         const int tasks = nbc * (2 * nbr - nbc + 1) / 2;
         int grid = std::min(G, tasks);
         int *abort = (int *)(ready + words - 1);
         const double *b = has_b ? d_b : nullptr;
         void *args[] = {&d_M, &n, &ld, (void *)&nrows, &b, &flags, &Dinv, &ready, &abort};
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(DF_THREADS), args,
+        e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(DF_THREADS), args,
                                             sizeof(DfShared), st);
         if (e != cudaSuccess) {
             irwls_set_error(-2, "CUDA error in chol_df (cooperative): %s", cudaGetErrorString(e));
             return -2;
         }
         irwls_count_launch(1);
+        if (has_b && cluster_sweep_for(n)) {
+            const int rc = chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, ready, words, chained);
+            if (rc) cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
+            return rc;
+        }
+        e = cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
+        if (e != cudaSuccess) {
+            irwls_set_error(-2, "CUDA error clearing the ready list: %s", cudaGetErrorString(e));
+            return -2;
+        }
     } else if (g_chol_path == 2) {
         irwls_set_error(-2, "the data-flow Cholesky needs a cooperative launch");
         return -2;
@@ -1143,7 +1163,7 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
         const int rc = chol_enqueue_panels(d_M, n, ld, nrows, flags, Dinv, st);
         if (rc) return rc;
     }
-    if (has_b) return chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st);
+    if (has_b) return chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, nullptr, 0, false);
     if (d_info && (e = cudaMemcpyAsync(d_info, flags, sizeof(int), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) {
         irwls_set_error(-2, "pivot status: %s", cudaGetErrorString(e));
         return -2;
@@ -1177,23 +1197,25 @@ int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, doubl
 // 2048, the cooperative one above, one CTA where neither can run. They give
 // the same bits.
 int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
-                           cudaStream_t st) {
+                           cudaStream_t st, unsigned *clear, size_t words, bool chained) {
     {
-        if (n <= 8 * SWB * NB && sweep_cluster_ok()) {
+        if (cluster_sweep_for(n)) {
             // two blocks a CTA, up to eight CTAs: one block's update holds the
             // FP64 units for 0.45 us, the chain of a block takes about 1.3
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(std::min(8, (n + 2 * NB - 1) / (2 * NB)));
             cfg.blockDim = dim3(256);
             cfg.stream = st;
-            cudaLaunchAttribute at[1];
+            cudaLaunchAttribute at[2];
             at[0].id = cudaLaunchAttributeClusterDimension;
             at[0].val.clusterDim.x = cfg.gridDim.x;
             at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = at;
-            cfg.numAttrs = 1;
+            cfg.numAttrs = chained ? 2 : 1;
             const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_sweep_cluster_kernel, (const double *)d_M, n, ld,
-                                                     (const double *)Dinv, d_x, flags, d_info);
+                                                     (const double *)Dinv, d_x, flags, d_info, clear, (int)words);
             if (e != cudaSuccess) {
                 irwls_set_error(-2, "CUDA error in chol_sweep (cluster): %s", cudaGetErrorString(e));
                 return -2;
@@ -1256,10 +1278,10 @@ extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_
     double *diag = (double *)irwls_ctx_scratch(0, (size_t)npanel * NB * NB * sizeof(double));
     if (!diag) return -3;
     // ready list of the data-flow path: the context's grow-only slot 3
-    unsigned *ready = (unsigned *)irwls_ctx_scratch(3, df_ready_words(n, d_x != nullptr) * sizeof(unsigned));
+    unsigned *ready = (unsigned *)irwls_ctx_scratch_zeroed(3, df_ready_words(n, d_x != nullptr) * sizeof(unsigned));
     if (!ready) return -3;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_CHOL);
-    int rc = chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, nullptr, irwls_stream(), ready);
+    int rc = chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, nullptr, irwls_stream(), ready, true);
     if (rc) return rc;
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_CHOL);
     return 0;

@@ -68,6 +68,8 @@ struct Ctx {
     char msg[512] = "";
     void *scratch[IRWLS_SCRATCH_SLOTS] = {};
     size_t scratch_bytes[IRWLS_SCRATCH_SLOTS] = {};
+    unsigned *post = nullptr;  // pinned words of irwls_ctx_post
+    unsigned post_seq = 0;
     int own_rng = 0;
     Rand31 rng;
 };
@@ -175,6 +177,7 @@ extern "C" void irwls_ctx_destroy(void *h) {
         if (c->scratch[k]) cudaFreeAsync(c->scratch[k], c->stream);
     cudaStreamSynchronize(c->stream);
     cudaFree(c->flags);
+    if (c->post) cudaFreeHost(c->post);
     cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -237,10 +240,62 @@ extern "C" void *irwls_ctx_scratch(int slot, size_t bytes) {
     return c->scratch[slot];
 }
 
+extern "C" int irwls_dev_host_alloc(void **p, size_t bytes);
+// The same with zeros in new memory (the users leave zeros behind).
+extern "C" void *irwls_ctx_scratch_zeroed(int slot, size_t bytes) {
+    Ctx *c = cur();
+    const bool fresh = bytes > c->scratch_bytes[slot];
+    void *p = irwls_ctx_scratch(slot, bytes);
+    if (p && fresh && cudaMemsetAsync(p, 0, bytes, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeAsync(c->scratch[slot], c->stream);
+        c->scratch[slot] = nullptr;
+        c->scratch_bytes[slot] = 0;
+        irwls_set_error(-2, "clearing %zu bytes of device scratch failed", bytes);
+        return nullptr;
+    }
+    return p;
+}
+
+// The context's pinned words for a kernel that posts one value (word 1) and its
+// number (word 0), and the next number; NULL: no memory.
+extern "C" unsigned *irwls_ctx_post(unsigned *seq) {
+    Ctx *c = cur();
+    if (!c->post) {
+        if (irwls_dev_host_alloc((void **)&c->post, 2 * sizeof(unsigned))) return nullptr;
+        c->post[0] = 0;
+    }
+    *seq = ++c->post_seq;
+    return c->post;
+}
+
 extern "C" int irwls_dev_sync(void) {
     cudaError_t e = cudaStreamSynchronize(cur()->stream);
     if (e != cudaSuccess) return cuda_fail(e, "stream synchronize");
     return 0;
+}
+
+// Waits until a kernel has posted `v` to *seq (post_seq). The stream is asked now
+// and then, so that a failed kernel ends the wait. bytes: what the host reads,
+// for the transfer counters.
+extern "C" void irwls_count_bytes(long long h2d, long long d2h);
+extern "C" int irwls_dev_wait_post(const unsigned *seq, unsigned v, size_t bytes) {
+    for (;;) {
+        for (int k = 0; k < 2000; ++k)
+            if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) == v) {
+                irwls_count_bytes(0, (long long)bytes);
+                return 0;
+            }
+        const cudaError_t e = cudaStreamQuery(cur()->stream);
+        if (e == cudaErrorNotReady) {
+            std::this_thread::yield();
+            continue;
+        }
+        if (e != cudaSuccess) return cuda_fail(e, "waiting for a kernel's result");
+        if (__atomic_load_n(seq, __ATOMIC_ACQUIRE) == v) continue;
+        irwls_set_error(-2, "a kernel ended without posting its result");
+        return -2;
+    }
 }
 
 extern "C" int irwls_dev_malloc(void **p, size_t bytes) {

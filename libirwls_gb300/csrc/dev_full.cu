@@ -181,6 +181,10 @@ __global__ void __launch_bounds__(NT) sub_init_kernel(irwls_sub_ws ws, const dou
         ws.stats->nW = 1.0;
         ws.stats->bmax = 0.0;
         ws.stats->bmin = 0.0;
+        ws.stats->best = 1e9;
+        ws.h_stats->nS1 = n1;
+        ws.h_stats->nS3 = n3;
+        post_seq(&ws.h_stats->seq, ws.seq);
     }
 }
 
@@ -371,14 +375,20 @@ __global__ void __launch_bounds__(NT) sub_update_kernel(irwls_sub_ws ws, double 
     if (threadIdx.x == 0) ws.cnt[0] = nl;
 }
 
-// a_i, groups, beta <- bnew, S1/S3 lists, G13[n1] (src/full-train.c:264-344).
+// a_i, groups, beta <- bnew, S1/S3 lists, G13[n1] (src/full-train.c:264-344), the
+// best iterate so far, and the iteration's results to the host.
 template <int NT>
 __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double C) {
     chain_wait();
     chain_open();
     __shared__ double buf[2][NT], part[2][4];
-    __shared__ int s_scan[32];
+    __shared__ int s_scan[32], s_better;
     const int w = ws.w;
+    if (threadIdx.x == 0) {
+        const double ratio = ws.stats->dW / ws.stats->nW;
+        s_better = ratio < ws.stats->best;
+        if (s_better) ws.stats->best = ratio;
+    }
     for (int i = threadIdx.x; i < w; i += NT) {
         const double yi = ws.y[i], ei = ws.e[i];
         const double ey = __dmul_rn(ei, yi);
@@ -398,6 +408,8 @@ __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double 
     }
     if (threadIdx.x == 0) ws.beta[w] = ws.bnew[w];
     __syncthreads();
+    if (s_better)
+        for (int i = threadIdx.x; i <= w; i += NT) ws.bbest[i] = ws.bnew[i];
     const int n1 = block_compact(w, [&](int i) { return ws.grp[i] == 1; },
                                  [&](int p, int i) {
                                      ws.S1[p] = i;
@@ -419,6 +431,14 @@ __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double 
         if (n3 > 0) ws.G13[n1] = g13;
         ws.stats->nS1 = n1;
         ws.stats->nS3 = n3;
+        irwls_sub_stats *h = ws.h_stats;
+        h->dW = ws.stats->dW;
+        h->nW = ws.stats->nW;
+        h->bmax = ws.stats->bmax;
+        h->bmin = ws.stats->bmin;
+        h->nS1 = n1;
+        h->nS3 = n3;
+        post_seq(&h->seq, ws.seq);
     }
 }
 
@@ -504,13 +524,15 @@ __global__ void __launch_bounds__(PC) norms_chunk_kernel(const double *__restric
     part[CT + t] = v2;
 }
 
-__global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restrict__ part, double *out2) {
+__global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restrict__ part, irwls_outer_counts *h,
+                                                         unsigned seq) {
     __shared__ double red[33];
     const double dW = chunk_tree_sum(part[threadIdx.x], red);
     const double nW = chunk_tree_sum(part[CT + threadIdx.x], red);
     if (threadIdx.x == 0) {
-        out2[0] = dW;
-        out2[1] = nW;
+        h->dW = dW;
+        h->nW = nW;
+        post_seq(&h->seq, seq);
     }
 }
 
@@ -591,7 +613,7 @@ __device__ __forceinline__ int classify_one(double bi, double ei, double yi, dou
 
 __global__ void __launch_bounds__(CT) classify_kernel(const double *__restrict__ bnew, const double *__restrict__ e,
                                                       const double *__restrict__ y, int l, double C, int *SW,
-                                                      int *SC, int *SIN, irwls_outer_counts *counts) {
+                                                      int *SC, int *SIN, irwls_outer_counts *h, unsigned seq) {
     __shared__ int s_scan[CT];
     __shared__ int first[6];
     if (threadIdx.x < 6) first[threadIdx.x] = 0x7fffffff;
@@ -611,9 +633,10 @@ __global__ void __launch_bounds__(CT) classify_kernel(const double *__restrict__
     const int nsc = block_compact(l, [&](int i) { return cat(i) == 1; }, [&](int p, int i) { SC[p] = i; }, s_scan);
     const int nin = block_compact(l, [&](int i) { return cat(i) == 0; }, [&](int p, int i) { SIN[p] = i; }, s_scan);
     if (threadIdx.x == 0) {
-        counts->nSW = nsw;
-        counts->nSC = nsc;
-        counts->nSIN = nin;
+        h->nSW = nsw;
+        h->nSC = nsc;
+        h->nSIN = nin;
+        post_seq(&h->seq, seq);
     }
 }
 
@@ -745,7 +768,7 @@ __global__ void __launch_bounds__(256) classify_count_kernel(const unsigned char
 __global__ void __launch_bounds__(256) classify_write_kernel(const unsigned char *__restrict__ code, int l,
                                                              const int *__restrict__ first,
                                                              const int *__restrict__ cnt, int nb, int *SW, int *SC,
-                                                             int *SIN, irwls_outer_counts *counts) {
+                                                             int *SIN, irwls_outer_counts *h, unsigned seq) {
     __shared__ int ws[3][8];
     int base[3];
     for (int k = 0; k < 3; ++k) {
@@ -754,9 +777,10 @@ __global__ void __launch_bounds__(256) classify_write_kernel(const unsigned char
         base[k] = bsum256(part, ws[0]);
     }
     if (blockIdx.x == nb - 1 && threadIdx.x == 0) {
-        counts->nSW = base[0] + cnt[3 * (nb - 1)];
-        counts->nSC = base[1] + cnt[3 * (nb - 1) + 1];
-        counts->nSIN = base[2] + cnt[3 * (nb - 1) + 2];
+        h->nSW = base[0] + cnt[3 * (nb - 1)];
+        h->nSC = base[1] + cnt[3 * (nb - 1) + 1];
+        h->nSIN = base[2] + cnt[3 * (nb - 1) + 2];
+        post_seq(&h->seq, seq);
     }
     int *const out[3] = {SW, SC, SIN};
     const int r0 = blockIdx.x * CB, r1 = min(l, r0 + CB);
@@ -906,6 +930,7 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
     if (cap <= SUB_K) rc |= irwls_dev_malloc((void **)&ws->K, nk * nk * sizeof(double));
     rc |= irwls_dev_malloc((void **)&ws->stats, sizeof(irwls_sub_stats));
     rc |= irwls_dev_host_alloc((void **)&ws->h_stats, sizeof(irwls_sub_stats));
+    if (ws->h_stats) memset(ws->h_stats, 0, sizeof(irwls_sub_stats));
     ws->map = ws->mapbuf;
     return rc ? -3 : 0;
 }
@@ -920,8 +945,13 @@ extern "C" void irwls_sub_release(irwls_sub_ws *ws) {
     memset(ws, 0, sizeof *ws);
 }
 
+extern "C" int irwls_sub_wait(irwls_sub_ws *ws) {
+    return irwls_dev_wait_post(&ws->h_stats->seq, ws->seq, sizeof(irwls_sub_stats));
+}
+
 extern "C" int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C) {
     const int w = ws->w;
+    ++ws->seq;
     if (w < 512) launch_chained(sub_init_kernel<512>, dim3(1), dim3(512), 0, *ws, X->y, C);
     else launch_chained(sub_init_kernel<CT>, dim3(1), dim3(CT), 0, *ws, X->y, C);
     IRWLS_LAUNCH_CHECK("sub_init");
@@ -1017,6 +1047,7 @@ extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, doubl
                                                  ws->e, ws->scal, ws->e))
             return -2;
     }
+    ++ws->seq;
     if (w < 512) launch_chained(sub_groups_kernel<512>, dim3(1), dim3(512), 0, *ws, C);
     else launch_chained(sub_groups_kernel<CT>, dim3(1), dim3(CT), 0, *ws, C);
     IRWLS_LAUNCH_CHECK("sub_groups");
@@ -1058,22 +1089,22 @@ extern "C" int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt,
     return 0;
 }
 
-extern "C" int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, double *d_out2) {
+extern "C" int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, irwls_outer_counts *h, unsigned seq) {
     double *part = (double *)irwls_ctx_scratch(2, (size_t)2 * CT * sizeof(double));
     if (!part) return -3;
     norms_chunk_kernel<<<CT / PC, PC, 0, irwls_stream()>>>(d_beta, d_bnew, n, part);
     IRWLS_LAUNCH_CHECK("norms_chunk");
-    norms_final_kernel<<<1, CT, 0, irwls_stream()>>>(part, d_out2);
+    norms_final_kernel<<<1, CT, 0, irwls_stream()>>>(part, h, seq);
     IRWLS_LAUNCH_CHECK("norms_final");
     return 0;
 }
 
 extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, const double *d_y, int l, double C,
-                                   int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *d_counts) {
+                                   int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *h, unsigned seq) {
     if (l <= CT) {
         // one round of one CTA is faster than four launches (at 4000 rows it
         // took 94 us: every row's FP64 tests four times on one SM)
-        classify_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_e, d_y, l, C, d_SW, d_SC, d_SIN, d_counts);
+        classify_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_e, d_y, l, C, d_SW, d_SC, d_SIN, h, seq);
         IRWLS_LAUNCH_CHECK("classify");
         return 0;
     }
@@ -1093,7 +1124,7 @@ extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, cons
     IRWLS_LAUNCH_CHECK("classify_code");
     classify_count_kernel<<<nb, 256, 0, irwls_stream()>>>(code, l, first, cnt);
     IRWLS_LAUNCH_CHECK("classify_count");
-    classify_write_kernel<<<nb, 256, 0, irwls_stream()>>>(code, l, first, cnt, nb, d_SW, d_SC, d_SIN, d_counts);
+    classify_write_kernel<<<nb, 256, 0, irwls_stream()>>>(code, l, first, cnt, nb, d_SW, d_SC, d_SIN, h, seq);
     IRWLS_LAUNCH_CHECK("classify_write");
     return 0;
 }

@@ -246,7 +246,7 @@ __device__ __forceinline__ uint32_t panel_bytes(int k, int NB, int p, int q) {
 
 __global__ void __launch_bounds__(WT, 1) ws_mixed_kernel(const double *__restrict__ H, int n1, int ld,
                                                        const double *__restrict__ rhs, double *__restrict__ x,
-                                                       int *__restrict__ flags) {
+                                                       int *__restrict__ flags, unsigned *post, unsigned seq) {
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ __align__(16) float sm[];
     __shared__ int bad_sh, flag_sh;
@@ -631,6 +631,8 @@ __global__ void __launch_bounds__(WT, 1) ws_mixed_kernel(const double *__restric
         int bad = 0;
         for (int r = 0; r < WC; ++r) bad |= *cl.map_shared_rank(&bad_sh, r);
         flags[2] = bad ? 1 : (converged ? 0 : 2);
+        post[1] = bad ? 1 : (converged ? 0 : 2);
+        post_seq(post, seq);
     }
     cl.sync();
 }
@@ -684,10 +686,12 @@ extern "C" int irwls_ws_mixed_max(void) { return cluster_ok() ? WNB * WB : 0; }
 // solution goes to x (n1 + 1 values). Returns 0 when solved, 1 when the FP32
 // factor or the refinement failed (x is then not written with a valid
 // solution and the caller solves in FP64), a negative code on a launch error.
-// Synchronizes the stream to read the outcome.
+// Waits for the outcome, which the kernel posts.
 extern "C" int irwls_ws_solve_mixed(const double *d_H, int n1, int ld, const double *d_rhs, double *d_x) {
     if (n1 < 1 || n1 > WNB * WB || ld < n1 + 1 || !cluster_ok()) return 1;
     int *flags = irwls_dev_flags();
+    unsigned seq, *post = irwls_ctx_post(&seq);
+    if (!post) return -3;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -701,19 +705,13 @@ extern "C" int irwls_ws_solve_mixed(const double *d_H, int n1, int ld, const dou
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_CHOL);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, ws_mixed_kernel, d_H, n1, ld, d_rhs, d_x, flags);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, ws_mixed_kernel, d_H, n1, ld, d_rhs, d_x, flags, post, seq);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_CHOL);
     if (e != cudaSuccess) {
         irwls_set_error(-2, "working-set cluster solve launch: %s", cudaGetErrorString(e));
         return -2;
     }
     IRWLS_LAUNCH_CHECK("ws_mixed");
-    int st = -1;
-    e = cudaMemcpyAsync(&st, flags + 2, sizeof(int), cudaMemcpyDeviceToHost, irwls_stream());
-    if (e == cudaSuccess) e = cudaStreamSynchronize(irwls_stream());
-    if (e != cudaSuccess) {
-        irwls_set_error(-2, "working-set cluster solve: %s", cudaGetErrorString(e));
-        return -2;
-    }
-    return st == 0 ? 0 : 1;
+    if (irwls_dev_wait_post(post, seq, sizeof(int))) return -2;
+    return post[1] == 0 ? 0 : 1;
 }

@@ -32,7 +32,7 @@ int *rpermute(int n) {
 static int run_sub(irwls_sub_ws *ws, const irwls_dev_set *X, const properties *props) {
     const double C = props->C;
     if (irwls_sub_init(ws, X, C)) return -1;
-    if (irwls_dev_d2h(ws->h_stats, ws->stats, sizeof(irwls_sub_stats)) || irwls_dev_sync()) return -1;
+    if (irwls_sub_wait(ws)) return -1;
     int n1 = ws->h_stats->nS1, n3 = ws->h_stats->nS3;
     int iter = 0, since_best = 0;
     double dW = 1e9, nW = 1.0, best = 1e9, bmax = 0.0, bmin = 0.0;
@@ -41,7 +41,7 @@ static int run_sub(irwls_sub_ws *ws, const irwls_dev_set *X, const properties *p
         /* G13 of the lists left by the previous iteration (zero before the first) */
         if (iter > 1 && irwls_sub_g13(ws, X, n1, n3)) return -1;
         if (irwls_sub_iterate(ws, X, C, n1, n3)) return -1;
-        if (irwls_dev_d2h(ws->h_stats, ws->stats, sizeof(irwls_sub_stats)) || irwls_dev_sync()) return -1;
+        if (irwls_sub_wait(ws)) return -1;
         const irwls_sub_stats *st = ws->h_stats;
         dW = st->dW;
         nW = st->nW;
@@ -49,8 +49,7 @@ static int run_sub(irwls_sub_ws *ws, const irwls_dev_set *X, const properties *p
         bmin = st->bmin;
         if (dW / nW < best) {
             best = dW / nW;
-            since_best = 0;
-            if (irwls_dev_d2d(ws->bbest, ws->bnew, (size_t)(ws->w + 1) * sizeof(double))) return -1;
+            since_best = 0;  /* (the kernels have copied the iterate to bbest) */
         } else {
             since_best += 1;
         }
@@ -105,10 +104,10 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         return -8;
     }
     int rc = 0;
-    double *e = NULL, *beta = NULL, *bnew = NULL, *cb = NULL, *dbias = NULL, *norms = NULL;
+    double *e = NULL, *beta = NULL, *bnew = NULL, *cb = NULL, *dbias = NULL;
     int *SW = NULL, *SIN = NULL, *SC = NULL, *lst = NULL, *cnt = NULL, *perm_d = NULL;
-    irwls_outer_counts *counts = NULL, *h_counts = NULL;
-    double *h_norms = NULL;
+    irwls_outer_counts *h_counts = NULL;
+    unsigned seq = 0;
     irwls_sub_ws ws;
     memset(&ws, 0, sizeof ws);
     const size_t L1 = (size_t)(l + 1);
@@ -137,16 +136,14 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     rc |= irwls_dev_malloc((void **)&bnew, L1 * sizeof(double));
     rc |= irwls_dev_malloc((void **)&cb, L1 * sizeof(double));
     rc |= irwls_dev_malloc((void **)&dbias, 2 * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&norms, 2 * sizeof(double));
     rc |= irwls_dev_malloc((void **)&SW, (W + 1) * sizeof(int));
     rc |= irwls_dev_malloc((void **)&SIN, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&SC, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&lst, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&perm_d, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&cnt, 2 * sizeof(int));
-    rc |= irwls_dev_malloc((void **)&counts, sizeof(irwls_outer_counts));
     rc |= irwls_dev_host_alloc((void **)&h_counts, sizeof(irwls_outer_counts));
-    rc |= irwls_dev_host_alloc((void **)&h_norms, 2 * sizeof(double));
+    if (h_counts) h_counts->seq = 0;
     rc |= irwls_sub_alloc(&ws, W);
     if (tcs) {
         rc |= irwls_dev_malloc((void **)&xflag, L1 * sizeof(int));
@@ -228,8 +225,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
             if (ex < 0 || (ex == 1 && irwls_dev_kernel_rowsum_n(X, NULL, l, X, lst, cnt, cb, NULL, NULL, -1, e, dbias, e)))
                 goto fail;
         }
-        if (irwls_full_norms(beta, bnew, l + 1, norms)) goto fail;
-        if (irwls_dev_d2h(h_norms, norms, 2 * sizeof(double)) || irwls_dev_sync()) goto fail;
+        if (irwls_full_norms(beta, bnew, l + 1, h_counts, ++seq)) goto fail;
+        if (irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(double))) goto fail;
         if (tcs) {
             /* a tensor-core wait that ran out left these errors stale: stop now */
             const int tc = irwls_tc_status();
@@ -239,7 +236,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
             }
             acc += eps * h_l1[0];
         }
-        const double ratio = h_norms[0] / h_norms[1];
+        const double ratio = h_counts->dW / h_counts->nW;
         if (ratio < props.Eta) stop = 1;
         if (irwls_dev_d2d(beta, bnew, L1 * sizeof(double))) goto fail;
         if (ratio < best) {
@@ -249,8 +246,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
             since_best += 1;
         }
         /* classification and the next working set (:540-643) */
-        if (irwls_full_classify(bnew, e, X->y, l, C, SW, SC, SIN, counts)) goto fail;
-        if (irwls_dev_d2h(h_counts, counts, sizeof(irwls_outer_counts)) || irwls_dev_sync()) goto fail;
+        if (irwls_full_classify(bnew, e, X->y, l, C, SW, SC, SIN, h_counts, ++seq)) goto fail;
+        if (irwls_dev_wait_post(&h_counts->seq, seq, 4 * sizeof(int))) goto fail;
         nSW = h_counts->nSW;
         nSIN = h_counts->nSIN;
         const int nSC = h_counts->nSC;
@@ -320,10 +317,9 @@ done:
     for (size_t k = 0; k < sizeof xbufs / sizeof xbufs[0]; k++) irwls_dev_free(xbufs[k]);
     irwls_dev_host_free(h_xcnt);
     irwls_dev_host_free(h_l1);
-    void *bufs[] = {e, beta, bnew, cb, dbias, norms, SW, SIN, SC, lst, perm_d, cnt, counts};
+    void *bufs[] = {e, beta, bnew, cb, dbias, SW, SIN, SC, lst, perm_d, cnt};
     for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
     irwls_dev_host_free(h_counts);
-    irwls_dev_host_free(h_norms);
     return rc ? -1 : 0;
 }
 

@@ -40,10 +40,14 @@ void irwls_ctx_bind(void *h);
 void irwls_ctx_destroy(void *h);
 int irwls_ctx_error(void *h, char *msg, int cap);
 void *irwls_ctx_scratch(int slot, size_t bytes);   /* grow-only, slots 0..3 */
+void *irwls_ctx_scratch_zeroed(int slot, size_t bytes);
 /* The context's random numbers: libc srand/rand in the default context, a
  * generator that reproduces them exactly in worker contexts. */
 void irwls_srand(unsigned seed);
 int irwls_rand(void);
+/* a kernel's result in pinned host memory: waits for its number */
+int irwls_dev_wait_post(const unsigned *seq, unsigned v, size_t bytes);
+unsigned *irwls_ctx_post(unsigned *seq);
 int irwls_dev_malloc(void **p, size_t bytes);
 int irwls_dev_free(void *p);
 int irwls_dev_h2d(void *d_dst, const void *h_src, size_t bytes);   /* async */
@@ -136,8 +140,9 @@ int irwls_dev_gemv(const double *d_A, const double *d_v, double *d_out, int size
 
 /* ---- full IRWLS steps (dev_full.cu) -------------------------------------- */
 typedef struct irwls_sub_stats {
-    double dW, nW, bmax, bmin;
-    int nS1, nS3, pad0, pad1;
+    double dW, nW, bmax, bmin, best;  /* best: the smallest dW / nW so far, of bbest */
+    int nS1, nS3;
+    unsigned seq, pad;
 } irwls_sub_stats;
 
 /* The inner-IRWLS device state on a working set of w rows; map[i] is the
@@ -151,7 +156,8 @@ typedef struct irwls_sub_ws {
     int *grp, *S1, *S3, *lst, *lloc, *gl1, *gl3, *cnt, *mapbuf;   /* lst, lloc: changed weights, as rows of X and of the set */
     int use13;            /* this iteration's G13 is not zero */
     irwls_sub_stats *stats;   /* device */
-    irwls_sub_stats *h_stats; /* pinned host mirror */
+    irwls_sub_stats *h_stats; /* pinned host mirror, written by the last kernel of a step */
+    unsigned seq;             /* number of the last step */
     int ldH;
     void *tcs;                /* precision form: the training's tensor-core set (NULL: FP64 throughout) */
 } irwls_sub_ws;
@@ -159,7 +165,7 @@ typedef struct irwls_sub_ws {
 int irwls_sub_alloc(irwls_sub_ws *ws, int cap);
 void irwls_sub_release(irwls_sub_ws *ws);
 /* a_i and the groups at entry (src/full-train.c:131-155); e, beta and map
- * must be set; stats->nS1/nS3 filled. */
+ * must be set; nS1 and nS3 posted (irwls_sub_wait). */
 int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C);
 /* G13 of the current S1/S3 lists (src/full-train.c:327-344), for the next
  * irwls_sub_iterate. */
@@ -167,21 +173,25 @@ int irwls_sub_g13(irwls_sub_ws *ws, const irwls_dev_set *X, int n1, int n3);
 /* One inner iteration: H and rhs, solve, weights, working-set error update,
  * a_i and groups (src/full-train.c:160-307). */
 int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, double C, int n1, int n3);
+/* the last step's results are in h_stats */
+int irwls_sub_wait(irwls_sub_ws *ws);
 
 /* Outer-loop steps (src/full-train.c:436-643). d_lst/d_cb/d_cnt are scratch
  * lists of at least l entries. */
 typedef struct irwls_outer_counts {
-    int nSW, nSIN, nSC, pad;
-} irwls_outer_counts;
+    double dW, nW;
+    int nSW, nSIN, nSC;
+    unsigned seq;  /* number of the last post */
+} irwls_outer_counts;  /* pinned: written by norms (dW, nW) and classify (the counts) */
 int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, const int *d_SIN, int nSIN,
                    const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN, void *exact);
 int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e, const double *d_beta, int l,
                          double *d_esub, double *d_bsub);
 int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt, const double *d_beta, int l,
                         double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_dbias);
-int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, double *d_out2);
+int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, irwls_outer_counts *h, unsigned seq);
 int irwls_full_classify(const double *d_bnew, const double *d_e, const double *d_y, int l, double C,
-                        int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *d_counts);
+                        int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *h, unsigned seq);
 int irwls_full_fill_ws(int *d_SW, int nSW, int *d_SIN, int nSIN, const int *d_SC, int nSC,
                        const int *d_perm, int space);
 
@@ -226,9 +236,16 @@ int irwls_par_gram_tc(const double *d_KSC, int m, const int *d_act, int nact, co
 int irwls_par_gram_reduce(const double *d_part, int P, int m, const double *d_KC, double *d_K1, int ldK1);
 int irwls_par_residual(const double *d_KSC, int l, int m, const double *d_beta, const double *d_y, double C,
                        double M, double *d_e, double *d_Da);
+/* one iteration's results in pinned host memory: delta writes dW and nW, weights
+ * nact and then the iteration's number */
+typedef struct irwls_par_post {
+    double dW, nW;
+    int nact;
+    unsigned seq;
+} irwls_par_post;
 int irwls_par_weights(const double *d_Da, const double *d_y, int l, int *d_act, double *d_sd, double *d_day,
-                      int *d_nact);
-int irwls_par_delta(const double *d_bnew, double *d_beta, int m, double *d_out2);
+                      irwls_par_post *h, unsigned seq);
+int irwls_par_delta(const double *d_bnew, double *d_beta, int m, irwls_par_post *h);
 
 /* Precision form of full IRWLS (dev_tc.cu): split-BF16 copy of a set and the
  * tensor-core error update out_i = (init_i - sum_j cb_j k(x_i, x_{idx_j})) -
