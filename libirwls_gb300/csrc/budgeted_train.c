@@ -206,7 +206,9 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
                          : irwls_par_gram_fp64(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P))
                 goto fail;
             g_gram_flops += (double)nact * (m + 1) * m;
-            if (irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)) goto fail;
+            if (digits && !mixed ? irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)
+                                 : irwls_dev_chol_solve_order(d_K1, m, ld, NULL, d_bnew))
+                goto fail;
             if (irwls_par_delta(d_bnew, d_beta, m, h_post)) goto fail;
             if (irwls_par_residual(d_KSC, l, m, d_beta, X->y, C, M, d_e, d_Da)) goto fail;
             if (irwls_par_weights(d_Da, X->y, l, d_act, d_sd, d_day, h_post, (unsigned)iter + 1)) goto fail;

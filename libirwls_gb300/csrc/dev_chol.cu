@@ -533,11 +533,15 @@ __device__ void factor_stream(DfShared &sh, const FactorPart &f, int nb, int k0,
 
 // ready: columns published of diag[j] at ready[j] (j < nbc), of tile L(i, j)
 // at ready[nbc + j * nbr + i]. b: the right-hand side (row n), or NULL when
-// it is in row n of M already.
+// it is in row n of M already. ninv: the leading diagonal blocks whose inverse the
+// sweep reads; of the others it gets the reciprocal pivots (the diagonal). The
+// last block's inverse, which nothing else hides, goes when the sweep substitutes
+// that block: 50 us a solve of order 64, with the inverse 59.
 __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restrict__ M, int n, int ld, int nrows,
                                                                 const double *__restrict__ b, int *__restrict__ flags,
                                                                 double *__restrict__ Dinv,
-                                                                unsigned *__restrict__ ready, int *__restrict__ abort) {
+                                                                unsigned *__restrict__ ready, int *__restrict__ abort,
+                                                                int ninv) {
     chain_open();  // (the sweep may be made resident; it waits for the whole of this)
     extern __shared__ __align__(16) unsigned char df_smem[];
     DfShared &sh = *(DfShared *)df_smem;
@@ -769,7 +773,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
                     if (lane < nc) M[(size_t)(c0 + lane) * ld + r0 + nc] = v;
                 }
                 // the inverse (for the backward sweep after this launch)
-                invert_columns(sh.T, sh.Di, sh.rp, nc);
+                if (j < ninv) invert_columns(sh.T, sh.Di, sh.rp, nc);
+                else if (tid < nc) sh.Di[tid][tid] = sh.rp[tid];
                 bar_sync<BAR_ALL, 256>();
                 for (int e = tid; e < NB * NB; e += 256) Dinv[(size_t)j * NB * NB + e] = sh.Di[e / NB][e % NB];
             } else {
@@ -914,6 +919,8 @@ __global__ void __launch_bounds__(256) chol_backsolve_coop_kernel(double *__rest
 // chain warps when x_(q+2) is in it. A dot product's four partial chains
 // (sweep_dot, sweep_row) run on four lanes, eight FMAs each, instead of one
 // after another on one: 65 cycles per FP64 instruction whatever the lanes.
+// subst: the last block by substitution with its L and reciprocal pivots, 5000
+// cycles once, instead of an inverse formed at the factorization's end.
 __device__ __forceinline__ double chains_sum(double a) {
     a += __shfl_xor_sync(0xffffffffu, a, 1);
     return a + __shfl_xor_sync(0xffffffffu, a, 2);  // (a0 + a1) + (a2 + a3)
@@ -923,6 +930,7 @@ constexpr int SWB = 8;                // blocks of a CTA
 constexpr int SWN = 8 * SWB;          // blocks of the largest order
 struct SweepShared {
     double z[SWB][NB], xb[SWN][NB], Di[2][NB][NB + 1];
+    double rp[NB];                  // reciprocal pivots of the last block (with subst)
     uint64_t got[SWN], ready[SWB];  // x_b has arrived; a block has all but its last update
 };
 __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double *__restrict__ M, int n, int ld,
@@ -930,7 +938,8 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
                                                                     double *__restrict__ x,
                                                                     const int *__restrict__ flags,
                                                                     int *__restrict__ info,
-                                                                    unsigned *__restrict__ clear, int words) {
+                                                                    unsigned *__restrict__ clear, int words,
+                                                                    int subst) {
     chain_wait();
     chain_open();
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -955,7 +964,18 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
     auto load_inv = [&](int b, int t0, int nt) {
         for (int t = t0; t < NB * NB; t += nt) sh.Di[b & 1][t / NB][t % NB] = Dinv[(size_t)b * NB * NB + t];
     };
-    if ((nblk - 1) % g == me) load_inv(nblk - 1, tid, 256);
+    if ((nblk - 1) % g == me) {
+        const int b = nblk - 1, nb = n - NB * b;
+        if (subst) {
+            for (int t = tid; t < NB * NB; t += 256) {
+                const int r = t % NB, c = t / NB;
+                if (c <= r && r < nb) sh.Di[b & 1][r][c] = M[(size_t)(NB * b + c) * ld + NB * b + r];
+            }
+            if (tid < nb) sh.rp[tid] = Dinv[(size_t)b * NB * NB + tid * NB + tid];
+        } else {
+            load_inv(b, tid, 256);
+        }
+    }
     if (info && me == 0 && tid == 0) *info = *flags;
     cl.sync();
     // this thread's values of rows of L_b^T for block q (4 k + ch)
@@ -991,10 +1011,25 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
                 const double(*D)[NB + 1] = sh.Di[b & 1];
                 const double *yb = sh.z[b / g];
                 double a = 0.0;
-                for (int k = 0; k < K; ++k) a = fma(D[t + 4 * k + ch][t], yb[t + 4 * k + ch], a);
-                if (ch == 0)
-                    for (int c = t + 4 * K; c < nb; ++c) a = fma(D[c][t], yb[c], a);
-                a = chains_sum(a);
+                if (subst && b == nblk - 1) {
+                    if (tid < 32) {
+                        double v = lane < nb ? sh.z[b / g][lane] : 0.0;
+                        for (int q = nb - 1; q >= 0; --q) {
+                            const double l = D[q][min(lane, q)];
+                            if (lane == q) v = v * sh.rp[q];
+                            const double xq = __shfl_sync(0xffffffffu, v, q);
+                            if (lane < q) v = fma(-l, xq, v);
+                        }
+                        if (lane < nb) sh.z[b / g][lane] = v;
+                    }
+                    asm volatile("bar.sync 1, 128;\n" ::: "memory");
+                    if (t < nb) a = yb[t];
+                } else {
+                    for (int k = 0; k < K; ++k) a = fma(D[t + 4 * k + ch][t], yb[t + 4 * k + ch], a);
+                    if (ch == 0)
+                        for (int c = t + 4 * K; c < nb; ++c) a = fma(D[c][t], yb[c], a);
+                    a = chains_sum(a);
+                }
                 if (t < nb) {
                     // lane ch of the row sends to CTAs ch, ch + 4
                     if (b > 0)
@@ -1105,7 +1140,7 @@ bool sweep_cluster_ok() {
 
 int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, double *Dinv, cudaStream_t st);
 int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
-                           cudaStream_t st, unsigned *clear, size_t words, bool chained);
+                           cudaStream_t st, unsigned *clear, size_t words, bool chained, bool subst);
 
 // Whether the cluster sweep takes order n.
 bool cluster_sweep_for(int n) { return n <= 8 * SWB * NB && sweep_cluster_ok(); }
@@ -1113,14 +1148,16 @@ bool cluster_sweep_for(int n) { return n <= 8 * SWB * NB && sweep_cluster_ok(); 
 // ready: the data-flow path's list (df_ready_words words, all zero; it is left all
 // zero, by the cluster sweep or a memset: clearing it before the factorization
 // instead cost each solve 4 us), or NULL for the multi-launch path. chained: the
-// sweep may be a chained launch (a stream of this library).
+// sweep may be a chained launch (a stream of this library). order: every block of the
+// sweep through its inverse (irwls_dev_chol_solve_order).
 // d_b: the right-hand side, or NULL when row n of M holds
 // it. The pivot status starts at zero here; it goes to d_info (or NULL) too.
 int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int *flags, double *Dinv, int *d_info,
-                 cudaStream_t st, unsigned *ready = nullptr, bool chained = false) {
+                 cudaStream_t st, unsigned *ready = nullptr, bool chained = false, bool order = false) {
     const int has_b = d_x != nullptr;
     const int nrows = n + has_b;
     const int G = ready && g_chol_path != 1 ? df_capacity() : 0;
+    const bool subst = !order && cluster_sweep_for(n);
     cudaError_t e = cudaSuccess;
     if (G > 0) {
         // one cooperative launch of the data-flow factorization
@@ -1130,7 +1167,8 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
         int grid = std::min(G, tasks);
         int *abort = (int *)(ready + words - 1);
         const double *b = has_b ? d_b : nullptr;
-        void *args[] = {&d_M, &n, &ld, (void *)&nrows, &b, &flags, &Dinv, &ready, &abort};
+        int ninv = has_b ? nbc - subst : 0;
+        void *args[] = {&d_M, &n, &ld, (void *)&nrows, &b, &flags, &Dinv, &ready, &abort, &ninv};
         e = cudaLaunchCooperativeKernel((const void *)chol_df_kernel, dim3(grid), dim3(DF_THREADS), args,
                                             sizeof(DfShared), st);
         if (e != cudaSuccess) {
@@ -1139,7 +1177,7 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
         }
         irwls_count_launch(1);
         if (has_b && cluster_sweep_for(n)) {
-            const int rc = chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, ready, words, chained);
+            const int rc = chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, ready, words, chained, subst);
             if (rc) cudaMemsetAsync(ready, 0, words * sizeof(unsigned), st);
             return rc;
         }
@@ -1163,7 +1201,7 @@ int chol_enqueue(double *d_M, int n, int ld, const double *d_b, double *d_x, int
         const int rc = chol_enqueue_panels(d_M, n, ld, nrows, flags, Dinv, st);
         if (rc) return rc;
     }
-    if (has_b) return chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, nullptr, 0, false);
+    if (has_b) return chol_enqueue_backsolve(d_M, n, ld, d_x, Dinv, flags, d_info, st, nullptr, 0, false, subst);
     if (d_info && (e = cudaMemcpyAsync(d_info, flags, sizeof(int), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) {
         irwls_set_error(-2, "pivot status: %s", cudaGetErrorString(e));
         return -2;
@@ -1197,7 +1235,7 @@ int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, doubl
 // 2048, the cooperative one above, one CTA where neither can run. They give
 // the same bits.
 int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
-                           cudaStream_t st, unsigned *clear, size_t words, bool chained) {
+                           cudaStream_t st, unsigned *clear, size_t words, bool chained, bool subst) {
     {
         if (cluster_sweep_for(n)) {
             // two blocks a CTA, up to eight CTAs: one block's update holds the
@@ -1215,7 +1253,7 @@ int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv
             cfg.attrs = at;
             cfg.numAttrs = chained ? 2 : 1;
             const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_sweep_cluster_kernel, (const double *)d_M, n, ld,
-                                                     (const double *)Dinv, d_x, flags, d_info, clear, (int)words);
+                                                     (const double *)Dinv, d_x, flags, d_info, clear, (int)words, (int)subst);
             if (e != cudaSuccess) {
                 irwls_set_error(-2, "CUDA error in chol_sweep (cluster): %s", cudaGetErrorString(e));
                 return -2;
@@ -1266,7 +1304,7 @@ extern "C" int irwls_dev_zero_upper(double *d_M, int n, int ld) {
     return 0;
 }
 
-extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_b, double *d_x) {
+static int chol_solve(double *d_M, int n, int ld, const double *d_b, double *d_x, bool order) {
     if (n <= 0) return 0;
     if (ld < n + 1) {
         irwls_set_error(-6, "Cholesky leading dimension %d < n + 1 = %d", ld, n + 1);
@@ -1281,10 +1319,21 @@ extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_
     unsigned *ready = (unsigned *)irwls_ctx_scratch_zeroed(3, df_ready_words(n, d_x != nullptr) * sizeof(unsigned));
     if (!ready) return -3;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_CHOL);
-    int rc = chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, nullptr, irwls_stream(), ready, true);
+    int rc = chol_enqueue(d_M, n, ld, d_b, d_x, flags, diag, nullptr, irwls_stream(), ready, true, order);
     if (rc) return rc;
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_CHOL);
     return 0;
+}
+
+extern "C" int irwls_dev_chol_solve(double *d_M, int n, int ld, const double *d_b, double *d_x) {
+    return chol_solve(d_M, n, ld, d_b, d_x, false);
+}
+
+// The same with the backward sweep's last block through its inverse as the others,
+// for callers whose results move far beyond its rounding (IRWLSpar on SGMA
+// centroids can multiply that by 10^8).
+extern "C" int irwls_dev_chol_solve_order(double *d_M, int n, int ld, const double *d_b, double *d_x) {
+    return chol_solve(d_M, n, ld, d_b, d_x, true);
 }
 
 extern "C" int irwls_chol_sweep_ctas(int n) { return coop_backsolve_ctas(n); }

@@ -23,6 +23,7 @@ def test_against_exact_products(l, m, nact, P):
     act = np.sort(rng.choice(l, nact, replace=False)).astype(np.int32)
     sd, day = rng.uniform(0.1, 30.0, nact), rng.standard_normal(nact)
     lib = load()
+    assert lib.irwls_dev_init() == 0
     lib.irwls_dev_malloc.argtypes = [C.POINTER(VP), C.c_size_t]
     lib.irwls_dev_h2d.argtypes = lib.irwls_dev_d2h.argtypes = [VP, VP, C.c_size_t]
     lib.irwls_dev_free.argtypes = [VP]

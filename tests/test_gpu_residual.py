@@ -19,6 +19,7 @@ def test_errors_and_weights(l, m):
     K, beta, y = rng.standard_normal((l, m)), rng.standard_normal(m), np.where(rng.random(l) < 0.5, -1.0, 1.0)
     cost, top = 3.0, 1e4
     lib = load()
+    assert lib.irwls_dev_init() == 0
     lib.irwls_dev_malloc.argtypes = [C.POINTER(VP), C.c_size_t]
     lib.irwls_dev_h2d.argtypes = lib.irwls_dev_d2h.argtypes = [VP, VP, C.c_size_t]
     lib.irwls_dev_free.argtypes = [VP]
