@@ -1,21 +1,12 @@
 // dev_predict.cu -- batched prediction f(x_i) = bias + sum_j w_j k(x_i, sv_j)
-// (reference src/LIBIRWLS-predict.c:56-131): small batches as an ordered kernel
-// row sum in FP64, the support vectors in the reference's order; large ones from
-// the tensor cores (dev_predict_tc.cu). The sign is taken on the device.
+// (reference src/LIBIRWLS-predict.c:56-131): small batches and linear kernels as
+// FP64 row sums (dev_tiles.cu), large RBF ones from the tensor cores
+// (dev_predict_tc.cu). The sign is taken on the device.
 #include <algorithm>
 
 #include "dev_common.cuh"
 
 namespace {
-
-__global__ void fill_kernel(double *p, int n, double v) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
-}
-
-__global__ void sign_kernel(double *p, int n) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        p[i] = (p[i] >= 0.0) ? 1.0 : -1.0;
-}
 
 // Linear-kernel fast path: W[c] = sum_j w_j sv_j[c]. Block b sums the
 // support vectors of chunk b (LW_CHUNK of them, model order) for every
@@ -93,23 +84,13 @@ extern "C" int irwls_predict_linear(const irwls_dev_set *T, int n, const irwls_d
 }
 
 // f_i of every row, or its sign: on the tensor cores where that path takes the
-// sizes and values (dev_predict_tc.cu), else as ordered FP64 row sums.
+// sizes and values (dev_predict_tc.cu), else on the FP64 pipe.
 extern "C" int irwls_predict_soft(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                                   double bias, int hard, double *d_out) {
     if (n <= 0) return 0;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_PREDICT);
     int rc = irwls_predict_exact(T, n, S, nSV, d_w, bias, hard, d_out);
-    const bool ordered = rc == 1;
-    if (ordered) {
-        fill_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n, bias);
-        IRWLS_LAUNCH_CHECK("fill");
-        rc = irwls_dev_predict_rowsum(T, n, S, nSV, d_w, d_out);
-    }
+    if (rc == 1) rc = irwls_dev_predict_rows(T, n, S, nSV, d_w, bias, hard, d_out);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_PREDICT);
-    if (rc) return rc;
-    if (hard && ordered) {
-        sign_kernel<<<ceil_div(n, 256), 256, 0, irwls_stream()>>>(d_out, n);
-        IRWLS_LAUNCH_CHECK("sign");
-    }
-    return 0;
+    return rc;
 }

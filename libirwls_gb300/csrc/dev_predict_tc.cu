@@ -575,9 +575,9 @@ int slice_grid(long long rows, int npb, int sms) {
 // features or weights that are not finite, values whose squares leave FP32's
 // range or whose y does not fit its fixed point, no room for the workspace, or
 // fewer than 500000 kernel values: the preparation and the host's wait for the
-// maxima cost about 60 us. A call with 250000 values (1000 vectors) took 202 us
-// there and 206 us here with 20 features a row, 180 and 180 with 11 of 54, 1109
-// and 817 with 300; one with 10^6 values 335 and 232, 345 and 199, 2724 and 997.
+// maxima cost about 60 us. A call with 500000 values (1000 vectors) took 190 us there
+// and 200 here with 20 features a row, 192 and 178 with 12 of 54, 1558 and 919 with
+// 300; with 250 vectors 202 and 208, 202 and 186, 1364 and 745.
 extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                                    double bias, int hard, double *d_out) {
     constexpr double MIN_VALUES = 5.0e5;

@@ -6,6 +6,8 @@
 // looked up against the dense A row, so stored zeros cost nothing. The work
 // is FP64-ALU bound on GB300, so the design minimises FP64 instructions per
 // kernel entry; memory traffic is a few bytes per entry and hits L1/L2.
+#include <algorithm>
+
 #include "dev_common.cuh"
 
 namespace {
@@ -57,11 +59,7 @@ __global__ void __launch_bounds__(kThreads) kernel_block_kernel(KView A, const i
 
 // Ordered row sums. CTA = R output rows x all B; B is swept in chunks of
 // JB = 1024 / R columns: every thread evaluates 4 terms into shared memory,
-// then one thread per row folds the chunk left to right. FUSED (linear kernels
-// in prediction): a stored value's product and addition are one rounding, which
-// halves the FP64 instructions that bound the kernel (9000 rows of 33 values against
-// 1501 vectors: 1068 us, 2000 with a multiply and an add).
-template <bool FUSED>
+// then one thread per row folds the chunk left to right.
 __global__ void __launch_bounds__(kThreads) kernel_rowsum_kernel(KView A, const int *__restrict__ ia, int nA, KView B,
                                                                  const int *__restrict__ ib, int nB,
                                                                  const int *__restrict__ nBp, int R,
@@ -91,8 +89,7 @@ __global__ void __launch_bounds__(kThreads) kernel_rowsum_kernel(KView A, const 
             if (jj < jn && i < nA) {
                 const int j = j0 + jj;
                 const int jb = ib ? ib[j] : j;
-                const double *a = sA + (size_t)r * A.ld;
-                const double kv = FUSED ? sparse_dot_fused(a, B, jb) : kentry(B, a, sQ[r], jb);
+                double kv = kentry(B, sA + (size_t)r * A.ld, sQ[r], jb);
                 term = cb ? __dmul_rn(cb[j], kv) : kv;
                 if (sa) term = __dmul_rn(term, sa[ia ? ia[i] : i]);
                 if (sb) term = __dmul_rn(term, sb[jb]);
@@ -110,6 +107,38 @@ __global__ void __launch_bounds__(kThreads) kernel_rowsum_kernel(KView A, const 
         __syncthreads();
     }
     if (folder) out[me] = tail ? __dsub_rn(acc, tail[0]) : acc;
+}
+
+// Prediction's row sums (and the sign with hard): 256 / R threads per row, thread t
+// the vectors t, t + 256 / R, ..., the threads' sums by a fixed tree. Nothing is
+// handed over or waited for before the end; the training's ordered sums fold each
+// row in one thread, 65 cycles a vector that a small batch leaves exposed (64 rows
+// of 20 values against 400 vectors: 11 us, ordered 27) and that use R lanes of the
+// FP64 pipe's 32. Linear kernels round once per stored value, half the FP64
+// instructions that bound the kernel (9000 rows of 33 values against 1501 vectors:
+// 932 us, ordered 2000, at the pipe's peak 840).
+__global__ void __launch_bounds__(kThreads) predict_rows_kernel(KView A, int nA, KView B, int nB, int R,
+                                                                const double *__restrict__ w, double bias, int hard,
+                                                                double *__restrict__ out) {
+    extern __shared__ double smem[];
+    __shared__ double sQ[8], red[8];
+    const int i0 = blockIdx.x * R;
+    stage_rows(smem, sQ, A, nullptr, i0, R, nA);
+    const int per = kThreads / R, r = threadIdx.x / per;
+    const double *a = smem + (size_t)r * A.ld;
+    double acc = 0.0;
+    if (i0 + r < nA)
+        for (int j = threadIdx.x % per; j < nB; j += per)
+            acc = fma(w[j], B.mode == IRWLS_K_LINEAR ? sparse_dot_fused(a, B, j) : kentry(B, a, sQ[r], j), acc);
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x < R && i0 + threadIdx.x < nA) {
+        double f = 0.0;
+        for (int k = 0; k < 8 / R; ++k) f += red[threadIdx.x * (8 / R) + k];
+        f += bias;
+        out[i0 + threadIdx.x] = hard ? (f >= 0.0 ? 1.0 : -1.0) : f;
+    }
 }
 
 }  // namespace
@@ -136,24 +165,30 @@ extern "C" int irwls_dev_kernel_block(const irwls_dev_set *A, const int *d_ia, i
     return irwls_dev_kernel_block_t(A, d_ia, nA, B, d_ib, nB, d_out, ld_out, 0);
 }
 
-static int rowsum_launch(const irwls_dev_set *A, const int *d_ia, int nA, const irwls_dev_set *B, const int *d_ib,
-                         int nB, const int *d_nB, const double *d_cb, const double *d_sa, const double *d_sb, int op,
-                         const double *d_init, const double *d_tail, double *d_out, bool fused) {
-    if (nA <= 0) return 0;
-    // rows per CTA: enough CTAs to cover the SMs twice, at most 8
+// Rows per CTA: enough CTAs to cover the SMs twice, at most 8; 0 and an error
+// where a row does not fit.
+static int rowsum_rows(const irwls_dev_set *A, int nA) {
     int R = 8;
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
     while (R > 1 && ceil_div(nA, R) < 2 * sms) R >>= 1;
     while (R > 1 && rows_per_cta(A->ld, R) < R) R >>= 1;
     if (rows_per_cta(A->ld, R) < R) {
         irwls_set_error(-5, "feature width %d is too wide for the shared-memory tile", A->width);
-        return -5;
+        return 0;
     }
+    return R;
+}
+
+static int rowsum_launch(const irwls_dev_set *A, const int *d_ia, int nA, const irwls_dev_set *B, const int *d_ib,
+                         int nB, const int *d_nB, const double *d_cb, const double *d_sa, const double *d_sb, int op,
+                         const double *d_init, const double *d_tail, double *d_out) {
+    if (nA <= 0) return 0;
+    const int R = rowsum_rows(A, nA);
+    if (!R) return -5;
     const size_t smem = ((size_t)R * A->ld + 8 + 1024) * sizeof(double);
-    auto kern = fused ? kernel_rowsum_kernel<true> : kernel_rowsum_kernel<false>;
-    if (smem > 48 * 1024) allow_smem(kern);
+    if (smem > 48 * 1024) allow_smem(kernel_rowsum_kernel);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
-    kern<<<ceil_div(nA, R), kThreads, smem, irwls_stream()>>>(
+    kernel_rowsum_kernel<<<ceil_div(nA, R), kThreads, smem, irwls_stream()>>>(
         kview(A), d_ia, nA, kview(B), d_ib, nB > 0 ? nB : 0, d_nB, R, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_ROWSUM);
     IRWLS_LAUNCH_CHECK("kernel_rowsum");
@@ -165,20 +200,27 @@ extern "C" int irwls_dev_kernel_rowsum(const irwls_dev_set *A, const int *d_ia, 
                                        const double *d_sb, int k_first, int op, const double *d_init,
                                        const double *d_tail, double *d_out) {
     (void)k_first;  // IEEE multiplication commutes: k*c and c*k round identically
-    return rowsum_launch(A, d_ia, nA, B, d_ib, nB, nullptr, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out,
-                         false);
+    return rowsum_launch(A, d_ia, nA, B, d_ib, nB, nullptr, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
 }
 
 extern "C" int irwls_dev_kernel_rowsum_n(const irwls_dev_set *A, const int *d_ia, int nA, const irwls_dev_set *B,
                                          const int *d_ib, const int *d_nB, const double *d_cb, const double *d_sa,
                                          const double *d_sb, int op, const double *d_init, const double *d_tail,
                                          double *d_out) {
-    return rowsum_launch(A, d_ia, nA, B, d_ib, 0, d_nB, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out, false);
+    return rowsum_launch(A, d_ia, nA, B, d_ib, 0, d_nB, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
 }
 
-// out_i = init_i + sum_j w_j k(A_i, B_j) in the order of j, for prediction.
-extern "C" int irwls_dev_predict_rowsum(const irwls_dev_set *A, int nA, const irwls_dev_set *B, int nB,
-                                        const double *d_w, double *d_out) {
-    return rowsum_launch(A, nullptr, nA, B, nullptr, nB, nullptr, d_w, nullptr, nullptr, +1, d_out, nullptr, d_out,
-                         A->mode == IRWLS_K_LINEAR && B->mode == IRWLS_K_LINEAR);
+// f_i = bias + sum_j w_j k(A_i, B_j) for prediction, or its sign. The rows per CTA as
+// for the ordered sums.
+extern "C" int irwls_dev_predict_rows(const irwls_dev_set *A, int nA, const irwls_dev_set *B, int nB,
+                                      const double *d_w, double bias, int hard, double *d_out) {
+    if (nA <= 0) return 0;
+    const int R = rowsum_rows(A, nA);
+    if (!R) return -5;
+    const size_t smem = (size_t)R * A->ld * sizeof(double);
+    if (smem > 40 * 1024) allow_smem(predict_rows_kernel);
+    predict_rows_kernel<<<ceil_div(nA, R), kThreads, smem, irwls_stream()>>>(kview(A), nA, kview(B), std::max(nB, 0), R,
+                                                                            d_w, bias, hard, d_out);
+    IRWLS_LAUNCH_CHECK("predict_rows");
+    return 0;
 }

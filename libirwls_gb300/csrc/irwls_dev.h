@@ -114,9 +114,9 @@ int irwls_dev_kernel_rowsum(const irwls_dev_set *A, const int *d_ia, int nA, con
                             const double *d_sb, int k_first, int op, const double *d_init,
                             const double *d_tail, double *d_out);
 /* Same with the B count read from device memory (*d_nB). */
-/* init in d_out; linear kernels with fused multiply-adds */
-int irwls_dev_predict_rowsum(const irwls_dev_set *A, int nA, const irwls_dev_set *B, int nB, const double *d_w,
-                             double *d_out);
+/* prediction's row sums or their signs (dev_tiles.cu) */
+int irwls_dev_predict_rows(const irwls_dev_set *A, int nA, const irwls_dev_set *B, int nB, const double *d_w,
+                           double bias, int hard, double *d_out);
 int irwls_dev_kernel_rowsum_n(const irwls_dev_set *A, const int *d_ia, int nA, const irwls_dev_set *B,
                               const int *d_ib, const int *d_nB, const double *d_cb, const double *d_sa,
                               const double *d_sb, int op, const double *d_init, const double *d_tail,
