@@ -32,11 +32,19 @@ constexpr int CT = 1024;
 // SGMA
 // --------------------------------------------------------------------------
 
+// The screened selection's candidates whose FP64 scores a step needs: need[0] of
+// them, their slots in ascending order from need[3] on; all for a larger need[0]
+// and without a screening.
+__device__ __forceinline__ int cand_count(const int *need) { return need ? min(need[0], NCAND) : NCAND; }
+__device__ __forceinline__ int cand_slot(const int *need, int c) {
+    return need && need[0] <= NCAND ? need[3 + c] : c;
+}
+
 // Per candidate: KNC row, forward then backward substitution with L, eta.
 // smem: v[s] (working vector), A row of the candidate (ld doubles).
-// With `need` (the screened selection) the kernel returns unless need[0] is
-// set; its CTAs from NCAND on then form the columns of KSC that no earlier
-// step formed (from built[0] on).
+// With `need` (the screened selection) only the candidates that it names are
+// solved, CTA c the c-th (row c of Z, its own row of W and eta); the CTAs from
+// NCAND on form the columns of KSC that no earlier step formed (from built[0] on).
 __global__ void __launch_bounds__(256) sgma_cand_kernel(KView X, const int *__restrict__ cand,
                                                         const int *__restrict__ cent, int s,
                                                         const double *__restrict__ L, int ldL,
@@ -64,7 +72,8 @@ __global__ void __launch_bounds__(256) sgma_cand_kernel(KView X, const int *__re
         }
         return;
     }
-    const int gc = cand[c];
+    if (c >= cand_count(need)) return;
+    const int slot = cand_slot(need, c), gc = cand[slot];
     for (int t = tid; t < X.ld; t += blockDim.x) sA[t] = X.X[(size_t)gc * X.ld + t];
     __syncthreads();
     const double qa = X.q[gc];
@@ -107,7 +116,7 @@ __global__ void __launch_bounds__(256) sgma_cand_kernel(KView X, const int *__re
         }
         __syncthreads();
     }
-    for (int e = tid; e < s; e += blockDim.x) W[(size_t)c * ldz + e] = v[e];
+    for (int e = tid; e < s; e += blockDim.x) W[(size_t)slot * ldz + e] = v[e];
     __syncthreads();
     // backward: L^T z = w
     for (int b = nblk - 1; b >= 0; --b) {
@@ -143,7 +152,7 @@ __global__ void __launch_bounds__(256) sgma_cand_kernel(KView X, const int *__re
         // eta = 1 - sum_e k_e z_e, left to right (src/budgeted-train.c:192-194)
         double val = 1.0;
         for (int e = 0; e < s; ++e) val = __dsub_rn(val, __dmul_rn(KN[(size_t)c * ldz + e], v[e]));
-        eta[c] = val;
+        eta[slot] = val;
     }
 }
 
@@ -365,12 +374,72 @@ __global__ void __launch_bounds__(256) linv_finish_kernel(const double *__restri
     }
 }
 
+// The scores below of up to 4 NB candidates: a thread per row of 64 and NB
+// candidates (c, c + 4, ...), K_nm read where it lies.
+template <int NB>
+__device__ __forceinline__ void score_few(const KView &X, int l, const int *__restrict__ cand, int s,
+                                          const double *__restrict__ KSC, const double *__restrict__ Z, int ldz,
+                                          double *__restrict__ part, const int *__restrict__ need, int ncand,
+                                          double (*red)[NCAND + 1]) {
+    const int tid = threadIdx.x, c = tid & 3, rr = tid >> 2;
+    const double *z[NB];
+    int gc[NB];
+    double sum[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const int j = min(c + 4 * b, ncand - 1);
+        z[b] = Z + (size_t)j * ldz;
+        gc[b] = cand[cand_slot(need, j)];
+        sum[b] = 0.0;
+    }
+    for (int i = 64 * blockIdx.x + rr; i < l; i += 64 * gridDim.x) {
+        double a[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) a[b] = 0.0;
+        int k = 0;
+        for (; k + 8 <= s; k += 8) {
+            double x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u] = KSC[(size_t)(k + u) * l + i];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int b = 0; b < NB; ++b) a[b] = fma(x[u], z[b][k + u], a[b]);
+        }
+        for (; k < s; ++k)
+#pragma unroll
+            for (int b = 0; b < NB; ++b) a[b] = fma(KSC[(size_t)k * l + i], z[b][k], a[b]);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const double r = a[b] - kentry(X, X.X + (size_t)gc[b] * X.ld, X.q[gc[b]], i);
+            sum[b] = fma(r, r, sum[b]);
+        }
+    }
+    // lanes of a warp hold 8 rows of each candidate
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        for (int o = 16; o >= 4; o >>= 1) sum[b] += __shfl_xor_sync(0xffffffffu, sum[b], o);
+        if ((tid & 31) < 4) red[tid >> 5][c + 4 * b] = sum[b];
+    }
+    __syncthreads();
+    if (tid < ncand) {
+        double t = 0.0;
+        for (int g = 0; g < 8; ++g) t += red[g][tid];
+        part[(size_t)blockIdx.x * NCAND + tid] = t;
+    }
+}
+
 // SGMA scores: for row tiles of GM rows and all 64 candidates,
 // acc[i][c] = sum_k KSC[k*l + i] Z[c*ldz + k], r = acc - k(cand_c, x_i), and
 // the sum of r^2 over the CTA's tiles goes to part[blockIdx.x][c].
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (a fixed order, so the
 // partial sums are deterministic); 32-row tiles keep the last round short.
-// K-steps of GK are double-buffered with cp.async.
+// K-steps of GK are double-buffered with cp.async. With `need` the candidates
+// that it names, up to 16 of them by score_few, whose FP64 work is that of their
+// number rounded up to 4, 8 or 16: the screening leaves two to four (100000 rows,
+// 600 centroids: in 176 steps of 600, 2.9 on average; the selection takes 0.24 s,
+// 2.5 with all 64 scored in every step). 200000 rows, 1000 centroids: 3.3 s, with
+// all 64 scored in the steps that ask 9.4.
 constexpr int GM = 32, GK = 16;
 __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const int *__restrict__ cand, int s,
                                                            const double *__restrict__ KSC,
@@ -384,8 +453,15 @@ __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const
     __shared__ double red[16][NCAND + 1];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;  // tx: candidate group, ty: row group
+    const int ncand = cand_count(need), nb = (ncand + 15) / 16;  // candidates, groups of 16
     const int ntiles = (l + GM - 1) / GM;
     const int nk = (s + GK - 1) / GK;
+    if (ncand <= 16) {
+        if (ncand <= 4) score_few<1>(X, l, cand, s, KSC, Z, ldz, part, need, ncand, red);
+        else if (ncand <= 8) score_few<2>(X, l, cand, s, KSC, Z, ldz, part, need, ncand, red);
+        else score_few<4>(X, l, cand, s, KSC, Z, ldz, part, need, ncand, red);
+        return;
+    }
     double ps[4] = {0.0, 0.0, 0.0, 0.0};
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const int i0 = tile * GM;
@@ -402,10 +478,10 @@ __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const
                 cp_async8(&As[buf][kk][r], ok ? (const void *)(KSC + (size_t)k * l + i) : (const void *)KSC,
                           ok ? 8 : 0);
             }
-            for (int t = tid; t < GK * NCAND; t += 256) {
+            for (int t = tid; t < GK * 16 * nb; t += 256) {
                 const int c = t / GK, kk = t % GK;
                 const int k = k0 + kk;
-                const bool ok = k < s;
+                const bool ok = k < s && c < ncand;
                 cp_async8(&Bs[buf][kk][c], ok ? (const void *)(Z + (size_t)c * ldz + k) : (const void *)Z,
                           ok ? 8 : 0);
             }
@@ -427,18 +503,20 @@ __global__ void __launch_bounds__(256, 2) sgma_gemm_kernel(KView X, int l, const
 #pragma unroll
                 for (int a = 0; a < 2; ++a) av[a] = As[buf][kk][ty + 16 * a];
 #pragma unroll
-                for (int b = 0; b < 4; ++b) bv[b] = Bs[buf][kk][tx + 16 * b];
+                for (int b = 0; b < 4; ++b) bv[b] = b < nb ? Bs[buf][kk][tx + 16 * b] : 0.0;
 #pragma unroll
-                for (int a = 0; a < 2; ++a)
+                for (int b = 0; b < 4; ++b)
+                    if (b < nb)
 #pragma unroll
-                    for (int b = 0; b < 4; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+                        for (int a = 0; a < 2; ++a) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
             }
             __syncthreads();
         }
         // epilogue: subtract the candidate kernel value, square, accumulate
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int gc = cand[tx + 16 * b];
+            if (tx + 16 * b >= ncand) break;
+            const int gc = cand[cand_slot(need, tx + 16 * b)];
             const double *arow = X.X + (size_t)gc * X.ld;
             const double qa = X.q[gc];
 #pragma unroll
@@ -472,20 +550,23 @@ __global__ void __launch_bounds__(NCAND) sgma_select_kernel(const double *__rest
     chain_open();
     if (need && !need[0]) return;
     __shared__ double sc[NCAND];
-    const int c = threadIdx.x;
+    const int c = threadIdx.x, ncand = cand_count(need);
     double v = 0.0;
-    for (int b = 0; b < nblk; ++b) v += part[(size_t)b * NCAND + c];
-    const double et = eta[c];
-    sc[c] = (et > 0.0) ? __dmul_rn(__ddiv_rn(1.0, et), v) : 0.0;
+    if (c < ncand) {
+        for (int b = 0; b < nblk; ++b) v += part[(size_t)b * NCAND + c];
+        const double et = eta[cand_slot(need, c)];
+        sc[c] = (et > 0.0) ? __dmul_rn(__ddiv_rn(1.0, et), v) : 0.0;
+    }
     __syncthreads();
     if (c == 0) {
         double val = sc[0];
         int bb = 0;
-        for (int i = 1; i < NCAND; ++i)
+        for (int i = 1; i < ncand; ++i)
             if (sc[i] > val) {
                 val = sc[i];
                 bb = i;
             }
+        bb = cand_slot(need, bb);
         cent[s] = cand[bb];
         best[0] = bb;
         bestval[s] = val;

@@ -528,8 +528,9 @@ constexpr int CAT_LD = 68;
 // step, 8: a margin for the rows not seen, 2^-19: the FP32 kernel values and
 // products), so sum r^2 over l rows is known to a factor 1 +- d,
 // d = 2x + x^2 + 2^-18, x = E / sqrt(sum r^2 / l). If another row's score can
-// reach the best one's within those bounds, or a bound is not finite, need[0]
-// asks for the FP64 scores of the step (irwls_sgma_rescore).
+// reach the best one's within those bounds, or a bound is not finite, need asks
+// for the FP64 scores of the candidates that can (irwls_sgma_rescore): need[0] is
+// their number (0: settled), need[3 ...] their slots in ascending order.
 __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__restrict__ part, int nblk,
                                                               const double *__restrict__ eta,
                                                               const int *__restrict__ cand, int s, int *cent,
@@ -596,10 +597,16 @@ __global__ void __launch_bounds__(1024) sgma_select_f32_kernel(const float *__re
         if (eps) {
             const float low = (float)sc[bb] * (1.f - dl[bb]);
             bool ask = !(low > 0.f);
-            for (int k = i; k < 64; k += 32)
-                ask |= k != bb && cand[k] != cb && !((float)sc[k] * (1.f + dl[k]) < low);
+            int at = 0;
+            for (int k = i; k < 64; k += 32) {
+                const bool in = k == bb || !((float)sc[k] * (1.f + dl[k]) < low);
+                ask |= in && k != bb && cand[k] != cb;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                if (in) need[3 + at + __popc(m & ((1u << i) - 1u))] = k;
+                at += __popc(m);
+            }
             ask = __any_sync(0xffffffffu, ask);
-            if (i == 0) need[0] = ask;
+            if (i == 0) need[0] = ask ? at : 0;
         }
     }
 }

@@ -115,10 +115,10 @@ static void draw_label_rows(const svm_dataset *ds, double want, int n, int *out)
 
 /* SGMA with tensor-core scores. screen = 0: the precision form. screen = 1:
  * the plain form -- the tensor-core scores and a measured bound of their error
- * settle the steps whose best candidate stands clear of the others; the other
- * steps (a fraction of a percent on the workloads) take the FP64 scores of
- * all 64 candidates on the device, with the columns of K_nm they need formed
- * then. The selection is the FP64 one either way. verbose == 1 prints the
+ * settle the steps whose best candidate stands clear of the others; in the other
+ * steps (a few percent at budgets of 100, nearly all late steps at 1000) the
+ * candidates that can still be the best take the FP64 scores on the device, with
+ * the columns of K_nm they need formed then. The selection is the FP64 one either way. verbose == 1 prints the
  * scores, so every step then takes the FP64 ones. */
 static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out, int screen) {
     const int m = props.size, l = ds->l;
@@ -140,7 +140,7 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     const int learn = !screen && g_proposer != NULL && X->mode != IRWLS_K_LINEAR && m > 2;
     const int trace = !screen && g_trace_feat != NULL && m > 2;
     double *d_KSC = NULL, *d_Z = NULL, *d_part64 = NULL;
-    int *d_need = NULL; /* need, the columns of K_nm formed, and the error measure (float bits) */
+    int *d_need = NULL; /* number of candidates to rescore, the columns of K_nm formed, the error measure (float bits), the slots */
     const int nf = irwls_mlp_feature_count(), pool = g_pool, half = g_pool / 2;
     void *F = irwls_f32_mirror(X);
     if (!F) {
@@ -180,7 +180,7 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
         rc |= irwls_dev_malloc((void **)&d_KSC, (size_t)l * m * sizeof(double));
         rc |= irwls_dev_malloc((void **)&d_Z, (size_t)64 * ldz * sizeof(double));
         rc |= irwls_dev_malloc((void **)&d_part64, (size_t)irwls_sgma_partials(l) * 64 * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_need, 3 * sizeof(int));
+        rc |= irwls_dev_malloc((void **)&d_need, 67 * sizeof(int));
     }
     if (learn || trace) {
         rc |= irwls_dev_malloc((void **)&d_probe, NPROBE * sizeof(int));
