@@ -862,9 +862,11 @@ __global__ void __launch_bounds__(256) exact_write_kernel(const double *__restri
 // e = y - K(:, SV) beta_SV - b in FP64 over all l rows (the exact error
 // vector that the incremental updates approximate).
 extern "C" int irwls_full_exact_errors(const irwls_dev_set *X, int l, const double *d_beta, int *d_lst, double *d_cb,
-                                       int *d_cnt, double *d_e) {
+                                       int *d_cnt, double *d_e, void *exact) {
     sv_list_kernel<<<1, CT, 0, irwls_stream()>>>(d_beta, l, d_lst, d_cb, d_cnt);
     IRWLS_LAUNCH_CHECK("sv_list");
+    const int rc = irwls_exact_rowsum(exact, nullptr, l, d_lst, d_cnt, l, d_cb, nullptr, -1, X->y, d_beta + l, d_e);
+    if (rc != 1) return rc;
     return irwls_dev_kernel_rowsum_n(X, nullptr, l, X, d_lst, d_cnt, d_cb, nullptr, nullptr, -1, X->y, d_beta + l,
                                      d_e);
 }

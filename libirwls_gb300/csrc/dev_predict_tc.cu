@@ -701,8 +701,8 @@ extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) 
     na = std::min(na, n);
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t sb = up(slice_bytes(n, npb)), ab = up(slice_bytes(na, npb)), n4 = up((size_t)n * 4), n8 = up((size_t)n * 8);
-    // partial sums: all rows in up to 16 chunks, or a list of rows against any
-    const size_t nparts = (size_t)GR * std::max<size_t>((size_t)n * 16, (size_t)na * ceil_div(n, PN));
+    // partial sums: all rows in up to 16 chunks, lists of up to 2048 rows in any number
+    const size_t nparts = (size_t)GR * std::max<size_t>((size_t)n * 16, (size_t)std::min(na, 2048) * ceil_div(n, PN));
     const size_t total = 2 * sb + ab + 3 * (n4 + n8) + 256 + up(nparts * sizeof(double));
     if (total > ((size_t)4 << 30)) return nullptr;
     ExactRows *E = (ExactRows *)calloc(1, sizeof(ExactRows));

@@ -121,10 +121,11 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
        solves, GIN and the in-set updates are the FP64 form's. */
     void *tcs = NULL;
     if (irwls_get_precision() == IRWLS_PRECISION_MIXED && !(tcs = irwls_tc_set_create(X, l, W))) return -1;
-    /* plain form: the row sums from the tensor cores where they are large enough
-       (at most W changed weights per update, or W rows); the errors are as close
-       to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu) */
-    void *exact = !tcs && (double)l * W >= 5.0e5 ? irwls_exact_rows_create(X, l, W) : NULL;
+    /* the FP64-accurate row sums from the tensor cores where they are large enough
+       (at most W changed weights per update, or W rows; in the precision form any
+       set of rows, on data without its exact-integer products); the errors are as
+       close to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu) */
+    void *exact = (double)l * W >= 5.0e5 && !(tcs && irwls_tc_set_exact(tcs)) ? irwls_exact_rows_create(X, l, tcs ? l : W) : NULL;
     const double band = 0.05, eps = 2e-5 * (tcs ? irwls_tc_set_kbound(tcs) : 1.0);
     int *xflag = NULL, *xmark = NULL, *xS = NULL, *xSnew = NULL, *svlst = NULL, *svcnt = NULL, *xcnt = NULL,
         *h_xcnt = NULL;
@@ -213,7 +214,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
                 /* at most nSW changed weights: exact tensor-core dot products
                    where the data allow them, else the FP64 kernels */
                 if (irwls_dev_gather(e, xS, nS, eS)) goto fail;
-                const int ex = irwls_tc_exact_rowsum(tcs, X, xS, nS, lst, 0, cnt, nSW, cb, NULL, NULL, -1, eS, dbias, eS);
+                int ex = irwls_tc_exact_rowsum(tcs, X, xS, nS, lst, 0, cnt, nSW, cb, NULL, NULL, -1, eS, dbias, eS);
+                if (ex == 1) ex = irwls_exact_rowsum(exact, xS, nS, lst, cnt, nSW, cb, NULL, -1, eS, dbias, eS);
                 if (ex < 0 ||
                     (ex == 1 && irwls_dev_kernel_rowsum_n(X, xS, nS, X, lst, cnt, cb, NULL, NULL, -1, eS, dbias, eS)))
                     goto fail;
@@ -274,7 +276,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
                error bound of the others nears the band */
             int all_exact = 0;
             if (acc > band / 5) {
-                if (irwls_full_exact_errors(X, l, bnew, svlst, svcb, svcnt, e)) goto fail;
+                if (irwls_full_exact_errors(X, l, bnew, svlst, svcb, svcnt, e, exact)) goto fail;
                 acc = 0.0;
                 all_exact = 1;
             }
@@ -289,8 +291,9 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
                     irwls_dev_d2h(h_xcnt, svcnt, sizeof(int)) || irwls_dev_sync())
                     goto fail;
                 const int nsv = h_xcnt[0];
-                const int ex = irwls_tc_exact_rowsum(tcs, X, xSnew, nnew, svlst, nsv, NULL, nsv, svcb, NULL, NULL, -1,
-                                                     eS, bnew + l, eS);
+                int ex = irwls_tc_exact_rowsum(tcs, X, xSnew, nnew, svlst, nsv, NULL, nsv, svcb, NULL, NULL, -1, eS,
+                                               bnew + l, eS);
+                if (ex == 1) ex = irwls_exact_rowsum(exact, xSnew, nnew, svlst, svcnt, nsv, svcb, NULL, -1, eS, bnew + l, eS);
                 if (ex < 0 || (ex == 1 && irwls_dev_kernel_rowsum_n(X, xSnew, nnew, X, svlst, svcnt, svcb, NULL, NULL,
                                                                     -1, eS, bnew + l, eS)))
                     goto fail;

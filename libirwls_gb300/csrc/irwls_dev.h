@@ -253,8 +253,9 @@ int irwls_par_delta(const double *d_bnew, double *d_beta, int m, irwls_par_post 
  * tail[0] over all of its rows, j < *d_n <= wmax. */
 void *irwls_tc_set_create(const irwls_dev_set *X, int rows, int wmax);
 /* e = y - K(:, SV) beta_SV - beta[l] in FP64 (dev_full.cu); lst/cb/cnt are scratch of l entries. */
+/* exact: irwls_exact_rows_create of the set, or NULL */
 int irwls_full_exact_errors(const irwls_dev_set *X, int l, const double *d_beta, int *d_lst, double *d_cb, int *d_cnt,
-                            double *d_e);
+                            double *d_e, void *exact);
 /* The exact-error row set of the precision form (dev_full.cu): S = support
  * vectors, rows with |e y| < band, and SW; Snew = rows of S not flagged
  * before (none when all_exact); counts = {|S|, |Snew|}. */
