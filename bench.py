@@ -10,7 +10,9 @@ step (the count the reference hard-codes).
 
 One step = one complete training (SGMA + IRWLSpar) of that workload. Both
 forms are timed in the same run, on the same resident dataset:
-  plain FP64 : the reference's arithmetic, the form the parity tests pin;
+  plain FP64 : FP64-accurate, the form the parity tests pin (SGMA screened on
+               the tensor cores and decided in FP64, the Gram from base-256
+               integer digit products);
   precision  : SGMA scores on the tensor cores from three bf16 pieces of Q
                and W (exactly their FP32 values), IRWLSpar's Gram from
                exact integer digit products on the tensor cores,
@@ -22,17 +24,13 @@ forms are timed in the same run, on the same resident dataset:
           out accuracy change <= 0.1%), else of the plain form; dataset
           resident on the GPU, CUDA events on the library's stream, L2
           flushed between steps. The plain form, the denominator of the
-          speed-up, takes 16 s per training: it is timed on min(K, 3) steps
-          after one warm-up.
+          speed-up, takes seconds per training: it is timed on min(K, 3)
+          steps after one warm-up.
   e2e   : the same form through the reference-facing C ABI (SGMA() +
           IRWLSpar() on the host svm_dataset), host-to-device copies of the
           dataset and device-to-host copies of the results included.
-  roofline: the dominant kernel of that form. Precision form: the tensor-core
-          Gram, its algorithmic work n_act (m + 1) m flops per IRWLSpar
-          iteration (the FP64 SYRK it replaces) against the measured
-          sustained bf16 peak; the rate of its bf16 digit-pair products is a
-          separate field. Plain form: the FP64 SGMA GEMM against a live FP64
-          probe.
+  roofline: the dominant kernel of that form, the SGMA score kernel: its
+          algorithmic bytes against the measured copy bandwidth.
   kernels : the other measured kernel rooflines of both forms.
   cpu_baseline: one complete training of the workload (SGMA to m = 1000,
           IRWLSpar to convergence) by the CPU restatement of the reference
@@ -90,7 +88,7 @@ METRIC = "train s at ≤1e-4 rel dual-obj err: mixed/batched/learned vs plain FP
 N_ROWS, BUDGET, GAMMA, COST, SEED = 200_000, 1000, 0.1, 100.0, 20240602
 # wall-clock budget of the reference arm's complete CPU trainings (at least one runs)
 REF_ARM_BUDGET_S = 240.0
-# the plain FP64 form (16 s per training of the budgeted workload) is timed on
+# the plain form (seconds per training of the budgeted workload) is timed on
 # at most this many steps after one warm-up
 PLAIN_STEPS = 3
 
@@ -499,43 +497,31 @@ def run_ours(args):
         return
 
     peaks, peak_src = measured_peaks()
-    fp64_peak = lib.irwls_fp64_peak_tflops(5)
     sgma_flops = sum(2.0 * args.rows * s * 64 for s in range(2, args.budget))
+    sus = peaks.get("bf16_tflops_sustained") or peaks.get("bf16_tflops")
     kernels = {}
-    if 0 in runs:
-        g_s = runs[0]["prof"]["sgma_scores"][0]
-        ach = sgma_flops / g_s / 1e12 if g_s > 0 else 0.0
-        kernels["sgma_gemm_kernel (plain FP64)"] = {
-            "bound": "fp64", "achieved": round(ach, 4), "peak": round(fp64_peak, 4), "unit": "TFLOP/s",
-            "frac": round(ach / fp64_peak, 4) if fp64_peak else None,
-            "share_of_step": round(g_s / runs[0]["s"], 4)}
-        gr_s = runs[0]["prof"]["irwls_gram"][0]
-        ach = runs[0]["gram_flops"] / gr_s / 1e12 if gr_s > 0 else 0.0
-        kernels["gram_kernel (plain FP64)"] = {
-            "bound": "fp64", "achieved": round(ach, 4), "peak": round(fp64_peak, 4), "unit": "TFLOP/s",
-            "frac": round(ach / fp64_peak, 4) if fp64_peak else None,
-            "share_of_step": round(gr_s / runs[0]["s"], 4)}
-    if 1 in runs:
-        gr_s = runs[1]["prof"]["irwls_gram"][0]
-        alg = runs[1]["gram_flops"] / gr_s / 1e12 if gr_s > 0 else 0.0
-        tc = runs[1]["gram_tc_flops"] / gr_s / 1e12 if gr_s > 0 else 0.0
-        sus = peaks.get("bf16_tflops_sustained") or peaks.get("bf16_tflops")
-        kernels["gram_tc_kernel (precision form, exact integer digit products on tcgen05)"] = {
+    names = {0: "plain form", 1: "precision form"}
+    for prec in forms:
+        run, name = runs[prec], names[prec]
+        gr_s = run["prof"]["irwls_gram"][0]
+        alg = run["gram_flops"] / gr_s / 1e12 if gr_s > 0 else 0.0
+        tc = run["gram_tc_flops"] / gr_s / 1e12 if gr_s > 0 else 0.0
+        kernels["gram_tc_kernel (%s, exact integer digit products on tcgen05)" % name] = {
             "bound": "tensor", "achieved": round(alg, 3), "peak": sus,
             "unit": "TFLOP/s algorithmic (n_act (m+1) m flops per IRWLSpar iteration, the FP64 SYRK replaced)",
             "frac": round(alg / sus, 4) if sus else None,
             "peak_source": peak_src + " bf16 sustained (the kernel runs inside a seconds-long training)",
             "digit_product_tflops": round(tc, 2),
             "digit_product_pipe_frac": round(tc / sus, 4) if sus else None,
-            "digit_products_per_algorithmic_product": round(runs[1]["gram_tc_flops"] / runs[1]["gram_flops"], 2)
-            if runs[1]["gram_flops"] else None,
-            "share_of_step": round(gr_s / runs[1]["s"], 4),
-            "slicing_share_of_step": round(runs[1]["prof"]["irwls_gram_slicing"][0] / runs[1]["s"], 4)}
-        sc_s = runs[1]["prof"]["sgma_scores"][0]
+            "digit_products_per_algorithmic_product": round(run["gram_tc_flops"] / run["gram_flops"], 2)
+            if run["gram_flops"] else None,
+            "share_of_step": round(gr_s / run["s"], 4),
+            "slicing_share_of_step": round(run["prof"]["irwls_gram_slicing"][0] / run["s"], 4)}
+        sc_s = run["prof"]["sgma_scores"][0]
         nl = max(1, args.budget - 2)  # score launches (orders 2 ... m - 1)
         sc_bytes = sum(score_launch_bytes(args.rows, s, hd) for s in range(2, args.budget))
         ach = sc_bytes / sc_s / 1e9 if sc_s > 0 else 0.0
-        kernels["sgma_tc_score_ws_kernel (precision form, tcgen05 on three bf16 pieces)"] = {
+        kernels["sgma_tc_score_ws_kernel (%s, tcgen05 on three bf16 pieces)" % name] = {
             "bound": "hbm", "achieved": round(ach, 1), "peak": peaks.get("hbm_gbs"),
             "unit": "GB/s algorithmic (per launch at order s: Q's three bf16 pieces of the s columns rounded up "
                     "to 32, read once; the 64 residuals of every row written; the rows' FP32 CSR read)",
@@ -543,7 +529,7 @@ def run_ours(args):
             "peak_source": peak_src + " HBM copy", "launches": nl,
             "avg_launch_us": round(sc_s / nl * 1e6, 2),
             "algorithmic_tflops": round(sgma_flops / sc_s / 1e12, 2) if sc_s > 0 else None,
-            "share_of_step": round(sc_s / runs[1]["s"], 4)}
+            "share_of_step": round(sc_s / run["s"], 4)}
     # roofline: the dominant kernel of the headline form
     if head == 1:
         k = kernels["sgma_tc_score_ws_kernel (precision form, tcgen05 on three bf16 pieces)"]
@@ -564,10 +550,8 @@ def run_ours(args):
         g["traffic_launch"] = {"launch": "last of 42 (active rows 62357)", "duration_ms": 1.517,
                                "traffic": 894986752 + 3068672, "algorithmic_bytes": 62357 * 1001 * 8}
     else:
-        k = kernels["sgma_gemm_kernel (plain FP64)"]
-        roofline = dict(k, kernel="sgma_gemm_kernel", traffic=None,
-                        peak_source="measured live: FP64 FMA-chain probe of the library "
-                                    "(irwls_fp64_peak_tflops); MEASURED_PEAKS.json has no FP64 figure")
+        k = kernels["sgma_tc_score_ws_kernel (plain form, tcgen05 on three bf16 pieces)"]
+        roofline = dict(k, kernel="sgma_tc_score_ws_kernel", traffic=None)
 
     accuracy, value, form = None, step_s, ("plain FP64" if head == 0 else "precision (mixed)")
     if forms == (0, 1):
@@ -809,7 +793,7 @@ def full_measure(args, lib, libc):
     value = r["s"]
     peak = lib.irwls_fp64_peak_tflops(3)
     roofline = {"bound": "latency" if head == 0 else "mixed",
-                "kernel": "kernel row sums (FP64 ordered) and Cholesky solves",
+                "kernel": "kernel row sums and Cholesky solves",
                 "achieved": None, "peak": round(peak, 4), "unit": "TFLOP/s", "frac": None, "traffic": None,
                 "share_of_step": {k: round(v[0] / value, 4) for k, v in r["prof"].items()},
                 "launches_per_step": {k: int(v[1]) for k, v in r["prof"].items()}}

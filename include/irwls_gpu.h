@@ -80,7 +80,11 @@ int irwls_ws_mixed_max(void);
 int irwls_gpu_available(void);
 
 /* Arithmetic of the training paths:
- * IRWLS_PRECISION_FP64 (default): FP64 throughout, reference parity;
+ * IRWLS_PRECISION_FP64 (default): FP64 accuracy throughout, reference parity.
+ * Large RBF row sums (predictions, the error updates of full training) and the
+ * IRWLSpar Gram from 128 centroids on come from exact integer digit products on
+ * the tensor cores, no further from a 64-bit evaluation than ordered FP64 sums;
+ * SGMA's scores are screened on the tensor cores and decided in FP64;
  * IRWLS_PRECISION_MIXED: the precision form -- SGMA candidate scores from
  * tensor-core products of three bf16 pieces per value (FP32 accuracy) on
  * the Nystrom features of the current centroids, with the K_mm

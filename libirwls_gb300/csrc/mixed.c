@@ -1,9 +1,10 @@
 /*
  * mixed.c -- host orchestration of the precision form of budgeted IRWLS
  * (same loops, exit tests and random draws as budgeted_train.c):
- *   SGMA: candidate kernel rows, the factor L of K_CC + jitter and its
- *         inverse (kept explicitly, as the reference keeps invKC) in FP64;
- *         the candidate solves W = K_CN L^-T as one FP64 GEMM; scores from
+ *   SGMA: candidate kernel rows and the factor L of K_CC + jitter in FP64;
+ *         the candidates' W = K_CN L^-T ahead of their steps by forward
+ *         substitution (dev_sgma_ahead.cu; proposed candidates and very
+ *         large budgets by the explicit inverse and an FP64 GEMM); scores from
  *         Q w on the tensor cores (Q = K_nm L^-T and W held as three bf16
  *         pieces each, exactly their FP32 values; six piece products, so
  *         Q w has FP32 accuracy), candidate kernel rows of the score
