@@ -24,10 +24,11 @@
 //
 // Against a 64-bit evaluation the decision values are within 2.5e-16 of their
 // size, the ordered FP64 sums within 1.5e-15 (20000 one-hot rows of 54 features,
-// 3000 vectors). Those take 5475 us of kernel time, this 480 us and 50 us of
-// preparation. Bound: the epilogue's integer instructions (about 130 per value,
-// 45 % of the issue slots, latency between them the rest); the MMAs (33 x 16
-// cycles per 16 features of a tile pair) run beside it.
+// 3000 vectors). Those take 5475 us of kernel time, this 456 us and 50 us of
+// preparation. Bound: the epilogue's integer instructions (about 120 per value,
+// 41 % of the issue slots, latency between them the rest); the MMAs (33 x 32
+// cycles per 16 features of a tile pair) run while the epilogue forms the kernel
+// values of the tile before (480 us when it held the accumulators for them).
 #include <cuda_bf16.h>
 #include <math.h>
 #include <stdint.h>
@@ -345,7 +346,7 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
         const long long ai = live ? p.at[row] : 0;
         double sum = 0.0, nw = 0.0;
         ulonglong2 ng = {0, 0};
-        long long T[MULTI ? CW : 1];
+        long long T[CW];
         // vector et of tile t into registers (past the end: weight 0, 2^-y <= 1)
         auto fetch = [&](int t) {
             const int j = PN * t + et;
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
             if (et < PN && jj + 1 < jn) fetch(j0 + jj + 1);
             if (MULTI)
 #pragma unroll
-                for (int c = 0; c < (MULTI ? CW : 1); ++c) T[c] = 0;
+                for (int c = 0; c < CW; ++c) T[c] = 0;
             for (int d = 0; d < nd; ++d, ++blk) {
                 // (this barrier also publishes the tile's vectors, and after it
                 // nobody reads the other buffer)
@@ -410,19 +411,19 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
                         // units of 2^(8 v - 8) for level v: pairs of levels in 32 bits
                         // (1, 2 and 3 x 2^21, 4 x 2^21 at most; see above for 3 and 2)
                         const long long th = (long long)(l[7] * 256 + l[6]) * 65536 + (l[5] * 256 + l[4]);
-                        long long t = (th << 24) + (long long)(l[3] * 256 + l[2]) * 256 + (l[1] + (l[0] >> 8));
-                        if constexpr (MULTI) {
-                            t += T[c4 + c];
-                            T[c4 + c] = t;
-                            if (d + 1 < nd) continue;
-                        }
-                        const int cc = CW * gr + c4 + c;
-                        const ulonglong2 a = ag[cc];
-                        const long long m = __mul64hi(t, (long long)a.y);
-                        const long long y = ai + (long long)a.x - (m >> shift);
-                        sum = fma(w[cc], exp2_fixed<FB>(y, p.fb, table), sum);
+                        const long long t = (th << 24) + (long long)(l[3] * 256 + l[2]) * 256 + (l[1] + (l[0] >> 8));
+                        T[c4 + c] = MULTI ? T[c4 + c] + t : t;
                     }
                 }
+            }
+            if (stop) break;
+            // the kernel values, while the next tile's products run
+#pragma unroll
+            for (int c = 0; c < CW; ++c) {
+                const ulonglong2 a = ag[CW * gr + c];
+                const long long m = __mul64hi(T[c], (long long)a.y);
+                const long long y = ai + (long long)a.x - (m >> shift);
+                sum = fma(w[CW * gr + c], exp2_fixed<FB>(y, p.fb, table), sum);
             }
         }
         if (stop) abort_flag = 1;
