@@ -518,9 +518,11 @@ __global__ void to_f32_kernel(const double *__restrict__ in, long long n, float 
 // groups for features that differ mod 8.
 constexpr int CAT_LD = 68;
 
-// Scores of the precision form: per candidate, the tile sums in 16 strided
-// groups with Kahan-compensated FP32 adds, the 16 group sums in FP64 in a
-// fixed order, score = sum / eta; strict ">" argmax, first index wins.
+// Scores of the precision form: per candidate, the score CTAs' sums in 16
+// strided groups with Kahan-compensated FP32 adds, the 16 group sums in FP64 in a
+// fixed order, score = sum / eta; strict ">" argmax, first index wins. One CTA reads
+// them all, so the score CTAs add up their tiles (469 tile sums at 60000 rows took
+// it 2 us longer).
 //
 // With eps (the plain form's screened selection) the scores only screen: the
 // residuals r = Q w - k carry an absolute error of at most about
@@ -950,6 +952,7 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
                                    sq[jt & 1], et, EPI);
         };
         TileRows T = {};
+        float psum = 0.f, pcomp = 0.f;  // threads et < 64: candidate et's sum over this CTA's tiles
         if (my_tiles > 0) T = stage(0, entries(0));
         int2 pn = entries(1);
         if (early) {
@@ -1015,13 +1018,18 @@ __global__ void __launch_bounds__(128 + 128 * EG, 1) sgma_tc_score_ws_kernel(
             }
             asm volatile("bar.sync 1, %0;\n" ::"r"(EPI));
             if (et < 64) {
-                // the candidate's four row-quarter sums, in a fixed order
+                // the candidate's four row-quarter sums, in a fixed order, added
+                // to those of this CTA's tiles before (compensated)
                 const float *w = &wred[4 * (et / CPG)][et % CPG];
-                part[(size_t)tile * 64 + et] = (w[0] + w[CPG]) + (w[2 * CPG] + w[3 * CPG]);
+                const float y = __fsub_rn((w[0] + w[CPG]) + (w[2 * CPG] + w[3 * CPG]), pcomp);
+                const float t = __fadd_rn(psum, y);
+                pcomp = __fsub_rn(__fsub_rn(t, psum), y);
+                psum = t;
             }
             asm volatile("bar.sync 1, %0;\n" ::"r"(EPI));
             T = Tn;
         }
+        if (et < 64) part[(size_t)blockIdx.x * 64 + et] = psum;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();
@@ -1155,6 +1163,11 @@ extern "C" int irwls_sgma_tc_fits(const irwls_dev_set *X) {
     return score_smem_fixed(X) + 2 * TcRing<64, QB_NP, WS_BK>::BYTES <= score_smem_limit();
 }
 
+// CTAs of the score kernel, each leaving one partial sum per candidate.
+extern "C" int irwls_sgma_tc_partials(int l) {
+    return std::max(1, std::min(ceil_div(l, TC_BM), irwls_num_sms() > 0 ? irwls_num_sms() : 148));
+}
+
 // early: as the kernel's.
 extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l, const int *d_cand, const void *Qb,
                                    int ldq, const void *Wb, int s, float *d_part, float *d_resid, int early) {
@@ -1194,8 +1207,7 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
                 break;
             }
     const size_t smem = fixed + 2 * xs + (size_t)ns * stage;
-    const int ntiles = ceil_div(l, TC_BM);
-    const int grid = std::max(1, std::min(ntiles, irwls_num_sms() > 0 ? irwls_num_sms() : 148));
+    const int grid = irwls_sgma_tc_partials(l);
     const KViewF kv = kviewf(X, (const F32Mirror *)F);
     const __nv_bfloat16 *qb = (const __nv_bfloat16 *)Qb, *wb = (const __nv_bfloat16 *)Wb;
     auto launch = [&](auto kern) {
@@ -1215,8 +1227,6 @@ extern "C" int irwls_sgma_tc_score(const irwls_dev_set *X, const void *F, int l,
     IRWLS_LAUNCH_CHECK("sgma_tc_score");
     return 0;
 }
-
-extern "C" int irwls_sgma_tc_partials(int l) { return ceil_div(l, TC_BM); }
 
 // eps, need: the screened selection's error measure and its answer, or NULL.
 extern "C" int irwls_sgma_tc_select(const float *d_part, int nblk, const double *d_eta, const int *d_cand, int s,

@@ -166,7 +166,7 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     rc |= irwls_dev_malloc((void **)&d_part, (size_t)nblk * 64 * sizeof(float));
     rc |= irwls_dev_malloc((void **)&d_val, (size_t)m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_rq, (size_t)l * 64 * sizeof(float));
-    const size_t qb_bytes = (size_t)nblk * 128 * ldq * 6; /* whole 128-row tiles, three pieces */
+    const size_t qb_bytes = (size_t)((l + 127) / 128) * 128 * ldq * 6; /* whole 128-row tiles, three pieces */
     rc |= irwls_dev_malloc(&Qb, qb_bytes);
     if (!ahead) rc |= irwls_dev_malloc(&Wb, (size_t)64 * ldq * 6);
     rc |= irwls_dev_malloc((void **)&lrow, (size_t)(m + 1) * sizeof(float));
