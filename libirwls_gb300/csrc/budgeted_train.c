@@ -191,7 +191,7 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     rc |= irwls_dev_h2d(d_idx, idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_memset(d_beta, 0, (size_t)m * sizeof(double));
     rc |= irwls_dev_memset(d_bbest, 0, (size_t)m * sizeof(double));
-    rc |= irwls_par_build(X, l, d_idx, m, d_KC, d_KSC, digits && !mixed);
+    rc |= irwls_par_build(X, l, d_idx, m, d_KC, d_KSC);
     rc |= irwls_par_first(X->y, l, M, d_act, d_sd, d_day);
     rc |= irwls_dev_sync();
     if (rc) goto done;

@@ -1059,15 +1059,11 @@ extern "C" int irwls_sgma_extend(const irwls_dev_set *X, int l, int s, const int
     return 0;
 }
 
-// exact: K_nm from the tensor cores where they take it (irwls_exact_block).
-extern "C" int irwls_par_build(const irwls_dev_set *X, int l, const int *d_idx, int m, double *d_KC, double *d_KSC,
-                               int exact) {
+extern "C" int irwls_par_build(const irwls_dev_set *X, int l, const int *d_idx, int m, double *d_KC, double *d_KSC) {
     if (irwls_dev_kernel_block_t(X, d_idx, m, X, d_idx, m, d_KC, m, 0)) return -2;
     add_diag_kernel<<<ceil_div(m, 256), 256, 0, irwls_stream()>>>(d_KC, m, 0.00001);
     IRWLS_LAUNCH_CHECK("add_diag");
     // KSC row-major l x m: out[row * m + centroid]
-    const int rc = exact ? irwls_exact_block(X, l, d_idx, m, d_KSC, m) : 1;
-    if (rc != 1) return rc;
     return irwls_dev_kernel_block_t(X, d_idx, m, X, nullptr, l, d_KSC, m, 1);
 }
 

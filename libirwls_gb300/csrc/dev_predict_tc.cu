@@ -231,15 +231,12 @@ struct PredictArgs {
     int fb, emax, shr;           // unit of y; the largest e_j; y's product part is
     unsigned long long g;        //   (T g_j 2^-64) 2^(e_i - shr) with g_j = g 2^(e_j - emax)
     double *part;                // [strip][row]: strips of P chunks x column groups
-    double *out;                 // kernel values, row i at out + i ldo
-    long long ldo;
 };
 
 // EW = 16 epilogue warps: 128 rows x 4 groups of 16 vectors. MULTI: more than
-// 96 features, several drains per tile pair. FB: as exp2_fixed. STORE: the kernel
-// values themselves to p.out.
-template <bool MULTI, int FB, bool STORE>
-__global__ void __launch_bounds__(64 + 32 * 16, 1) predict_tc_kernel(PredictArgs p, int *flags) {
+// 96 features, several drains per tile pair. FB: as exp2_fixed.
+template <bool MULTI, int FB>
+__global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArgs p, int *flags) {
     constexpr int EW = 16, CW = PN / (EW / 4);  // columns of a group
     extern __shared__ __align__(1024) unsigned char p_smem[];
     __shared__ __align__(8) uint64_t full[PNS], empty[PNS], accf, acce, done;
@@ -341,9 +338,8 @@ __global__ void __launch_bounds__(64 + 32 * 16, 1) predict_tc_kernel(PredictArgs
             if (!mbar_wait(smem_u32(&done), 0u)) abort_flag = 1;
         }
         __syncwarp();
-    } else {
-        // (a warp reads the accumulator rows 32 (warp % 4) ...)
-        const int qr = warp & 3, gr = (warp - 2) >> 2, et = threadIdx.x - 64;
+    } else if (warp >= 4) {
+        const int qr = warp & 3, gr = (warp - 4) >> 2, et = threadIdx.x - 128;
         const int row = PM * I + 32 * qr + lane;
         const bool live = row < p.n;
         const int shift = live ? min(p.shr - p.et[row], 63) : 63;
@@ -354,7 +350,7 @@ __global__ void __launch_bounds__(64 + 32 * 16, 1) predict_tc_kernel(PredictArgs
         // vector et of tile t into registers (past the end: weight 0, 2^-y <= 1)
         auto fetch = [&](int t) {
             const int j = PN * t + et;
-            nw = !STORE && j < nsv ? p.w[j] : 0.0;
+            nw = j < nsv ? p.w[j] : 0.0;
             ng.x = j < nsv ? (unsigned long long)p.as[j] : 1ULL << 62;
             ng.y = j < nsv ? p.g >> min(p.emax - p.es[j], 63) : 0;
         };
@@ -427,17 +423,11 @@ __global__ void __launch_bounds__(64 + 32 * 16, 1) predict_tc_kernel(PredictArgs
                 const ulonglong2 a = ag[CW * gr + c];
                 const long long m = __mul64hi(T[c], (long long)a.y);
                 const long long y = ai + (long long)a.x - (m >> shift);
-                const double k = exp2_fixed<FB>(y, p.fb, table);
-                if constexpr (STORE) {
-                    const int j = PN * (j0 + jj) + CW * gr + c;
-                    if (live && j < nsv) p.out[(size_t)row * p.ldo + j] = k;
-                } else {
-                    sum = fma(w[CW * gr + c], k, sum);
-                }
+                sum = fma(w[CW * gr + c], exp2_fixed<FB>(y, p.fb, table), sum);
             }
         }
         if (stop) abort_flag = 1;
-        if (!STORE && live && !stop) p.part[(size_t)(z * (EW / 4) + gr) * p.n + row] = sum;
+        if (live && !stop) p.part[(size_t)(z * (EW / 4) + gr) * p.n + row] = sum;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();
@@ -557,12 +547,11 @@ int best_chunks(int it, int nt, int sms, long long most = 1 << 30) {
 
 constexpr int GR = 4;  // strips of a chunk (column groups of predict_tc_kernel)
 
-template <bool STORE>
 void launch_predict(const PredictArgs &a, int tiles) {
-    auto kern = a.npb > PDRAIN ? (a.fb == 56 ? predict_tc_kernel<true, 56, STORE> : predict_tc_kernel<true, 0, STORE>)
-                               : (a.fb == 56 ? predict_tc_kernel<false, 56, STORE> : predict_tc_kernel<false, 0, STORE>);
+    auto kern = a.npb > PDRAIN ? (a.fb == 56 ? predict_tc_kernel<true, 56> : predict_tc_kernel<true, 0>)
+                               : (a.fb == 56 ? predict_tc_kernel<false, 56> : predict_tc_kernel<false, 0>);
     allow_smem(kern);
-    kern<<<dim3(tiles, a.P), 64 + 32 * 16, (size_t)PNS * P_STAGE + 1024, irwls_stream()>>>(a, irwls_dev_flags());
+    kern<<<dim3(tiles, a.P), 128 + 32 * 16, (size_t)PNS * P_STAGE + 1024, irwls_stream()>>>(a, irwls_dev_flags());
     irwls_count_launch(1);
 }
 
@@ -665,7 +654,7 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
         a.at = at + r0;
         row_slice_kernel<<<slice_grid((long long)tiles * PM, npb, sms), 256, 0, irwls_stream()>>>(T->X + (size_t)r0 * T->ld, T->ld, T->width, rows, et + r0, tiles * PM, npb, dT);
         irwls_count_launch(1);
-        launch_predict<false>(a, tiles);
+        launch_predict(a, tiles);
         predict_finish_kernel<<<ceil_div(rows, 256), 256, 0, irwls_stream()>>>(a.part, P * GR, rows, bias, hard, d_out + r0);
         irwls_count_launch(1);
         rc = irwls_check_launch("predict_tc");
@@ -795,42 +784,10 @@ extern "C" int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d
     a.w = d_cb;
     a.part = E->part;
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
-    launch_predict<false>(a, it);
+    launch_predict(a, it);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_ROWSUM);
     rowsum_finish_kernel<<<ceil_div(nA, 256), 256, 0, irwls_stream()>>>(E->part, a.P * GR, nA, d_ia, d_sa, op, d_init,
                                                                        d_tail, d_out);
     irwls_count_launch(1);
     return irwls_check_launch("exact_rowsum");
-}
-
-// out[i ldo + j] = k(x_i, x_idx[j]) for i < n, j < m (idx: any rows of the set),
-// FP64-accurate; 1 where
-// irwls_exact_rows_create declines or below 500000 values (the caller then takes the
-// FP64 kernel: 50000 x 300 of 12 stored values 1200 us there, 194 here and about 60
-// of preparation).
-extern "C" int irwls_exact_block(const irwls_dev_set *X, int n, const int *d_idx, int m, double *d_out, long long ldo) {
-    if (m < 1 || n < 1 || (double)n * m < 5.0e5 || std::max(m, n) > X->n_rows) return 1;
-    ExactRows *E = (ExactRows *)irwls_exact_rows_create(X, X->n_rows, 1);
-    if (!E) return 1;
-    gather_slices_kernel<<<slice_grid((long long)m * PS, E->npb, E->sms), 256, 0, irwls_stream()>>>(
-        (const uint4 *)E->S, E->ex, E->q, E->npb, d_idx, m, nullptr, (uint4 *)E->bS, E->bex, E->bq);
-    irwls_count_launch(1);
-    PredictArgs a = E->p;
-    const int it = ceil_div(n, PM), nt = ceil_div(m, PN);
-    a.per = ceil_div(nt, best_chunks(it, nt, E->sms));
-    a.P = ceil_div(nt, a.per);
-    a.T = E->S;
-    a.et = E->ex;
-    a.at = E->q;
-    a.S = E->bS;
-    a.es = E->bex;
-    a.as = E->bq;
-    a.n = n;
-    a.nsv = m;
-    a.out = d_out;
-    a.ldo = ldo;
-    launch_predict<true>(a, it);
-    const int rc = irwls_check_launch("exact_block");
-    irwls_exact_rows_free(E);
-    return rc;
 }

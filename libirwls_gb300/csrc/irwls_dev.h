@@ -209,7 +209,7 @@ int irwls_sgma_select(const double *d_part, int l, const double *d_eta, const in
 int irwls_sgma_extend(const irwls_dev_set *X, int l, int s, const int *d_cent, const int *d_best,
                       const double *d_W, int ldz, double *d_L, int ldL, double *d_KSC);
 /* IRWLSpar: KC row-major m x m, KSC row-major l x m. */
-int irwls_par_build(const irwls_dev_set *X, int l, const int *d_idx, int m, double *d_KC, double *d_KSC, int exact);
+int irwls_par_build(const irwls_dev_set *X, int l, const int *d_idx, int m, double *d_KC, double *d_KSC);
 int irwls_par_first(const double *d_y, int l, double M, int *d_act, double *d_sd, double *d_day);
 size_t irwls_par_gram_part_bytes(int m, int P);
 /* The Gram on the tensor cores (dev_gram_tc.cu): A' as exact integer digits
@@ -310,8 +310,6 @@ void irwls_exact_rows_free(void *h);
 int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d_ib, const int *d_nB, int nBmax,
                        const double *d_cb, const double *d_sa, int op, const double *d_init, const double *d_tail,
                        double *d_out);
-/* kernel values against listed rows of the set (IRWLSpar's K_nm, plain form) */
-int irwls_exact_block(const irwls_dev_set *X, int n, const int *d_idx, int m, double *d_out, long long ldo);
 size_t irwls_predict_linear_scratch(int width, int nsv);
 int irwls_predict_linear(const irwls_dev_set *T, int n, const irwls_dev_set *S, int nSV, const double *d_w,
                          double bias, int hard, double *d_W, double *d_out);
