@@ -659,6 +659,8 @@ __global__ void __launch_bounds__(GT_MAX) gram_kernel(const double *__restrict__
                                                       int nact, const double *__restrict__ sd,
                                                       const double *__restrict__ day, int chunk,
                                                       double *__restrict__ part) {
+    chain_wait();
+    chain_open();
     const int z = blockIdx.x;
     const int p0 = z * chunk, p1 = min(nact, p0 + chunk);
     __shared__ __align__(16) double A[2][TK][GW];
@@ -734,6 +736,8 @@ __global__ void __launch_bounds__(GT_MAX) gram_kernel(const double *__restrict__
 // part_z; row m = K2 = sum_z part_z[m][:].
 __global__ void gram_reduce_kernel(const double *__restrict__ part, int P, int m, const double *__restrict__ KC,
                                    double *__restrict__ K1, int ld) {
+    chain_wait();
+    chain_open();
     const long long total = (long long)(m + 1) * m;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
@@ -759,6 +763,8 @@ __global__ void __launch_bounds__(256) residual_kernel(const double *__restrict_
                                                        const double *__restrict__ beta, const double *__restrict__ y,
                                                        double C, double M, double *__restrict__ e,
                                                        double *__restrict__ Da) {
+    chain_wait();
+    chain_open();
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int i0 = RROWS * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); i0 < l; i0 += RROWS * nw) {
@@ -822,6 +828,8 @@ __device__ __forceinline__ int block_sum256(int v, int *ws) {
 
 __global__ void __launch_bounds__(256) weights_count_kernel(const double *__restrict__ Da, int l,
                                                             int *__restrict__ cnt) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[8];
     const int r0 = blockIdx.x * WB, r1 = min(l, r0 + WB);
     int c = 0;
@@ -835,6 +843,8 @@ __global__ void __launch_bounds__(256) weights_write_kernel(const double *__rest
                                                             int *__restrict__ act, double *__restrict__ sd,
                                                             double *__restrict__ day, irwls_par_post *h,
                                                             unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[8];
     __shared__ int woff[8];
     int part = 0;
@@ -887,6 +897,8 @@ __global__ void first_weights_kernel(const double *__restrict__ y, int l, double
 // dW = |bnew - beta|^2, nW = |bnew|^2 (chunked, fixed order), beta <- bnew.
 __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bnew, double *beta, int m,
                                                    irwls_par_post *h) {
+    chain_wait();
+    chain_open();
     __shared__ double red[33];
     const int ch = (m + CT - 1) / CT;
     const int b = threadIdx.x * ch, e = min(m, b + ch);
@@ -1078,8 +1090,8 @@ extern "C" size_t irwls_par_gram_part_bytes(int m, int P) { return (size_t)P * (
 // K1 = KC + the sum of P Gram partials (the last step of both digit forms).
 extern "C" int irwls_par_gram_reduce(const double *d_part, int P, int m, const double *d_KC, double *d_K1, int ldK1) {
     const long long tot = (long long)(m + 1) * m;
-    gram_reduce_kernel<<<(int)std::min<long long>(ceil_div(tot, 256), 65535), 256, 0, irwls_stream()>>>(
-        d_part, P, m, d_KC, d_K1, ldK1);
+    launch_chained(gram_reduce_kernel, dim3((int)std::min<long long>(ceil_div(tot, 256), 65535)), dim3(256), 0, d_part,
+                   P, m, d_KC, d_K1, ldK1);
     IRWLS_LAUNCH_CHECK("gram_reduce");
     return 0;
 }
@@ -1107,13 +1119,13 @@ extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act,
     }
     const int wpc = ceil_div(W, ns);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
-    gram_kernel<<<dim3(P, ceil_div(W, wpc)), 32 * wpc, 0, irwls_stream()>>>(d_KSC, m, d_act, nact, d_sd, d_day, chunk,
-                                                                          d_part);
+    launch_chained(gram_kernel, dim3(P, ceil_div(W, wpc)), dim3(32 * wpc), 0, d_KSC, m, d_act, nact, d_sd, d_day, chunk,
+                   d_part);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
     IRWLS_LAUNCH_CHECK("gram");
     const long long total = (long long)(m + 1) * m;
-    gram_reduce_kernel<<<(int)std::min<long long>(ceil_div(total, 256), 65535), 256, 0, irwls_stream()>>>(
-        d_part, P, m, d_KC, d_K1, ldK1);
+    launch_chained(gram_reduce_kernel, dim3((int)std::min<long long>(ceil_div(total, 256), 65535)), dim3(256), 0,
+                   d_part, P, m, d_KC, d_K1, ldK1);
     IRWLS_LAUNCH_CHECK("gram_reduce");
     return 0;
 }
@@ -1121,7 +1133,7 @@ extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act,
 extern "C" int irwls_par_residual(const double *d_KSC, int l, int m, const double *d_beta, const double *d_y, double C,
                                   double M, double *d_e, double *d_Da) {
     const int blocks = std::min(ceil_div(l, 8 * RROWS), 8 * (irwls_num_sms() > 0 ? irwls_num_sms() : 148));
-    residual_kernel<<<blocks, 256, 0, irwls_stream()>>>(d_KSC, l, m, d_beta, d_y, C, M, d_e, d_Da);
+    launch_chained(residual_kernel, dim3(blocks), dim3(256), 0, d_KSC, l, m, d_beta, d_y, C, M, d_e, d_Da);
     IRWLS_LAUNCH_CHECK("residual");
     return 0;
 }
@@ -1131,15 +1143,15 @@ extern "C" int irwls_par_weights(const double *d_Da, const double *d_y, int l, i
     const int nb = std::max(1, ceil_div(l, WB));
     int *cnt = (int *)irwls_ctx_scratch(2, (size_t)nb * sizeof(int));
     if (!cnt) return -3;
-    weights_count_kernel<<<nb, 256, 0, irwls_stream()>>>(d_Da, l, cnt);
+    launch_chained(weights_count_kernel, dim3(nb), dim3(256), 0, d_Da, l, cnt);
     IRWLS_LAUNCH_CHECK("weights_count");
-    weights_write_kernel<<<nb, 256, 0, irwls_stream()>>>(d_Da, d_y, l, cnt, nb, d_act, d_sd, d_day, h, seq);
+    launch_chained(weights_write_kernel, dim3(nb), dim3(256), 0, d_Da, d_y, l, cnt, nb, d_act, d_sd, d_day, h, seq);
     IRWLS_LAUNCH_CHECK("weights_write");
     return 0;
 }
 
 extern "C" int irwls_par_delta(const double *d_bnew, double *d_beta, int m, irwls_par_post *h) {
-    delta_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_beta, m, h);
+    launch_chained(delta_kernel, dim3(1), dim3(CT), 0, d_bnew, d_beta, m, h);
     IRWLS_LAUNCH_CHECK("delta");
     return 0;
 }

@@ -25,6 +25,9 @@ int irwls_num_sms();
 // chain_open() after its chain_wait(), so before chain_wait() a kernel may read
 // what was complete before the kernel before it, and touch nothing else in
 // global memory. chain_open() lets the next chained kernel be scheduled.
+// The kernels of the training loops' outer passes, some of them a few us long,
+// spent 1 to 2 us each on being scheduled; chained: full training of 700 x 54
+// 18.46 -> 17.86 ms, the budget of 50000 x 300 23.03 -> 22.64 ms.
 // Outside a chained launch both are no-ops.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void chain_open() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }

@@ -448,6 +448,8 @@ __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double 
 // sum of the weights of every inactive sample (src/full-train.c:436-456).
 __global__ void gather_ws_kernel(const int *__restrict__ SW, int nSW, const double *__restrict__ e,
                                  const double *__restrict__ beta, int l, double *esub, double *bsub) {
+    chain_wait();
+    chain_open();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= nSW; i += gridDim.x * blockDim.x) {
         if (i < nSW) {
             esub[i] = e[SW[i]];
@@ -464,6 +466,8 @@ __global__ void __launch_bounds__(CT) apply_ws_kernel(const int *__restrict__ SW
                                                       const double *__restrict__ bt, const double *__restrict__ beta,
                                                       int l, double *bnew, int *lst, double *cb, int *cnt,
                                                       double *dbias) {
+    chain_wait();
+    chain_open();
     __shared__ int s_scan[CT];
     for (int i = threadIdx.x; i < nSW; i += CT) bnew[SW[i]] = bt[i];
     if (threadIdx.x == 0) {
@@ -513,6 +517,8 @@ __device__ double chunk_tree_sum(double v, double *red) {
 // dW = sum (beta - bnew)^2 and nW = sum beta^2 (src/full-train.c:512-520).
 __global__ void __launch_bounds__(PC) norms_chunk_kernel(const double *__restrict__ beta,
                                                          const double *__restrict__ bnew, int n, double *part) {
+    chain_wait();
+    chain_open();
     const int t = blockIdx.x * PC + threadIdx.x, ch = (n + CT - 1) / CT, b = t * ch, e = min(n, b + ch);
     double v1 = 0.0, v2 = 0.0;
     for (int i = b; i < e; ++i) {
@@ -526,6 +532,8 @@ __global__ void __launch_bounds__(PC) norms_chunk_kernel(const double *__restric
 
 __global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restrict__ part, irwls_outer_counts *h,
                                                          unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ double red[33];
     const double dW = chunk_tree_sum(part[threadIdx.x], red);
     const double nW = chunk_tree_sum(part[CT + threadIdx.x], red);
@@ -542,6 +550,8 @@ __global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restric
 // the sums, pass 3 writes each chunk's entries at its offset.
 __global__ void __launch_bounds__(PC) gin_chunk_kernel(const int *__restrict__ SIN, int nSIN,
                                                        const double *__restrict__ bnew, int *ccount, double *csum) {
+    chain_wait();
+    chain_open();
     const int t = blockIdx.x * PC + threadIdx.x, ch = (nSIN + CT - 1) / CT, b = t * ch, e = min(nSIN, b + ch);
     int c = 0;
     double v = 0.0;
@@ -556,6 +566,8 @@ __global__ void __launch_bounds__(PC) gin_chunk_kernel(const int *__restrict__ S
 
 __global__ void __launch_bounds__(CT) gin_scan_kernel(int *ccount, const double *__restrict__ csum, int *cnt,
                                                       double *GIN, int nSW) {
+    chain_wait();
+    chain_open();
     __shared__ int s_scan[CT];
     __shared__ double red[33];
     const int total = block_exclusive_scan(s_scan, ccount[threadIdx.x]);
@@ -570,6 +582,8 @@ __global__ void __launch_bounds__(CT) gin_scan_kernel(int *ccount, const double 
 __global__ void __launch_bounds__(PC) gin_write_kernel(const int *__restrict__ SIN, int nSIN,
                                                        const double *__restrict__ bnew,
                                                        const int *__restrict__ coffset, int *lst, double *cb) {
+    chain_wait();
+    chain_open();
     const int t = blockIdx.x * PC + threadIdx.x, ch = (nSIN + CT - 1) / CT, b = t * ch, e = min(nSIN, b + ch);
     int off = coffset[t];
     for (int o = b; o < e; ++o) {
@@ -614,6 +628,8 @@ __device__ __forceinline__ int classify_one(double bi, double ei, double yi, dou
 __global__ void __launch_bounds__(CT) classify_kernel(const double *__restrict__ bnew, const double *__restrict__ e,
                                                       const double *__restrict__ y, int l, double C, int *SW,
                                                       int *SC, int *SIN, irwls_outer_counts *h, unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ int s_scan[CT];
     __shared__ int first[6];
     if (threadIdx.x < 6) first[threadIdx.x] = 0x7fffffff;
@@ -642,6 +658,8 @@ __global__ void __launch_bounds__(CT) classify_kernel(const double *__restrict__
 
 __global__ void fill_ws_kernel(int *SW, int nSW, int *SIN, int nSIN, const int *__restrict__ SC, int nSC,
                                const int *__restrict__ perm, int space) {
+    chain_wait();
+    chain_open();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nSC; i += gridDim.x * blockDim.x) {
         const int v = SC[perm ? perm[i] : i];
         if (i < space) SW[nSW + i] = v;
@@ -728,6 +746,8 @@ __device__ __forceinline__ void ordered_round(const bool (&member)[NL], int i, i
 __global__ void classify_code_kernel(const double *__restrict__ bnew, const double *__restrict__ e,
                                      const double *__restrict__ y, int l, double C, unsigned char *__restrict__ code,
                                      int *__restrict__ first) {
+    chain_wait();
+    chain_open();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < l; i += gridDim.x * blockDim.x) {
         int slot = -1;
         const int c = classify_one(bnew[i], e[i], y[i], C, &slot);
@@ -752,6 +772,8 @@ __device__ __forceinline__ int classify_list(unsigned char v, int i, const int *
 
 __global__ void __launch_bounds__(256) classify_count_kernel(const unsigned char *__restrict__ code, int l,
                                                              const int *__restrict__ first, int *__restrict__ cnt) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[8];
     const int r0 = blockIdx.x * CB, r1 = min(l, r0 + CB);
     int c[3] = {0, 0, 0};
@@ -769,6 +791,8 @@ __global__ void __launch_bounds__(256) classify_write_kernel(const unsigned char
                                                              const int *__restrict__ first,
                                                              const int *__restrict__ cnt, int nb, int *SW, int *SC,
                                                              int *SIN, irwls_outer_counts *h, unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[3][8];
     int base[3];
     for (int k = 0; k < 3; ++k) {
@@ -793,6 +817,8 @@ __global__ void __launch_bounds__(256) classify_write_kernel(const unsigned char
 }
 
 __global__ void fill_int_kernel(int *p, int n, int v) {
+    chain_wait();
+    chain_open();
     for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = v;
 }
 
@@ -1064,11 +1090,11 @@ extern "C" int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, 
     if (!sc) return -3;
     double *csum = (double *)sc;
     int *ccount = (int *)(sc + (size_t)CT * sizeof(double));
-    gin_chunk_kernel<<<CT / PC, PC, 0, irwls_stream()>>>(d_SIN, nSIN, d_bnew, ccount, csum);
+    launch_chained(gin_chunk_kernel, dim3(CT / PC), dim3(PC), 0, d_SIN, nSIN, d_bnew, ccount, csum);
     IRWLS_LAUNCH_CHECK("gin_chunk");
-    gin_scan_kernel<<<1, CT, 0, irwls_stream()>>>(ccount, csum, d_cnt, d_GIN, nSW);
+    launch_chained(gin_scan_kernel, dim3(1), dim3(CT), 0, ccount, csum, d_cnt, d_GIN, nSW);
     IRWLS_LAUNCH_CHECK("gin_scan");
-    gin_write_kernel<<<CT / PC, PC, 0, irwls_stream()>>>(d_SIN, nSIN, d_bnew, ccount, d_lst, d_cb);
+    launch_chained(gin_write_kernel, dim3(CT / PC), dim3(PC), 0, d_SIN, nSIN, d_bnew, ccount, d_lst, d_cb);
     IRWLS_LAUNCH_CHECK("gin_write");
     const int rc = irwls_exact_rowsum(exact, d_SW, nSW, d_lst, d_cnt, nSIN, d_cb, X->y, +1, nullptr, nullptr, d_GIN);
     if (rc != 1) return rc;
@@ -1078,7 +1104,8 @@ extern "C" int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, 
 
 extern "C" int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e, const double *d_beta, int l,
                                     double *d_esub, double *d_bsub) {
-    gather_ws_kernel<<<ceil_div(nSW + 1, 256), 256, 0, irwls_stream()>>>(d_SW, nSW, d_e, d_beta, l, d_esub, d_bsub);
+    launch_chained(gather_ws_kernel, dim3(ceil_div(nSW + 1, 256)), dim3(256), 0, d_SW, nSW, d_e, d_beta, l, d_esub,
+                   d_bsub);
     IRWLS_LAUNCH_CHECK("gather_ws");
     return 0;
 }
@@ -1086,7 +1113,8 @@ extern "C" int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e,
 extern "C" int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt, const double *d_beta, int l,
                                    double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_dbias) {
     if (irwls_dev_d2d(d_bnew, d_beta, (size_t)(l + 1) * sizeof(double))) return -2;
-    apply_ws_kernel<<<1, CT, 0, irwls_stream()>>>(d_SW, nSW, d_bt, d_beta, l, d_bnew, d_lst, d_cb, d_cnt, d_dbias);
+    launch_chained(apply_ws_kernel, dim3(1), dim3(CT), 0, d_SW, nSW, d_bt, d_beta, l, d_bnew, d_lst, d_cb, d_cnt,
+                   d_dbias);
     IRWLS_LAUNCH_CHECK("apply_ws");
     return 0;
 }
@@ -1094,9 +1122,9 @@ extern "C" int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt,
 extern "C" int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, irwls_outer_counts *h, unsigned seq) {
     double *part = (double *)irwls_ctx_scratch(2, (size_t)2 * CT * sizeof(double));
     if (!part) return -3;
-    norms_chunk_kernel<<<CT / PC, PC, 0, irwls_stream()>>>(d_beta, d_bnew, n, part);
+    launch_chained(norms_chunk_kernel, dim3(CT / PC), dim3(PC), 0, d_beta, d_bnew, n, part);
     IRWLS_LAUNCH_CHECK("norms_chunk");
-    norms_final_kernel<<<1, CT, 0, irwls_stream()>>>(part, h, seq);
+    launch_chained(norms_final_kernel, dim3(1), dim3(CT), 0, part, h, seq);
     IRWLS_LAUNCH_CHECK("norms_final");
     return 0;
 }
@@ -1106,7 +1134,7 @@ extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, cons
     if (l <= CT) {
         // one round of one CTA is faster than four launches (at 4000 rows it
         // took 94 us: every row's FP64 tests four times on one SM)
-        classify_kernel<<<1, CT, 0, irwls_stream()>>>(d_bnew, d_e, d_y, l, C, d_SW, d_SC, d_SIN, h, seq);
+        launch_chained(classify_kernel, dim3(1), dim3(CT), 0, d_bnew, d_e, d_y, l, C, d_SW, d_SC, d_SIN, h, seq);
         IRWLS_LAUNCH_CHECK("classify");
         return 0;
     }
@@ -1118,15 +1146,15 @@ extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, cons
     if (!sc) return -3;
     int *cnt = (int *)sc, *first = (int *)(sc + cbytes);
     unsigned char *code = sc + cbytes + fbytes;
-    fill_int_kernel<<<1, 32, 0, irwls_stream()>>>(first, 6, 0x7fffffff);
+    launch_chained(fill_int_kernel, dim3(1), dim3(32), 0, first, 6, 0x7fffffff);
     IRWLS_LAUNCH_CHECK("classify_first");
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
-    classify_code_kernel<<<std::min(ceil_div(l, 256), 8 * sms), 256, 0, irwls_stream()>>>(d_bnew, d_e, d_y, l, C,
-                                                                                         code, first);
+    launch_chained(classify_code_kernel, dim3(std::min(ceil_div(l, 256), 8 * sms)), dim3(256), 0, d_bnew, d_e, d_y, l,
+                   C, code, first);
     IRWLS_LAUNCH_CHECK("classify_code");
-    classify_count_kernel<<<nb, 256, 0, irwls_stream()>>>(code, l, first, cnt);
+    launch_chained(classify_count_kernel, dim3(nb), dim3(256), 0, code, l, first, cnt);
     IRWLS_LAUNCH_CHECK("classify_count");
-    classify_write_kernel<<<nb, 256, 0, irwls_stream()>>>(code, l, first, cnt, nb, d_SW, d_SC, d_SIN, h, seq);
+    launch_chained(classify_write_kernel, dim3(nb), dim3(256), 0, code, l, first, cnt, nb, d_SW, d_SC, d_SIN, h, seq);
     IRWLS_LAUNCH_CHECK("classify_write");
     return 0;
 }
@@ -1134,7 +1162,8 @@ extern "C" int irwls_full_classify(const double *d_bnew, const double *d_e, cons
 extern "C" int irwls_full_fill_ws(int *d_SW, int nSW, int *d_SIN, int nSIN, const int *d_SC, int nSC,
                                   const int *d_perm, int space) {
     if (nSC <= 0) return 0;
-    fill_ws_kernel<<<ceil_div(nSC, 256), 256, 0, irwls_stream()>>>(d_SW, nSW, d_SIN, nSIN, d_SC, nSC, d_perm, space);
+    launch_chained(fill_ws_kernel, dim3(ceil_div(nSC, 256)), dim3(256), 0, d_SW, nSW, d_SIN, nSIN, d_SC, nSC, d_perm,
+                   space);
     IRWLS_LAUNCH_CHECK("fill_ws");
     return 0;
 }

@@ -131,6 +131,8 @@ __global__ void __launch_bounds__(256) gram_colmax_kernel(const double *__restri
                                                           const double *__restrict__ sd,
                                                           const double *__restrict__ day,
                                                           unsigned long long *__restrict__ cmax) {
+    chain_wait();
+    chain_open();
     const int p0 = blockIdx.x * GCM, p1 = min(nact, p0 + GCM);
     const int c = 256 * blockIdx.y + threadIdx.x;
     if (c > m) return;
@@ -191,6 +193,8 @@ __global__ void __launch_bounds__(256) gram_slice_kernel(const double *__restric
                                                          const double *__restrict__ day,
                                                          const unsigned long long *__restrict__ cmax, int ncols,
                                                          int npb, __nv_bfloat16 *__restrict__ S) {
+    chain_wait();
+    chain_open();
     constexpr int HALF = GramDigits<BITS>::HALF;
     __shared__ uint16_t bf[2 * HALF + 1];  // bf16 bits of -HALF ... HALF
     for (int t = threadIdx.x; t <= 2 * HALF; t += 256) {
@@ -275,6 +279,8 @@ template <int BITS>
 __global__ void __launch_bounds__(G_THREADS, 1) gram_tc_kernel(const __nv_bfloat16 *__restrict__ S, int npb, int spc,
                                                                int m, const unsigned long long *__restrict__ cmax,
                                                                double *__restrict__ part, int *flags) {
+    chain_wait();
+    chain_open();
     using Cfg = GramDigits<BITS>;
     constexpr int LOW = Cfg::LOW, LEVELS = Cfg::LEVELS, GSCALE = Cfg::GSCALE, GDRAIN = Cfg::GDRAIN;
     const int J = blockIdx.x, I = blockIdx.y, z = blockIdx.z;
@@ -494,8 +500,8 @@ int gram_run(const double *d_KSC, int m, const int *d_act, int nact, const doubl
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM_SLICE);
     if (irwls_dev_memset(cmax, 0, (size_t)(m + 1) * sizeof(unsigned long long))) return -1;
     if (nact > 0) {
-        gram_colmax_kernel<<<dim3(ceil_div(nact, GCM), ceil_div(m + 1, 256)), 256, 0, irwls_stream()>>>(
-            d_KSC, m, d_act, nact, d_sd, d_day, cmax);
+        launch_chained(gram_colmax_kernel, dim3(ceil_div(nact, GCM), ceil_div(m + 1, 256)), dim3(256), 0, d_KSC, m,
+                       d_act, nact, d_sd, d_day, cmax);
         IRWLS_LAUNCH_CHECK("gram_colmax");
     }
     const size_t smem = (size_t)GNS * G_STAGE + 1024;
@@ -510,13 +516,13 @@ int gram_run(const double *d_KSC, int m, const int *d_act, int nact, const doubl
         pz = ceil_div(npb, spc);
         if (irwls_prof_on() && n > 0) irwls_prof_begin(IRWLS_PROF_GRAM_SLICE);
         const long long items = (long long)ct * GM * npb * 2;
-        gram_slice_kernel<BITS><<<(int)std::min<long long>(ceil_div(items, 256), 16LL * sms), 256, 0, irwls_stream()>>>(
-            d_KSC, m, d_act + a, rows, d_sd + a, d_day + a, cmax, ct * GM, npb, S);
+        launch_chained(gram_slice_kernel<BITS>, dim3((int)std::min<long long>(ceil_div(items, 256), 16LL * sms)),
+                       dim3(256), 0, d_KSC, m, d_act + a, rows, d_sd + a, d_day + a, cmax, ct * GM, npb, S);
         if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM_SLICE);
         IRWLS_LAUNCH_CHECK("gram_slice");
         if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
-        gram_tc_kernel<BITS><<<dim3(nt, ct, pz), G_THREADS, smem, irwls_stream()>>>(
-            S, npb, spc, m, cmax, d_part + (size_t)parts * (m + 1) * m, irwls_dev_flags());
+        launch_chained(gram_tc_kernel<BITS>, dim3(nt, ct, pz), dim3(G_THREADS), smem, S, npb, spc, m, cmax,
+                       d_part + (size_t)parts * (m + 1) * m, irwls_dev_flags());
         g_tc_flops += (double)tiles * npb * GBK * GM * GN * 2.0 * Cfg::GPAIRS;
         if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
         IRWLS_LAUNCH_CHECK("gram_tc");

@@ -450,6 +450,8 @@ __global__ void predict_finish_kernel(const double *__restrict__ part, int strip
 __global__ void rowsum_finish_kernel(const double *__restrict__ part, int strips, int n, const int *__restrict__ ia,
                                      const double *__restrict__ sa, int op, const double *init,  // may alias out
                                      const double *__restrict__ tail, double *out) {
+    chain_wait();
+    chain_open();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     double f = 0.0;
@@ -468,6 +470,8 @@ __global__ void __launch_bounds__(256) gather_slices_kernel(const uint4 *__restr
                                                             const int *__restrict__ idx, int n,
                                                             const int *__restrict__ np, uint4 *__restrict__ oS,
                                                             int *__restrict__ oex, long long *__restrict__ oa) {
+    chain_wait();
+    chain_open();
     if (np) n = np[0];
     constexpr int TILE = PS * PPIECE / 8;  // 16-byte units of a 16-feature block of a tile
     const int units = npb * PS * 2;        // of a row
@@ -765,12 +769,12 @@ extern "C" int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d
     a.per = ceil_div(nt, best_chunks(it, nt, E->sms, (long long)(E->nparts / GR / nA)));
     a.P = ceil_div(nt, a.per);
     if (d_ia) {
-        gather_slices_kernel<<<slice_grid((long long)nA * PS, E->npb, E->sms), 256, 0, irwls_stream()>>>(
-            (const uint4 *)E->S, E->ex, E->q, E->npb, d_ia, nA, nullptr, (uint4 *)E->aS, E->aex, E->aq);
+        launch_chained(gather_slices_kernel, dim3(slice_grid((long long)nA * PS, E->npb, E->sms)), dim3(256), 0,
+                       (const uint4 *)E->S, E->ex, E->q, E->npb, d_ia, nA, nullptr, (uint4 *)E->aS, E->aex, E->aq);
         irwls_count_launch(1);
     }
-    gather_slices_kernel<<<slice_grid((long long)nBmax * PS, E->npb, E->sms), 256, 0, irwls_stream()>>>(
-        (const uint4 *)E->S, E->ex, E->q, E->npb, d_ib, nBmax, d_nB, (uint4 *)E->bS, E->bex, E->bq);
+    launch_chained(gather_slices_kernel, dim3(slice_grid((long long)nBmax * PS, E->npb, E->sms)), dim3(256), 0,
+                   (const uint4 *)E->S, E->ex, E->q, E->npb, d_ib, nBmax, d_nB, (uint4 *)E->bS, E->bex, E->bq);
     irwls_count_launch(1);
     a.T = d_ia ? E->aS : E->S;
     a.et = d_ia ? E->aex : E->ex;
@@ -786,8 +790,8 @@ extern "C" int irwls_exact_rowsum(void *h, const int *d_ia, int nA, const int *d
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
     launch_predict(a, it);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_ROWSUM);
-    rowsum_finish_kernel<<<ceil_div(nA, 256), 256, 0, irwls_stream()>>>(E->part, a.P * GR, nA, d_ia, d_sa, op, d_init,
-                                                                       d_tail, d_out);
+    launch_chained(rowsum_finish_kernel, dim3(ceil_div(nA, 256)), dim3(256), 0, E->part, a.P * GR, nA, d_ia, d_sa, op,
+                   d_init, d_tail, d_out);
     irwls_count_launch(1);
     return irwls_check_launch("exact_rowsum");
 }

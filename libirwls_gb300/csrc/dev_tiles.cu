@@ -68,6 +68,8 @@ __global__ void __launch_bounds__(kThreads) kernel_rowsum_kernel(KView A, const 
                                                                  const double *__restrict__ sb, int op,
                                                                  const double *init,  // may alias out
                                                                  const double *__restrict__ tail, double *out) {
+    chain_wait();
+    chain_open();
     extern __shared__ double smem[];
     double *sA = smem;
     double *sQ = smem + (size_t)R * A.ld;
@@ -188,8 +190,8 @@ static int rowsum_launch(const irwls_dev_set *A, const int *d_ia, int nA, const 
     const size_t smem = ((size_t)R * A->ld + 8 + 1024) * sizeof(double);
     if (smem > 48 * 1024) allow_smem(kernel_rowsum_kernel);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_ROWSUM);
-    kernel_rowsum_kernel<<<ceil_div(nA, R), kThreads, smem, irwls_stream()>>>(
-        kview(A), d_ia, nA, kview(B), d_ib, nB > 0 ? nB : 0, d_nB, R, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
+    launch_chained(kernel_rowsum_kernel, dim3(ceil_div(nA, R)), dim3(kThreads), smem, kview(A), d_ia, nA, kview(B),
+                   d_ib, nB > 0 ? nB : 0, d_nB, R, d_cb, d_sa, d_sb, op, d_init, d_tail, d_out);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_ROWSUM);
     IRWLS_LAUNCH_CHECK("kernel_rowsum");
     return 0;
