@@ -202,8 +202,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         ws.w = nSW;
         ws.map = SW;
         ws.tcs = tcs;
-        if (irwls_full_gather_ws(SW, nSW, e, beta, l, ws.e, ws.beta)) goto fail;
-        if (irwls_dev_memset(ws.bbest, 0, (size_t)(nSW + 1) * sizeof(double))) goto fail;
+        if (irwls_full_gather_ws(SW, nSW, e, beta, l, ws.e, ws.beta, ws.bbest)) goto fail;
         if (run_sub(&ws, X, &props)) goto fail;
         /* betaNew over the working set; e -= K(:, SW) (betaNew - beta) - dbias (:488-510) */
         if (irwls_full_apply_ws(SW, nSW, ws.bbest, beta, l, bnew, lst, cb, cnt, dbias)) goto fail;
@@ -227,8 +226,11 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
             if (ex < 0 || (ex == 1 && irwls_dev_kernel_rowsum_n(X, NULL, l, X, lst, cnt, cb, NULL, NULL, -1, e, dbias, e)))
                 goto fail;
         }
-        if (irwls_full_norms(beta, bnew, l + 1, h_counts, ++seq)) goto fail;
-        if (irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(double))) goto fail;
+        /* the norms (and beta = betaNew), the classification and the next working set
+           (:512-520, :540-643): the second posts last, one wait for both */
+        if (irwls_full_norms(SW, nSW, beta, bnew, l, h_counts, ++seq)) goto fail;
+        if (irwls_full_classify(bnew, e, X->y, l, C, SW, SC, SIN, h_counts, ++seq)) goto fail;
+        if (irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(double) + 4 * sizeof(int))) goto fail;
         if (tcs) {
             /* a tensor-core wait that ran out left these errors stale: stop now */
             const int tc = irwls_tc_status();
@@ -240,16 +242,12 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         }
         const double ratio = h_counts->dW / h_counts->nW;
         if (ratio < props.Eta) stop = 1;
-        if (irwls_dev_d2d(beta, bnew, L1 * sizeof(double))) goto fail;
         if (ratio < best) {
             best = ratio;
             since_best = 0;
         } else {
             since_best += 1;
         }
-        /* classification and the next working set (:540-643) */
-        if (irwls_full_classify(bnew, e, X->y, l, C, SW, SC, SIN, h_counts, ++seq)) goto fail;
-        if (irwls_dev_wait_post(&h_counts->seq, seq, 4 * sizeof(int))) goto fail;
         nSW = h_counts->nSW;
         nSIN = h_counts->nSIN;
         const int nSC = h_counts->nSC;

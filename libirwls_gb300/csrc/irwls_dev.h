@@ -183,14 +183,15 @@ typedef struct irwls_outer_counts {
     double dW, nW;
     int nSW, nSIN, nSC;
     unsigned seq;  /* number of the last post */
-} irwls_outer_counts;  /* pinned: written by norms (dW, nW) and classify (the counts) */
+} irwls_outer_counts;  /* pinned: written by norms (dW, nW), then classify (the counts) */
 int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, const int *d_SIN, int nSIN,
                    const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN, void *exact);
 int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e, const double *d_beta, int l,
-                         double *d_esub, double *d_bsub);
+                         double *d_esub, double *d_bsub, double *d_bbest);
 int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt, const double *d_beta, int l,
                         double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_dbias);
-int irwls_full_norms(const double *d_beta, const double *d_bnew, int n, irwls_outer_counts *h, unsigned seq);
+int irwls_full_norms(const int *d_SW, int nSW, double *d_beta, const double *d_bnew, int l, irwls_outer_counts *h,
+                     unsigned seq);
 int irwls_full_classify(const double *d_bnew, const double *d_e, const double *d_y, int l, double C,
                         int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *h, unsigned seq);
 int irwls_full_fill_ws(int *d_SW, int nSW, int *d_SIN, int nSIN, const int *d_SC, int nSC,
