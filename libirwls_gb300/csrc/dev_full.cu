@@ -536,10 +536,15 @@ __global__ void __launch_bounds__(PC) norms_chunk_kernel(const double *__restric
 // Then beta = bnew, which differ in the working set and the bias only (a copy of
 // all of it each way and the clearing of bbest broke the chain of kernels three
 // times a pass: full training of 700 x 54 17.75 -> 17.31 ms without them and with
-// one wait of the host for the norms and the lists).
+// one wait of the host for the norms and the lists). The precision form's error
+// bound and status go with the post, and exact_write_kernel and sv_list_kernel post
+// their counts: copies and waits for these took 80 us a pass of 20000 images
+// (10.04 -> 9.60 ms).
 __global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restrict__ part, irwls_outer_counts *h,
                                                          unsigned seq, const int *__restrict__ SW, int nSW, int l,
-                                                         double *beta, const double *__restrict__ bnew) {
+                                                         double *beta, const double *__restrict__ bnew,
+                                                         const double *__restrict__ dbias,
+                                                         const int *__restrict__ flags) {
     chain_wait();
     chain_open();
     __shared__ double red[33];
@@ -548,6 +553,8 @@ __global__ void __launch_bounds__(CT) norms_final_kernel(const double *__restric
     if (threadIdx.x == 0) {
         h->dW = dW;
         h->nW = nW;
+        h->l1 = dbias[1];
+        h->tc = flags[1];
         post_seq(&h->seq, seq);
         beta[l] = bnew[l];
     }
@@ -680,18 +687,24 @@ __global__ void fill_ws_kernel(int *SW, int nSW, int *SIN, int nSIN, const int *
 
 __global__ void gather_kernel(const double *__restrict__ src, const int *__restrict__ idx, int n,
                               double *__restrict__ dst) {
+    chain_wait();
+    chain_open();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dst[k] = src[idx[k]];
 }
 
 __global__ void scatter_kernel(const double *__restrict__ src, const int *__restrict__ idx, int n,
                                double *__restrict__ dst) {
+    chain_wait();
+    chain_open();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dst[idx[k]] = src[k];
 }
 
 // Precision form: the support vectors (beta != 0 over the l samples) as a
 // compact list with their weights, in index order.
 __global__ void __launch_bounds__(CT) sv_list_kernel(const double *__restrict__ beta, int l, int *lst, double *cb,
-                                                     int *cnt) {
+                                                     int *cnt, irwls_outer_counts *h, unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ int s_scan[CT];
     const int n = block_compact(l, [&](int i) { return beta[i] != 0.0; },
                                 [&](int p, int i) {
@@ -699,7 +712,13 @@ __global__ void __launch_bounds__(CT) sv_list_kernel(const double *__restrict__ 
                                     cb[p] = beta[i];
                                 },
                                 s_scan);
-    if (threadIdx.x == 0) cnt[0] = n;
+    if (threadIdx.x == 0) {
+        cnt[0] = n;
+        if (h) {
+            h->nsv = n;
+            post_seq(&h->seq, seq);
+        }
+    }
 }
 
 // ---- multi-block ordered compactions over all l rows ------------------------
@@ -833,6 +852,8 @@ __global__ void fill_int_kernel(int *p, int n, int v) {
 }
 
 __global__ void mark_kernel(const int *__restrict__ SW, int nSW, int *__restrict__ mark, int v) {
+    chain_wait();
+    chain_open();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nSW; k += gridDim.x * blockDim.x) mark[SW[k]] = v;
 }
 
@@ -850,6 +871,8 @@ __global__ void __launch_bounds__(256) exact_count_kernel(const double *__restri
                                                           const double *__restrict__ beta, int l,
                                                           const int *__restrict__ mark, double band, int all_exact,
                                                           const int *__restrict__ flag, int *__restrict__ cnt) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[8];
     const int r0 = blockIdx.x * CB, r1 = min(l, r0 + CB);
     int cs = 0, cn = 0;
@@ -870,7 +893,9 @@ __global__ void __launch_bounds__(256) exact_write_kernel(const double *__restri
                                                           const double *__restrict__ beta, int l,
                                                           const int *__restrict__ mark, double band, int all_exact,
                                                           int *__restrict__ flag, const int *__restrict__ cnt, int nb,
-                                                          int *S, int *Snew, int *counts) {
+                                                          int *S, int *Snew, irwls_outer_counts *h, unsigned seq) {
+    chain_wait();
+    chain_open();
     __shared__ int ws[2][8];
     int base[2];
     for (int k = 0; k < 2; ++k) {
@@ -879,8 +904,9 @@ __global__ void __launch_bounds__(256) exact_write_kernel(const double *__restri
         base[k] = bsum256(part, ws[0]);
     }
     if (blockIdx.x == nb - 1 && threadIdx.x == 0) {
-        counts[0] = base[0] + cnt[2 * (nb - 1)];
-        counts[1] = base[1] + cnt[2 * (nb - 1) + 1];
+        h->nS = base[0] + cnt[2 * (nb - 1)];
+        h->nnew = base[1] + cnt[2 * (nb - 1) + 1];
+        post_seq(&h->seq, seq);
     }
     int *const out[2] = {S, Snew};
     const int r0 = blockIdx.x * CB, r1 = min(l, r0 + CB);
@@ -899,7 +925,7 @@ __global__ void __launch_bounds__(256) exact_write_kernel(const double *__restri
 // vector that the incremental updates approximate).
 extern "C" int irwls_full_exact_errors(const irwls_dev_set *X, int l, const double *d_beta, int *d_lst, double *d_cb,
                                        int *d_cnt, double *d_e, void *exact) {
-    sv_list_kernel<<<1, CT, 0, irwls_stream()>>>(d_beta, l, d_lst, d_cb, d_cnt);
+    launch_chained(sv_list_kernel, dim3(1), dim3(CT), 0, d_beta, l, d_lst, d_cb, d_cnt, nullptr, 0u);
     IRWLS_LAUNCH_CHECK("sv_list");
     const int rc = irwls_exact_rowsum(exact, nullptr, l, d_lst, d_cnt, l, d_cb, nullptr, -1, X->y, d_beta + l, d_e);
     if (rc != 1) return rc;
@@ -907,29 +933,32 @@ extern "C" int irwls_full_exact_errors(const irwls_dev_set *X, int l, const doub
                                      d_e);
 }
 
-extern "C" int irwls_full_sv_list(const double *d_beta, int l, int *d_lst, double *d_cb, int *d_cnt) {
-    sv_list_kernel<<<1, CT, 0, irwls_stream()>>>(d_beta, l, d_lst, d_cb, d_cnt);
+extern "C" int irwls_full_sv_list(const double *d_beta, int l, int *d_lst, double *d_cb, int *d_cnt,
+                                  irwls_outer_counts *h, unsigned seq) {
+    launch_chained(sv_list_kernel, dim3(1), dim3(CT), 0, d_beta, l, d_lst, d_cb, d_cnt, h, seq);
     IRWLS_LAUNCH_CHECK("sv_list");
     return 0;
 }
 
 extern "C" int irwls_full_exact_set(const double *d_e, const double *d_y, const double *d_beta, int l,
                                     const int *d_SW, int nSW, double band, int all_exact, int *d_flag, int *d_mark,
-                                    int *d_S, int *d_Snew, int *d_counts) {
+                                    int *d_S, int *d_Snew, irwls_outer_counts *h, unsigned seq) {
     const int nb = std::max(1, ceil_div(l, CB));
     int *cnt = (int *)irwls_ctx_scratch(2, (size_t)2 * nb * sizeof(int));
     if (!cnt) return -3;
     if (nSW > 0) {
-        mark_kernel<<<ceil_div(nSW, 256), 256, 0, irwls_stream()>>>(d_SW, nSW, d_mark, 1);
+        launch_chained(mark_kernel, dim3(ceil_div(nSW, 256)), dim3(256), 0, d_SW, nSW, d_mark, 1);
         IRWLS_LAUNCH_CHECK("exact_mark");
     }
-    exact_count_kernel<<<nb, 256, 0, irwls_stream()>>>(d_e, d_y, d_beta, l, d_mark, band, all_exact, d_flag, cnt);
+    launch_chained(exact_count_kernel, dim3(nb), dim3(256), 0, d_e, d_y, d_beta, l, d_mark, band, all_exact, d_flag,
+                   cnt);
     IRWLS_LAUNCH_CHECK("exact_count");
-    exact_write_kernel<<<nb, 256, 0, irwls_stream()>>>(d_e, d_y, d_beta, l, d_mark, band, all_exact, d_flag, cnt,
-                                                       nb, d_S, d_Snew, d_counts);
+    launch_chained(exact_write_kernel, dim3(nb), dim3(256), 0, d_e, d_y, d_beta, l, d_mark, band, all_exact, d_flag,
+                   cnt,
+                   nb, d_S, d_Snew, h, seq);
     IRWLS_LAUNCH_CHECK("exact_write");
     if (nSW > 0) {
-        mark_kernel<<<ceil_div(nSW, 256), 256, 0, irwls_stream()>>>(d_SW, nSW, d_mark, 0);
+        launch_chained(mark_kernel, dim3(ceil_div(nSW, 256)), dim3(256), 0, d_SW, nSW, d_mark, 0);
         IRWLS_LAUNCH_CHECK("exact_unmark");
     }
     return 0;
@@ -937,14 +966,14 @@ extern "C" int irwls_full_exact_set(const double *d_e, const double *d_y, const 
 
 extern "C" int irwls_dev_gather(const double *d_src, const int *d_idx, int n, double *d_dst) {
     if (n <= 0) return 0;
-    gather_kernel<<<std::min(ceil_div(n, 256), 1024), 256, 0, irwls_stream()>>>(d_src, d_idx, n, d_dst);
+    launch_chained(gather_kernel, dim3(std::min(ceil_div(n, 256), 1024)), dim3(256), 0, d_src, d_idx, n, d_dst);
     IRWLS_LAUNCH_CHECK("gather");
     return 0;
 }
 
 extern "C" int irwls_dev_scatter(const double *d_src, const int *d_idx, int n, double *d_dst) {
     if (n <= 0) return 0;
-    scatter_kernel<<<std::min(ceil_div(n, 256), 1024), 256, 0, irwls_stream()>>>(d_src, d_idx, n, d_dst);
+    launch_chained(scatter_kernel, dim3(std::min(ceil_div(n, 256), 1024)), dim3(256), 0, d_src, d_idx, n, d_dst);
     IRWLS_LAUNCH_CHECK("scatter");
     return 0;
 }
@@ -1129,12 +1158,13 @@ extern "C" int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt,
 }
 
 extern "C" int irwls_full_norms(const int *d_SW, int nSW, double *d_beta, const double *d_bnew, int l,
-                                irwls_outer_counts *h, unsigned seq) {
+                                const double *d_dbias, irwls_outer_counts *h, unsigned seq) {
     double *part = (double *)irwls_ctx_scratch(2, (size_t)2 * CT * sizeof(double));
     if (!part) return -3;
     launch_chained(norms_chunk_kernel, dim3(CT / PC), dim3(PC), 0, d_beta, d_bnew, l + 1, part);
     IRWLS_LAUNCH_CHECK("norms_chunk");
-    launch_chained(norms_final_kernel, dim3(1), dim3(CT), 0, part, h, seq, d_SW, nSW, l, d_beta, d_bnew);
+    launch_chained(norms_final_kernel, dim3(1), dim3(CT), 0, part, h, seq, d_SW, nSW, l, d_beta, d_bnew,
+                   d_dbias, irwls_dev_flags());
     IRWLS_LAUNCH_CHECK("norms_final");
     return 0;
 }

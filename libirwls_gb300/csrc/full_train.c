@@ -105,8 +105,9 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     }
     int rc = 0;
     double *e = NULL, *beta = NULL, *bnew = NULL, *cb = NULL, *dbias = NULL;
-    int *SW = NULL, *SIN = NULL, *SC = NULL, *lst = NULL, *cnt = NULL, *perm_d = NULL;
-    irwls_outer_counts *h_counts = NULL;
+    int *SW = NULL, *SIN = NULL, *SC = NULL, *lst = NULL, *cnt = NULL;
+    irwls_outer_counts *h_counts = NULL;  /* in one pinned block with the permutation of the candidates */
+    int *h_perm = NULL;
     unsigned seq = 0;
     irwls_sub_ws ws;
     memset(&ws, 0, sizeof ws);
@@ -127,9 +128,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
        close to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu) */
     void *exact = (double)l * W >= 5.0e5 && !(tcs && irwls_tc_set_exact(tcs)) ? irwls_exact_rows_create(X, l, tcs ? l : W) : NULL;
     const double band = 0.05, eps = 2e-5 * (tcs ? irwls_tc_set_kbound(tcs) : 1.0);
-    int *xflag = NULL, *xmark = NULL, *xS = NULL, *xSnew = NULL, *svlst = NULL, *svcnt = NULL, *xcnt = NULL,
-        *h_xcnt = NULL;
-    double *eS = NULL, *svcb = NULL, *h_l1 = NULL;
+    int *xflag = NULL, *xmark = NULL, *xS = NULL, *xSnew = NULL, *svlst = NULL, *svcnt = NULL;
+    double *eS = NULL, *svcb = NULL;
     int nS = 0;
     double acc = 0.0;
     rc |= irwls_dev_malloc((void **)&e, L1 * sizeof(double));
@@ -141,10 +141,12 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     rc |= irwls_dev_malloc((void **)&SIN, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&SC, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&lst, L1 * sizeof(int));
-    rc |= irwls_dev_malloc((void **)&perm_d, L1 * sizeof(int));
     rc |= irwls_dev_malloc((void **)&cnt, 2 * sizeof(int));
-    rc |= irwls_dev_host_alloc((void **)&h_counts, sizeof(irwls_outer_counts));
-    if (h_counts) h_counts->seq = 0;
+    rc |= irwls_dev_host_alloc((void **)&h_counts, sizeof(irwls_outer_counts) + L1 * sizeof(int));
+    if (h_counts) {
+        h_counts->seq = 0;
+        h_perm = (int *)(h_counts + 1);
+    }
     rc |= irwls_sub_alloc(&ws, W);
     if (tcs) {
         rc |= irwls_dev_malloc((void **)&xflag, L1 * sizeof(int));
@@ -153,11 +155,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         rc |= irwls_dev_malloc((void **)&xSnew, L1 * sizeof(int));
         rc |= irwls_dev_malloc((void **)&svlst, L1 * sizeof(int));
         rc |= irwls_dev_malloc((void **)&svcnt, 2 * sizeof(int));
-        rc |= irwls_dev_malloc((void **)&xcnt, 2 * sizeof(int));
         rc |= irwls_dev_malloc((void **)&eS, L1 * sizeof(double));
         rc |= irwls_dev_malloc((void **)&svcb, L1 * sizeof(double));
-        rc |= irwls_dev_host_alloc((void **)&h_xcnt, 2 * sizeof(int));
-        rc |= irwls_dev_host_alloc((void **)&h_l1, sizeof(double));
         if (!rc) {
             rc |= irwls_dev_memset(xflag, 0, L1 * sizeof(int));
             rc |= irwls_dev_memset(xmark, 0, L1 * sizeof(int));
@@ -186,11 +185,10 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         if (rc) goto done;
         if (tcs) {
             /* e = y is exact everywhere: S is the first working set */
-            rc |= irwls_full_exact_set(e, X->y, bnew, l, SW, nSW, band, 1, xflag, xmark, xS, xSnew, xcnt);
-            rc |= irwls_dev_d2h(h_xcnt, xcnt, 2 * sizeof(int));
-            rc |= irwls_dev_sync();
+            rc |= irwls_full_exact_set(e, X->y, bnew, l, SW, nSW, band, 1, xflag, xmark, xS, xSnew, h_counts, ++seq);
+            if (!rc) rc = irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(int));
             if (rc) goto done;
-            nS = h_xcnt[0];
+            nS = h_counts->nS;
         }
     }
 
@@ -220,7 +218,7 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
                     goto fail;
             }
             if (irwls_tc_kernel_rowsum(tcs, lst, cnt, cb, e, dbias, e)) goto fail;
-            if (irwls_dev_scatter(eS, xS, nS, e) || irwls_dev_d2h(h_l1, dbias + 1, sizeof(double))) goto fail;
+            if (irwls_dev_scatter(eS, xS, nS, e)) goto fail;
         } else {
             const int ex = irwls_exact_rowsum(exact, NULL, l, lst, cnt, nSW, cb, NULL, -1, e, dbias, e);
             if (ex < 0 || (ex == 1 && irwls_dev_kernel_rowsum_n(X, NULL, l, X, lst, cnt, cb, NULL, NULL, -1, e, dbias, e)))
@@ -228,17 +226,17 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         }
         /* the norms (and beta = betaNew), the classification and the next working set
            (:512-520, :540-643): the second posts last, one wait for both */
-        if (irwls_full_norms(SW, nSW, beta, bnew, l, h_counts, ++seq)) goto fail;
+        if (irwls_full_norms(SW, nSW, beta, bnew, l, dbias, h_counts, ++seq)) goto fail;
         if (irwls_full_classify(bnew, e, X->y, l, C, SW, SC, SIN, h_counts, ++seq)) goto fail;
-        if (irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(double) + 4 * sizeof(int))) goto fail;
+        if (irwls_dev_wait_post(&h_counts->seq, seq, 3 * sizeof(double) + 5 * sizeof(int))) goto fail;
         if (tcs) {
             /* a tensor-core wait that ran out left these errors stale: stop now */
-            const int tc = irwls_tc_status();
+            const int tc = h_counts->tc ? irwls_tc_status() : 0;
             if (tc) {
                 irwls_set_error(-13, "a tensor-core pipeline wait of the error update ran out (code %d)", tc);
                 goto fail;
             }
-            acc += eps * h_l1[0];
+            acc += eps * h_counts->l1;
         }
         const double ratio = h_counts->dW / h_counts->nW;
         if (ratio < props.Eta) stop = 1;
@@ -261,11 +259,12 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         } else {
             int *perm = rpermute(nSC);
             const int space = W - nSW;
-            int r2 = irwls_dev_h2d(perm_d, perm, nSC * sizeof(int));
-            r2 |= irwls_full_fill_ws(SW, nSW, SIN, nSIN, SC, nSC, perm_d, space);
-            r2 |= irwls_dev_sync();  /* perm is pageable host memory: finish the copy before freeing it */
+            /* read by the kernel from the pinned block; the classification that ends the
+               next pass comes after it */
+            memcpy(h_perm, perm, (size_t)nSC * sizeof(int));
             free(perm);
-            if (r2) goto fail;
+            irwls_count_bytes((long long)nSC * (long long)sizeof(int), 0);
+            if (irwls_full_fill_ws(SW, nSW, SIN, nSIN, SC, nSC, h_perm, space)) goto fail;
             nSW += space;
             nSIN += nSC - space;
         }
@@ -278,17 +277,18 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
                 acc = 0.0;
                 all_exact = 1;
             }
-            if (irwls_full_exact_set(e, X->y, bnew, l, SW, nSW, band, all_exact, xflag, xmark, xS, xSnew, xcnt) ||
-                irwls_dev_d2h(h_xcnt, xcnt, 2 * sizeof(int)) || irwls_dev_sync())
+            if (irwls_full_exact_set(e, X->y, bnew, l, SW, nSW, band, all_exact, xflag, xmark, xS, xSnew, h_counts,
+                                     ++seq) ||
+                irwls_dev_wait_post(&h_counts->seq, seq, 2 * sizeof(int)))
                 goto fail;
-            nS = h_xcnt[0];
-            const int nnew = h_xcnt[1];
+            nS = h_counts->nS;
+            const int nnew = h_counts->nnew;
             if (nnew > 0) {
                 /* rows entering S: e = y - sum over the support vectors - b */
-                if (irwls_full_sv_list(bnew, l, svlst, svcb, svcnt) || irwls_dev_gather(X->y, xSnew, nnew, eS) ||
-                    irwls_dev_d2h(h_xcnt, svcnt, sizeof(int)) || irwls_dev_sync())
+                if (irwls_full_sv_list(bnew, l, svlst, svcb, svcnt, h_counts, ++seq) ||
+                    irwls_dev_gather(X->y, xSnew, nnew, eS) || irwls_dev_wait_post(&h_counts->seq, seq, sizeof(int)))
                     goto fail;
-                const int nsv = h_xcnt[0];
+                const int nsv = h_counts->nsv;
                 int ex = irwls_tc_exact_rowsum(tcs, X, xSnew, nnew, svlst, nsv, NULL, nsv, svcb, NULL, NULL, -1, eS,
                                                bnew + l, eS);
                 if (ex == 1) ex = irwls_exact_rowsum(exact, xSnew, nnew, svlst, svcnt, nsv, svcb, NULL, -1, eS, bnew + l, eS);
@@ -314,11 +314,9 @@ done:
     irwls_sub_release(&ws);
     irwls_tc_set_free(tcs);
     irwls_exact_rows_free(exact);
-    void *xbufs[] = {xflag, xmark, xS, xSnew, svlst, svcnt, xcnt, eS, svcb};
+    void *xbufs[] = {xflag, xmark, xS, xSnew, svlst, svcnt, eS, svcb};
     for (size_t k = 0; k < sizeof xbufs / sizeof xbufs[0]; k++) irwls_dev_free(xbufs[k]);
-    irwls_dev_host_free(h_xcnt);
-    irwls_dev_host_free(h_l1);
-    void *bufs[] = {e, beta, bnew, cb, dbias, SW, SIN, SC, lst, perm_d, cnt};
+    void *bufs[] = {e, beta, bnew, cb, dbias, SW, SIN, SC, lst, cnt};
     for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
     irwls_dev_host_free(h_counts);
     return rc ? -1 : 0;

@@ -56,6 +56,7 @@ int irwls_dev_d2d(void *d_dst, const void *d_src, size_t bytes);   /* async */
 int irwls_dev_memset(void *d_dst, int byte, size_t bytes);         /* async */
 int irwls_dev_workspace(size_t bytes, void **d_ws);   /* grow-only scratch */
 void irwls_dev_release_workspace(void);
+void irwls_count_bytes(long long h2d, long long d2h);  /* the transfer counters */
 int irwls_dev_host_alloc(void **p, size_t bytes);      /* pinned host memory */
 void irwls_dev_host_free(void *p);
 
@@ -180,18 +181,19 @@ int irwls_sub_wait(irwls_sub_ws *ws);
 /* Outer-loop steps (src/full-train.c:436-643). d_lst/d_cb/d_cnt are scratch
  * lists of at least l entries. */
 typedef struct irwls_outer_counts {
-    double dW, nW;
-    int nSW, nSIN, nSC;
+    double dW, nW, l1;  /* l1, tc: the update's sum |beta change| and its tensor-core status */
+    int nSW, nSIN, nSC, tc;
+    int nS, nnew, nsv;  /* the exact set, the rows entering it, the support vectors */
     unsigned seq;  /* number of the last post */
-} irwls_outer_counts;  /* pinned: written by norms (dW, nW), then classify (the counts) */
+} irwls_outer_counts;  /* pinned: written by norms (to l1, and tc), then classify (the lists), exact_set and sv_list */
 int irwls_full_gin(const irwls_dev_set *X, const int *d_SW, int nSW, const int *d_SIN, int nSIN,
                    const double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_GIN, void *exact);
 int irwls_full_gather_ws(const int *d_SW, int nSW, const double *d_e, const double *d_beta, int l,
                          double *d_esub, double *d_bsub, double *d_bbest);
 int irwls_full_apply_ws(const int *d_SW, int nSW, const double *d_bt, const double *d_beta, int l,
                         double *d_bnew, int *d_lst, double *d_cb, int *d_cnt, double *d_dbias);
-int irwls_full_norms(const int *d_SW, int nSW, double *d_beta, const double *d_bnew, int l, irwls_outer_counts *h,
-                     unsigned seq);
+int irwls_full_norms(const int *d_SW, int nSW, double *d_beta, const double *d_bnew, int l, const double *d_dbias,
+                     irwls_outer_counts *h, unsigned seq);
 int irwls_full_classify(const double *d_bnew, const double *d_e, const double *d_y, int l, double C,
                         int *d_SW, int *d_SC, int *d_SIN, irwls_outer_counts *h, unsigned seq);
 int irwls_full_fill_ws(int *d_SW, int nSW, int *d_SIN, int nSIN, const int *d_SC, int nSC,
@@ -259,10 +261,12 @@ int irwls_full_exact_errors(const irwls_dev_set *X, int l, const double *d_beta,
                             double *d_e, void *exact);
 /* The exact-error row set of the precision form (dev_full.cu): S = support
  * vectors, rows with |e y| < band, and SW; Snew = rows of S not flagged
- * before (none when all_exact); counts = {|S|, |Snew|}. */
+ * before (none when all_exact); posts |S| and |Snew|. */
 int irwls_full_exact_set(const double *d_e, const double *d_y, const double *d_beta, int l, const int *d_SW, int nSW,
-                         double band, int all_exact, int *d_flag, int *d_mark, int *d_S, int *d_Snew, int *d_counts);
-int irwls_full_sv_list(const double *d_beta, int l, int *d_lst, double *d_cb, int *d_cnt);   /* beta != 0, i < l */
+                         double band, int all_exact, int *d_flag, int *d_mark, int *d_S, int *d_Snew,
+                         irwls_outer_counts *h, unsigned seq);
+int irwls_full_sv_list(const double *d_beta, int l, int *d_lst, double *d_cb, int *d_cnt, irwls_outer_counts *h,
+                       unsigned seq);   /* beta != 0, i < l; posts their number */
 int irwls_dev_gather(const double *d_src, const int *d_idx, int n, double *d_dst);    /* dst[k] = src[idx[k]] */
 int irwls_dev_scatter(const double *d_src, const int *d_idx, int n, double *d_dst);   /* dst[idx[k]] = src[k] */
 /* Bound on |k(x_i, x_j)| over the set (1 for RBF, max q for linear). */
