@@ -178,23 +178,10 @@ __global__ void __launch_bounds__(256) row_slice_kernel(const double *__restrict
     }
 }
 
-// log2(e) gamma q in units of 2^-fb: |q| = M 2^(E - 1075), times cg 2^-ec.
 __global__ void row_norms_kernel(const double *__restrict__ q, int n, unsigned long long cg, int ec, int fb,
                                  long long *__restrict__ a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned long long b = (unsigned long long)__double_as_longlong(q[i]);
-    const int E = (int)((b >> 52) & 0x7ff);
-    long long v = 0;
-    if (E != 0) {
-        const unsigned long long M = ((b & ((1ULL << 52) - 1)) | (1ULL << 52)) << 11;  // q = M 2^(E - 1086)
-        const unsigned long long h = __umul64hi(M, cg);                               // M cg 2^-64
-        const int sh = -(E - 1086 + 64 - ec + fb);                                    // value = h 2^-sh
-        if (sh <= 0) v = (long long)(h << min(-sh, 1));  // (bounded by the choice of fb: not reached)
-        else if (sh < 64) v = (long long)((h >> (sh - 1)) + 1 >> 1);
-        if (b >> 63) v = -v;
-    }
-    a[i] = v;
+    if (i < n) a[i] = fixed_scaled(q[i], cg, ec, fb);
 }
 
 // The same of the row's own fixed point, for raw rows (their kernel is that of the
@@ -490,18 +477,6 @@ __global__ void __launch_bounds__(256) gather_slices_kernel(const uint4 *__restr
             oa[i] = a[r];
         }
     }
-}
-
-// gamma log2(e) = g 2^-e with g in [2^62, 2^63): the 53-bit mantissa of gamma
-// times log2(e) 2^62, exactly.
-void scaled_gamma(double gamma, unsigned long long *g, int *e) {
-    int x;
-    const double m = frexp(gamma, &x);  // gamma = m 2^x, m in [0.5, 1)
-    unsigned __int128 p = (unsigned __int128)(unsigned long long)(m * 9007199254740992.0) * 0x5c551d94ae0bf85eULL;
-    int s = 0;  // gamma log2(e) = p 2^(x - 53 - 62)
-    while ((p >> s) >> 63) ++s;
-    *g = (unsigned long long)(p >> s);
-    *e = 115 - x - s;
 }
 
 size_t slice_bytes(long long rows, int npb) { return (size_t)((rows + PM - 1) / PM) * npb * PS * PPIECE * 2; }

@@ -9,6 +9,7 @@
 // double (worst of 20000 random arguments against 60 digits: 5.5 x 2^-62), so
 // the double is within 0.52 ulp; CUDA's exp() is within 1 ulp.
 #pragma once
+#include <math.h>
 #include <stdint.h>
 
 // 2^63 2^(-i / 16) and 2^63 2^(-i / 256), i < 16, rounded to nearest
@@ -58,4 +59,32 @@ __device__ __forceinline__ double exp2_fixed(long long y, int fb, const unsigned
         if (n < -1020) bits = 0x7ff0000000000000LL;
     }
     return __longlong_as_double(bits);
+}
+
+// log2(e) gamma q in units of 2^-fb: |q| = M 2^(E - 1075), times cg 2^-ec.
+__device__ __forceinline__ long long fixed_scaled(double q, unsigned long long cg, int ec, int fb) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(q);
+    const int E = (int)((b >> 52) & 0x7ff);
+    long long v = 0;
+    if (E != 0) {
+        const unsigned long long M = ((b & ((1ULL << 52) - 1)) | (1ULL << 52)) << 11;  // q = M 2^(E - 1086)
+        const unsigned long long h = __umul64hi(M, cg);                               // M cg 2^-64
+        const int sh = -(E - 1086 + 64 - ec + fb);                                    // value = h 2^-sh
+        if (sh <= 0) v = (long long)(h << min(-sh, 1));  // (bounded by the choice of fb: not reached)
+        else if (sh < 64) v = (long long)((h >> (sh - 1)) + 1 >> 1);
+        if (b >> 63) v = -v;
+    }
+    return v;
+}
+
+// gamma log2(e) = g 2^-e with g in [2^62, 2^63): the 53-bit mantissa of gamma
+// times log2(e) 2^62, exactly.
+inline void scaled_gamma(double gamma, unsigned long long *g, int *e) {
+    int x;
+    const double m = frexp(gamma, &x);  // gamma = m 2^x, m in [0.5, 1)
+    unsigned __int128 p = (unsigned __int128)(unsigned long long)(m * 9007199254740992.0) * 0x5c551d94ae0bf85eULL;
+    int s = 0;  // gamma log2(e) = p 2^(x - 53 - 62)
+    while ((p >> s) >> 63) ++s;
+    *g = (unsigned long long)(p >> s);
+    *e = 115 - x - s;
 }
