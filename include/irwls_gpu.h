@@ -266,7 +266,7 @@ double irwls_fp32_peak_tflops(int reps);
  * d_b: right-hand side (n doubles, device) copied into row n, or NULL if row n
  * already holds it. d_x: solution (n doubles, device), or NULL to factor only.
  * d_info: NULL, or a device int that receives the first failed pivot
- * (1-based, 0 if none). stream: a cudaStream_t, or NULL for the default
+ * (1-based, 0 if none; -1: a bounded wait ran out and x is no solution). stream: a cudaStream_t, or NULL for the default
  * stream; the call only enqueues work on it.
  *
  * Limit: n <= 4096; larger orders are rejected (-11, see
@@ -292,6 +292,11 @@ int irwls_chol_sweep_ctas(int n);
  * multi-launch sequence; 2: the data-flow launch only. Both give the same
  * bits. */
 void irwls_debug_chol_path(int mode);
+/* Test hook, no counterpart in the reference: the polls after which a wait of the
+ * solves' cluster sweep (orders up to 2048) runs out; 0: at once, below: the default
+ * 2^26. The solve then ends as usual but reports -1 in d_info (allocation-free
+ * solve), and the other calls fail with -13. */
+void irwls_debug_sweep_wait(long long polls);
 
 #ifdef __cplusplus
 }

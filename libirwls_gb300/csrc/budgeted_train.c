@@ -213,6 +213,10 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
             if (irwls_par_residual(d_KSC, l, m, d_beta, X->y, C, M, d_e, d_Da)) goto fail;
             if (irwls_par_weights(d_Da, X->y, l, d_act, d_sd, d_day, h_post, (unsigned)iter + 1)) goto fail;
             if (irwls_dev_wait_post(&h_post->seq, (unsigned)iter + 1, 2 * sizeof(double) + sizeof(int))) goto fail;
+            if (h_post->tc) {
+                irwls_set_error(-13, "a bounded wait of the Gram or of the solve ran out (code %d)", irwls_tc_status());
+                goto fail;
+            }
             dW = h_post->dW;
             nW = h_post->nW;
             nact = h_post->nact;
@@ -232,13 +236,6 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
         g_last_nact = nact;
     }
     if (irwls_dev_d2h(weights_out, d_bbest, (size_t)m * sizeof(double)) || irwls_dev_sync()) goto fail;
-    if (digits) {
-        const int tc = irwls_tc_status();
-        if (tc) {
-            irwls_set_error(-13, "a tensor-core pipeline wait of the Gram ran out (code %d)", tc);
-            goto fail;
-        }
-    }
     goto done;
 fail:
     rc = -1;

@@ -896,12 +896,13 @@ __global__ void first_weights_kernel(const double *__restrict__ y, int l, double
 
 // dW = |bnew - beta|^2, nW = |bnew|^2 (chunked, fixed order), beta <- bnew.
 __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bnew, double *beta, int m,
-                                                   irwls_par_post *h) {
+                                                   irwls_par_post *h, const int *__restrict__ flags) {
     chain_wait();
     chain_open();
     __shared__ double red[33];
     const int ch = (m + CT - 1) / CT;
     const int b = threadIdx.x * ch, e = min(m, b + ch);
+    const int tc = flags[1];
     double vd = 0.0, vn = 0.0;
     for (int i = b; i < e; ++i) {
         const double d = __dsub_rn(bnew[i], beta[i]);
@@ -915,6 +916,7 @@ __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bn
     if (threadIdx.x == 0) {
         h->dW = dW;
         h->nW = nW;
+        h->tc = tc;
         __threadfence_system();
     }
 }
@@ -1151,7 +1153,7 @@ extern "C" int irwls_par_weights(const double *d_Da, const double *d_y, int l, i
 }
 
 extern "C" int irwls_par_delta(const double *d_bnew, double *d_beta, int m, irwls_par_post *h) {
-    launch_chained(delta_kernel, dim3(1), dim3(CT), 0, d_bnew, d_beta, m, h);
+    launch_chained(delta_kernel, dim3(1), dim3(CT), 0, d_bnew, d_beta, m, h, irwls_dev_flags());
     IRWLS_LAUNCH_CHECK("delta");
     return 0;
 }

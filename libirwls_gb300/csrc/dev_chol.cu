@@ -921,6 +921,13 @@ __global__ void __launch_bounds__(256) chol_backsolve_coop_kernel(double *__rest
 // after another on one: 65 cycles per FP64 instruction whatever the lanes.
 // subst: the last block by substitution with its L and reciprocal pivots, 5000
 // cycles once, instead of an inverse formed at the factorization's end.
+//
+// The waits are bounded, by `limit` polls. A thread whose wait runs out goes on
+// without waiting, on whatever it has: every barrier is reached by all its threads
+// and every x_b is sent, so nobody else is left standing, and the pivot status -1
+// and the status word CHOL_WAIT_CODE tell the caller that x is not a solution. A CTA
+// leaves when all that was sent to it has arrived: a store still under way would
+// land in the shared memory of whatever runs there next.
 __device__ __forceinline__ double chains_sum(double a) {
     a += __shfl_xor_sync(0xffffffffu, a, 1);
     return a + __shfl_xor_sync(0xffffffffu, a, 2);  // (a0 + a1) + (a2 + a3)
@@ -936,10 +943,10 @@ struct SweepShared {
 __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double *__restrict__ M, int n, int ld,
                                                                     const double *__restrict__ Dinv,
                                                                     double *__restrict__ x,
-                                                                    const int *__restrict__ flags,
+                                                                    int *__restrict__ flags,
                                                                     int *__restrict__ info,
                                                                     unsigned *__restrict__ clear, int words,
-                                                                    int subst) {
+                                                                    int subst, long long limit) {
     chain_wait();
     chain_open();
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -976,7 +983,6 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
             load_inv(b, tid, 256);
         }
     }
-    if (info && me == 0 && tid == 0) *info = *flags;
     cl.sync();
     // this thread's values of rows of L_b^T for block q (4 k + ch)
     auto load_row = [&](int q, int b, double *v) {
@@ -1002,10 +1008,10 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
         a = chains_sum(a);
         if (ch == 0) sh.z[q / g][row] = sh.z[q / g][row] - a;
     };
+    bool ok = true;
     if (tid < 128) {
         double pre[8];
-        bool ok = true;
-        for (int b = nblk - 1; b >= 0 && ok; --b) {
+        for (int b = nblk - 1; b >= 0; --b) {
             if (b % g == me) {
                 const int nb = min(NB, n - NB * b), t = row, K = t < nb ? (nb - t) / 4 : 0;
                 const double(*D)[NB + 1] = sh.Di[b & 1];
@@ -1054,23 +1060,21 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
                 load_inv(b - 1, tid, 128);
                 load_row(b - 1, b, pre);
                 // x_(b+1) and all before it are in the block (none when b is the last)
-                if (b + 1 < nblk) ok = mbar_wait(smem_u32(&sh.ready[(b - 1) / g]), 0u);
-                ok = ok && mbar_wait(smem_u32(&sh.got[b]), 0u);
+                if (b + 1 < nblk) ok = ok && mbar_wait(smem_u32(&sh.ready[(b - 1) / g]), 0u, limit);
+                ok = ok && mbar_wait(smem_u32(&sh.got[b]), 0u, limit);
                 update(b - 1, b, pre);
                 asm volatile("bar.sync 1, 128;\n" ::: "memory");
             }
         }
     } else {
-        bool ok = true;
-        for (int b = nblk - 1; b >= 2 && ok; --b) {
+        for (int b = nblk - 1; b >= 2; --b) {
             // this CTA's blocks q <= b - 2, the next to be handed over first
             int q = b - 2 - ((b - 2 - me) % g + g) % g;
             if (q < 0) continue;
             double v[8];
             load_row(q, b, v);
-            ok = mbar_wait(smem_u32(&sh.got[b]), 0u);
-            if ((b - 1) % g == me) ok = ok && mbar_wait(smem_u32(&sh.got[b - 1]), 0u);
-            if (!ok) break;
+            ok = ok && mbar_wait(smem_u32(&sh.got[b]), 0u, limit);
+            if ((b - 1) % g == me) ok = ok && mbar_wait(smem_u32(&sh.got[b - 1]), 0u, limit);
             for (; q >= 0; q -= g) {
                 update(q, b, v);
                 if (q == b - 2) {
@@ -1081,8 +1085,18 @@ __global__ void __launch_bounds__(256, 1) chol_sweep_cluster_kernel(const double
             }
         }
     }
-    cl.sync();  // no CTA leaves while others may send to it
+    // every x_b but x_0 goes to every CTA
+    if (tid > 0 && tid < nblk && !mbar_wait(smem_u32(&sh.got[tid]), 0u)) ok = false;
+    if (!ok) {
+        atomicExch(flags, -1);
+        atomicExch(flags + 1, CHOL_WAIT_CODE | 0x10000 | me);
+    }
+    cl.sync();  // (all have reported)
+    if (info && me == 0 && tid == 0) *info = atomicAdd(flags, 0);
 }
+
+// Polls of a sweep's waits (irwls_debug_sweep_wait).
+std::atomic<long long> g_sweep_wait{TC_WAIT_LIMIT};
 
 // CTAs of the cooperative sweep for order n on the current device, or 0 when
 // they cannot all be resident at once (the single-CTA sweep is used then).
@@ -1139,7 +1153,7 @@ bool sweep_cluster_ok() {
 }
 
 int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, double *Dinv, cudaStream_t st);
-int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
+int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, int *flags, int *d_info,
                            cudaStream_t st, unsigned *clear, size_t words, bool chained, bool subst);
 
 // Whether the cluster sweep takes order n.
@@ -1234,7 +1248,7 @@ int chol_enqueue_panels(double *d_M, int n, int ld, int nrows, int *flags, doubl
 // The backward sweep L^T x = z (z in row n of M): the cluster form up to order
 // 2048, the cooperative one above, one CTA where neither can run. They give
 // the same bits.
-int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, const int *flags, int *d_info,
+int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv, int *flags, int *d_info,
                            cudaStream_t st, unsigned *clear, size_t words, bool chained, bool subst) {
     {
         if (cluster_sweep_for(n)) {
@@ -1253,7 +1267,8 @@ int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv
             cfg.attrs = at;
             cfg.numAttrs = chained ? 2 : 1;
             const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_sweep_cluster_kernel, (const double *)d_M, n, ld,
-                                                     (const double *)Dinv, d_x, flags, d_info, clear, (int)words, (int)subst);
+                                                     (const double *)Dinv, d_x, flags, d_info, clear, (int)words, (int)subst,
+                                                     g_sweep_wait.load());
             if (e != cudaSuccess) {
                 irwls_set_error(-2, "CUDA error in chol_sweep (cluster): %s", cudaGetErrorString(e));
                 return -2;
@@ -1342,6 +1357,11 @@ extern "C" int irwls_chol_sweep_ctas(int n) { return coop_backsolve_ctas(n); }
 // possible (default), 1 = the multi-launch factorization, 2 = data flow only.
 extern "C" void irwls_debug_chol_path(int mode) { g_chol_path = mode >= 0 && mode <= 2 ? mode : 0; }
 
+// Test hook: polls of the cluster sweep's waits (0: each runs out at once; below: the
+// default).
+extern "C" void irwls_debug_sweep_wait(long long polls) { g_sweep_wait.store(polls >= 0 ? polls : TC_WAIT_LIMIT); }
+
+// -1 in *info: a bounded wait of the solve ran out.
 extern "C" int irwls_dev_pivot_status(int *info) {
     *info = 0;
     cudaError_t e = cudaMemcpyAsync(info, irwls_dev_flags(), sizeof(int), cudaMemcpyDeviceToHost, irwls_stream());

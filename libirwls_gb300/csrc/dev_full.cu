@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double 
     __shared__ double buf[2][NT], part[2][4];
     __shared__ int s_scan[32], s_better;
     const int w = ws.w;
+    const int tc = ws.flags[1];  // (here, so that the post does not wait for it)
     if (threadIdx.x == 0) {
         const double ratio = ws.stats->dW / ws.stats->nW;
         s_better = ratio < ws.stats->best;
@@ -438,6 +439,7 @@ __global__ void __launch_bounds__(NT) sub_groups_kernel(irwls_sub_ws ws, double 
         h->bmin = ws.stats->bmin;
         h->nS1 = n1;
         h->nS3 = n3;
+        h->tc = tc;
         post_seq(&h->seq, ws.seq);
     }
 }
@@ -998,6 +1000,7 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
     rc |= irwls_dev_malloc((void **)&ws->stats, sizeof(irwls_sub_stats));
     rc |= irwls_dev_host_alloc((void **)&ws->h_stats, sizeof(irwls_sub_stats));
     if (ws->h_stats) memset(ws->h_stats, 0, sizeof(irwls_sub_stats));
+    ws->flags = irwls_dev_flags();
     ws->map = ws->mapbuf;
     return rc ? -3 : 0;
 }

@@ -43,6 +43,11 @@ static int run_sub(irwls_sub_ws *ws, const irwls_dev_set *X, const properties *p
         if (irwls_sub_iterate(ws, X, C, n1, n3)) return -1;
         if (irwls_sub_wait(ws)) return -1;
         const irwls_sub_stats *st = ws->h_stats;
+        if (st->tc) {
+            irwls_set_error(-13, "a bounded wait of a working-set system or an error update ran out (code %d)",
+                            irwls_tc_status());
+            return -1;
+        }
         dW = st->dW;
         nW = st->nW;
         bmax = st->bmax;

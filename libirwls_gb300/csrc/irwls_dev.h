@@ -144,7 +144,8 @@ int irwls_dev_gemv(const double *d_A, const double *d_v, double *d_out, int size
 typedef struct irwls_sub_stats {
     double dW, nW, bmax, bmin, best;  /* best: the smallest dW / nW so far, of bbest */
     int nS1, nS3;
-    unsigned seq, pad;
+    unsigned seq;
+    int tc;  /* a bounded wait of this or an earlier kernel ran out (the status word) */
 } irwls_sub_stats;
 
 /* The inner-IRWLS device state on a working set of w rows; map[i] is the
@@ -160,6 +161,7 @@ typedef struct irwls_sub_ws {
     irwls_sub_stats *stats;   /* device */
     irwls_sub_stats *h_stats; /* pinned host mirror, written by the last kernel of a step */
     unsigned seq;             /* number of the last step */
+    const int *flags;         /* the context's status words */
     int ldH;
     void *tcs;                /* precision form: the training's tensor-core set (NULL: FP64 throughout) */
 } irwls_sub_ws;
@@ -240,12 +242,13 @@ int irwls_par_gram_tc(const double *d_KSC, int m, const int *d_act, int nact, co
 int irwls_par_gram_reduce(const double *d_part, int P, int m, const double *d_KC, double *d_K1, int ldK1);
 int irwls_par_residual(const double *d_KSC, int l, int m, const double *d_beta, const double *d_y, double C,
                        double M, double *d_e, double *d_Da);
-/* one iteration's results in pinned host memory: delta writes dW and nW, weights
- * nact and then the iteration's number */
+/* one iteration's results in pinned host memory: delta writes dW, nW and tc (the status
+ * word of the bounded waits before it), weights nact and then the iteration's number */
 typedef struct irwls_par_post {
     double dW, nW;
     int nact;
     unsigned seq;
+    int tc, pad;
 } irwls_par_post;
 int irwls_par_weights(const double *d_Da, const double *d_y, int l, int *d_act, double *d_sd, double *d_day,
                       irwls_par_post *h, unsigned seq);

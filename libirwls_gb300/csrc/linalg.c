@@ -56,6 +56,10 @@ static int block_solve(double *matrix, int r, int ro, int co, int n, const doubl
     }
     int info = 0;
     if (!rc) rc |= irwls_dev_pivot_status(&info);
+    if (!rc && info < 0) {
+        irwls_set_error(-13, "a bounded wait of the order-%d solve ran out (code %d)", n, irwls_tc_status());
+        rc = -13;
+    }
     if (!rc && info)
         irwls_set_warning(IRWLS_WARN_PIVOT,
                           "pivot %d of the order-%d system is not positive: it is stored without its square root "

@@ -25,9 +25,9 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t da, uint64_t db
         "l"(da), "l"(db), "r"(idesc), "r"(acc));
 }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long long limit = TC_WAIT_LIMIT) {
     uint32_t done = 0;
-    for (long long it = 0; it < TC_WAIT_LIMIT && !done; ++it) {
+    for (long long it = 0; it < limit && !done; ++it) {
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(done)
