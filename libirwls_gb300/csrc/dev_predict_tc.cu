@@ -18,7 +18,8 @@
 //    the levels combine to the integer T = sum N N' 2^-48 (the dropped levels
 //    weigh below 2^-61 sigma sigma' per feature).
 // 3. y = log2(e) gamma (q_i + q_j) - 2 log2(e) gamma sigma_i sigma_j 2^-62 T
-//    in 64-bit fixed point (its unit 2^-56, or below 2^-56 of the largest term), then
+//    in 64-bit fixed point (its unit 2^-56, or below 2^-56 of the largest term, but
+//    no coarser than FP64 sums of the nearest rows: fixed_point_of), then
 //    2^-y by exp2_fixed. The value times w_j is added in FP64, in vector order
 //    per strip of 16 of every 64 vectors; the strips' sums in a fixed order.
 //
@@ -57,9 +58,12 @@ static_assert((5LL * 256 + 6) * PDRAIN * PK * 128 * 128 < (1LL << 31), "levels 3
 // Element offset of (row r of the 128-row tile, k of the 16-feature block) in a piece.
 __device__ __forceinline__ int ppiece_off(int r, int k) { return (r >> 3) * 128 + (k >> 3) * 64 + (r & 7) * 8 + (k & 7); }
 
+constexpr int TOPS = 4;  // words of a set's maxima (row_scales_kernel)
+
 // Per row: e with 2^e >= |x| (-2000: a zero row), and over the set the largest
-// |q| (with q) and the largest |x|^2 (floats rounded up a little, as bits) and, with w,
-// the high half of the largest |w|; with rp that of infinity where a row's
+// |q| (with q) and the largest |x|^2 (floats rounded up a little, as bits), with w
+// the high half of the largest |w|, and with q the complement of the smallest |q|
+// (rounded down); with rp that of infinity where a row's
 // indices do not increase (a vector that names a feature twice: its products add
 // both). One warp per row.
 __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restrict__ X, int ld, int width,
@@ -67,9 +71,9 @@ __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restric
                                                          const double *__restrict__ w, const int *__restrict__ rp,
                                                          const int *__restrict__ ci, int n, int *__restrict__ ex,
                                                          unsigned *__restrict__ top) {
-    __shared__ unsigned big[3];
+    __shared__ unsigned big[TOPS];
     const int lane = threadIdx.x & 31;
-    if (threadIdx.x < 3) big[threadIdx.x] = 0;
+    if (threadIdx.x < TOPS) big[threadIdx.x] = 0;
     __syncthreads();
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const double *row = X + (size_t)i * ld;
@@ -109,13 +113,16 @@ __global__ void __launch_bounds__(256) row_scales_kernel(const double *__restric
             ex[i] = E == 0 ? -2000 : e + max(grow, 0);
             // (the order of non-negative floats is that of their bits; an
             // overflow to infinity makes the caller take the other path)
-            if (q) atomicMax(big, __float_as_uint(fabsf((float)q[i]) * up));
+            if (q) {
+                atomicMax(big, __float_as_uint(fabsf((float)q[i]) * up));
+                atomicMax(big + 3, ~__float_as_uint(fabsf((float)q[i]) * 0.999f));
+            }
             atomicMax(big + 1, __float_as_uint(E == 0 ? 0.f : ldexpf(rho * up, 2 * e)));
             if (w || bad) atomicMax(big + 2, bad ? 0x7ff00000u : (unsigned)__double2hiint(w[i]) & 0x7fffffffu);
         }
     }
     __syncthreads();
-    if (threadIdx.x < 3 && big[threadIdx.x]) atomicMax(top + threadIdx.x, big[threadIdx.x]);
+    if (threadIdx.x < TOPS && big[threadIdx.x]) atomicMax(top + threadIdx.x, big[threadIdx.x]);
 }
 
 // round(x 2^(55 - e)) for |x| <= 2^e, ties away from zero.
@@ -482,7 +489,12 @@ __global__ void __launch_bounds__(256) gather_slices_kernel(const uint4 *__restr
 size_t slice_bytes(long long rows, int npb) { return (size_t)((rows + PM - 1) / PM) * npb * PS * PPIECE * 2; }
 
 // The fixed point of y from the maxima of the two sets (row_scales_kernel: |q|,
-// |x|^2 and, for the vectors, |w|), and cg 2^-ec = gamma log2(e); false: not for it.
+// |x|^2, for the vectors |w|, and the smallest |q|), and cg 2^-ec = gamma log2(e);
+// false: not for it. One unit serves all pairs, and the largest norms set it: a unit
+// above 2^-53 is taken only where it is below half an ulp of c (q_i + q_j), which FP64
+// sums round to, for the smallest norms too. (One row of |x|^2 = 10^7 among rows of 10,
+// gamma 0.1: unit 2^-40, the other rows' values 3.5e-14 off, in FP64 3.4e-17. Rows of
+// 400 to 450 apart by 1, gamma 0.25: unit 2^-51, 3.7e-17 off, in FP64 1.8e-15.)
 // Raw rows (no q) take it in units of 2^-53 at most: there it is as close as the
 // differences' squares summed in FP64 (units of y each, about 3 to a value's 1 to
 // 2 ulp), in larger units close rows would not be.
@@ -502,7 +514,17 @@ bool fixed_point_of(double gamma, bool raw, const float *ht, const float *hs, Pr
     a->emax = hs[1] > 0.f ? (ilogb((double)hs[1]) >> 1) + 1 : -74;
     // y's product part = 2 c 2^(e_i + e_j) 2^-62 T 2^fb; no left shift in it
     a->fb = std::min(a->fb, *ec - 3 - ei - a->emax);
-    if (a->fb < (raw ? 53 : 32)) return false;
+    if (a->fb < 53) {
+        unsigned low[2];
+        float qmin[2];
+        memcpy(low, ht + 3, sizeof low[0]);
+        memcpy(low + 1, hs + 3, sizeof low[0]);
+        for (int k = 0; k < 2; ++k) low[k] = ~low[k];
+        memcpy(qmin, low, sizeof qmin);
+        if (raw || a->fb < 32 ||
+            !(ldexp(1.0, 54 - a->fb) <= gamma * 1.4426950408889634 * ((double)qmin[0] + (double)qmin[1])))
+            return false;
+    }
     a->g = *cg;
     a->shr = *ec - 3 - a->fb - a->emax;
     return true;
@@ -553,7 +575,7 @@ int slice_grid(long long rows, int npb, int sms) {
 // are not for it (the caller then sums on the FP64 pipe): not the RBF kernel, more than 12288 features (what the FP64 path takes) or 4 GB of vector
 // slices, a vector that names a feature twice, a gamma outside (1e-30, 1e6),
 // features or weights that are not finite, values whose squares leave FP32's
-// range or whose y does not fit its fixed point, no room for the workspace, or
+// range or whose y does not fit a fixed point as fine as FP64, no room for the workspace, or
 // fewer than 500000 kernel values: the preparation and the host's wait for the
 // maxima cost about 60 us. A call with 500000 values (1000 vectors) took 190 us there
 // and 200 here with 20 features a row, 192 and 178 with 12 of 54, 1558 and 919 with
@@ -592,7 +614,7 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     int *et = (int *)(ws + off_et), *es = (int *)(ws + off_es);
     long long *at = (long long *)(ws + ((off_at + 255) & ~(size_t)255)), *as = (long long *)(ws + ((off_as + 255) & ~(size_t)255));
     unsigned *top = (unsigned *)(ws + ((off_top + 255) & ~(size_t)255));
-    int rc = irwls_dev_memset(top, 0, 6 * sizeof(unsigned));
+    int rc = irwls_dev_memset(top, 0, 2 * TOPS * sizeof(unsigned));
     auto fail = [&](int code) {
         irwls_dev_free(ws);
         return code;
@@ -603,17 +625,17 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
                                                      et, top);
     irwls_count_launch(1);
     row_scales_kernel<<<gs, 256, 0, irwls_stream()>>>(S->X, S->ld, S->width, raw ? nullptr : S->q, d_w, raw ? nullptr : S->rp, S->ci,
-                                                     nSV, es, top + 3);
+                                                     nSV, es, top + TOPS);
     irwls_count_launch(1);
     row_slice_kernel<<<slice_grid((long long)ceil_div(nSV, PM) * PM, npb, sms), 256, 0, irwls_stream()>>>(S->X, S->ld, S->width, nSV, es, ceil_div(nSV, PM) * PM, npb, dS);
     irwls_count_launch(1);
     if ((rc = irwls_check_launch("predict_prepare"))) return fail(rc);
-    float h[6];
+    float h[2 * TOPS];
     if (irwls_dev_d2h(h, top, sizeof h) || irwls_dev_sync()) return fail(-2);
     PredictArgs a = {};
     unsigned long long cg;
     int ec;
-    if (!fixed_point_of(gamma, raw, h, h + 3, &a, &cg, &ec)) return fail(1);
+    if (!fixed_point_of(gamma, raw, h, h + TOPS, &a, &cg, &ec)) return fail(1);
     launch_norms(T, raw, n, et, cg, ec, a.fb, at);
     launch_norms(S, raw, nSV, es, cg, ec, a.fb, as);
     a.T = dT;
@@ -707,8 +729,8 @@ extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) 
     E->part = (double *)w;
     E->nparts = nparts;
     E->n = n, E->npb = npb, E->na = na, E->sms = sms;
-    float h[3];
-    int rc = irwls_dev_memset(top, 0, 3 * sizeof(unsigned));
+    float h[TOPS];
+    int rc = irwls_dev_memset(top, 0, TOPS * sizeof(unsigned));
     row_scales_kernel<<<std::min(ceil_div(n, 8), 4 * sms), 256, 0, irwls_stream()>>>(X->X, X->ld, X->width,
                                                                                   raw ? nullptr : X->q, nullptr,
                                                                                   raw ? nullptr : X->rp, X->ci, n,
