@@ -193,20 +193,27 @@ __global__ void row_norms_kernel(const double *__restrict__ q, int n, unsigned l
 
 // The same of the row's own fixed point, for raw rows (their kernel is that of the
 // differences: FP64 norms would leave c |x|^2 2^-53 of them, the integers leave
-// units of y): T_ii = sum N N 2^-48, in the products' unit. A warp per row.
+// units of y): T_ii = sum N N 2^-48, in the products' unit, summed to 2^-32 of it
+// before it is rounded (a product's floor per feature put all of a set's values
+// 3.2e-15 off at 784 features). A warp per row.
 __global__ void __launch_bounds__(256) row_norms_raw_kernel(const double *__restrict__ X, int ld, int width, int n,
                                                             const int *__restrict__ ex, unsigned long long cg, int ec,
                                                             int fb, long long *__restrict__ a) {
     const int lane = threadIdx.x & 31;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const int e = ex[i];
-        long long T = 0;
+        long long T = 0, low = 0;
         if (e > -2000)
             for (int t = lane; t < width; t += 32) {
                 const long long N = fixed55(X[(size_t)i * ld + t], e) << 8;
                 T += __mul64hi(N, N);
+                low += (unsigned long long)(N * N) >> 32;
             }
-        for (int o = 16; o > 0; o >>= 1) T += __shfl_xor_sync(0xffffffffu, T, o);
+        for (int o = 16; o > 0; o >>= 1) {
+            T += __shfl_xor_sync(0xffffffffu, T, o);
+            low += __shfl_xor_sync(0xffffffffu, low, o);
+        }
+        T += (low + (1LL << 31)) >> 32;
         // c |x|^2 2^fb = T cg 2^(2 e - 62 - ec + fb)
         const int sh = -(2 * e + 2 - ec + fb);
         const long long m = (long long)__umul64hi((unsigned long long)T, cg);
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(128 + 32 * 16, 1) predict_tc_kernel(PredictArg
             if (et < PN && jj + 1 < jn) fetch(j0 + jj + 1);
             if (MULTI)
 #pragma unroll
-                for (int c = 0; c < CW; ++c) T[c] = 0;
+                for (int c = 0; c < CW; ++c) T[c] = nd >> 1;  // (l[0] >> 8 takes half a unit off per drain)
             for (int d = 0; d < nd; ++d, ++blk) {
                 // (this barrier also publishes the tile's vectors, and after it
                 // nobody reads the other buffer)
@@ -495,11 +502,18 @@ size_t slice_bytes(long long rows, int npb) { return (size_t)((rows + PM - 1) / 
 // sums round to, for the smallest norms too. (One row of |x|^2 = 10^7 among rows of 10,
 // gamma 0.1: unit 2^-40, the other rows' values 3.5e-14 off, in FP64 3.4e-17. Rows of
 // 400 to 450 apart by 1, gamma 0.25: unit 2^-51, 3.7e-17 off, in FP64 1.8e-15.)
-// Raw rows (no q) take it in units of 2^-53 at most: there it is as close as the
-// differences' squares summed in FP64 (units of y each, about 3 to a value's 1 to
-// 2 ulp), in larger units close rows would not be.
-bool fixed_point_of(double gamma, bool raw, const float *ht, const float *hs, PredictArgs *a, unsigned long long *cg,
-                    int *ec) {
+// Raw rows (no q) take it in units of 2^-56, from 16 features on 2^-55: there it is as
+// close as the differences' squares summed in FP64 (rms of a value at a common offset
+// of the rows: 3.4e-17 and 3.4e-17 in FP64 at 20 features and 2^-55, 3.8e-17 and
+// 3.3e-17 at 4), in larger units it is not (2^-53: 7.5e-17). And the products' dropped levels
+// weigh 0.083 units of T per feature in a row's product with itself or a row near it (the
+// digits agree), where the norms have them whole: y is off by
+// 0.17 width c sigma^2 2^-62 there, where differences give 0 (784 features and an
+// exponent of 62: all values 3.2e-15 off; FP64 sums 6e-17). Raw rows are taken while
+// that stays below 2^-54: width times the exponent up to 1536 (3.5e-17 and 3.5e-17 in
+// FP64 at 1320, 4.2e-17 and 3.7e-17 at 1960).
+bool fixed_point_of(double gamma, bool raw, int width, const float *ht, const float *hs, PredictArgs *a,
+                    unsigned long long *cg, int *ec) {
     unsigned wtop;
     memcpy(&wtop, hs + 2, sizeof wtop);
     if (!(ht[1] < 1e30f && hs[1] < 1e30f) || wtop >= 0x7ff00000u) return false;
@@ -514,17 +528,19 @@ bool fixed_point_of(double gamma, bool raw, const float *ht, const float *hs, Pr
     a->emax = hs[1] > 0.f ? (ilogb((double)hs[1]) >> 1) + 1 : -74;
     // y's product part = 2 c 2^(e_i + e_j) 2^-62 T 2^fb; no left shift in it
     a->fb = std::min(a->fb, *ec - 3 - ei - a->emax);
-    if (a->fb < 53) {
+    if (!raw && a->fb < 53) {
         unsigned low[2];
         float qmin[2];
         memcpy(low, ht + 3, sizeof low[0]);
         memcpy(low + 1, hs + 3, sizeof low[0]);
-        for (int k = 0; k < 2; ++k) low[k] = ~low[k];
+        for (unsigned &v : low) v = ~v;
         memcpy(qmin, low, sizeof qmin);
-        if (raw || a->fb < 32 ||
+        if (a->fb < 32 ||
             !(ldexp(1.0, 54 - a->fb) <= gamma * 1.4426950408889634 * ((double)qmin[0] + (double)qmin[1])))
             return false;
     }
+    // (sigma^2 is at most 4 |x|^2, so c sigma^2 at most ym)
+    if (raw && (a->fb < (width < 16 ? 56 : 55) || ym * width > 1536.0)) return false;
     a->g = *cg;
     a->shr = *ec - 3 - a->fb - a->emax;
     return true;
@@ -635,7 +651,7 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     PredictArgs a = {};
     unsigned long long cg;
     int ec;
-    if (!fixed_point_of(gamma, raw, h, h + TOPS, &a, &cg, &ec)) return fail(1);
+    if (!fixed_point_of(gamma, raw, width, h, h + TOPS, &a, &cg, &ec)) return fail(1);
     launch_norms(T, raw, n, et, cg, ec, a.fb, at);
     launch_norms(S, raw, nSV, es, cg, ec, a.fb, as);
     a.T = dT;
@@ -742,7 +758,7 @@ extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) 
     rc = rc || irwls_check_launch("exact_rows") || irwls_dev_d2h(h, top, sizeof h) || irwls_dev_sync();
     unsigned long long cg;
     int ec;
-    if (rc || !fixed_point_of(gamma, raw, h, h, &E->p, &cg, &ec)) {
+    if (rc || !fixed_point_of(gamma, raw, X->width, h, h, &E->p, &cg, &ec)) {
         irwls_exact_rows_free(E);
         return nullptr;
     }
