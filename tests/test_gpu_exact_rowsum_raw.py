@@ -17,8 +17,8 @@ N, NB = 2000, 300
 
 
 # width, the exponent of twice a row's norm (about; the largest is up to 1.7 times that), the spread of the rows; whether they are for this path
-@pytest.mark.parametrize("d,top,spread,taken", [(20, 15, 1.0, True), (40, 30, 0.2, True), (100, 17, 0.2, True),
-                                                (97, 4, 1.0, True), (4, 12, 0.2, True), (4, 45, 0.2, False),
+@pytest.mark.parametrize("d,top,spread,taken", [(20, 15, 1.0, True), (40, 30, 0.2, True), (100, 12, 0.2, True),
+                                                (97, 4, 1.0, True), (100, 17, 0.2, False), (4, 12, 0.2, True), (4, 45, 0.2, False),
                                                 (20, 45, 0.2, True), (20, 90, 0.2, False), (200, 120, 0.2, False),
                                                 (784, 62, 0.2, False), (784, 120, 1.0, False), (2000, 16, 0.2, False)])
 def test_values(d, top, spread, taken):
