@@ -187,6 +187,7 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     rc |= irwls_dev_host_alloc((void **)&h_post, sizeof(irwls_par_post));
     if (rc) goto done;
     h_post->seq = 0;
+    h_post->tc = 0;
     double M = 10000.0;
     rc |= irwls_dev_h2d(d_idx, idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_memset(d_beta, 0, (size_t)m * sizeof(double));

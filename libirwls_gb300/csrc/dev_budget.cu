@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(CT) delta_kernel(const double *__restrict__ bn
     if (threadIdx.x == 0) {
         h->dW = dW;
         h->nW = nW;
-        h->tc = tc;
+        if (tc) h->tc = tc;  // (zero before)
         __threadfence_system();
     }
 }

@@ -146,6 +146,7 @@ typedef struct irwls_sub_stats {
     int nS1, nS3;
     unsigned seq;
     int tc;  /* a bounded wait of this or an earlier kernel ran out (the status word) */
+    int unordered, pad;  /* cnt[1] */
 } irwls_sub_stats;
 
 /* The inner-IRWLS device state on a working set of w rows; map[i] is the
@@ -158,6 +159,7 @@ typedef struct irwls_sub_ws {
     double *K;            /* kernel matrix of the working set, w x w (NULL: too large to keep) */
     int *grp, *S1, *S3, *lst, *lloc, *gl1, *gl3, *cnt, *mapbuf;   /* lst, lloc: changed weights, as rows of X and of the set */
     int use13;            /* this iteration's G13 is not zero */
+    int ordered;          /* cnt[1] says whether a row of the set names a feature twice or out of order */
     irwls_sub_stats *stats;   /* device */
     irwls_sub_stats *h_stats; /* pinned host mirror, written by the last kernel of a step */
     unsigned seq;             /* number of the last step */
