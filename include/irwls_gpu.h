@@ -33,6 +33,9 @@ enum { IRWLS_WARN_PIVOT = 1 };
  * disarms). The call that meets it fails with -3, as when the runtime refuses
  * memory, and the library stays usable. */
 void irwls_debug_fail_alloc(long long n);
+/* Test hook, no counterpart in the reference: device allocations of more than
+ * `bytes` are refused from now on, as where memory is short (0: none is). */
+void irwls_debug_alloc_limit(size_t bytes);
 /* Test hook, no counterpart in the reference: the poll limit of every bounded
  * wait of the precision form's full-IRWLS error-update kernel (<= 0: the
  * default, 2^26 polls) and a stall switch with which that kernel's MMA thread

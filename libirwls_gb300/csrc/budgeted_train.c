@@ -34,7 +34,8 @@ int *randomCentroids(svm_dataset dataset, properties props) {
 }
 
 int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out);
-int irwls_sgma_screened_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out);
+int irwls_sgma_screened_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, const int *cand,
+                            int *cent_out);
 
 /* Candidate draws of every SGMA step s >= 2 (src/budgeted-train.c:157-167):
  * candidate i must carry label (i % 2) * 2 - 1. */
@@ -64,13 +65,14 @@ int irwls_sgma_dev(const irwls_dev_set *X, const svm_dataset *ds, properties pro
     const int m = props.size, l = ds->l;
     if (m <= 0) return 0;
     if (irwls_get_precision() == IRWLS_PRECISION_MIXED) return irwls_sgma_mixed_dev(X, ds, props, cent_out);
-    {
-        const int rc = irwls_sgma_screened_dev(X, ds, props, cent_out);
-        if (rc != -100) return rc;
-    }
     int *cand = irwls_draw_sgma_candidates(ds, m);
     if (!cand) return -1;
-    int rc = 0;
+    int rc = irwls_sgma_screened_dev(X, ds, props, cand, cent_out);
+    if (rc != -100) {
+        free(cand);
+        return rc;
+    }
+    rc = 0;
     int *d_cand = NULL, *d_cent = NULL, *d_best = NULL;
     double *d_L = NULL, *d_KSC = NULL, *d_W = NULL, *d_Z = NULL, *d_KN = NULL, *d_eta = NULL, *d_part = NULL,
            *d_val = NULL;

@@ -257,6 +257,9 @@ extern "C" void irwls_rand_sequence(unsigned seed, int n, int *out) {
 // on fails as if the runtime had refused it (nothing is allocated).
 static std::atomic<long long> g_fail_alloc{0};
 extern "C" void irwls_debug_fail_alloc(long long n) { g_fail_alloc.store(n > 0 ? n : 0); }
+// Device allocations above this are refused, as where memory is short.
+static std::atomic<size_t> g_alloc_limit{~(size_t)0};
+extern "C" void irwls_debug_alloc_limit(size_t bytes) { g_alloc_limit.store(bytes ? bytes : ~(size_t)0); }
 static bool injected_alloc_failure() {
     long long v = g_fail_alloc.load();
     while (v > 0)
@@ -343,22 +346,24 @@ extern "C" int irwls_dev_wait_post(const unsigned *seq, unsigned v, size_t bytes
     }
 }
 
-extern "C" int irwls_dev_malloc(void **p, size_t bytes) {
+// NULL, or why not.
+static const char *try_malloc(void **p, size_t bytes) {
     *p = nullptr;
-    if (bytes == 0) bytes = 16;
-    if (injected_alloc_failure()) {
-        irwls_set_error(-3, "device allocation of %zu bytes failed (injected failure)", bytes);
-        return -3;
-    }
-    cudaError_t e = pool_malloc(p, bytes, cur());
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        irwls_set_error(-3, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
-        *p = nullptr;
-        return -3;
-    }
-    return 0;
+    if (injected_alloc_failure() || bytes > g_alloc_limit.load()) return "injected failure";
+    const cudaError_t e = pool_malloc(p, bytes ? bytes : 16, cur());
+    if (e == cudaSuccess) return nullptr;
+    cudaGetLastError();
+    *p = nullptr;
+    return cudaGetErrorString(e);
 }
+extern "C" int irwls_dev_malloc(void **p, size_t bytes) {
+    const char *why = try_malloc(p, bytes);
+    if (!why) return 0;
+    irwls_set_error(-3, "device allocation of %zu bytes failed: %s", bytes, why);
+    return -3;
+}
+// For what a call can do without: a refusal is no error of the call.
+extern "C" int irwls_dev_malloc_try(void **p, size_t bytes) { return try_malloc(p, bytes) ? -3 : 0; }
 extern "C" int irwls_dev_free(void *p) {
     if (p) cudaFreeAsync(p, cur()->stream);
     return 0;

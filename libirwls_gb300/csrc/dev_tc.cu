@@ -1093,14 +1093,15 @@ __global__ void __launch_bounds__(256) q_column_direct_kernel(KViewF X, int l, c
 
 }  // namespace
 
-extern "C" void *irwls_f32_mirror(const irwls_dev_set *X) {
+// quiet: no room is no error.
+extern "C" void *irwls_f32_mirror(const irwls_dev_set *X, int quiet) {
     F32Mirror *f = (F32Mirror *)calloc(1, sizeof(F32Mirror));
     if (!f) return nullptr;
     const long long nx = (long long)X->n_rows * X->ld;
     int rc = 0;
-    rc |= irwls_dev_malloc((void **)&f->X, (size_t)(nx > 0 ? nx : 1) * sizeof(float));
-    rc |= irwls_dev_malloc((void **)&f->cv, (size_t)(X->nnz > 0 ? X->nnz : 1) * sizeof(float));
-    rc |= irwls_dev_malloc((void **)&f->q, (size_t)(X->n_rows > 0 ? X->n_rows : 1) * sizeof(float));
+    rc |= irwls_dev_malloc_try((void **)&f->X, (size_t)(nx > 0 ? nx : 1) * sizeof(float));
+    rc |= irwls_dev_malloc_try((void **)&f->cv, (size_t)(X->nnz > 0 ? X->nnz : 1) * sizeof(float));
+    rc |= irwls_dev_malloc_try((void **)&f->q, (size_t)(X->n_rows > 0 ? X->n_rows : 1) * sizeof(float));
     if (!rc) {
         const int g = 4 * (irwls_num_sms() > 0 ? irwls_num_sms() : 148);
         const double *src[3] = {X->X, X->cv, X->q};
@@ -1118,7 +1119,7 @@ extern "C" void *irwls_f32_mirror(const irwls_dev_set *X) {
         irwls_dev_free(f->cv);
         irwls_dev_free(f->q);
         free(f);
-        irwls_set_error(-3, "cannot create the FP32 copy of the dataset");
+        if (!quiet) irwls_set_error(-3, "cannot create the FP32 copy of the dataset");
         return nullptr;
     }
     return f;

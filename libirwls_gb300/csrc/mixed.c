@@ -62,7 +62,7 @@ int irwls_q_column(const irwls_dev_set *X, const void *F, int l, const int *d_ce
                    int ldq, float *d_qn);
 int irwls_q_column_resid(int l, const float *d_rq, const int *d_best, int s, const float *lrow, void *Qb, int ldq,
                          float *d_qn);
-void *irwls_f32_mirror(const irwls_dev_set *X);
+void *irwls_f32_mirror(const irwls_dev_set *X, int quiet);
 void irwls_f32_mirror_free(void *h);
 void irwls_f32_mirror_view(const void *h, const float **X, const float **q);
 int irwls_learn_features(const float *X, int ld, int width, int raw, const float *q, float ng, const double *y,
@@ -121,11 +121,11 @@ static void draw_label_rows(const svm_dataset *ds, double want, int n, int *out)
  * candidates that can still be the best take the FP64 scores on the device, with
  * the columns of K_nm they need formed then. The selection is the FP64 one either way. verbose == 1 prints the
  * scores, so every step then takes the FP64 ones. */
-static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out, int screen) {
+static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, const int *cand, int *cent_out,
+                       int screen) {
     const int m = props.size, l = ds->l;
-    if (m <= 0) return 0;
-    int *cand = irwls_draw_sgma_candidates(ds, m);
-    if (!cand) return -1;
+    /* the plain form without the memory for its screening takes the FP64 scores of all */
+    int (*const take)(void **, size_t) = screen ? irwls_dev_malloc_try : irwls_dev_malloc;
     const int ldq = round_up(m, 128), ldL = m, ldz = m;
     const int nblk = irwls_sgma_tc_partials(l);
     int rc = 0;
@@ -143,57 +143,56 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
     double *d_KSC = NULL, *d_Z = NULL, *d_part64 = NULL;
     int *d_need = NULL; /* number of candidates to rescore, the columns of K_nm formed, the error measure (float bits), the slots */
     const int nf = irwls_mlp_feature_count(), pool = g_pool, half = g_pool / 2;
-    void *F = irwls_f32_mirror(X);
-    if (!F) {
-        free(cand);
-        return -1;
-    }
-    /* the candidates' rows ahead of their steps (dev_sgma_ahead.cu), where the
-       candidates are known then and the workspace (64 m (8 m + 6 ldq) bytes) is
-       at most 4 GB, m about 2100, and can be had; else the explicit inverse */
-    if (!learn && irwls_sgma_ahead_bytes(m, ldq) <= (size_t)4 << 30 &&
-        irwls_dev_malloc(&ahead, irwls_sgma_ahead_bytes(m, ldq))) {
-        irwls_clear_error();
-        ahead = NULL;
-    }
-    rc |= irwls_dev_malloc((void **)&d_cand, (size_t)m * 64 * sizeof(int));
-    rc |= irwls_dev_malloc((void **)&d_cent, (size_t)m * sizeof(int));
-    rc |= irwls_dev_malloc((void **)&d_best, sizeof(int));
-    rc |= irwls_dev_malloc((void **)&d_L, (size_t)m * ldL * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_W, (size_t)64 * ldz * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_KN, (size_t)64 * ldz * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_eta, 64 * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_part, (size_t)nblk * 64 * sizeof(float));
-    rc |= irwls_dev_malloc((void **)&d_val, (size_t)m * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_rq, (size_t)l * 64 * sizeof(float));
+    void *F = irwls_f32_mirror(X, screen);
+    if (!F) return screen ? -100 : -1;
+    rc |= take((void **)&d_cand, (size_t)m * 64 * sizeof(int));
+    rc |= take((void **)&d_cent, (size_t)m * sizeof(int));
+    rc |= take((void **)&d_best, sizeof(int));
+    rc |= take((void **)&d_L, (size_t)m * ldL * sizeof(double));
+    rc |= take((void **)&d_W, (size_t)64 * ldz * sizeof(double));
+    rc |= take((void **)&d_KN, (size_t)64 * ldz * sizeof(double));
+    rc |= take((void **)&d_eta, 64 * sizeof(double));
+    rc |= take((void **)&d_part, (size_t)nblk * 64 * sizeof(float));
+    rc |= take((void **)&d_val, (size_t)m * sizeof(double));
+    rc |= take((void **)&d_rq, (size_t)l * 64 * sizeof(float));
     const size_t qb_bytes = (size_t)((l + 127) / 128) * 128 * ldq * 6; /* whole 128-row tiles, three pieces */
-    rc |= irwls_dev_malloc(&Qb, qb_bytes);
-    if (!ahead) rc |= irwls_dev_malloc(&Wb, (size_t)64 * ldq * 6);
-    rc |= irwls_dev_malloc((void **)&lrow, (size_t)(m + 1) * sizeof(float));
-    if (!ahead) {
-        rc |= irwls_dev_malloc((void **)&d_Linv, (size_t)m * ldL * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_wpart, irwls_sgma_wpart_count(m) * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_lpart, irwls_sgma_lpart_count(m) * sizeof(double));
-    }
-    rc |= irwls_dev_malloc((void **)&d_qn, (size_t)(l + 2) * sizeof(float));
-    rc |= irwls_dev_malloc((void **)&d_resid, sizeof(double));
+    rc |= take(&Qb, qb_bytes);
+    rc |= take((void **)&lrow, (size_t)(m + 1) * sizeof(float));
+    rc |= take((void **)&d_qn, (size_t)(l + 2) * sizeof(float));
+    rc |= take((void **)&d_resid, sizeof(double));
     if (screen) {
-        rc |= irwls_dev_malloc((void **)&d_KSC, (size_t)l * m * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_Z, (size_t)64 * ldz * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_part64, (size_t)irwls_sgma_partials(l) * 64 * sizeof(double));
-        rc |= irwls_dev_malloc((void **)&d_need, 67 * sizeof(int));
+        rc |= take((void **)&d_KSC, (size_t)l * m * sizeof(double));
+        rc |= take((void **)&d_Z, (size_t)64 * ldz * sizeof(double));
+        rc |= take((void **)&d_part64, (size_t)irwls_sgma_partials(l) * 64 * sizeof(double));
+        rc |= take((void **)&d_need, 67 * sizeof(int));
     }
     if (learn || trace) {
-        rc |= irwls_dev_malloc((void **)&d_probe, NPROBE * sizeof(int));
-        rc |= irwls_dev_malloc((void **)&d_F, (size_t)pool * nf * sizeof(float));
+        rc |= take((void **)&d_probe, NPROBE * sizeof(int));
+        rc |= take((void **)&d_F, (size_t)pool * nf * sizeof(float));
     }
     if (learn) {
-        rc |= irwls_dev_malloc((void **)&d_pool, (size_t)m * pool * sizeof(int));
-        rc |= irwls_dev_malloc((void **)&d_pred, (size_t)pool * sizeof(float));
+        rc |= take((void **)&d_pool, (size_t)m * pool * sizeof(int));
+        rc |= take((void **)&d_pred, (size_t)pool * sizeof(float));
     }
     if (trace) {
-        rc |= irwls_dev_malloc((void **)&d_tfeat, (size_t)(m - 2) * NCAND * nf * sizeof(float));
-        rc |= irwls_dev_malloc((void **)&d_tscore, (size_t)(m - 2) * NCAND * sizeof(float));
+        rc |= take((void **)&d_tfeat, (size_t)(m - 2) * NCAND * nf * sizeof(float));
+        rc |= take((void **)&d_tscore, (size_t)(m - 2) * NCAND * sizeof(float));
+    }
+    /* after all that the call cannot do without: the candidates' rows ahead of their
+       steps (dev_sgma_ahead.cu), where the candidates are known then and the workspace
+       (64 m (8 m + 6 ldq) bytes) is at most 4 GB, m about 2100, and can be had; else
+       the explicit inverse */
+    if (!rc && (learn || irwls_sgma_ahead_bytes(m, ldq) > (size_t)4 << 30 ||
+                irwls_dev_malloc_try(&ahead, irwls_sgma_ahead_bytes(m, ldq)))) {
+        ahead = NULL;
+        rc |= take(&Wb, (size_t)64 * ldq * 6);
+        rc |= take((void **)&d_Linv, (size_t)m * ldL * sizeof(double));
+        rc |= take((void **)&d_wpart, irwls_sgma_wpart_count(m) * sizeof(double));
+        rc |= take((void **)&d_lpart, irwls_sgma_lpart_count(m) * sizeof(double));
+    }
+    if (rc && screen) {
+        rc = -100;
+        goto done;
     }
     if (rc) goto done;
     {
@@ -305,7 +304,6 @@ static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties
         free(val);
     }
 done:
-    free(cand);
     {
         void *bufs[] = {d_cand, d_cent, d_best, d_L, d_W, d_KN, d_eta, d_part, d_val, d_rq, Qb, Wb, lrow,
                         d_Linv, d_wpart, d_lpart, d_qn, d_resid, d_probe, d_F, d_pool, d_pred, d_tfeat, d_tscore,
@@ -313,21 +311,28 @@ done:
         for (size_t k = 0; k < sizeof bufs / sizeof bufs[0]; k++) irwls_dev_free(bufs[k]);
         irwls_f32_mirror_free(F);
     }
-    return rc ? -1 : 0;
+    return rc == -100 ? -100 : rc ? -1 : 0;
 }
 
 int irwls_sgma_mixed_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out) {
-    return sgma_tc_dev(X, ds, props, cent_out, 0);
+    if (props.size <= 0) return 0;
+    int *cand = irwls_draw_sgma_candidates(ds, props.size);
+    if (!cand) return -1;
+    const int rc = sgma_tc_dev(X, ds, props, cand, cent_out, 0);
+    free(cand);
+    return rc;
 }
 
-/* The plain form through the screened selection; -100 when it does not apply:
- * a linear kernel (Q is not bounded there), a feature width beyond the score
- * kernel's tile, or K_nm and Q together above 96 GB (the FP64 selection needs
- * K_nm alone). */
-int irwls_sgma_screened_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, int *cent_out) {
+/* The plain form through the screened selection, with the steps' candidates; -100
+ * when it does not apply, with nothing done and no error recorded: a linear kernel (Q
+ * is not bounded there), a feature width beyond the score kernel's tile, K_nm and Q
+ * together above 96 GB, or not the memory for it (the FP64 selection needs K_nm
+ * alone). */
+int irwls_sgma_screened_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, const int *cand,
+                            int *cent_out) {
     const double bytes = (double)ds->l * (14.0 * round_up(props.size, 128) + 256.0);
     if (X->mode == IRWLS_K_LINEAR || !irwls_sgma_tc_fits(X) || bytes > 96e9) return -100;
-    return sgma_tc_dev(X, ds, props, cent_out, 1);
+    return sgma_tc_dev(X, ds, props, cand, cent_out, 1);
 }
 
 /* Records the features and exact scores of the candidates of a precision-form
