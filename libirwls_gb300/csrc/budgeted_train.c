@@ -137,6 +137,18 @@ void irwls_record_run_info(int par_iterations, int active_rows) {
     g_last_nact = active_rows;
 }
 
+/* Split-K chunks of the Gram: in FP64 about eight CTAs per SM and 64 x 64 lower
+ * tile with at least 512 rows each, at most 64; for the digits three times as
+ * many at most, of which it takes as many as fill the SMs. */
+static int gram_chunks(int l, int m, int digits) {
+    const int tiles = ((m + 64) / 64) * ((m + 63) / 64 + 1) / 2;
+    int P = ((digits ? 24 : 8) * 152 + tiles - 1) / tiles;
+    if (P > l / (digits ? 256 : 512)) P = l / (digits ? 256 : 512);
+    if (P < 1) P = 1;
+    if (P > (digits ? 128 : 64)) P = digits ? 128 : 64;
+    return P;
+}
+
 /* IRWLSpar on a resident dataset; weights_out gets betaBest (m values). */
 int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties props, double *weights_out) {
     const int m = props.size;
@@ -150,35 +162,27 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     const int ld = m + 1;
     /* The Gram runs on the tensor cores through exact integer digits of the
        active rows (dev_gram_tc.cu): base 256 in the plain form (FP64
-       accuracy), base 128 in the precision form. P bounds the split-K chunks,
-       of which it takes as many as fill the SMs. The plain form keeps the
+       accuracy), base 128 in the precision form. The plain form keeps the
        FP64 product below 128 centroids (one 128-column tile): IRWLS can
        multiply a change of rounding in K1 by 10^8 (20000 rows, 100 SGMA
        centroids: any other split of the same FP64 sums moves the weights by
        1e-9 to 1e-8), and the product is small enough there to keep its
-       order and its chunks, about eight per SM and 64 x 64 lower tile with at
-       least 512 rows each (20000 x 100: 0.27 ms). At 50000 x 300 it took 2.55 ms
+       order and its chunks (20000 x 100: 0.27 ms). At 50000 x 300 it took 2.55 ms
        per iteration, three quarters of the training; the digits, with their
-       slicing, take 0.20. */
-    const int sms = 152;
-    const int tiles = ((m + 64) / 64) * ((m + 63) / 64 + 1) / 2;
+       slicing, take 0.20. Where their workspace cannot be had (up to 4 GB, and
+       more partials) the FP64 product serves them too. */
     const int mixed = irwls_get_precision() == IRWLS_PRECISION_MIXED;
-    const int digits = mixed || m >= 128;
+    const int large = !mixed && m >= 128;
+    int digits = mixed || large;
     void *d_A = NULL;
-    int P = ((digits ? 24 : 8) * sms + tiles - 1) / tiles;
-    if (P > l / (digits ? 256 : 512)) P = l / (digits ? 256 : 512);
-    if (P < 1) P = 1;
-    if (P > (digits ? 128 : 64)) P = digits ? 128 : 64;
-    if (digits) {
-        if (!mixed && P < irwls_par_gram_min_parts(l, m)) P = irwls_par_gram_min_parts(l, m);
-        rc |= irwls_dev_malloc(&d_A, mixed ? irwls_par_gram_tc_bytes(l, m) : irwls_par_gram_bytes(l, m));
-    }
+    int P = gram_chunks(l, m, digits);
+    if (large && P < irwls_par_gram_min_parts(l, m)) P = irwls_par_gram_min_parts(l, m);
+    if (mixed) rc |= irwls_dev_malloc(&d_A, irwls_par_gram_tc_bytes(l, m));
     rc |= irwls_dev_malloc((void **)&d_idx, (size_t)m * sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_act, (size_t)l * sizeof(int));
     rc |= irwls_dev_malloc((void **)&d_KC, (size_t)m * m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_KSC, (size_t)l * m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_K1, (size_t)ld * ld * sizeof(double));
-    rc |= irwls_dev_malloc((void **)&d_part, irwls_par_gram_part_bytes(m, P));
     rc |= irwls_dev_malloc((void **)&d_sd, (size_t)l * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_day, (size_t)l * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_e, (size_t)l * sizeof(double));
@@ -187,6 +191,15 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
     rc |= irwls_dev_malloc((void **)&d_bnew, (size_t)m * sizeof(double));
     rc |= irwls_dev_malloc((void **)&d_bbest, (size_t)m * sizeof(double));
     rc |= irwls_dev_host_alloc((void **)&h_post, sizeof(irwls_par_post));
+    if (rc) goto done;
+    if (large && (irwls_dev_malloc_try(&d_A, irwls_par_gram_bytes(l, m)) ||
+                  irwls_dev_malloc_try((void **)&d_part, irwls_par_gram_part_bytes(m, P)))) {
+        irwls_dev_free(d_A);
+        d_A = NULL;
+        digits = 0;
+        P = gram_chunks(l, m, 0);
+    }
+    if (!d_part) rc |= irwls_dev_malloc((void **)&d_part, irwls_par_gram_part_bytes(m, P));
     if (rc) goto done;
     h_post->seq = 0;
     h_post->tc = 0;
@@ -209,8 +222,8 @@ int irwls_par_dev(const irwls_dev_set *X, int l, const int *idx, properties prop
                          : irwls_par_gram_fp64(d_KSC, m, d_act, nact, d_sd, d_day, d_KC, d_K1, ld, d_part, P))
                 goto fail;
             g_gram_flops += (double)nact * (m + 1) * m;
-            if (digits && !mixed ? irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)
-                                 : irwls_dev_chol_solve_order(d_K1, m, ld, NULL, d_bnew))
+            if (large ? irwls_dev_chol_solve(d_K1, m, ld, NULL, d_bnew)
+                      : irwls_dev_chol_solve_order(d_K1, m, ld, NULL, d_bnew))
                 goto fail;
             if (irwls_par_delta(d_bnew, d_beta, m, h_post)) goto fail;
             if (irwls_par_residual(d_KSC, l, m, d_beta, X->y, C, M, d_e, d_Da)) goto fail;

@@ -732,6 +732,83 @@ __global__ void __launch_bounds__(GT_MAX) gram_kernel(const double *__restrict__
     }
 }
 
+// The same from 128 columns on, where the digits' workspace cannot be had
+// (budgeted_train.c): 64 x 64 tiles (bi, bj), bi >= bj, of the lower triangle, a
+// thread 4 x 4 values of its tile. 2.55 ms an iteration of 50000 x 300, the digits 0.20.
+constexpr int TT = 64;
+__global__ void __launch_bounds__(256) gram_wide_kernel(const double *__restrict__ KSC, int m,
+                                                        const int *__restrict__ act, int nact,
+                                                        const double *__restrict__ sd, const double *__restrict__ day,
+                                                        int chunk, double *__restrict__ part) {
+    chain_wait();
+    chain_open();
+    const int bj = blockIdx.x, bi = blockIdx.y, z = blockIdx.z;
+    if (bi < bj) return;
+    const int r0 = bi * TT, c0 = bj * TT;  // output rows (0..m), output cols (0..m-1)
+    const int p0 = z * chunk, p1 = min(nact, p0 + chunk);
+    __shared__ __align__(16) double Ai[2][TK][TT + 1];
+    __shared__ __align__(16) double Aj[2][TK][TT + 1];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    double acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
+    auto load = [&](int buf, int p) {
+        for (int t = tid; t < TK * TT; t += 256) {
+            const int kk = t / TT, cc = t % TT, pp = p + kk;
+            const int ci = r0 + cc, cj = c0 + cc;
+            const bool in = pp < p1;
+            const double *row = in ? KSC + (size_t)act[pp] * m : KSC;
+            const bool ki = in && ci < m, di = in && ci == m, kj = in && cj < m;
+            cp_async8(&Ai[buf][kk][cc], ki ? row + ci : di ? day + pp : KSC, ki || di ? 8 : 0);
+            cp_async8(&Aj[buf][kk][cc], kj ? row + cj : KSC, kj ? 8 : 0);
+        }
+        cp_async_commit();
+    };
+    if (p0 < p1) load(0, p0);
+    int it = 0;
+    for (int p = p0; p < p1; p += TK, ++it) {
+        const int buf = it & 1;
+        if (p + TK < p1) {
+            load(buf ^ 1, p + TK);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
+        }
+        for (int t = tid; t < TK * TT; t += 256) {  // each thread scales what it copied
+            const int kk = t / TT, cc = t % TT;
+            if (p + kk < p1) {
+                const double sc = sd[p + kk];
+                if (r0 + cc < m) Ai[buf][kk][cc] = __dmul_rn(sc, Ai[buf][kk][cc]);
+                if (c0 + cc < m) Aj[buf][kk][cc] = __dmul_rn(sc, Aj[buf][kk][cc]);
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < TK; ++kk) {
+            double ai[4], aj[4];
+#pragma unroll
+            for (int a = 0; a < 4; ++a) ai[a] = Ai[buf][kk][ty + 16 * a];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) aj[b] = Aj[buf][kk][tx + 16 * b];
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+#pragma unroll
+                for (int b = 0; b < 4; ++b) acc[a][b] = fma(ai[a], aj[b], acc[a][b]);
+        }
+        __syncthreads();
+    }
+    double *out = part + (size_t)z * (m + 1) * m;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int r = r0 + ty + 16 * a, c = c0 + tx + 16 * b;
+            if (r <= m && c < m && c <= r) out[(size_t)r * m + c] = acc[a][b];
+        }
+}
+
 // K1 (column-major, leading dimension ld >= m + 1, lower part) = KC + sum_z
 // part_z; row m = K2 = sum_z part_z[m][:].
 __global__ void gram_reduce_kernel(const double *__restrict__ part, int P, int m, const double *__restrict__ KC,
@@ -1101,10 +1178,6 @@ extern "C" int irwls_par_gram_reduce(const double *d_part, int P, int m, const d
 extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act, int nact, const double *d_sd,
                                    const double *d_day, const double *d_KC, double *d_K1, int ldK1, double *d_part,
                                    int P) {
-    if (m > 127) {
-        irwls_set_error(-5, "the FP64 Gram takes fewer than 128 columns");
-        return -5;
-    }
     const int chunk = nact > 0 ? ceil_div(nact, P) : 1;
     // micro-tiles of the lower triangle, in warps; CTAs per chunk so that the
     // busiest SM has the least to do (8 multiply-adds per warp and row, and the
@@ -1121,8 +1194,12 @@ extern "C" int irwls_par_gram_fp64(const double *d_KSC, int m, const int *d_act,
     }
     const int wpc = ceil_div(W, ns);
     if (irwls_prof_on()) irwls_prof_begin(IRWLS_PROF_GRAM);
-    launch_chained(gram_kernel, dim3(P, ceil_div(W, wpc)), dim3(32 * wpc), 0, d_KSC, m, d_act, nact, d_sd, d_day, chunk,
-                   d_part);
+    if (m > 127)
+        launch_chained(gram_wide_kernel, dim3(ceil_div(m, TT), ceil_div(m + 1, TT), P), dim3(256), 0, d_KSC, m, d_act,
+                       nact, d_sd, d_day, chunk, d_part);
+    else
+        launch_chained(gram_kernel, dim3(P, ceil_div(W, wpc)), dim3(32 * wpc), 0, d_KSC, m, d_act, nact, d_sd, d_day,
+                       chunk, d_part);
     if (irwls_prof_on()) irwls_prof_end(IRWLS_PROF_GRAM);
     IRWLS_LAUNCH_CHECK("gram");
     const long long total = (long long)(m + 1) * m;
