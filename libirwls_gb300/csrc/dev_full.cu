@@ -1010,16 +1010,20 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
                     &ws->mapbuf};
     for (int **p : ints) rc |= irwls_dev_malloc((void **)p, nd * sizeof(int));
     rc |= irwls_dev_malloc((void **)&ws->H, nd * nd * sizeof(double));
-    // the kernel matrix of working sets up to SUB_K rows (134 MB at most)
-    // (the six first violators can exceed a working set below six)
-    const size_t nk = (size_t)cap + 6;
-    if (cap <= SUB_K) rc |= irwls_dev_malloc((void **)&ws->K, nk * nk * sizeof(double));
     rc |= irwls_dev_malloc((void **)&ws->stats, sizeof(irwls_sub_stats));
     rc |= irwls_dev_host_alloc((void **)&ws->h_stats, sizeof(irwls_sub_stats));
     if (ws->h_stats) memset(ws->h_stats, 0, sizeof(irwls_sub_stats));
     ws->flags = irwls_dev_flags();
     ws->map = ws->mapbuf;
     return rc ? -3 : 0;
+}
+
+// The kernel matrix of working sets up to SUB_K rows (134 MB at most; the six first
+// violators can exceed a working set below six), after everything that the training
+// cannot do without: where it cannot be had, each iteration forms its values.
+extern "C" void irwls_sub_keep(irwls_sub_ws *ws) {
+    const size_t nk = (size_t)ws->cap + 6;
+    if (ws->cap > SUB_K || irwls_dev_malloc_try((void **)&ws->K, nk * nk * sizeof(double))) ws->K = nullptr;
 }
 
 extern "C" void irwls_sub_release(irwls_sub_ws *ws) {

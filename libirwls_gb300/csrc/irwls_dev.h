@@ -157,7 +157,7 @@ typedef struct irwls_sub_ws {
     int cap;
     int *map;             /* device, w entries (points at mapbuf or a caller list) */
     double *a, *e, *beta, *bnew, *bsol, *bbest, *G13, *rhs, *GIN, *y, *dlt, *scal, *H;
-    double *K;            /* kernel matrix of the working set, w x w (NULL: too large to keep) */
+    double *K;            /* kernel matrix of the working set, w x w (NULL: not kept) */
     int *grp, *S1, *S3, *lst, *lloc, *gl1, *gl3, *cnt, *mapbuf;   /* lst, lloc: changed weights, as rows of X and of the set */
     int use13;            /* this iteration's G13 is not zero */
     int ordered;          /* cnt[1] says whether a row of the set names a feature twice or out of order */
@@ -170,6 +170,7 @@ typedef struct irwls_sub_ws {
 } irwls_sub_ws;
 
 int irwls_sub_alloc(irwls_sub_ws *ws, int cap);
+void irwls_sub_keep(irwls_sub_ws *ws);   /* K, where it can be had */
 void irwls_sub_release(irwls_sub_ws *ws);
 /* a_i and the groups at entry (src/full-train.c:131-155); e, beta and map
  * must be set; nS1 and nS3 posted (irwls_sub_wait). */
