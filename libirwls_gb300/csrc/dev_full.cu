@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(NT) sub_init_kernel(irwls_sub_ws ws, const dou
     __shared__ int s_scan[32];
     chain_wait();
     chain_open();
-    const int w = ws.w, all = ws.cnt[1];
+    const int w = ws.w;
     for (int i = threadIdx.x; i < w; i += NT) {
         const double yi = yg[ws.map[i]];
         ws.y[i] = yi;
@@ -184,7 +184,6 @@ __global__ void __launch_bounds__(NT) sub_init_kernel(irwls_sub_ws ws, const dou
         ws.stats->best = 1e9;
         ws.h_stats->nS1 = n1;
         ws.h_stats->nS3 = n3;
-        if (all) ws.h_stats->unordered = all;  // (zero before)
         post_seq(&ws.h_stats->seq, ws.seq);
     }
 }
@@ -240,44 +239,44 @@ __global__ void build_border_kernel(irwls_sub_ws ws, int n1) {
 // 81 us per inner iteration, against 31 us once and 5 us to read them). Row i,
 // columns j <= i, and their mirror images: both orders of a pair give the same
 // bits (the raw form's squares; the norm form's products of shared entries in
-// index order) -- but not where a row names a feature twice or out of order
-// (cnt[1]): its dense copy keeps the last entry, its list has both, and a value
-// depends on which row is read as which. Then all w x w values are formed, row i
-// dense and row j by its list, and H takes them as its lower part has them.
+// index order) -- but not where a row names a feature twice or out of order: its
+// dense copy keeps the last entry, its list has both, and a value depends on which
+// row is read as which. Then ALL w x w values are formed, row i dense and row j by
+// its list, and H takes them as its lower part has them.
+template <bool ALL>
 __global__ void __launch_bounds__(64) sub_kmat_kernel(irwls_sub_ws ws, KView X) {
     chain_wait();
     chain_open();
     extern __shared__ double sA[];
     const int i = blockIdx.y, w = ws.w;
-    const bool all = ws.cnt[1] != 0;
-    if (!all && (int)blockIdx.x * 64 > i) return;
+    if (!ALL && (int)blockIdx.x * 64 > i) return;
     const int gi = ws.map[i];
     for (int t = threadIdx.x; t < X.ld; t += 64) sA[t] = X.X[(size_t)gi * X.ld + t];
     __syncthreads();
     const int j = blockIdx.x * 64 + threadIdx.x;
-    if (j >= w || (!all && j > i)) return;
+    if (j >= w || (!ALL && j > i)) return;
     const double kv = kentry(X, sA, X.q[gi], ws.map[j]);
     ws.K[(size_t)i * w + j] = kv;
-    if (!all) ws.K[(size_t)j * w + i] = kv;
+    if (!ALL) ws.K[(size_t)j * w + i] = kv;
 }
 
-// cnt[1] of the training's rows: some row's indices do not increase.
-__global__ void __launch_bounds__(256) sub_order_kernel(KView X, int n, int *cnt) {
+// *out is set where some row's indices do not increase.
+__global__ void __launch_bounds__(256) sub_order_kernel(KView X, int n, int *out) {
     chain_wait();
     chain_open();
     const int lane = threadIdx.x & 31;
     bool bad = false;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5)
         for (int p = X.rp[i] + 1 + lane; p < X.rp[i + 1]; p += 32) bad |= X.ci[p] <= X.ci[p - 1];
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(cnt + 1, 1);
+    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(out, 1);
 }
 
 // One iteration's system from K (src/full-train.c:165-186, :327-344): CTA
 // j < n1 writes column j of H (rows j .. n1 - 1, the border row) and
 // rhs_j = 1 - G13_j - GIN_j with G13_j = sum over S3 of C k y_j y_o (use13),
-// CTA n1 the border's corner. all: K is not symmetric (sub_kmat_kernel).
-__global__ void __launch_bounds__(128) sub_system_kernel(irwls_sub_ws ws, double C, int n1, int n3, int use13,
-                                                         int all) {
+// CTA n1 the border's corner. ALL: as sub_kmat_kernel.
+template <bool ALL>
+__global__ void __launch_bounds__(128) sub_system_kernel(irwls_sub_ws ws, double C, int n1, int n3, int use13) {
     chain_wait();
     chain_open();
     __shared__ double red[4];
@@ -295,7 +294,7 @@ __global__ void __launch_bounds__(128) sub_system_kernel(irwls_sub_ws ws, double
     double *col = ws.H + (size_t)j * ws.ldH;
     for (int i = j + threadIdx.x; i < n1; i += 128) {
         const int li = ws.S1[i];
-        double h = __dmul_rn(__dmul_rn(all ? ws.K[(size_t)li * w + lj] : row[li], ws.y[li]), yj);
+        double h = __dmul_rn(__dmul_rn(ALL ? ws.K[(size_t)li * w + lj] : row[li], ws.y[li]), yj);
         if (i == j) h = __dadd_rn(h, __ddiv_rn(1.0, ws.a[lj]));
         col[i] = h;
     }
@@ -1020,10 +1019,21 @@ extern "C" int irwls_sub_alloc(irwls_sub_ws *ws, int cap) {
 
 // The kernel matrix of working sets up to SUB_K rows (134 MB at most; the six first
 // violators can exceed a working set below six), after everything that the training
-// cannot do without: where it cannot be had, each iteration forms its values.
-extern "C" void irwls_sub_keep(irwls_sub_ws *ws) {
+// cannot do without: where it cannot be had, each iteration forms its values. The rows
+// are looked over here, once: h_stats->unordered holds after the stream's next
+// synchronisation.
+extern "C" int irwls_sub_keep(irwls_sub_ws *ws, const irwls_dev_set *X) {
     const size_t nk = (size_t)ws->cap + 6;
-    if (ws->cap > SUB_K || irwls_dev_malloc_try((void **)&ws->K, nk * nk * sizeof(double))) ws->K = nullptr;
+    if (ws->cap > SUB_K || irwls_dev_malloc_try((void **)&ws->K, nk * nk * sizeof(double))) {
+        ws->K = nullptr;
+        return 0;
+    }
+    if (X->mode == IRWLS_K_RAW_RBF || X->n_rows < 1) return 0;
+    if (irwls_dev_memset(ws->cnt, 0, sizeof(int))) return -2;
+    launch_chained(sub_order_kernel, dim3(std::min(ceil_div(X->n_rows, 8), 1024)), dim3(256), 0, kview(X), X->n_rows,
+                   ws->cnt);
+    IRWLS_LAUNCH_CHECK("sub_order");
+    return irwls_dev_d2h(&ws->h_stats->unordered, ws->cnt, sizeof(int));
 }
 
 extern "C" void irwls_sub_release(irwls_sub_ws *ws) {
@@ -1042,16 +1052,6 @@ extern "C" int irwls_sub_wait(irwls_sub_ws *ws) {
 
 extern "C" int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C) {
     const int w = ws->w;
-    if (!ws->ordered) {
-        // once per training, as the rows stay
-        if (irwls_dev_memset(ws->cnt, 0, 2 * sizeof(int))) return -2;
-        if (ws->K && X->mode != IRWLS_K_RAW_RBF && X->n_rows > 0) {
-            launch_chained(sub_order_kernel, dim3(std::min(ceil_div(X->n_rows, 8), 1024)), dim3(256), 0, kview(X),
-                           X->n_rows, ws->cnt);
-            IRWLS_LAUNCH_CHECK("sub_order");
-        }
-        ws->ordered = 1;
-    }
     ++ws->seq;
     if (w < 512) launch_chained(sub_init_kernel<512>, dim3(1), dim3(512), 0, *ws, X->y, C);
     else launch_chained(sub_init_kernel<CT>, dim3(1), dim3(CT), 0, *ws, X->y, C);
@@ -1064,9 +1064,9 @@ extern "C" int irwls_sub_init(irwls_sub_ws *ws, const irwls_dev_set *X, double C
     if (ex < 0) return -2;
     if (ex == 1) {
         const size_t smem = (size_t)X->ld * sizeof(double);
-        if (smem > 48 * 1024)
-            allow_smem(sub_kmat_kernel);
-        launch_chained(sub_kmat_kernel, dim3(ceil_div(w, 64), w), dim3(64), smem, *ws, kview(X));
+        const auto kern = ws->h_stats->unordered ? sub_kmat_kernel<true> : sub_kmat_kernel<false>;
+        if (smem > 48 * 1024) allow_smem(kern);
+        launch_chained(kern, dim3(ceil_div(w, 64), w), dim3(64), smem, *ws, kview(X));
         IRWLS_LAUNCH_CHECK("sub_kmat");
     }
     return 0;
@@ -1114,8 +1114,7 @@ static int sub_system_direct(irwls_sub_ws *ws, const irwls_dev_set *X, int n1) {
 extern "C" int irwls_sub_iterate(irwls_sub_ws *ws, const irwls_dev_set *X, double C, int n1, int n3) {
     const int n = n1 + 1, w = ws->w;
     if (ws->K) {
-        launch_chained(sub_system_kernel, dim3(n1 + 1), dim3(128), 0, *ws, C, n1, n3, ws->use13,
-                       ws->h_stats->unordered);
+        launch_chained(ws->h_stats->unordered ? sub_system_kernel<true> : sub_system_kernel<false>, dim3(n1 + 1), dim3(128), 0, *ws, C, n1, n3, ws->use13);
         IRWLS_LAUNCH_CHECK("sub_system");
     } else if (sub_system_direct(ws, X, n1)) {
         return -2;

@@ -72,7 +72,7 @@ double *subIRWLS(svm_dataset dataset, properties props, double *GIN, double *e, 
     irwls_sub_ws ws;
     double *out = NULL;
     if (irwls_sub_alloc(&ws, l > 0 ? l : 1)) goto done_x;
-    irwls_sub_keep(&ws);
+    if (irwls_sub_keep(&ws, &X)) goto done_ws;
     ws.w = l;
     {
         int *ident = (int *)malloc((l > 0 ? l : 1) * sizeof(int));
@@ -169,7 +169,8 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
         }
     }
     if (rc) goto done;
-    irwls_sub_keep(&ws);
+    rc |= irwls_sub_keep(&ws, X);
+    if (rc) goto done;
 
     /* initial working set: every tenth sample, up to W (src/full-train.c:411-423) */
     int nSW = 0, nSIN = 0;

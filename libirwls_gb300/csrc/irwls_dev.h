@@ -147,7 +147,7 @@ typedef struct irwls_sub_stats {
     int nS1, nS3;
     unsigned seq;
     int tc;  /* a bounded wait of this or an earlier kernel ran out (the status word) */
-    int unordered, pad;  /* cnt[1] */
+    int unordered, pad;  /* host: some row names a feature twice or out of order (irwls_sub_keep) */
 } irwls_sub_stats;
 
 /* The inner-IRWLS device state on a working set of w rows; map[i] is the
@@ -160,7 +160,6 @@ typedef struct irwls_sub_ws {
     double *K;            /* kernel matrix of the working set, w x w (NULL: not kept) */
     int *grp, *S1, *S3, *lst, *lloc, *gl1, *gl3, *cnt, *mapbuf;   /* lst, lloc: changed weights, as rows of X and of the set */
     int use13;            /* this iteration's G13 is not zero */
-    int ordered;          /* cnt[1] says whether a row of the set names a feature twice or out of order */
     irwls_sub_stats *stats;   /* device */
     irwls_sub_stats *h_stats; /* pinned host mirror, written by the last kernel of a step */
     unsigned seq;             /* number of the last step */
@@ -170,7 +169,7 @@ typedef struct irwls_sub_ws {
 } irwls_sub_ws;
 
 int irwls_sub_alloc(irwls_sub_ws *ws, int cap);
-void irwls_sub_keep(irwls_sub_ws *ws);   /* K, where it can be had */
+int irwls_sub_keep(irwls_sub_ws *ws, const irwls_dev_set *X);   /* K, where it can be had; the caller synchronises */
 void irwls_sub_release(irwls_sub_ws *ws);
 /* a_i and the groups at entry (src/full-train.c:131-155); e, beta and map
  * must be set; nS1 and nS3 posted (irwls_sub_wait). */
