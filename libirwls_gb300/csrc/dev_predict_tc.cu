@@ -622,10 +622,8 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     const size_t off_as = off_at + (size_t)n * 8 + 256, off_top = off_as + (size_t)nSV * 8 + 256;
     const size_t off_part = (off_top + 1024) & ~(size_t)255;
     unsigned char *ws = nullptr;
-    if (irwls_dev_malloc((void **)&ws, off_part + (size_t)P * GR * rn * sizeof(double))) {
-        irwls_clear_error();  // (no room for it: the ordered sums need none)
-        return 1;
-    }
+    if (irwls_dev_malloc_try((void **)&ws, off_part + (size_t)P * GR * rn * sizeof(double)))
+        return 1;  // (no room for it: the FP64 rows need none)
     __nv_bfloat16 *dT = (__nv_bfloat16 *)ws, *dS = (__nv_bfloat16 *)(ws + off_s);
     int *et = (int *)(ws + off_et), *es = (int *)(ws + off_es);
     long long *at = (long long *)(ws + ((off_at + 255) & ~(size_t)255)), *as = (long long *)(ws + ((off_as + 255) & ~(size_t)255));
@@ -708,7 +706,8 @@ extern "C" void irwls_exact_rows_free(void *h) {
 }
 
 // Rows 0 ... n - 1 of X for row sums of all or up to na listed rows against lists
-// of rows; NULL where irwls_predict_exact would return 1, or above 4 GB.
+// of rows; NULL where irwls_predict_exact would return 1, or above 4 GB, and where a
+// launch or a copy failed: an error is recorded then, and only then.
 extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) {
     const double gamma = -X->neg_gamma;
     const bool raw = X->mode == IRWLS_K_RAW_RBF;
@@ -724,9 +723,8 @@ extern "C" void *irwls_exact_rows_create(const irwls_dev_set *X, int n, int na) 
     const size_t total = 2 * sb + ab + 3 * (n4 + n8) + 256 + up(nparts * sizeof(double));
     if (total > ((size_t)4 << 30)) return nullptr;
     ExactRows *E = (ExactRows *)calloc(1, sizeof(ExactRows));
-    if (!E) return nullptr;
-    if (irwls_dev_malloc((void **)&E->ws, total)) {
-        irwls_clear_error();
+    if (!E) return nullptr;  // (as without room on the device)
+    if (irwls_dev_malloc_try((void **)&E->ws, total)) {
         free(E);
         return nullptr;
     }

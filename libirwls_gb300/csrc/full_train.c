@@ -131,8 +131,9 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     /* the FP64-accurate row sums from the tensor cores where they are large enough
        (at most W changed weights per update, or W rows; in the precision form any
        set of rows, on data without its exact-integer products); the errors are as
-       close to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu) */
-    void *exact = (double)l * W >= 5.0e5 && !(tcs && irwls_tc_set_exact(tcs)) ? irwls_exact_rows_create(X, l, tcs ? l : W) : NULL;
+       close to 64 bits as the ordered FP64 sums' (dev_predict_tc.cu). Up to 4 GB, after
+       all that the training cannot do without */
+    void *exact = NULL;
     const double band = 0.05, eps = 2e-5 * (tcs ? irwls_tc_set_kbound(tcs) : 1.0);
     int *xflag = NULL, *xmark = NULL, *xS = NULL, *xSnew = NULL, *svlst = NULL, *svcnt = NULL;
     double *eS = NULL, *svcb = NULL;
@@ -170,6 +171,10 @@ int irwls_full_train_dev(const irwls_dev_set *X, int l, properties props, double
     }
     if (rc) goto done;
     rc |= irwls_sub_keep(&ws, X);
+    if (!rc && (double)l * W >= 5.0e5 && !(tcs && irwls_tc_set_exact(tcs))) {
+        exact = irwls_exact_rows_create(X, l, tcs ? l : W);
+        if (!exact && irwls_get_error() < 0) rc = -2;
+    }
     if (rc) goto done;
 
     /* initial working set: every tenth sample, up to W (src/full-train.c:411-423) */
