@@ -111,33 +111,60 @@ __global__ void __launch_bounds__(kThreads) kernel_rowsum_kernel(KView A, const 
     if (folder) out[me] = tail ? __dsub_rn(acc, tail[0]) : acc;
 }
 
-// Prediction's row sums (and the sign with hard): 256 / R threads per row, thread t
-// the vectors t, t + 256 / R, ..., the threads' sums by a fixed tree. Nothing is
-// handed over or waited for before the end; the training's ordered sums fold each
-// row in one thread, 65 cycles a vector that a small batch leaves exposed (64 rows
-// of 20 values against 400 vectors: 11 us, ordered 27) and that use R lanes of the
-// FP64 pipe's 32. Linear kernels round once per stored value, half the FP64
-// instructions that bound the kernel (9000 rows of 33 values against 1501 vectors:
-// 932 us, ordered 2000, at the pipe's peak 840).
+// Prediction's row sums (and the sign with hard). A row has 8 groups of 32 chains,
+// chain 32 g + lane the vectors 32 g + lane, + 256, ...; a warp has the groups g, g +
+// 8 / R, ... of one row (8 / R warps a row), one after another, and adds up a group's
+// lanes as a butterfly does (16 apart, 8 apart, ...), two groups at a time as long as
+// there are two: halves of the warp keep different ones. The groups' sums in order. So what a row
+// gets does not depend on R, that is on the rows beside it. Nothing is handed
+// over or waited for before the end; the training's ordered sums fold each row in
+// one thread, 65 cycles a vector that a small batch leaves exposed (64 rows of 20
+// values against 400 vectors: 11 us, ordered 27) and that use R lanes of the FP64
+// pipe's 32. Linear kernels round once per stored value, half the FP64 instructions
+// that bound the kernel (9000 rows of 33 values against 1501 vectors: 932 us, ordered
+// 2000, at the pipe's peak 840).
 __global__ void __launch_bounds__(kThreads) predict_rows_kernel(KView A, int nA, KView B, int nB, int R,
                                                                 const double *__restrict__ w, double bias, int hard,
                                                                 double *__restrict__ out) {
     extern __shared__ double smem[];
-    __shared__ double sQ[8], red[8];
+    __shared__ double sQ[8], red[8][8];
     const int i0 = blockIdx.x * R;
     stage_rows(smem, sQ, A, nullptr, i0, R, nA);
-    const int per = kThreads / R, r = threadIdx.x / per;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpr = 8 / R, r = warp / wpr;
     const double *a = smem + (size_t)r * A.ld;
-    double acc = 0.0;
-    if (i0 + r < nA)
-        for (int j = threadIdx.x % per; j < nB; j += per)
-            acc = fma(w[j], B.mode == IRWLS_K_LINEAR ? sparse_dot_fused(a, B, j) : kentry(B, a, sQ[r], j), acc);
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    auto merge = [&](double low, double high, int o) {  // the lanes with bit o take the second group
+        const bool up = lane & o;
+        return (up ? high : low) + __shfl_xor_sync(0xffffffffu, up ? low : high, o);
+    };
+    double t = 0.0, h0 = 0.0, h1 = 0.0, h2 = 0.0;
+#pragma unroll 1
+    for (int n = 0; n < R; ++n) {
+        // group wpr k, k: n with its log2(R) bits in reverse, so that merged groups are R / 2, R / 4, ... apart
+        const int k = (int)(__brev((unsigned)n) >> 29) * R >> 3;
+        t = 0.0;
+        if (i0 + r < nA)
+            for (int j = 32 * (warp % wpr + wpr * k) + lane; j < nB; j += kThreads)
+                t = fma(w[j], B.mode == IRWLS_K_LINEAR ? sparse_dot_fused(a, B, j) : kentry(B, a, sQ[r], j), t);
+        if (!(n & 1)) {
+            h0 = t;
+        } else {
+            t = merge(h0, t, 16);
+            if (!(n & 2)) {
+                h1 = t;
+            } else {
+                t = merge(h1, t, 8);
+                if (!(n & 4)) h2 = t;
+                else t = merge(h2, t, 4);
+            }
+        }
+    }
+    for (int o = 16 / R; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const int part = 32 / R;  // lanes of a group
+    if (lane % part == 0) red[r][warp % wpr + wpr * (lane / part)] = t;
     __syncthreads();
     if (threadIdx.x < R && i0 + threadIdx.x < nA) {
         double f = 0.0;
-        for (int k = 0; k < 8 / R; ++k) f += red[threadIdx.x * (8 / R) + k];
+        for (int g = 0; g < 8; ++g) f += red[threadIdx.x][g];
         f += bias;
         out[i0 + threadIdx.x] = hard ? (f >= 0.0 ? 1.0 : -1.0) : f;
     }
