@@ -36,6 +36,9 @@ void irwls_debug_fail_alloc(long long n);
 /* Test hook, no counterpart in the reference: device allocations of more than
  * `bytes` are refused from now on, as where memory is short (0: none is). */
 void irwls_debug_alloc_limit(size_t bytes);
+/* Pinned host memory that the library keeps for the next dataset uploads: at
+ * most four buffers of 64 MB, until freeMemory. */
+long long irwls_staging_bytes(void);
 /* Test hook, no counterpart in the reference: the poll limit of every bounded
  * wait of the precision form's full-IRWLS error-update kernel (<= 0: the
  * default, 2^26 polls) and a stall switch with which that kernel's MMA thread

@@ -412,6 +412,7 @@ extern "C" int irwls_dev_workspace(size_t bytes, void **d_ws) {
     *d_ws = irwls_ctx_scratch(1, bytes);
     return *d_ws ? 0 : -3;
 }
+static void stages_release();
 extern "C" void irwls_dev_release_workspace(void) {
     Ctx *c = cur();
     if (c->scratch[1]) cudaFreeAsync(c->scratch[1], c->stream);
@@ -421,6 +422,7 @@ extern "C" void irwls_dev_release_workspace(void) {
         cudaStreamSynchronize(c->stream);
         cudaMemPoolTrimTo(c->pool, 0);
     }
+    stages_release();
 }
 
 // ---------------------------------------------------------------------------
@@ -454,7 +456,7 @@ extern "C" int irwls_check_labels(const svm_dataset *ds, int n_rows) {
 namespace {
 
 // Pinned staging buffers, kept for the next upload: at most kStageKeep of them,
-// each at most kStageBytes. An upload has its buffer to itself, from any thread
+// each at most kStageBytes, until irwls_dev_release_workspace. An upload has its buffer to itself, from any thread
 // or context, and gives it back with an event behind its copy on its stream;
 // the next user takes one whose event has passed (or waits for it), so an
 // upload itself does not wait. (Copies of pageable memory will not do instead:
@@ -469,10 +471,16 @@ struct Stage {
 std::mutex g_stage_mutex;
 std::vector<Stage> g_stages;
 
+void stage_free(const Stage &s) {
+    cudaEventDestroy(s.done);
+    irwls_dev_host_free(s.p);
+}
+
 int stage_take(size_t bytes, Stage *out) {
     int wait = -1;
     {
         std::lock_guard<std::mutex> lock(g_stage_mutex);
+        g_stages.reserve(kStageKeep + 1);  // (giving back then needs no memory)
         int full = 0;
         for (size_t k = 0; k < g_stages.size(); ++k) {
             if (g_stages[k].bytes < bytes) continue;
@@ -487,7 +495,12 @@ int stage_take(size_t bytes, Stage *out) {
         }
     }
     cudaGetLastError();  // (a query that was not ready is no error)
-    if (wait == 1 && cudaEventSynchronize(out->done) != cudaSuccess) return cuda_fail(cudaGetLastError(), "staging");
+    if (wait == 1 && cudaEventSynchronize(out->done) != cudaSuccess) {
+        const int rc = cuda_fail(cudaGetLastError(), "staging");
+        stage_free(*out);
+        *out = {nullptr, 0, nullptr};
+        return rc;
+    }
     if (wait >= 0) return 0;
     size_t cap = bytes;
     if (bytes <= kStageBytes)  // the next power of two, so that slightly larger sets reuse it
@@ -496,6 +509,7 @@ int stage_take(size_t bytes, Stage *out) {
     if (irwls_dev_host_alloc(&out->p, cap)) return -3;
     if (cudaEventCreateWithFlags(&out->done, cudaEventDisableTiming) != cudaSuccess) {
         irwls_dev_host_free(out->p);
+        out->p = nullptr;
         return cuda_fail(cudaGetLastError(), "staging event");
     }
     return 0;
@@ -520,11 +534,20 @@ int stage_give(Stage s) {
     }
     if (drop.p) {
         if (cudaEventSynchronize(drop.done) != cudaSuccess) rc = -2;
-        cudaEventDestroy(drop.done);
-        irwls_dev_host_free(drop.p);
+        stage_free(drop);
     }
     return rc;
 }
+// A buffer in use: given back also where an exception ends the upload.
+struct StageHold {
+    Stage s = {nullptr, 0, nullptr};
+    int give() {
+        const Stage t = s;
+        s.p = nullptr;
+        return stage_give(t);
+    }
+    ~StageHold() { give(); }
+};
 
 // fn(first row, last row, chunk) over `n` rows in `chunks` contiguous chunks,
 // taken in turn by the caller and helpers - 1 other threads. The caller waits for
@@ -554,6 +577,29 @@ void over_rows(int n, int chunks, int helpers, std::function<void(int, int, int)
     team->work();
     while (team->done.load() < chunks) std::this_thread::yield();
 }
+
+}  // namespace
+
+// The kept buffers given back (those in use come back later and are kept then).
+static void stages_release() {
+    std::vector<Stage> all;
+    {
+        std::lock_guard<std::mutex> lock(g_stage_mutex);
+        all.swap(g_stages);
+    }
+    for (const Stage &s : all) {
+        cudaEventSynchronize(s.done);
+        stage_free(s);
+    }
+}
+extern "C" long long irwls_staging_bytes(void) {
+    std::lock_guard<std::mutex> lock(g_stage_mutex);
+    long long b = 0;
+    for (const Stage &s : g_stages) b += (long long)s.bytes;
+    return b;
+}
+
+namespace {
 
 // The dense rows by feature index from the CSR: a warp per row writes its
 // zeros, then its entries (a row whose indices do not increase may name one
@@ -657,9 +703,9 @@ static int upload_rows_(svm_sample *const *rows, const double *q, const double *
                  rb = round256((n + 1) * sizeof(int)), ib = round256((size_t)nnz * sizeof(int));
     const size_t pack = 2 * qb + vb + rb + ib;   // q, y, cv, rp, ci
     const size_t head = raw ? xbytes : 0;        // the raw rows go over as they are
-    Stage st = {nullptr, 0, nullptr};
-    if (stage_take(head + pack, &st)) return -3;
-    unsigned char *h = (unsigned char *)st.p;
+    StageHold stage;
+    if (stage_take(head + pack, &stage.s)) return -3;
+    unsigned char *h = (unsigned char *)stage.s.p;
     double *hX = (double *)h, *hq = (double *)(h + head), *hy = (double *)(h + head + qb),
            *hcv = (double *)(h + head + 2 * qb);
     int *hrp = (int *)(h + head + 2 * qb + vb), *hci = (int *)(h + head + 2 * qb + vb + rb);
@@ -704,7 +750,7 @@ static int upload_rows_(svm_sample *const *rows, const double *q, const double *
             rc |= irwls_check_launch("dense_rows");
         }
     }
-    rc |= stage_give(st);
+    rc |= stage.give();
     if (rc) {
         irwls_dev_release(out);
         return rc < 0 ? rc : -3;
