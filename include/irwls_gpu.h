@@ -90,7 +90,8 @@ int irwls_gpu_available(void);
  * Large RBF row sums (predictions, the error updates of full training) and the
  * IRWLSpar Gram from 128 centroids on come from exact integer digit products on
  * the tensor cores, no further from a 64-bit evaluation than ordered FP64 sums;
- * SGMA's scores are screened on the tensor cores and decided in FP64;
+ * SGMA's candidates are screened by tensor-core scores with an error measured on
+ * sampled rows, and by FP64 scores where that does not settle a step;
  * IRWLS_PRECISION_MIXED: the precision form -- SGMA candidate scores from
  * tensor-core products of three bf16 pieces per value (FP32 accuracy) on
  * the Nystrom features of the current centroids, with the K_mm

@@ -115,12 +115,13 @@ static void draw_label_rows(const svm_dataset *ds, double want, int n, int *out)
 }
 
 /* SGMA with tensor-core scores. screen = 0: the precision form. screen = 1:
- * the plain form -- the tensor-core scores and a measured bound of their error
- * settle the steps whose best candidate stands clear of the others; in the other
+ * the plain form -- the tensor-core scores and an estimate of their error, measured
+ * on the sampled candidates (dev_tc.cu), settle the steps whose best candidate stands clear of the others; in the other
  * steps (a few percent at budgets of 100, nearly all late steps at 1000) the
  * candidates that can still be the best take the FP64 scores on the device, with
- * the columns of K_nm they need formed then. The selection is the FP64 one either way. verbose == 1 prints the
- * scores, so every step then takes the FP64 ones. */
+ * the columns of K_nm they need formed then. The selection is the FP64 one as far as
+ * the estimate holds. verbose == 1 prints the scores, so every step then takes the
+ * FP64 ones. */
 static int sgma_tc_dev(const irwls_dev_set *X, const svm_dataset *ds, properties props, const int *cand, int *cent_out,
                        int screen) {
     const int m = props.size, l = ds->l;
