@@ -316,8 +316,9 @@ def measured_peaks():
 def timed_trainings(lib, libc, res, p, steps, warmup, cent, w, precision, clocks=None):
     """`warmup` untimed then `steps` timed trainings of one form on the
     resident dataset (L2 flushed before each; CUDA events on the library's
-    stream). Returns mean seconds, per-stage profile, launches and the clock
-    record."""
+    stream), then one more with the stages' events, which keep chained kernels
+    from starting early. Returns mean seconds, per-stage profile, launches and
+    the clock record."""
     lib.irwls_set_precision(precision)
 
     def step():
@@ -327,8 +328,6 @@ def timed_trainings(lib, libc, res, p, steps, warmup, cent, w, precision, clocks
 
     for _ in range(warmup):
         step()
-    lib.irwls_profile_enable(1)
-    lib.irwls_profile_reset()
     launches0 = lib.irwls_kernel_launches()
     lib.irwls_gram_tc_flops(1)
     if clocks:
@@ -341,13 +340,18 @@ def timed_trainings(lib, libc, res, p, steps, warmup, cent, w, precision, clocks
         times.append(lib.irwls_timer_stop() / 1000.0)
     clk = clocks.stop() if clocks else None
     launches = lib.irwls_kernel_launches() - launches0
-    prof = {name: profile_read(lib, slot, steps) for name, slot in PROFILE_SLOTS.items()}
+    tc_flops = lib.irwls_gram_tc_flops(1) / max(steps, 1)
+    lib.irwls_profile_enable(1)
+    lib.irwls_profile_reset()
+    lib.irwls_l2_flush(512 << 20)
+    step()
+    prof = {name: profile_read(lib, slot, 1) for name, slot in PROFILE_SLOTS.items()}
     lib.irwls_profile_enable(0)
     iters, nact = C.c_int(), C.c_int()
     lib.irwls_last_run_info(C.byref(iters), C.byref(nact))
     return {"s": statistics.mean(times), "prof": prof, "launches": launches / max(steps, 1), "clocks": clk,
             "iters": iters.value, "nact": nact.value, "gram_flops": lib.irwls_last_gram_flops(),
-            "gram_tc_flops": lib.irwls_gram_tc_flops(1) / max(steps, 1), "steps": steps, "warmup": warmup}
+            "gram_tc_flops": tc_flops, "steps": steps, "warmup": warmup}
 
 
 def end_to_end(lib, libc, hd, p, args, precision, ref_cent, steps):
@@ -720,8 +724,6 @@ def full_measure(args, lib, libc):
 
         for _ in range(args.warmup):
             step()
-        lib.irwls_profile_enable(1)
-        lib.irwls_profile_reset()
         launches0 = lib.irwls_kernel_launches()
         clocks = Clocks(0) if prec == forms[-1] else None
         if clocks:
@@ -733,11 +735,13 @@ def full_measure(args, lib, libc):
             step()
             times.append(lib.irwls_timer_stop() / 1000.0)
         clk = clocks.stop() if clocks else None
-        prof = {name: profile_read(lib, slot, args.steps) for name, slot in (("kernel_rowsums", 2),
-                                                                             ("cholesky_solves", 3))}
+        launches = lib.irwls_kernel_launches() - launches0
+        lib.irwls_profile_enable(1)  # (the stages in a step of their own, as timed_trainings)
+        lib.irwls_profile_reset()
+        step()
+        prof = {name: profile_read(lib, slot, 1) for name, slot in (("kernel_rowsums", 2), ("cholesky_solves", 3))}
         lib.irwls_profile_enable(0)
-        runs[prec] = {"s": statistics.mean(times), "launches": lib.irwls_kernel_launches() - launches0,
-                      "clocks": clk, "prof": prof}
+        runs[prec] = {"s": statistics.mean(times), "launches": launches, "clocks": clk, "prof": prof}
         betas[prec] = beta.copy()
     lib.irwls_resident_free(res)
     e2e = {}
