@@ -36,6 +36,10 @@ void irwls_debug_fail_alloc(long long n);
 /* Test hook, no counterpart in the reference: device allocations of more than
  * `bytes` are refused from now on, as where memory is short (0: none is). */
 void irwls_debug_alloc_limit(size_t bytes);
+/* Test hook, no counterpart in the reference: the rows of the plain Gram and of
+ * tensor-core predictions are taken in slabs of `bytes` of digit slices (0: 4 and
+ * 2 GB). */
+void irwls_debug_slab_bytes(size_t bytes);
 /* Pinned host memory that the library keeps for the next dataset uploads: at
  * most four buffers of 64 MB, until freeMemory. */
 long long irwls_staging_bytes(void);

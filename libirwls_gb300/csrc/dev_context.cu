@@ -260,6 +260,14 @@ extern "C" void irwls_debug_fail_alloc(long long n) { g_fail_alloc.store(n > 0 ?
 // Device allocations above this are refused, as where memory is short.
 static std::atomic<size_t> g_alloc_limit{~(size_t)0};
 extern "C" void irwls_debug_alloc_limit(size_t bytes) { g_alloc_limit.store(bytes ? bytes : ~(size_t)0); }
+// Bytes of digit slices at a time where rows are taken in slabs: `normal`, or what a
+// test has set.
+static std::atomic<size_t> g_slab_bytes{0};
+extern "C" void irwls_debug_slab_bytes(size_t bytes) { g_slab_bytes.store(bytes); }
+extern "C" size_t irwls_slab_bytes(size_t normal) {
+    const size_t b = g_slab_bytes.load();
+    return b ? b : normal;
+}
 static bool injected_alloc_failure() {
     long long v = g_fail_alloc.load();
     while (v > 0)

@@ -537,7 +537,7 @@ int gram_run(const double *d_KSC, int m, const int *d_act, int nact, const doubl
 constexpr size_t SLAB_BYTES = 4ULL << 30;
 int slab_rows(int m) {
     const size_t per = slices_bytes(GBK, m);  // one 16-row block of every column tile
-    return (int)std::min<size_t>(std::max<size_t>(SLAB_BYTES / per, 1) * GBK, 1u << 30);
+    return (int)std::min<size_t>(std::max<size_t>(irwls_slab_bytes(SLAB_BYTES) / per, 1) * GBK, 1u << 30);
 }
 
 }  // namespace

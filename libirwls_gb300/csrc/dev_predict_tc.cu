@@ -611,7 +611,7 @@ extern "C" int irwls_predict_exact(const irwls_dev_set *T, int n, const irwls_de
     if (!(gamma > 1e-30 && gamma < 1e6)) return 1;
     const int sms = irwls_num_sms() > 0 ? irwls_num_sms() : 148;
     // rows per slab: 2 GB of slices
-    const long long tiles_fit = std::max<long long>(1, ((long long)2 << 30) / (long long)slice_bytes(PM, npb));
+    const long long tiles_fit = std::max<long long>(1, (long long)(irwls_slab_bytes((size_t)2 << 30) / slice_bytes(PM, npb)));
     const int slab = (int)std::min<long long>((long long)PM * tiles_fit, (long long)ceil_div(n, PM) * PM);
     const int nt = ceil_div(nSV, PN), it = ceil_div(std::min(n, slab), PM);
     const int per = ceil_div(nt, best_chunks(it, nt, sms)), P = ceil_div(nt, per);

@@ -49,6 +49,7 @@ int irwls_rand(void);
 int irwls_dev_wait_post(const unsigned *seq, unsigned v, size_t bytes);
 unsigned *irwls_ctx_post(unsigned *seq);
 int irwls_dev_malloc(void **p, size_t bytes);
+size_t irwls_slab_bytes(size_t normal);
 int irwls_dev_malloc_try(void **p, size_t bytes);   /* the same, a refusal not recorded as an error */
 int irwls_dev_free(void *p);
 int irwls_dev_h2d(void *d_dst, const void *h_src, size_t bytes);   /* async */
