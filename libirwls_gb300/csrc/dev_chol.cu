@@ -346,6 +346,10 @@ __global__ void zero_upper_kernel(double *__restrict__ M, int n, int ld) {
 // ---------------------------------------------------------------------------
 constexpr long long DF_WAIT_LIMIT = 1LL << 22;
 constexpr int CHOL_WAIT_CODE = 0x40000000;
+// polls of the computing warps for the loader, which gives up after DF_WAIT_LIMIT polls of
+// L2 (1300 cycles each) or TC_WAIT_LIMIT of its own barrier: 16 times those
+constexpr long long COMPUTE_WAIT_LIMIT = 16 * TC_WAIT_LIMIT;
+static_assert(COMPUTE_WAIT_LIMIT >= 256 * DF_WAIT_LIMIT, "the loader's verdict comes first");
 constexpr int DFC = 4;               // columns per published step
 constexpr int DFQ = NB / DFC;        // steps of a tile
 constexpr int DFR = 6;               // ring slots of steps
@@ -686,9 +690,11 @@ __global__ void __launch_bounds__(DF_THREADS, 1) chol_df_kernel(double *__restri
     const bool third = tid < NB * (NB + 1) / 2 - 512;
     const int r = tid % NB, u = tid / NB;
     bool good = true;
-    // the slot of the next step, or false when the loader gave up
+    // the slot of the next step, or false when the loader gave up. The loader's bounds
+    // end first and it always says which: a thread that gave up by itself would leave
+    // the others at the next barrier.
     auto take = [&](int s) {
-        return mbar_wait(smem_u32(&sh.full[s]), (unsigned)(step / DFR) & 1u) && !sh.bad[s];
+        return mbar_wait(smem_u32(&sh.full[s]), (unsigned)(step / DFR) & 1u, COMPUTE_WAIT_LIMIT) && !sh.bad[s];
     };
     auto give = [&](int s) {
         __syncwarp();
