@@ -870,11 +870,7 @@ size_t df_ready_words(int n, int has_b) {
     return nbc + nbc * nbr + 1;
 }
 
-// Enqueues the whole factorization (and the solve when has_b) on `st`, with
-// Dinv holding ceil(n/32) blocks of 32x32 doubles. Row n of M (the
-// right-hand side) is scratch on return: which backward sweep runs decides
-// what it holds.
-// The same backward sweep on several CTAs (a cooperative launch): thread t
+// The backward sweep of chol_backsolve_kernel on several CTAs (a cooperative launch): thread t
 // of CTA k owns row 256 k + t of z, which is row n of M updated in place.
 // Per 32-row block from the bottom, every CTA forms x_b = D_b^-T y_b in
 // shared memory from the block's rows of z (final since the previous block),
@@ -1165,6 +1161,9 @@ int chol_enqueue_backsolve(double *d_M, int n, int ld, double *d_x, double *Dinv
 // Whether the cluster sweep takes order n.
 bool cluster_sweep_for(int n) { return n <= 8 * SWB * NB && sweep_cluster_ok(); }
 
+// Enqueues the whole factorization (and the solve with d_x) on `st`, with Dinv
+// holding ceil(n/32) blocks of 32x32 doubles. Row n of M (the right-hand side) is
+// scratch on return: which backward sweep runs decides what it holds.
 // ready: the data-flow path's list (df_ready_words words, all zero; it is left all
 // zero, by the cluster sweep or a memset: clearing it before the factorization
 // instead cost each solve 4 us), or NULL for the multi-launch path. chained: the
